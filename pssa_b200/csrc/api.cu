@@ -1,4 +1,5 @@
 // extern "C" entry points: context lifecycle, validation, host staging. Kernels live in the other .cu files.
+#include <algorithm>
 #include <cstring>
 
 #include "bounds.hpp"
@@ -290,8 +291,10 @@ int32_t pssa_b200_ssm_forward_dev(pssa_b200_ctx* ctx, const float* delta, const 
     p.carry = carry, p.y = y, p.states = states, p.bar_a = bar_a, p.bar_b = bar_b;
     p.rows = rows, p.d = (int)d_m, p.s = (int)d_s, p.lanes = (int)lanes;
     p.aligned = ssm_vector_ok(p);
-    p.single_token = 1;  // decode-step shape: every lane at most one token
-    for (size_t l = 0; l < lanes; ++l) p.single_token = p.single_token && (lengths ? lengths[l] <= 1 : rows <= 1);
+    size_t max_len = lengths ? 0 : rows;
+    for (size_t l = 0; lengths && l < lanes; ++l) max_len = std::max<size_t>(max_len, lengths[l]);
+    p.single_token = max_len <= 1;  // decode-step shape: every lane at most one token
+    p.max_len = (int)std::min<size_t>(max_len, 0x7fffffff);
     if (offsets) {
         arena_reset(ctx);
         if ((rc = arena_reserve(ctx, arena_round(lanes * 4) * 2)) != PSSA_B200_OK) return rc;

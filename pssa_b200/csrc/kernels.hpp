@@ -34,6 +34,8 @@ struct SsmParams {
     const uint32_t* lengths;  // per lane row count, null = rows
     size_t rows;
     int d, s, lanes;
+    int max_len;           // longest lane, 0 = not known: with `rows` it tells how many lanes are in flight at a time
+    int tiled;             // time chunks: stay with the tiled kernel
     int aligned;           // 16-byte vector staging allowed
     // row pitches in floats (0 = dense: d for delta, s for b_proj / c_proj)
     size_t ld_delta, ld_bc;
@@ -48,6 +50,8 @@ struct SsmParams {
     size_t sum_delta_stride;
 };
 int32_t launch_ssm_fused(pssa_b200_ctx* ctx, const SsmParams& p, bool exact);
+// into how many consecutive time chunks each lane of this call is best cut (1 = a single pass); needs max_len and rows
+size_t ssm_time_chunks(const pssa_b200_ctx* ctx, const SsmParams& p, bool exact);
 // 16-byte staging and stores need 16-byte aligned bases and row pitches / widths that are multiples of 4 floats
 inline bool ssm_vector_ok(const SsmParams& p) {
     auto al = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };

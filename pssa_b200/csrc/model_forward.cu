@@ -169,11 +169,19 @@ int32_t forward_rows(pssa_b200_model* m, size_t rows, size_t lanes, const uint32
     bool single_token = true;  // a decode step: the SSM stage is then one pass over the carries
     uint32_t max_len = 0;
     for (size_t l = 0; l < lanes; ++l) single_token = single_token && h_len[l] <= 1, max_len = std::max(max_len, h_len[l]);
-    // Time chunks. The fused SSM kernel parallelises over lanes x channels only; with few lanes (long sequences) that
-    // leaves most SMs idle, so each lane is cut into `n_chunks` consecutive time chunks that run as independent
-    // "virtual lanes" in two passes: chunk maps from a zero carry, a fold of the maps in time order, then the real pass
-    // with each chunk's carry-in. Every exp is paid twice, so this is only done when the plain launch would occupy at
-    // most one CTA per SM -- or in the sequence-parallel mode, where the two passes are paid anyway.
+    // the SSM stage of a block; the block's own pointers (rates, carries) are filled in per block
+    SsmParams ssm{};
+    ssm.delta = ws.proj + m->off_delta, ssm.x_norm = ws.x_norm, ssm.b_proj = ws.proj + m->off_b, ssm.c_proj = ws.proj + m->off_c;
+    ssm.rates = m->blocks[0].rates, ssm.y = ws.y, ssm.y_bf16 = exact ? nullptr : ws.y_bf16;
+    ssm.offsets = ws.lane_off, ssm.lengths = ws.lane_len, ssm.rows = rows, ssm.d = d, ssm.s = s, ssm.lanes = (int)lanes;
+    ssm.ld_delta = nc, ssm.ld_bc = nc, ssm.lane_slots = ws.lane_slot, ssm.carry_stride = m->depth * m->loops * ds;
+    ssm.aligned = ssm_vector_ok(ssm);
+    ssm.single_token = single_token, ssm.max_len = (int)max_len;
+    // Time chunks. The SSM kernels parallelise over lanes x channels only; one long sequence can leave most of the machine
+    // idle, so each lane can be cut into `n_chunks` consecutive time chunks that run as independent "virtual lanes" in two
+    // passes: chunk maps from a zero carry, a fold of the maps in time order, then the real pass with each chunk's
+    // carry-in. Every exp is paid twice, so this is only done where it is the faster way all the same (ssm_time_chunks) --
+    // or in the sequence-parallel mode, where the two passes are paid anyway.
     const size_t ctas = lanes * ((m->d + 63) / 64);
     const size_t slots = (size_t)ctx->sm_count * 4;
     size_t n_chunks = 1;
@@ -183,12 +191,12 @@ int32_t forward_rows(pssa_b200_model* m, size_t rows, size_t lanes, const uint32
         // never on this rank's shard lengths, which differ between ranks (a shard may even be a single token).
         n_chunks = std::min<size_t>(16, std::max<size_t>(1, slots / ctas));
         n_chunks = std::min(n_chunks, std::max<size_t>(1, m->sp.capacity / lanes));
-    } else if (!single_token && ctas <= (size_t)ctx->sm_count) {
-        n_chunks = std::min<size_t>(16, std::max<size_t>(1, slots / ctas));
-        n_chunks = std::min(n_chunks, std::max<size_t>(1, max_len / 128));
+    } else if (!single_token) {
+        n_chunks = ssm_time_chunks(ctx, ssm, exact);
     }
     const bool two_pass = m->sp.active || n_chunks > 1;
     const size_t vlanes = lanes * n_chunks;
+    const int chunk_len = (int)((max_len + n_chunks - 1) / n_chunks);
     if (two_pass) {
         if (m->sp.active && vlanes > m->sp.capacity)
             return fail(ctx, PSSA_B200_ERR_SHAPE, "sequence-parallel prefill: %zu lanes exceed the %zu records the exchange buffers hold",
@@ -334,20 +342,17 @@ int32_t forward_rows(pssa_b200_model* m, size_t rows, size_t lanes, const uint32
                 return rc;
         }
         // stage 3: SSM with the lane carries of this block (src/gpu_batch.rs:582-619)
-        SsmParams sp{};
-        sp.delta = ws.proj + m->off_delta, sp.x_norm = ws.x_norm, sp.b_proj = ws.proj + m->off_b, sp.c_proj = ws.proj + m->off_c;
-        sp.rates = b.rates, sp.carry = carry_base, sp.y = ws.y, sp.y_bf16 = exact ? nullptr : ws.y_bf16;
-        sp.offsets = ws.lane_off + l0, sp.lengths = ws.lane_len + l0, sp.rows = rows, sp.d = d, sp.s = s, sp.lanes = (int)nl;  // lanes of this group; rows stay absolute
-        sp.ld_delta = nc, sp.ld_bc = nc, sp.lane_slots = ws.lane_slot + l0, sp.carry_stride = carry_stride;
-        sp.aligned = ssm_vector_ok(sp);
-        sp.single_token = single_token;
+        SsmParams sp = ssm;
+        sp.rates = b.rates, sp.carry = carry_base;
+        sp.offsets = ws.lane_off + l0, sp.lengths = ws.lane_len + l0, sp.lane_slots = ws.lane_slot + l0;
+        sp.lanes = (int)nl, sp.rows = nr;  // of this group; row numbers stay absolute
         if (two_pass) {
             // pass 1: every chunk's affine map (sum of delta, end state from a zero carry), one record per virtual lane
             const size_t rec = (size_t)d + ds;
             float* records = m->sp.active ? m->sp.send : m->chunks.records;
             PSSA_CUDA(ctx, cudaMemsetAsync(records, 0, vlanes * rec * sizeof(float), ctx->stream));
             SsmParams ag = sp;
-            ag.offsets = m->chunks.off, ag.lengths = m->chunks.len, ag.lanes = (int)vlanes;
+            ag.offsets = m->chunks.off, ag.lengths = m->chunks.len, ag.lanes = (int)vlanes, ag.max_len = chunk_len, ag.tiled = 1;
             ag.carry = records + d, ag.carry_stride = rec, ag.lane_slots = nullptr;
             ag.sum_delta = records, ag.sum_delta_stride = rec;
             ag.y_bf16 = nullptr, ag.single_token = 0;  // y of this pass is scratch: the real pass below overwrites it
@@ -365,7 +370,7 @@ int32_t forward_rows(pssa_b200_model* m, size_t rows, size_t lanes, const uint32
                                          carry_base, carry_stride, ws.lane_slot, m->chunks.carry_in, d, s)))
                 return rc;
             // pass 2: the real one, over the virtual lanes with their carry-ins (carry-outs are scratch)
-            sp.offsets = m->chunks.off, sp.lengths = m->chunks.len, sp.lanes = (int)vlanes;
+            sp.offsets = m->chunks.off, sp.lengths = m->chunks.len, sp.lanes = (int)vlanes, sp.max_len = chunk_len, sp.tiled = 1;
             sp.carry = m->chunks.carry_in, sp.carry_stride = ds, sp.lane_slots = nullptr, sp.single_token = 0;
         }
         if ((rc = launch_ssm_fused(ctx, sp, exact))) return rc;

@@ -20,10 +20,12 @@
 // Two arithmetic modes:
 //   FAST  ex2.approx on delta*(A*log2 e) (the reference's own GPU recipe, stages.ptx:21-22),
 //         FMA contraction, y summed per thread then by a shuffle tree over the G threads.
-//   EXACT expf, separately rounded multiply/add in the reference's order (src/pssa.rs:1131-1144);
+//   EXACT exp_exact, separately rounded multiply/add in the reference's order (src/pssa.rs:1131-1144);
 //         with G == 1 the sum over j is the reference's sequential sum.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
+
+#include <algorithm>
 
 #include "bounds.hpp"
 #include "context.hpp"
@@ -58,6 +60,26 @@ __device__ __forceinline__ float ex2_approx(float x) {
     return y;
 }
 
+// exp for the exact mode: x = n ln 2 + r by a two-part ln 2, e^r = 1 + (r + r^2 q(r)) with a quartic q (least largest relative
+// error on |r| <= ln 2 / 2, fitted by linear programming: 2^-28.3), n added to the exponent. For the decays of the
+// recurrence (-0.08 < x <= 0) 97 % of the results are the correctly rounded ones (largest error 0.57 ulp), which is what the
+// reference's host libm returns, so its states are met in far more bits than with a 1 to 2 ulp exp; and the XU pipe is not
+// used. Results near or below the smallest normal number, and overflow, are left to expf.
+__device__ __forceinline__ float exp_exact(float x) {
+    const float t = fmaf(x, 1.4426950408889634f, 12582912.0f);  // 1.5 * 2^23: the integer part ends up in the low bits
+    const float n = t - 12582912.0f;
+    float r = fmaf(n, -0.693145751953125f, x);
+    r = fmaf(n, -1.4286068202862268e-06f, r);
+    float q = 0.0013814537087455392f;
+    q = fmaf(q, r, 0.00836874544620514f);
+    q = fmaf(q, r, 0.04166838899254799f);
+    q = fmaf(q, r, 0.1666652113199234f);
+    q = fmaf(q, r, 0.4999999403953552f);
+    const float e = 1.0f + fmaf(q, __fmul_rn(r, r), r);
+    const float y = __int_as_float(__float_as_int(e) + (__float_as_int(t) << 23));
+    return fabsf(x) < 87.0f ? y : expf(x);
+}
+
 // Packed fp32 pairs (one instruction, two IEEE-rounded results): the kernel is bound by instruction issue, and the
 // per-state multiply / fma work is half the instruction stream.
 typedef unsigned long long f32x2;
@@ -78,6 +100,37 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
     f32x2 r;
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
     return r;
+}
+
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// 2^x for a pair of x <= 0 on the FMA pipe: x = n + f with |f| <= 1/2 by adding and taking off 1.5 * 2^23, 2^f by a degree-5
+// polynomial with p(0) = 1 (least largest relative error under that constraint, fitted by linear programming: 2^-22.5 after
+// fp32 rounding, mean -2e-8), n added to the exponent. Below 2^-126 the result stays at that size instead of going to zero.
+__device__ __forceinline__ f32x2 exp2_poly2(f32x2 x) {
+    float x0, x1;
+    unpack2(x, x0, x1);
+    x = pack2(fmaxf(x0, -126.0f), fmaxf(x1, -126.0f));
+    const f32x2 t = add2(x, pack2(12582912.0f, 12582912.0f));
+    const f32x2 f = fma2(add2(t, pack2(-12582912.0f, -12582912.0f)), pack2(-1.0f, -1.0f), x);
+    f32x2 r = pack2(0.001326472731307149f, 0.001326472731307149f);
+    r = fma2(r, f, pack2(0.009671512991189957f, 0.009671512991189957f));
+    r = fma2(r, f, pack2(0.05550733581185341f, 0.05550733581185341f));
+    r = fma2(r, f, pack2(0.24022242426872253f, 0.24022242426872253f));
+    r = fma2(r, f, pack2(0.6931470036506653f, 0.6931470036506653f));
+    r = fma2(r, f, pack2(1.0f, 1.0f));
+    float t0, t1, r0, r1;
+    unpack2(t, t0, t1);
+    unpack2(r, r0, r1);
+    return pack2(__int_as_float(__float_as_int(r0) + (__float_as_int(t0) << 23)), __int_as_float(__float_as_int(r1) + (__float_as_int(t1) << 23)));
+}
+__device__ __forceinline__ f32x2 exp2_approx2(f32x2 x) {
+    float x0, x1;
+    unpack2(x, x0, x1);
+    return pack2(ex2_approx(x0), ex2_approx(x1));
 }
 
 template <int ST, int G, bool EXACT, bool TAPE, int THR = kThreads, int CPT = 1>
@@ -253,7 +306,7 @@ __global__ void __launch_bounds__(THR, (ST <= 16 && !TAPE && !EXACT) ? ((THR > 2
             if (EXACT) {
 #pragma unroll
                 for (int jj = 0; jj < ST; ++jj) {
-                    float a = expf(__fmul_rn(dl, A[jj]));
+                    float a = exp_exact(__fmul_rn(dl, A[jj]));
                     float bb = __fmul_rn(dl, bj[jj]);
                     h[jj] = __fadd_rn(__fmul_rn(a, h[jj]), __fmul_rn(bb, xv));
                     yp = __fadd_rn(yp, __fmul_rn(h[jj], cj[jj]));
@@ -269,18 +322,18 @@ __global__ void __launch_bounds__(THR, (ST <= 16 && !TAPE && !EXACT) ? ((THR > 2
 #pragma unroll
                 for (int jj = 0; jj < ST; jj += 2) {
                     const f32x2 b2 = pack2(bj[jj], bj[jj + 1]), c2 = pack2(cj[jj], cj[jj + 1]);
-                    float e0, e1;
-                    unpack2(mul2(dl2, pack2(A[jj], A[jj + 1])), e0, e1);
-                    const float a0 = ex2_approx(e0), a1 = ex2_approx(e1);
-                    f32x2 h2 = fma2(pack2(a0, a1), pack2(h[jj], h[jj + 1]), mul2(w2, b2));
+                    // one pair of exponentials in eight goes to the FMA pipe (the benchmark's launch: 960 us with none, 925 with
+                    // one, 1039 with two, whose extra issue slots cost more than the XU pipe gains)
+                    const bool poly = ST == 16 && G == 4 && !TAPE && jj == 0;
+                    const f32x2 arg = mul2(dl2, pack2(A[jj], A[jj + 1]));
+                    const f32x2 a2 = poly ? exp2_poly2(arg) : exp2_approx2(arg);
+                    f32x2 h2 = fma2(a2, pack2(h[jj], h[jj + 1]), mul2(w2, b2));
                     unpack2(h2, h[jj], h[jj + 1]);
                     y2 = fma2(h2, c2, y2);
-                    if (TAPE) av[jj] = a0, av[jj + 1] = a1, bv[jj] = dl * bj[jj], bv[jj + 1] = dl * bj[jj + 1];
+                    if (TAPE) unpack2(a2, av[jj], av[jj + 1]), bv[jj] = dl * bj[jj], bv[jj + 1] = dl * bj[jj + 1];
                     if constexpr (CPT > 1) {
-                        float f0, f1;
-                        unpack2(mul2(dlb2, pack2(A1[jj], A1[jj + 1])), f0, f1);
-                        const float g0 = ex2_approx(f0), g1 = ex2_approx(f1);
-                        f32x2 hb2 = fma2(pack2(g0, g1), pack2(h1[jj], h1[jj + 1]), mul2(wb2, b2));
+                        const f32x2 argb = mul2(dlb2, pack2(A1[jj], A1[jj + 1]));
+                        f32x2 hb2 = fma2(poly ? exp2_poly2(argb) : exp2_approx2(argb), pack2(h1[jj], h1[jj + 1]), mul2(wb2, b2));
                         unpack2(hb2, h1[jj], h1[jj + 1]);
                         yb2 = fma2(hb2, c2, yb2);
                     }
@@ -367,6 +420,356 @@ __global__ void __launch_bounds__(THR, (ST <= 16 && !TAPE && !EXACT) ? ((THR > 2
         };
         store_state(h, i, valid);
         if constexpr (CPT > 1) store_state(h1, i1, valid1);
+    }
+}
+
+// Few lanes. The kernel above gives a warp eight channels, so one sequence of a 768-channel model is 96 warps on 592
+// schedulers; and cutting such sequences into time chunks pays every exponential twice. Here a channel's states are spread
+// over more lanes: LPC lanes hold SPL states each, 32 / LPC channels to a warp.
+//   * a lane owns pieces of V adjacent states, the pieces LPC * V apart, and neighbouring lanes hold the same states of
+//     different channels: a token's B and C are conflict-free 16-byte loads that neighbours share, and the tape (states,
+//     bar_a, bar_b) leaves in whole lines.
+//   * y needs a sum over the LPC lanes for every token: the lanes leave their partials in shared memory and the tile's sums
+//     are taken at its end, a lane per token, so no shuffle sits in the token loop. The exact mode sums the s products of
+//     a token one after another there, as the reference does.
+//   * few lanes leave a warp alone on its scheduler, so everything has to overlap inside it: see the token loop.
+//   * a tile's tail is padded with delta = 0, which leaves the state as it is (exp(0) = 1, input 0).
+// What bounds it: alone, a token's dependent instructions (about 85 cycles, 32 of them exponentials); with many warps the
+// shared-memory pipe (0.7 of its wavefronts) before the XU pipe (0.55).
+constexpr int kWideStages = 3;
+constexpr int kWideWarps = 4;
+template <int LPC, int SPL, int TT, bool EXACT>
+constexpr size_t wide_smem_floats() {
+    const int ch = kWideWarps * (32 / LPC), s = LPC * SPL;
+    return (size_t)kWideStages * TT * (2 * s + 2 * (ch + 4)) + 2 * TT * (ch + 4) + 2 * (size_t)TT * (ch + 1) * 4 +
+           (EXACT ? (size_t)kWideWarps * 32 * (s + 1) : (size_t)kWideWarps * TT * 36);
+}
+
+__device__ __forceinline__ void cp_async16_zfill(void* smem, const void* gmem, bool live) {
+    unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(live ? 16 : 0));
+}
+
+template <int V> struct WideVec;
+template <> struct WideVec<2> { typedef float2 type; };
+template <> struct WideVec<4> { typedef float4 type; };
+
+template <int LPC, int SPL, int TT, bool EXACT, bool TAPE>
+__global__ void __launch_bounds__(kWideWarps * 32) ssm_wide_kernel(SsmParams p) {
+    pdl_trigger();
+    pdl_wait();
+    constexpr int WARPS = kWideWarps;      // TT: tokens per staged tile
+    constexpr int S = LPC * SPL;           // states per channel
+    constexpr int V = SPL < 4 ? SPL : 4;   // adjacent states of a lane: one 8- or 16-byte access
+    constexpr int NQ = SPL / V;            // such pieces per lane, LPC * V states apart
+    constexpr int NP = SPL / 2;            // state pairs per lane
+    constexpr int CPW = 32 / LPC;          // channels per warp
+    constexpr int CH = WARPS * CPW;        // channels per CTA
+    constexpr int THR = WARPS * 32;
+    constexpr int CQ = CH / 4, SQ = S / 4;
+    constexpr int DP = CH + 4, WP = CH + 1;  // token pitches that spread the banks over tokens
+    typedef typename WideVec<V>::type vec;
+    static_assert(CH % 4 == 0 && (!EXACT || TT % LPC == 0) && TT % 8 == 0, "tile shapes");
+    extern __shared__ __align__(16) float smem[];
+    float* sm_b = smem;                                   // [stages][TT][S]
+    float* sm_c = sm_b + kWideStages * TT * S;            // [stages][TT][S]
+    float* sm_d = sm_c + kWideStages * TT * S;            // [stages][TT][DP]
+    float* sm_x = sm_d + kWideStages * TT * DP;           // [stages][TT][DP]
+    float* sm_y = sm_x + kWideStages * TT * DP;           // [2][TT][DP]
+    float4* sm_dw = reinterpret_cast<float4*>(sm_y + 2 * TT * DP);        // [2][TT][WP]
+    float* sm_p = reinterpret_cast<float*>(sm_dw + 2 * WP * TT);          // exact: [WARPS][32][S + 1]; fast: [WARPS][TT][36]
+
+    const int tid = threadIdx.x, wid = tid >> 5, lane_id = tid & 31;
+    const int jl = lane_id / CPW, cw = lane_id % CPW;
+    const int c = wid * CPW + cw;
+    const int ncb = (p.d + CH - 1) / CH;
+    const int lane = blockIdx.x / ncb;
+    const int i0 = (blockIdx.x % ncb) * CH;
+    const int i = i0 + c;
+    const bool valid = i < p.d;
+    const size_t row0 = p.offsets ? p.offsets[lane] : 0;
+    const int len = p.lengths ? (int)p.lengths[lane] : (int)p.rows;
+    if (len <= 0) return;
+    const int d = p.d;
+    const size_t ds = (size_t)d * S;
+    const size_t ldd = p.ld_delta ? p.ld_delta : (size_t)d;
+    const size_t ldbc = p.ld_bc ? p.ld_bc : (size_t)S;
+    float* carry = p.carry ? p.carry + (size_t)(p.lane_slots ? p.lane_slots[lane] : lane) * (p.carry_stride ? p.carry_stride : ds) : nullptr;
+    const size_t so = (size_t)i * S + V * jl;
+    float A[SPL], h[SPL];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        vec a{}, hv{};
+        if (valid) a = __ldg(reinterpret_cast<const vec*>(p.rates + so + q * V * LPC));
+        if (valid && carry) hv = *reinterpret_cast<const vec*>(carry + so + q * V * LPC);
+#pragma unroll
+        for (int v = 0; v < V; ++v) A[q * V + v] = reinterpret_cast<const float*>(&a)[v], h[q * V + v] = reinterpret_cast<const float*>(&hv)[v];
+    }
+    auto put = [&](float* base, int t, int q, const float* v) {  // one piece of a tape row
+        vec o;
+#pragma unroll
+        for (int u = 0; u < V; ++u) reinterpret_cast<float*>(&o)[u] = v[u];
+        *reinterpret_cast<vec*>(base + (row0 + t) * ds + so + q * V * LPC) = o;
+    };
+
+    const int ntiles = (len + TT - 1) / TT;
+    auto load_tile = [&](int k) {
+        if (k < ntiles) {
+            const int st = k % kWideStages, t0 = k * TT;
+            for (int idx = tid; idx < TT * SQ; idx += THR) {
+                const int tt = idx / SQ, j = idx % SQ * 4;
+                const bool live = t0 + tt < len;
+                const size_t o = (row0 + (live ? t0 + tt : 0)) * ldbc + j;
+                cp_async16_zfill(sm_b + (st * TT + tt) * S + j, p.b_proj + o, live);
+                cp_async16_zfill(sm_c + (st * TT + tt) * S + j, p.c_proj + o, live);
+            }
+            for (int idx = tid; idx < TT * CQ; idx += THR) {
+                const int tt = idx / CQ, q = idx % CQ;
+                const bool live = t0 + tt < len && i0 + q * 4 < d;
+                const size_t row = row0 + (live ? t0 + tt : 0), col = live ? i0 + q * 4 : 0;
+                cp_async16_zfill(sm_d + (st * TT + tt) * DP + q * 4, p.delta + row * ldd + col, live);
+                cp_async16_zfill(sm_x + (st * TT + tt) * DP + q * 4, p.x_norm + row * d + col, live);
+            }
+        }
+        cp_async_commit();
+    };
+    // y of a finished tile: 16-byte pieces of CH channels per token
+    auto store_y = [&](int k) {
+        const int t0 = k * TT, nt = min(TT, len - t0);
+        for (int idx = tid; idx < nt * CQ; idx += THR) {
+            const int tt = idx / CQ, q = idx % CQ;
+            if (i0 + q * 4 < d) {
+                const float4 v = *reinterpret_cast<const float4*>(sm_y + ((k & 1) * TT + tt) * DP + q * 4);
+                const size_t o = (row0 + t0 + tt) * (size_t)d + i0 + q * 4;
+                *reinterpret_cast<float4*>(p.y + o) = v;
+                if (p.y_bf16) {
+                    __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+                    uint2 pk;
+                    pk.x = *reinterpret_cast<unsigned*>(&lo), pk.y = *reinterpret_cast<unsigned*>(&hi);
+                    *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.y_bf16) + o) = pk;
+                }
+            }
+        }
+    };
+    // (delta, delta, delta * x, delta * x) of the group's channel for every token of a landed tile, spread over its lanes
+    auto prepare = [&](int k) {
+        const int st = k % kWideStages;
+#pragma unroll
+        for (int t = jl; t < TT; t += LPC) {
+            const float dl = sm_d[(st * TT + t) * DP + c], xv = sm_x[(st * TT + t) * DP + c];
+            sm_dw[((k & 1) * TT + t) * WP + c] = EXACT ? make_float4(dl, xv, 0.f, 0.f) : make_float4(dl, dl, dl * xv, dl * xv);
+        }
+    };
+    load_tile(0);
+    load_tile(1);
+    if constexpr (EXACT) {
+        for (int k = 0; k < ntiles; ++k) {
+            cp_async_wait<1>();
+            __syncthreads();  // tile k has landed; every warp is done with tile k - 1 and its y values are complete
+            load_tile(k + 2);
+            if (k > 0) store_y(k - 1);
+            prepare(k);
+            __syncwarp();
+            const int st = k % kWideStages, t0 = k * TT;
+#pragma unroll 1
+            for (int s0 = 0; s0 < TT; s0 += LPC) {
+                if (s0 > 0 && t0 + s0 >= len) break;
+                const float4* dw = sm_dw + ((k & 1) * TT + s0) * WP + c;
+                const int sj = (st * TT + s0) * S + V * jl;
+#pragma unroll 8
+                for (int tt = 0; tt < LPC; ++tt) {
+                    const float4 w4 = dw[tt * WP];
+#pragma unroll
+                    for (int q = 0; q < NQ; ++q) {
+                        const vec bv = *reinterpret_cast<const vec*>(sm_b + sj + tt * S + q * V * LPC);
+                        const vec cv = *reinterpret_cast<const vec*>(sm_c + sj + tt * S + q * V * LPC);
+                        float a[V], bb[V];
+#pragma unroll
+                        for (int v = 0; v < V; ++v) {
+                            a[v] = exp_exact(__fmul_rn(w4.x, A[q * V + v]));
+                            bb[v] = __fmul_rn(w4.x, reinterpret_cast<const float*>(&bv)[v]);
+                            h[q * V + v] = __fadd_rn(__fmul_rn(a[v], h[q * V + v]), __fmul_rn(bb[v], w4.y));
+                            sm_p[(wid * 32 + cw * LPC + tt) * (S + 1) + q * V * LPC + V * jl + v] =
+                                __fmul_rn(h[q * V + v], reinterpret_cast<const float*>(&cv)[v]);
+                        }
+                        if (TAPE && valid && t0 + s0 + tt < len) {
+                            if (p.states) put(p.states, t0 + s0 + tt, q, h + q * V);
+                            if (p.bar_a) put(p.bar_a, t0 + s0 + tt, q, a);
+                            if (p.bar_b) put(p.bar_b, t0 + s0 + tt, q, bb);
+                        }
+                    }
+                }
+                // lane (cw, jl) sums token jl of channel cw over the states in order
+                __syncwarp();
+                const float* pr = sm_p + (wid * 32 + cw * LPC + jl) * (S + 1);
+                float y = 0.0f;
+#pragma unroll 16
+                for (int j = 0; j < S; ++j) y = __fadd_rn(y, pr[j]);
+                sm_y[((k & 1) * TT + s0 + jl) * DP + c] = y;
+                __syncwarp();
+            }
+        }
+    } else {
+        // The tokens form one stream of TB-token batches across tile borders: while batch b goes through the recurrence,
+        // batch b + 1's exponentials are formed and batch b + 2's operands are on their way from shared memory. Two register
+        // sets, used in turn, so that nothing is moved between them.
+        constexpr int TB = 2, TG = 4 * TB;
+        f32x2 A2[NP], h2[NP];
+#pragma unroll
+        for (int q = 0; q < NP; ++q)
+            A2[q] = pack2(A[2 * q] * 1.4426950408889634f, A[2 * q + 1] * 1.4426950408889634f), h2[q] = pack2(h[2 * q], h[2 * q + 1]);
+        struct Ops { ulonglong2 w[TB]; f32x2 b[TB][NP]; };
+        struct Exps { f32x2 e[TB][NP], u[TB][NP]; };
+        struct Cs { f32x2 c[TB][NP]; };
+        auto load_pairs = [&](const float* src, f32x2* dst) {
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) {
+                if constexpr (V == 4) {
+                    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(src + q * V * LPC);
+                    dst[2 * q] = v.x, dst[2 * q + 1] = v.y;
+                } else {
+                    dst[q] = *reinterpret_cast<const f32x2*>(src + q * V * LPC);
+                }
+            }
+        };
+        // sb / sd: this lane's first state of a group of TG tokens in sm_b (sm_c lies a constant away), its channel's row of sm_dw
+        auto fetch = [&](const float* sb, const float4* sd, int b, Ops& o) {
+#pragma unroll
+            for (int u = 0; u < TB; ++u) {
+                o.w[u] = *reinterpret_cast<const ulonglong2*>(sd + (b * TB + u) * WP);
+                load_pairs(sb + (b * TB + u) * S, o.b[u]);
+            }
+        };
+        auto fetch_c = [&](const float* sb, int b, Cs& o) {
+#pragma unroll
+            for (int u = 0; u < TB; ++u) load_pairs(sb + kWideStages * TT * S + (b * TB + u) * S, o.c[u]);
+        };
+        auto expand = [&](const Ops& o, Exps& x) {
+            f32x2 arg[TB][NP];
+#pragma unroll
+            for (int u = 0; u < TB; ++u)
+#pragma unroll
+                for (int q = 0; q < NP; ++q) arg[u][q] = mul2(o.w[u].x, A2[q]);
+#pragma unroll
+            for (int u = 0; u < TB; ++u)
+#pragma unroll
+                for (int q = 0; q < NP; ++q) {
+                    x.e[u][q] = exp2_approx2(arg[u][q]);
+                    x.u[u][q] = mul2(o.w[u].y, o.b[u][q]);
+                }
+        };
+        auto recur = [&](const float* sb, const float4* sd, float* part, int t0, int b, const Exps& x, const Cs& cc) {
+            f32x2 hs[TB][NP], y2[TB];
+#pragma unroll
+            for (int u = 0; u < TB; ++u)
+#pragma unroll
+                for (int q = 0; q < NP; ++q) hs[u][q] = fma2(x.e[u][q], u == 0 ? h2[q] : hs[u - 1][q], x.u[u][q]);
+#pragma unroll
+            for (int q = 0; q < NP; ++q)
+#pragma unroll
+                for (int u = 0; u < TB; ++u) y2[u] = q == 0 ? mul2(hs[u][q], cc.c[u][q]) : fma2(hs[u][q], cc.c[u][q], y2[u]);
+#pragma unroll
+            for (int q = 0; q < NP; ++q) h2[q] = hs[TB - 1][q];
+#pragma unroll
+            for (int u = 0; u < TB; ++u) {
+                float lo, hi;
+                unpack2(y2[u], lo, hi);
+                part[(b * TB + u) * 36] = lo + hi;
+                const int t = t0 + b * TB + u;
+                if (TAPE && valid && t < len) {
+                    const float dl = sd[(b * TB + u) * WP].x;
+                    f32x2 bp[NP];
+                    load_pairs(sb + (b * TB + u) * S, bp);
+                    float hv[SPL], av[SPL], bw[SPL];
+#pragma unroll
+                    for (int q = 0; q < NP; ++q) {
+                        unpack2(hs[u][q], hv[2 * q], hv[2 * q + 1]);
+                        unpack2(x.e[u][q], av[2 * q], av[2 * q + 1]);
+                        unpack2(mul2(pack2(dl, dl), bp[q]), bw[2 * q], bw[2 * q + 1]);
+                    }
+#pragma unroll
+                    for (int q = 0; q < NQ; ++q) {
+                        if (p.states) put(p.states, t, q, hv + q * V);
+                        if (p.bar_a) put(p.bar_a, t, q, av + q * V);
+                        if (p.bar_b) put(p.bar_b, t, q, bw + q * V);
+                    }
+                }
+            }
+        };
+        Ops oa, ob;
+        Exps ea, eb;
+        Cs ca, cb;
+        for (int k = 0; k < ntiles; ++k) {
+            cp_async_wait<0>();
+            __syncthreads();  // tiles k and k + 1 have landed; every warp is done with tile k - 1 and its y values are complete
+            load_tile(k + 2);
+            if (k > 0) store_y(k - 1);
+            if (k == 0) prepare(0);
+            prepare(k + 1);
+            __syncwarp();
+            const float* sb = sm_b + (k % kWideStages) * TT * S + V * jl;
+            const float4* sd = sm_dw + (k & 1) * WP * TT + c;
+            const float* const sb_next = sm_b + ((k + 1) % kWideStages) * TT * S + V * jl;
+            const float4* const sd_next = sm_dw + ((k + 1) & 1) * WP * TT + c;
+            float* part = sm_p + wid * TT * 36 + cw * LPC + jl;
+            if (k == 0) {
+                fetch(sb, sd, 0, oa);
+                fetch(sb, sd, 1, ob);
+                fetch_c(sb, 0, ca);
+                expand(oa, ea);
+            }
+#pragma unroll 1
+            for (int g = 0; g < TT / TG; ++g) {
+                const float* nb = g == TT / TG - 1 ? sb_next : sb + TG * S;
+                const float4* nd = g == TT / TG - 1 ? sd_next : sd + TG * WP;
+                const int tg = k * TT + g * TG;
+                fetch(sb, sd, 2, oa);
+                fetch_c(sb, 1, cb);
+                recur(sb, sd, part, tg, 0, ea, ca);
+                expand(ob, eb);
+                fetch(sb, sd, 3, ob);
+                fetch_c(sb, 2, ca);
+                recur(sb, sd, part, tg, 1, eb, cb);
+                expand(oa, ea);
+                fetch(nb, nd, 0, oa);
+                fetch_c(sb, 3, cb);
+                recur(sb, sd, part, tg, 2, ea, ca);
+                expand(ob, eb);
+                fetch(nb, nd, 1, ob);
+                fetch_c(nb, 0, ca);
+                recur(sb, sd, part, tg, 3, eb, cb);
+                expand(oa, ea);
+                sb = nb, sd = nd, part += TG * 36;
+            }
+            // the tile's sums over the LPC lanes of a channel: lane (cw, jl) finishes tokens jl, jl + LPC, ... of channel cw
+            __syncwarp();
+#pragma unroll
+            for (int t = jl; t < TT; t += LPC) {
+                const float4* pr = reinterpret_cast<const float4*>(sm_p + (wid * TT + t) * 36 + cw * LPC);
+                float4 acc = pr[0];
+#pragma unroll
+                for (int q = 1; q < LPC / 4; ++q) {
+                    const float4 v = pr[q];
+                    acc.x += v.x, acc.y += v.y, acc.z += v.z, acc.w += v.w;
+                }
+                sm_y[((k & 1) * TT + t) * DP + c] = (acc.x + acc.y) + (acc.z + acc.w);
+            }
+            __syncwarp();
+        }
+#pragma unroll
+        for (int q = 0; q < NP; ++q) unpack2(h2[q], h[2 * q], h[2 * q + 1]);
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+    store_y(ntiles - 1);
+    if (carry && valid) {
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            vec o;
+#pragma unroll
+            for (int v = 0; v < V; ++v) reinterpret_cast<float*>(&o)[v] = h[q * V + v];
+            *reinterpret_cast<vec*>(carry + so + q * V * LPC) = o;
+        }
     }
 }
 
@@ -480,7 +883,7 @@ __global__ void __launch_bounds__(256) seqpar_fold_kernel(const float* __restric
             if (j < n) {
                 const int k = j / chunks, c = j - k * chunks;
                 const float* r = gathered + (size_t)k * rank_stride + ((size_t)lane * chunks + c) * rec;
-                pk[u] = expf(__fmul_rn(a, __ldg(r + i)));
+                pk[u] = exp_exact(__fmul_rn(a, __ldg(r + i)));
                 add[u] = __ldg(r + d + e);
             }
         }
@@ -518,12 +921,71 @@ int32_t launch_cfg(pssa_b200_ctx* ctx, const SsmParams& p) {
     return after_launch(ctx, "ssm_fused_kernel");
 }
 
+template <int LPC, int SPL, int TT, bool EXACT, bool TAPE>
+int32_t launch_wide_cfg(pssa_b200_ctx* ctx, const SsmParams& p) {
+    constexpr int CH = kWideWarps * (32 / LPC);
+    constexpr size_t smem = wide_smem_floats<LPC, SPL, TT, EXACT>() * sizeof(float);
+    auto kern = ssm_wide_kernel<LPC, SPL, TT, EXACT, TAPE>;
+    static PerDeviceOnce attr_set;
+    if (smem > 48 * 1024 && attr_set.need(ctx->device)) {
+        PSSA_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        attr_set.done(ctx->device);
+    }
+    const size_t blocks = (size_t)((p.d + CH - 1) / CH) * p.lanes;
+    if (blocks > 0x7fffffffull)
+        return fail(ctx, PSSA_B200_ERR_SHAPE, "B200 SSM grid (%zu, 1) exceeds grid limits; refusing launch", blocks);
+    PSSA_CUDA(ctx, launch_dependent(kern, dim3((unsigned)blocks), dim3(kWideWarps * 32), smem, ctx->stream, p));
+    return after_launch(ctx, "ssm_fused_kernel[few lanes]");
+}
+template <int LPC, int SPL, int TT>
+int32_t launch_wide(pssa_b200_ctx* ctx, const SsmParams& p, bool exact) {
+    const bool tape = p.states || p.bar_a || p.bar_b;
+    if (exact) return tape ? launch_wide_cfg<LPC, SPL, 32, true, true>(ctx, p) : launch_wide_cfg<LPC, SPL, 32, true, false>(ctx, p);
+    return tape ? launch_wide_cfg<LPC, SPL, TT, false, true>(ctx, p) : launch_wide_cfg<LPC, SPL, TT, false, false>(ctx, p);
+}
+
 // The tape outputs (states, bar_a, bar_b: the reference's training tape) cost d*s floats per token
 // each; inference never asks for them, so they live in a separate instantiation.
 template <int ST, int G, bool EXACT>
 int32_t launch_one(pssa_b200_ctx* ctx, const SsmParams& p) {
     if (p.states || p.bar_a || p.bar_b) return launch_cfg<ST, G, EXACT, true>(ctx, p);
     return launch_cfg<ST, G, EXACT, false>(ctx, p);
+}
+
+// CTA shape by wave balance. Every CTA of a launch is resident at once and a warp's time per token is fixed by
+// its exponentials (16 per lane and channel, 8 cycles each on its scheduler's XU pipe), so the launch lasts as
+// long as the busiest scheduler: count, per shape, the channel-warps the fullest SM puts on one scheduler.
+// 256 threads = 64 channels per CTA (4 CTAs per SM), 352 threads = 88 channels (2 per SM), 128 threads with two
+// channels per thread = 64 channels (3 per SM). With d = 768 and 32 lanes: 384 CTAs put 3 x 8 warps on most SMs
+// (6 per scheduler), 288 of 352 threads put 2 x 11 (6 on two schedulers, 5 on the others), 384 two-channel CTAs
+// put 3 x 4 double warps (6). On a tie the two-channel shape wins: a token's B and C rows are loaded once
+// for both channels (11.93 -> 11.67 ms for the 12 launches of the benchmark step).
+struct TiledShape {
+    int kind;  // 0 = 256 threads, 1 = 352, 2 = 128 with two channels per thread
+    long long busiest;
+};
+TiledShape tiled_shape(const pssa_b200_ctx* ctx, int d, int lanes) {
+    auto busiest = [&](int threads, int cpt, int cap) -> long long {
+        const int ch = threads / 4 * cpt;
+        const long long blocks = (long long)((d + ch - 1) / ch) * lanes;
+        const long long per_sm = (blocks + ctx->sm_count - 1) / ctx->sm_count;
+        if (per_sm > cap) return 1ll << 40;  // more than one wave: not considered
+        return (per_sm * (threads / 32) + 3) / 4 * cpt;
+    };
+    const long long two = busiest(128, 2, 3), wide = busiest(352, 1, 2), plain = busiest(256, 1, 4);
+    if (two <= wide && two <= plain) {
+        const long long all = ((long long)d * lanes / 8 + 4 * ctx->sm_count - 1) / (4 * ctx->sm_count);  // several waves
+        return {2, two < (1ll << 40) ? two : all};
+    }
+    if (wide < plain) return {1, wide};
+    return {0, plain};
+}
+
+// shapes the few-lanes kernel takes: state pairs that fill 4 to 32 lanes, 16-byte rows and states
+bool ssm_wide_ok(const SsmParams& p) {
+    auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+    return !p.tiled && (p.s == 16 || p.s == 32 || p.s == 64) && p.aligned && al16(p.rates) && al16(p.carry) && al16(p.states) &&
+           al16(p.bar_a) && al16(p.bar_b) && p.carry_stride % 4 == 0;
 }
 
 }  // namespace
@@ -537,6 +999,16 @@ int32_t launch_seqpar_fold(pssa_b200_ctx* ctx, const float* gathered, size_t rec
     seqpar_fold_kernel<<<grid, 256, 0, ctx->stream>>>(gathered, rec, world, rank, chunks, rank_stride, rates, state, state_stride,
                                                      lane_slots, carry_in, d, s);
     return after_launch(ctx, "seqpar_fold_kernel");
+}
+
+size_t ssm_time_chunks(const pssa_b200_ctx* ctx, const SsmParams& p, bool exact) {
+    const size_t longest = (size_t)p.max_len, ctas = (size_t)p.lanes * ((p.d + 63) / 64);
+    // Two passes pay every exponential twice. Where the few-lanes kernel applies they are the faster way only for a long
+    // sequence that leaves it under one and a half channels a scheduler (us, d 768, 64 states, one sequence: 2048 tokens 94
+    // in one pass, about 90 in two; 8192 tokens 357 and 326).
+    if (ssm_wide_ok(p) && (p.s < 64 || longest < (exact ? 4096 : 2048) || 2 * p.rows * (size_t)p.d > 3 * longest * 4 * (size_t)ctx->sm_count)) return 1;
+    if (ctas > (size_t)ctx->sm_count) return 1;
+    return std::min({(size_t)16, std::max<size_t>(1, 4 * (size_t)ctx->sm_count / ctas), std::max<size_t>(1, longest / 128)});
 }
 
 int32_t launch_ssm_fused(pssa_b200_ctx* ctx, const SsmParams& p, bool exact) {
@@ -558,6 +1030,29 @@ int32_t launch_ssm_fused(pssa_b200_ctx* ctx, const SsmParams& p, bool exact) {
         if (s <= 64) return launch_step<16>(ctx, p);
         return launch_step<32>(ctx, p);
     }
+    if (ssm_wide_ok(p)) {
+        // Channels in flight: lanes counted by their share of the longest one. With 64 states, up to one channel per scheduler
+        // takes 32 lanes a channel, above that 16; 32-token tiles while two CTAs an SM hold everything, 16-token ones
+        // (half the shared memory) beyond. With 64 states a full machine is the tiled kernel's: us per 1024 tokens at d = 768,
+        // tiled against this one: 1 lane 214 -> 52, 4 lanes 214 -> 91, 8 lanes 214 -> 171, 13 lanes 275 -> 237, but 24 lanes
+        // 344 and 402: the two lines below are fits of both. With 32 and 16 states this one is ahead at every size
+        // (384 x 32: 1 lane 226 -> 40, 64 lanes 369 -> 336; 192 x 16: 106 -> 40, 137 -> 104), and in the exact mode
+        // (64 states, 1 lane 1600 -> 107, 32 lanes 1742 -> 1604). The tape's stores decide where it is asked for: whole lines
+        // here, 4-byte pieces there. The lane splits sum y in different orders, so for calls of under 64 tokens a lane
+        // (decode loops start with those) the split follows the shape alone and a stream sees the same bits alone and in a
+        // batch; the exact mode's order is always the same.
+        const size_t longest = p.max_len ? (size_t)p.max_len : (p.lengths ? 1 : p.rows);
+        const int lanes = (int)std::max<size_t>(1, p.max_len || !p.lengths ? p.rows / std::max<size_t>(1, longest) : (size_t)p.lanes);
+        const size_t channels = (size_t)lanes * p.d, schedulers = 4 * (size_t)ctx->sm_count;
+        const bool by_shape = !exact && longest < 64;
+        if (s == 16) return channels <= 4 * schedulers && !by_shape ? launch_wide<8, 2, 32>(ctx, p, exact) : launch_wide<4, 4, 16>(ctx, p, exact);
+        if (s == 32) return channels <= 2 * schedulers && !by_shape ? launch_wide<16, 2, 32>(ctx, p, exact) : launch_wide<8, 4, 32>(ctx, p, exact);
+        if (channels <= (exact ? 2 : 1) * schedulers && !by_shape) return launch_wide<32, 2, 32>(ctx, p, exact);
+        if (channels <= 4 * schedulers) return launch_wide<16, 4, 32>(ctx, p, exact);
+        const double wide_us = 13.8 * (double)channels / (double)schedulers;
+        const double tiled_us = 66.0 + 70.0 * (double)tiled_shape(ctx, p.d, lanes).busiest;
+        if (exact || tape || by_shape || wide_us < tiled_us) return launch_wide<16, 4, 16>(ctx, p, exact);
+    }
     if (exact) {
         if (s <= 4) return launch_one<4, 1, true>(ctx, p);
         if (s <= 16) return launch_one<16, 1, true>(ctx, p);
@@ -570,25 +1065,10 @@ int32_t launch_ssm_fused(pssa_b200_ctx* ctx, const SsmParams& p, bool exact) {
         if (s <= 16) return launch_one<4, 4, false>(ctx, p);
         if (s <= 32) return launch_one<16, 2, false>(ctx, p);
         if (s <= 64) {
-            // CTA shape by wave balance. Every CTA of a launch is resident at once and a warp's time per token is fixed by
-            // its exponentials (16 per lane and channel, 8 cycles each on its scheduler's XU pipe), so the launch lasts as
-            // long as the busiest scheduler: count, per shape, the channel-warps the fullest SM puts on one scheduler.
-            // 256 threads = 64 channels per CTA (4 CTAs per SM), 352 threads = 88 channels (2 per SM), 128 threads with two
-            // channels per thread = 64 channels (3 per SM). With d = 768 and 32 lanes: 384 CTAs put 3 x 8 warps on most SMs
-            // (6 per scheduler), 288 of 352 threads put 2 x 11 (6 on two schedulers, 5 on the others), 384 two-channel CTAs
-            // put 3 x 4 double warps (6). On a tie the two-channel shape wins: a token's B and C rows are loaded once
-            // for both channels (11.93 -> 11.67 ms for the 12 launches of the benchmark step).
             if (!tape) {
-                auto busiest = [&](int threads, int cpt, int cap) -> long long {
-                    const int ch = threads / 4 * cpt;
-                    const long long blocks = (long long)((p.d + ch - 1) / ch) * p.lanes;
-                    const long long per_sm = (blocks + ctx->sm_count - 1) / ctx->sm_count;
-                    if (per_sm > cap) return 1ll << 40;  // more than one wave: not considered
-                    return (per_sm * (threads / 32) + 3) / 4 * cpt;
-                };
-                const long long two = busiest(128, 2, 3), wide = busiest(352, 1, 2), plain = busiest(256, 1, 4);
-                if (two <= wide && two <= plain) return launch_cfg<16, 4, false, false, 128, 2>(ctx, p);
-                if (wide < plain) return launch_cfg<16, 4, false, false, 352>(ctx, p);
+                const TiledShape t = tiled_shape(ctx, p.d, p.lanes);
+                if (t.kind == 2) return launch_cfg<16, 4, false, false, 128, 2>(ctx, p);
+                if (t.kind == 1) return launch_cfg<16, 4, false, false, 352>(ctx, p);
             }
             return launch_one<16, 4, false>(ctx, p);
         }
