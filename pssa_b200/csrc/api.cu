@@ -4,6 +4,7 @@
 
 #include "bounds.hpp"
 #include "context.hpp"
+#include "host_io.hpp"
 #include "kernels.hpp"
 
 namespace pssa {
@@ -48,16 +49,6 @@ void profile_record(pssa_b200_ctx* ctx, const char* kernel) {
     ctx->prof_names.push_back(kernel);
     ctx->prof_chain.push_back(ctx->chain);
 }
-
-// RAII device buffers for the host-pointer entry points (freed on every exit path)
-struct DeviceBuf {
-    void* p = nullptr;
-    ~DeviceBuf() {
-        if (p) cudaFree(p);
-    }
-    cudaError_t alloc(size_t bytes) { return cudaMalloc(&p, bytes ? bytes : 1); }
-    float* f() const { return (float*)p; }
-};
 }  // namespace pssa
 
 using namespace pssa;
@@ -96,6 +87,7 @@ int32_t pssa_b200_ctx_create(int32_t device, pssa_b200_ctx** out) {
         delete ctx;
         return cuda_fail(nullptr, e, "status word allocation");
     }
+    host_io_create();
     *out = ctx;
     return PSSA_B200_OK;
 }
@@ -104,6 +96,7 @@ void pssa_b200_ctx_destroy(pssa_b200_ctx* ctx) {
     if (!ctx) return;
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
+    host_io_destroy(ctx);
     if (ctx->arena) cudaFree(ctx->arena);
     if (ctx->status_dev) cudaFree(ctx->status_dev);
     cudaFree(ctx->resident.y), cudaFree(ctx->resident.states), cudaFree(ctx->resident.bar_a), cudaFree(ctx->resident.bar_b);
@@ -189,20 +182,11 @@ int32_t pssa_b200_affine_scan(pssa_b200_ctx* ctx, float* scan_a, float* scan_b, 
     if (rc != PSSA_B200_OK) return rc;
     if (!scan_a || !scan_b) return fail(ctx, PSSA_B200_ERR_INVALID_ARGUMENT, "B200 affine scan: null buffer");
     PSSA_CUDA(ctx, cudaSetDevice(ctx->device));
-    DeviceBuf da, db;
-    PSSA_CUDA(ctx, da.alloc(elems * 4));
-    PSSA_CUDA(ctx, db.alloc(elems * 4));
-    PSSA_CUDA(ctx, cudaMemcpyAsync(da.p, scan_a, elems * 4, cudaMemcpyHostToDevice, ctx->stream));
-    PSSA_CUDA(ctx, cudaMemcpyAsync(db.p, scan_b, elems * 4, cudaMemcpyHostToDevice, ctx->stream));
-    rc = launch_scan_maps(ctx, da.f(), db.f(), lanes, len, stride, ctx->scan_chunks);
-    if (rc != PSSA_B200_OK) {
-        cudaStreamSynchronize(ctx->stream);
-        return rc;
-    }
-    PSSA_CUDA(ctx, cudaMemcpyAsync(scan_a, da.p, elems * 4, cudaMemcpyDeviceToHost, ctx->stream));
-    PSSA_CUDA(ctx, cudaMemcpyAsync(scan_b, db.p, elems * 4, cudaMemcpyDeviceToHost, ctx->stream));
-    PSSA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    return PSSA_B200_OK;
+    HostCall call(ctx);
+    const int ia = call.inout(scan_a, scan_a, elems * 4), ib = call.inout(scan_b, scan_b, elems * 4);
+    if ((rc = call.upload())) return rc;
+    if ((rc = launch_scan_maps(ctx, call.f(ia), call.f(ib), lanes, len, stride, ctx->scan_chunks))) return rc;
+    return call.download(nullptr);
 }
 
 int32_t pssa_b200_scan_states_dev(pssa_b200_ctx* ctx, const float* a, const float* b, const float* h0, float* h,
@@ -224,26 +208,16 @@ int32_t pssa_b200_scan_states(pssa_b200_ctx* ctx, const float* a, const float* b
     if (rc != PSSA_B200_OK) return rc;
     if (!a || !b || !h) return fail(ctx, PSSA_B200_ERR_INVALID_ARGUMENT, "B200 scan states: null buffer");
     PSSA_CUDA(ctx, cudaSetDevice(ctx->device));
-    size_t row = lanes * stride * 4;
-    DeviceBuf da, db, dh0, dlast;
-    PSSA_CUDA(ctx, da.alloc(elems * 4));
-    PSSA_CUDA(ctx, db.alloc(elems * 4));
-    if (h0) PSSA_CUDA(ctx, dh0.alloc(row));
-    if (h_last) PSSA_CUDA(ctx, dlast.alloc(row));
-    PSSA_CUDA(ctx, cudaMemcpyAsync(da.p, a, elems * 4, cudaMemcpyHostToDevice, ctx->stream));
-    PSSA_CUDA(ctx, cudaMemcpyAsync(db.p, b, elems * 4, cudaMemcpyHostToDevice, ctx->stream));
-    if (h0) PSSA_CUDA(ctx, cudaMemcpyAsync(dh0.p, h0, row, cudaMemcpyHostToDevice, ctx->stream));
+    const size_t row = lanes * stride * 4;
+    HostCall call(ctx);
     // states overwrite the device copy of b: the output needs no third device array
-    rc = launch_scan_states(ctx, da.f(), db.f(), h0 ? dh0.f() : nullptr, db.f(), h_last ? dlast.f() : nullptr, lanes,
-                            len, stride, ctx->scan_chunks);
-    if (rc != PSSA_B200_OK) {
-        cudaStreamSynchronize(ctx->stream);
+    const int ia = call.in(a, elems * 4), ib = call.inout(b, h, elems * 4), i0 = h0 ? call.in(h0, row) : -1;
+    const int il = h_last ? call.out(h_last, row) : -1;
+    if ((rc = call.upload())) return rc;
+    if ((rc = launch_scan_states(ctx, call.f(ia), call.f(ib), h0 ? call.f(i0) : nullptr, call.f(ib), h_last ? call.f(il) : nullptr, lanes, len,
+                                 stride, ctx->scan_chunks)))
         return rc;
-    }
-    PSSA_CUDA(ctx, cudaMemcpyAsync(h, db.p, elems * 4, cudaMemcpyDeviceToHost, ctx->stream));
-    if (h_last) PSSA_CUDA(ctx, cudaMemcpyAsync(h_last, dlast.p, row, cudaMemcpyDeviceToHost, ctx->stream));
-    PSSA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    return PSSA_B200_OK;
+    return call.download(nullptr);
 }
 
 int32_t pssa_b200_scan_states_noalloc_dev(pssa_b200_ctx* ctx, const float* a, const float* b, const float* h0, float* h,
@@ -318,40 +292,19 @@ int32_t pssa_b200_ssm_forward(pssa_b200_ctx* ctx, const float* delta, const floa
     if (!delta || !b_proj || !c_proj || !x_norm || !rates || !initial || !y_ssm)
         return fail(ctx, PSSA_B200_ERR_INVALID_ARGUMENT, "B200 SSM forward: null buffer");
     PSSA_CUDA(ctx, cudaSetDevice(ctx->device));
-    DeviceBuf d_delta, d_b, d_c, d_x, d_rates, d_carry, d_y, d_states, d_ba, d_bb;
-    size_t tape = seq_len * sh.stride * 4;
-    PSSA_CUDA(ctx, d_delta.alloc(sh.token_m * 4));
-    PSSA_CUDA(ctx, d_x.alloc(sh.token_m * 4));
-    PSSA_CUDA(ctx, d_y.alloc(sh.token_m * 4));
-    PSSA_CUDA(ctx, d_b.alloc(sh.token_s * 4));
-    PSSA_CUDA(ctx, d_c.alloc(sh.token_s * 4));
-    PSSA_CUDA(ctx, d_rates.alloc(sh.stride * 4));
-    PSSA_CUDA(ctx, d_carry.alloc(sh.stride * 4));
-    if (states) PSSA_CUDA(ctx, d_states.alloc(tape));
-    if (bar_a) PSSA_CUDA(ctx, d_ba.alloc(tape));
-    if (bar_b) PSSA_CUDA(ctx, d_bb.alloc(tape));
-    cudaStream_t st = ctx->stream;
-    PSSA_CUDA(ctx, cudaMemcpyAsync(d_delta.p, delta, sh.token_m * 4, cudaMemcpyHostToDevice, st));
-    PSSA_CUDA(ctx, cudaMemcpyAsync(d_x.p, x_norm, sh.token_m * 4, cudaMemcpyHostToDevice, st));
-    PSSA_CUDA(ctx, cudaMemcpyAsync(d_b.p, b_proj, sh.token_s * 4, cudaMemcpyHostToDevice, st));
-    PSSA_CUDA(ctx, cudaMemcpyAsync(d_c.p, c_proj, sh.token_s * 4, cudaMemcpyHostToDevice, st));
-    PSSA_CUDA(ctx, cudaMemcpyAsync(d_rates.p, rates, sh.stride * 4, cudaMemcpyHostToDevice, st));
-    PSSA_CUDA(ctx, cudaMemcpyAsync(d_carry.p, initial, sh.stride * 4, cudaMemcpyHostToDevice, st));
-    rc = pssa_b200_ssm_forward_dev(ctx, d_delta.f(), d_b.f(), d_c.f(), d_x.f(), d_rates.f(), d_carry.f(), d_y.f(),
-                                   states ? d_states.f() : nullptr, bar_a ? d_ba.f() : nullptr,
-                                   bar_b ? d_bb.f() : nullptr, nullptr, nullptr, 1, seq_len, d_m, d_s, flags);
-    if (rc != PSSA_B200_OK) {
-        cudaStreamSynchronize(st);
-        return rc;
-    }
-    PSSA_CUDA(ctx, cudaMemcpyAsync(y_ssm, d_y.p, sh.token_m * 4, cudaMemcpyDeviceToHost, st));
-    if (states) {
-        memcpy(states, initial, sh.stride * 4);
-        PSSA_CUDA(ctx, cudaMemcpyAsync(states + sh.stride, d_states.p, tape, cudaMemcpyDeviceToHost, st));
-    }
-    if (bar_a) PSSA_CUDA(ctx, cudaMemcpyAsync(bar_a, d_ba.p, tape, cudaMemcpyDeviceToHost, st));
-    if (bar_b) PSSA_CUDA(ctx, cudaMemcpyAsync(bar_b, d_bb.p, tape, cudaMemcpyDeviceToHost, st));
-    PSSA_CUDA(ctx, cudaStreamSynchronize(st));
+    const size_t tape = seq_len * sh.stride * 4;
+    HostCall call(ctx);
+    const int i_delta = call.in(delta, sh.token_m * 4), i_x = call.in(x_norm, sh.token_m * 4), i_b = call.in(b_proj, sh.token_s * 4),
+              i_c = call.in(c_proj, sh.token_s * 4), i_rates = call.in(rates, sh.stride * 4), i_carry = call.in(initial, sh.stride * 4);
+    const int i_y = call.out(y_ssm, sh.token_m * 4), i_st = states ? call.out(states + sh.stride, tape) : -1,
+              i_ba = bar_a ? call.out(bar_a, tape) : -1, i_bb = bar_b ? call.out(bar_b, tape) : -1;
+    if ((rc = call.upload())) return rc;
+    rc = pssa_b200_ssm_forward_dev(ctx, call.f(i_delta), call.f(i_b), call.f(i_c), call.f(i_x), call.f(i_rates), call.f(i_carry), call.f(i_y),
+                                   states ? call.f(i_st) : nullptr, bar_a ? call.f(i_ba) : nullptr, bar_b ? call.f(i_bb) : nullptr, nullptr,
+                                   nullptr, 1, seq_len, d_m, d_s, flags);
+    if (rc != PSSA_B200_OK) return rc;
+    if ((rc = call.download(nullptr))) return rc;
+    if (states) memcpy(states, initial, sh.stride * 4);
     return PSSA_B200_OK;
 }
 
@@ -471,35 +424,17 @@ int32_t pssa_b200_memory_read(pssa_b200_ctx* ctx, const float* q, int32_t q_is_e
     if (!q || !keys || !norm_sq || !values || !m_val)
         return fail(ctx, PSSA_B200_ERR_INVALID_ARGUMENT, "B200 memory read: null buffer");
     PSSA_CUDA(ctx, cudaSetDevice(ctx->device));
-    DeviceBuf dq, dkeys, dns, dvals, dpnc, dqn, dw, dm, dmin;
-    cudaStream_t st = ctx->stream;
-    PSSA_CUDA(ctx, dq.alloc(rows * d_key * 4));
-    PSSA_CUDA(ctx, dkeys.alloc(capacity * d_key * 4));
-    PSSA_CUDA(ctx, dns.alloc(capacity * 4));
-    PSSA_CUDA(ctx, dvals.alloc(capacity * d_val * 4));
-    PSSA_CUDA(ctx, dpnc.alloc(rows * d_key * 4));
-    PSSA_CUDA(ctx, dqn.alloc(rows * 4));
-    PSSA_CUDA(ctx, dw.alloc(rows * capacity * 4));
-    PSSA_CUDA(ctx, dm.alloc(rows * d_val * 4));
-    PSSA_CUDA(ctx, dmin.alloc(rows * 4));
-    PSSA_CUDA(ctx, cudaMemcpyAsync(dq.p, q, rows * d_key * 4, cudaMemcpyHostToDevice, st));
-    PSSA_CUDA(ctx, cudaMemcpyAsync(dkeys.p, keys, capacity * d_key * 4, cudaMemcpyHostToDevice, st));
-    PSSA_CUDA(ctx, cudaMemcpyAsync(dns.p, norm_sq, capacity * 4, cudaMemcpyHostToDevice, st));
-    PSSA_CUDA(ctx, cudaMemcpyAsync(dvals.p, values, capacity * d_val * 4, cudaMemcpyHostToDevice, st));
-    PSSA_CUDA(ctx, cudaMemsetAsync(dw.p, 0, rows * capacity * 4, st));
-    rc = pssa_b200_memory_read_dev(ctx, dq.f(), q_is_euclidean, dkeys.f(), dns.f(), dvals.f(), rows, d_key, d_val,
-                                   capacity, count, tau, top_k, dpnc.f(), dqn.f(), dw.f(), dm.f(), dmin.f(), flags);
-    if (rc != PSSA_B200_OK) {
-        cudaStreamSynchronize(st);
-        return rc;
-    }
-    if (q_pnc) PSSA_CUDA(ctx, cudaMemcpyAsync(q_pnc, dpnc.p, rows * d_key * 4, cudaMemcpyDeviceToHost, st));
-    if (q_norm) PSSA_CUDA(ctx, cudaMemcpyAsync(q_norm, dqn.p, rows * 4, cudaMemcpyDeviceToHost, st));
-    if (weights) PSSA_CUDA(ctx, cudaMemcpyAsync(weights, dw.p, rows * capacity * 4, cudaMemcpyDeviceToHost, st));
-    PSSA_CUDA(ctx, cudaMemcpyAsync(m_val, dm.p, rows * d_val * 4, cudaMemcpyDeviceToHost, st));
-    if (min_dist) PSSA_CUDA(ctx, cudaMemcpyAsync(min_dist, dmin.p, rows * 4, cudaMemcpyDeviceToHost, st));
-    PSSA_CUDA(ctx, cudaStreamSynchronize(st));
-    return PSSA_B200_OK;
+    HostCall call(ctx);
+    const int i_q = call.in(q, rows * d_key * 4), i_k = call.in(keys, capacity * d_key * 4), i_n = call.in(norm_sq, capacity * 4),
+              i_v = call.in(values, capacity * d_val * 4);
+    const int i_pnc = call.out(q_pnc, rows * d_key * 4), i_qn = call.out(q_norm, rows * 4), i_w = call.out(weights, rows * capacity * 4),
+              i_m = call.out(m_val, rows * d_val * 4), i_md = call.out(min_dist, rows * 4);
+    if ((rc = call.upload())) return rc;
+    PSSA_CUDA(ctx, cudaMemsetAsync(call.f(i_w), 0, rows * capacity * 4, ctx->stream));
+    rc = pssa_b200_memory_read_dev(ctx, call.f(i_q), q_is_euclidean, call.f(i_k), call.f(i_n), call.f(i_v), rows, d_key, d_val, capacity, count, tau,
+                                   top_k, call.f(i_pnc), call.f(i_qn), call.f(i_w), call.f(i_m), call.f(i_md), flags);
+    if (rc != PSSA_B200_OK) return rc;
+    return call.download(nullptr);
 }
 
 // ------------------------------------------------------------------ bank write and plastic fast weights
@@ -590,27 +525,12 @@ int32_t pssa_b200_gemm_xwt(pssa_b200_ctx* ctx, const float* x, const float* w, s
     if (rc) return rc;
     if (!x || !w || !out) return fail(ctx, PSSA_B200_ERR_INVALID_ARGUMENT, "GEMM: null buffer");
     PSSA_CUDA(ctx, cudaSetDevice(ctx->device));
-    DeviceBuf dx, dw, dout;
-    cudaStream_t st = ctx->stream;
-    PSSA_CUDA(ctx, dx.alloc(rows * k * 4));
-    PSSA_CUDA(ctx, dw.alloc(n * k * 4));
-    PSSA_CUDA(ctx, dout.alloc(rows * n * 4));
-    PSSA_CUDA(ctx, cudaMemcpyAsync(dx.p, x, rows * k * 4, cudaMemcpyHostToDevice, st));
-    PSSA_CUDA(ctx, cudaMemcpyAsync(dw.p, w, n * k * 4, cudaMemcpyHostToDevice, st));
-    if (epilogue == PSSA_B200_EPI_ADD_OUT) PSSA_CUDA(ctx, cudaMemcpyAsync(dout.p, out, rows * n * 4, cudaMemcpyHostToDevice, st));
-    rc = pssa_b200_gemm_xwt_dev(ctx, dx.f(), dw.f(), rows, n, k, dout.f(), n, epilogue, alpha, precision);
-    if (rc == PSSA_B200_OK) {
-        int status = 0;
-        PSSA_CUDA(ctx, cudaMemcpyAsync(&status, ctx->status_dev, sizeof(int), cudaMemcpyDeviceToHost, st));
-        PSSA_CUDA(ctx, cudaStreamSynchronize(st));
-        if (status != 0) {
-            cudaMemsetAsync(ctx->status_dev, 0, sizeof(int), st);
-            return fail(ctx, status, "B200 GEMM: a bounded device-side wait expired");
-        }
-        PSSA_CUDA(ctx, cudaMemcpyAsync(out, dout.p, rows * n * 4, cudaMemcpyDeviceToHost, st));
-    }
-    PSSA_CUDA(ctx, cudaStreamSynchronize(st));
-    return rc;
+    HostCall call(ctx);
+    const int i_x = call.in(x, rows * k * 4), i_w = call.in(w, n * k * 4);
+    const int i_o = epilogue == PSSA_B200_EPI_ADD_OUT ? call.inout(out, out, rows * n * 4) : call.out(out, rows * n * 4);
+    if ((rc = call.upload())) return rc;
+    if ((rc = pssa_b200_gemm_xwt_dev(ctx, call.f(i_x), call.f(i_w), rows, n, k, call.f(i_o), n, epilogue, alpha, precision))) return rc;
+    return call.download("B200 GEMM");
 }
 
 int32_t pssa_b200_ctx_profile_begin(pssa_b200_ctx* ctx) {

@@ -19,7 +19,10 @@ struct pssa_b200_ctx {
     char* arena = nullptr;
     size_t arena_bytes = 0;
     size_t arena_used = 0;
-    // pinned staging for the host-pointer entry points
+    // host-pointer entry points (host_io.hpp): device region of their arrays, pinned staging
+    char *io = nullptr, *pinned = nullptr;
+    size_t io_bytes = 0, pinned_bytes = 0;
+    std::vector<cudaEvent_t> io_events;
     std::string error;
     std::string label;
     uint64_t launches = 0;

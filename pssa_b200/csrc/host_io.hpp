@@ -1,0 +1,57 @@
+// Host arrays in and out of the entry points that take host pointers.
+//
+// A call's inputs lie side by side in one device region and go over in one copy from pinned memory, its outputs come back
+// the same way; the device region and the pinned buffer belong to the context and are kept from call to call up to a bound.
+// A cudaMalloc / cudaFree pair per array and a pageable copy each was most of such a call: 128 x 192 x 192 product 97 -> 60 us,
+// memory stage of 128 tokens 537 -> 314 us. Large outputs are copied out of the pinned buffer by a few threads while the
+// next piece is on its way (one thread moves 18 GB/s, the link 52).
+#pragma once
+#include <cstddef>
+#include <cstdint>
+#include <vector>
+
+#include "context.hpp"
+
+namespace pssa {
+
+class HostCall {
+  public:
+    explicit HostCall(pssa_b200_ctx* ctx) : ctx_(ctx) {}
+    ~HostCall();
+    HostCall(const HostCall&) = delete;
+    HostCall& operator=(const HostCall&) = delete;
+    // declare every array first; each returns its index. `host` may be null: a device array without a host side
+    int in(const void* host, size_t bytes) { return add(host, nullptr, bytes); }
+    int out(void* host, size_t bytes) { return add(nullptr, host, bytes); }
+    int inout(const void* src, void* dst, size_t bytes) { return add(src, dst, bytes); }
+    int scratch(size_t bytes) { return add(nullptr, nullptr, bytes); }
+    int32_t upload();  // allocates the device region and enqueues the inputs
+    float* f(int i) const { return reinterpret_cast<float*>(base_ + arrays_[i].off); }
+    // Waits for the stream and brings the outputs back. With `what` the host arrays stay untouched when a bounded device-side
+    // wait has expired, whose status and `what` then become the error.
+    int32_t download(const char* what);
+
+  private:
+    struct Array {
+        const void* src;
+        void* dst;
+        size_t bytes, off;
+    };
+    int add(const void* src, void* dst, size_t bytes) {
+        arrays_.push_back({src, dst, bytes, 0});
+        return (int)arrays_.size() - 1;
+    }
+    pssa_b200_ctx* ctx_;
+    std::vector<Array> arrays_;
+    char* base_ = nullptr;
+    bool own_ = false;  // the region is this call's alone (above the kept bound)
+};
+
+// device -> host through the context's pinned buffer, in stream order; waits for the stream
+int32_t copy_to_host(pssa_b200_ctx* ctx, void* dst, const void* src_dev, size_t bytes);
+// pinned host memory of the context, at least `bytes`, valid until the next call; waits for the stream when it has to grow
+int32_t pinned_reserve(pssa_b200_ctx* ctx, size_t bytes);
+void host_io_create();  // once per context
+void host_io_destroy(pssa_b200_ctx* ctx);
+
+}  // namespace pssa

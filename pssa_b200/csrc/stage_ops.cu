@@ -8,20 +8,12 @@
 
 #include "bounds.hpp"
 #include "context.hpp"
+#include "host_io.hpp"
 #include "kernels.hpp"
 
 using namespace pssa;
 
 namespace {
-
-struct DevBuf {
-    void* p = nullptr;
-    ~DevBuf() {
-        if (p) cudaFree(p);
-    }
-    cudaError_t alloc(size_t bytes) { return cudaMalloc(&p, bytes ? bytes : 1); }
-    float* f() const { return (float*)p; }
-};
 
 // src/cuda/stage_bounds.rs:67-152 for the memory stage: every product must fit the u32 element index of the kernels
 int32_t memory_stage_shape(pssa_b200_ctx* ctx, size_t seq_len, size_t d_m, size_t d_k, size_t d_val, size_t capacity, size_t count,
@@ -76,32 +68,22 @@ int32_t pssa_b200_memory_forward(pssa_b200_ctx* ctx, const float* x_norm, const 
         !weights || !m_val || !g_mem || !m_proj || !m_inj)
         return fail(ctx, PSSA_B200_ERR_INVALID_ARGUMENT, "B200 memory forward: null buffer");
     PSSA_CUDA(ctx, cudaSetDevice(ctx->device));
-    cudaStream_t st = ctx->stream;
     const size_t T = seq_len, f = sizeof(float);
-    struct In { const float* host; size_t n; DevBuf buf; };
-    In in[] = {{x_norm, T * d_m, {}}, {y_ssm, T * d_m, {}}, {w_qx, d_k * d_m, {}}, {w_qh, d_k * d_m, {}}, {w_gate, d_m * d_m, {}},
-               {w_proj, d_m * d_val, {}}, {keys, capacity * d_k, {}}, {norm_sq, capacity, {}}, {values, capacity * d_val, {}}};
-    for (auto& i : in) {
-        PSSA_CUDA(ctx, i.buf.alloc(i.n * f));
-        PSSA_CUDA(ctx, cudaMemcpyAsync(i.buf.p, i.host, i.n * f, cudaMemcpyHostToDevice, st));
-    }
-    struct Out { float* host; size_t n; DevBuf buf; };
-    Out out[] = {{q_euc, T * d_k, {}}, {q_pnc, T * d_k, {}}, {q_norm, T, {}}, {weights, T * capacity, {}}, {m_val, T * d_val, {}},
-                 {g_mem, T * d_m, {}}, {m_proj, T * d_m, {}}, {m_inj, T * d_m, {}}};
-    for (auto& o : out) PSSA_CUDA(ctx, o.buf.alloc(o.n * f));
-    PSSA_CUDA(ctx, cudaMemsetAsync(out[3].buf.p, 0, out[3].n * f, st));
-    rc = pssa_b200_memory_forward_dev(ctx, in[0].buf.f(), in[1].buf.f(), in[2].buf.f(), in[3].buf.f(), in[4].buf.f(), in[5].buf.f(),
-                                      in[6].buf.f(), in[7].buf.f(), in[8].buf.f(), seq_len, d_m, d_k, d_val, capacity, count, tau,
-                                      out[0].buf.f(), out[1].buf.f(), out[2].buf.f(), out[3].buf.f(), out[4].buf.f(), out[5].buf.f(),
-                                      out[6].buf.f(), out[7].buf.f(), precision);
-    if (rc == PSSA_B200_OK) rc = pssa_b200_ctx_poll_status(ctx);  // a bounded wait that expired leaves the outputs untouched
-    if (rc != PSSA_B200_OK) {
-        cudaStreamSynchronize(st);
-        return rc;
-    }
-    for (auto& o : out) PSSA_CUDA(ctx, cudaMemcpyAsync(o.host, o.buf.p, o.n * f, cudaMemcpyDeviceToHost, st));
-    PSSA_CUDA(ctx, cudaStreamSynchronize(st));
-    return PSSA_B200_OK;
+    HostCall call(ctx);
+    const int in[] = {call.in(x_norm, T * d_m * f),      call.in(y_ssm, T * d_m * f),       call.in(w_qx, d_k * d_m * f),
+                      call.in(w_qh, d_k * d_m * f),      call.in(w_gate, d_m * d_m * f),    call.in(w_proj, d_m * d_val * f),
+                      call.in(keys, capacity * d_k * f), call.in(norm_sq, capacity * f),    call.in(values, capacity * d_val * f)};
+    const int out[] = {call.out(q_euc, T * d_k * f),     call.out(q_pnc, T * d_k * f),      call.out(q_norm, T * f),
+                       call.out(weights, T * capacity * f), call.out(m_val, T * d_val * f), call.out(g_mem, T * d_m * f),
+                       call.out(m_proj, T * d_m * f),    call.out(m_inj, T * d_m * f)};
+    if ((rc = call.upload())) return rc;
+    PSSA_CUDA(ctx, cudaMemsetAsync(call.f(out[3]), 0, T * capacity * f, ctx->stream));
+    rc = pssa_b200_memory_forward_dev(ctx, call.f(in[0]), call.f(in[1]), call.f(in[2]), call.f(in[3]), call.f(in[4]), call.f(in[5]), call.f(in[6]),
+                                      call.f(in[7]), call.f(in[8]), seq_len, d_m, d_k, d_val, capacity, count, tau, call.f(out[0]),
+                                      call.f(out[1]), call.f(out[2]), call.f(out[3]), call.f(out[4]), call.f(out[5]), call.f(out[6]),
+                                      call.f(out[7]), precision);
+    if (rc != PSSA_B200_OK) return rc;
+    return call.download("B200 memory forward");
 }
 
 int32_t pssa_b200_ssm_forward_resident(pssa_b200_ctx* ctx, const float* delta, const float* delta_raw, const float* b_proj,
@@ -132,25 +114,15 @@ int32_t pssa_b200_ssm_forward_resident(pssa_b200_ctx* ctx, const float* delta, c
         PSSA_CUDA(ctx, cudaMalloc((void**)&r.bar_b, seq_len * stride * 4));
         r.capacity_rows = rows_m, r.capacity_stride = tape;
     }
-    DevBuf dd, db, dc, dx, dr;
-    PSSA_CUDA(ctx, dd.alloc(rows_m * 4));
-    PSSA_CUDA(ctx, dx.alloc(rows_m * 4));
-    PSSA_CUDA(ctx, db.alloc(rows_s * 4));
-    PSSA_CUDA(ctx, dc.alloc(rows_s * 4));
-    PSSA_CUDA(ctx, dr.alloc(stride * 4));
-    PSSA_CUDA(ctx, cudaMemcpyAsync(dd.p, delta, rows_m * 4, cudaMemcpyHostToDevice, st));
-    PSSA_CUDA(ctx, cudaMemcpyAsync(dx.p, x_norm, rows_m * 4, cudaMemcpyHostToDevice, st));
-    PSSA_CUDA(ctx, cudaMemcpyAsync(db.p, b_proj, rows_s * 4, cudaMemcpyHostToDevice, st));
-    PSSA_CUDA(ctx, cudaMemcpyAsync(dc.p, c_proj, rows_s * 4, cudaMemcpyHostToDevice, st));
-    PSSA_CUDA(ctx, cudaMemcpyAsync(dr.p, rates, stride * 4, cudaMemcpyHostToDevice, st));
+    HostCall call(ctx);
+    const int i_d = call.in(delta, rows_m * 4), i_x = call.in(x_norm, rows_m * 4), i_b = call.in(b_proj, rows_s * 4), i_c = call.in(c_proj, rows_s * 4),
+              i_r = call.in(rates, stride * 4), i_h = call.in(initial, stride * 4);
+    if ((rc = call.upload())) return rc;
     // states row 0 = the initial carry (src/gpu_batch.rs:392-437); rows 1.. = state after each token
-    PSSA_CUDA(ctx, cudaMemcpyAsync(r.states, initial, stride * 4, cudaMemcpyHostToDevice, st));
-    DevBuf carry;
-    PSSA_CUDA(ctx, carry.alloc(stride * 4));
-    PSSA_CUDA(ctx, cudaMemcpyAsync(carry.p, r.states, stride * 4, cudaMemcpyDeviceToDevice, st));
-    rc = pssa_b200_ssm_forward_dev(ctx, dd.f(), db.f(), dc.f(), dx.f(), dr.f(), carry.f(), r.y, r.states + stride, r.bar_a, r.bar_b, nullptr,
-                                   nullptr, 1, seq_len, d_m, d_s, flags);
-    PSSA_CUDA(ctx, cudaStreamSynchronize(st));  // the staged inputs are freed on return
+    PSSA_CUDA(ctx, cudaMemcpyAsync(r.states, call.f(i_h), stride * 4, cudaMemcpyDeviceToDevice, st));
+    rc = pssa_b200_ssm_forward_dev(ctx, call.f(i_d), call.f(i_b), call.f(i_c), call.f(i_x), call.f(i_r), call.f(i_h), r.y, r.states + stride, r.bar_a,
+                                   r.bar_b, nullptr, nullptr, 1, seq_len, d_m, d_s, flags);
+    PSSA_CUDA(ctx, cudaStreamSynchronize(st));  // the staging region is the next call's
     if (rc != PSSA_B200_OK) return rc;
     r.seq_len = seq_len, r.d_m = d_m, r.d_s = d_s, r.valid = true;
     return PSSA_B200_OK;
@@ -171,13 +143,11 @@ int32_t pssa_b200_memory_forward_after_ssm(pssa_b200_ctx* ctx, const float* x_no
     cudaStream_t st = ctx->stream;
     const size_t stride = r.d_m * r.d_s;
     // publish the resident tape first: it stays recoverable even if the memory stage fails (src/cuda/stages.rs:737-771)
-    std::vector<float> y_host(seq_len * d_m);
-    PSSA_CUDA(ctx, cudaMemcpyAsync(y_host.data(), r.y, seq_len * d_m * 4, cudaMemcpyDeviceToHost, st));
-    if (states) PSSA_CUDA(ctx, cudaMemcpyAsync(states, r.states, (seq_len + 1) * stride * 4, cudaMemcpyDeviceToHost, st));
-    if (bar_a) PSSA_CUDA(ctx, cudaMemcpyAsync(bar_a, r.bar_a, seq_len * stride * 4, cudaMemcpyDeviceToHost, st));
-    if (bar_b) PSSA_CUDA(ctx, cudaMemcpyAsync(bar_b, r.bar_b, seq_len * stride * 4, cudaMemcpyDeviceToHost, st));
-    PSSA_CUDA(ctx, cudaStreamSynchronize(st));
-    std::memcpy(y_ssm, y_host.data(), y_host.size() * 4);
+    int32_t rc_copy = copy_to_host(ctx, y_ssm, r.y, seq_len * d_m * 4);
+    if (!rc_copy && states) rc_copy = copy_to_host(ctx, states, r.states, (seq_len + 1) * stride * 4);
+    if (!rc_copy && bar_a) rc_copy = copy_to_host(ctx, bar_a, r.bar_a, seq_len * stride * 4);
+    if (!rc_copy && bar_b) rc_copy = copy_to_host(ctx, bar_b, r.bar_b, seq_len * stride * 4);
+    if (rc_copy) return rc_copy;
     int32_t rc = pssa_b200_memory_forward(ctx, x_norm, y_ssm, w_qx, w_qh, w_gate, w_proj, keys, norm_sq, values, seq_len, d_m, d_k, d_val,
                                           capacity, count, tau, q_euc, q_pnc, q_norm, weights, m_val, g_mem, m_proj, m_inj, precision);
     if (rc == PSSA_B200_OK) r.valid = false;  // consumed

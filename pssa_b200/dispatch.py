@@ -218,7 +218,7 @@ class B200Dispatch:
 
     # ---- stage-level operators with the reference's argument lists (src/backend.rs:1186-1289, 1342-1385)
     def _memory_outputs(self, seq_len, d_m, d_k, d_val, capacity):
-        z = lambda *shape: np.zeros(shape, np.float32)  # noqa: E731
+        z = lambda *shape: np.empty(shape, np.float32)  # noqa: E731
         return dict(q_euc=z(seq_len, d_k), q_pnc=z(seq_len, d_k), q_norm=z(seq_len), weights=z(seq_len, capacity),
                     m_val=z(seq_len, d_val), g_mem=z(seq_len, d_m), m_proj=z(seq_len, d_m), m_inj=z(seq_len, d_m))
 

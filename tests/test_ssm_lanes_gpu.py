@@ -40,9 +40,8 @@ def test_few_lanes_matches_the_ordered_recurrence(gpu, d, s, lengths, exact):
     gpu.ssm_forward_dev(*t[:5], c2, y2, offsets, lengths, rows, d, s, states=states, exact=exact)
     torch.cuda.synchronize()
     tol = 5e-6 if exact else REL_TOL
-    got = y.cpu().numpy()
+    assert chan_err(y.cpu().numpy(), ref_y, 0) <= tol
     for off, ln in zip(offsets, lengths):
-        assert chan_err(got[off:off + ln], ref_y[off:off + ln], 0) <= tol
         if ln:  # the tape's last row is the carry out
             assert torch.equal(states[off + ln - 1], c2[[i for i in range(n) if offsets[i] == off and lengths[i]][0]])
     assert chan_err(t[5].cpu().numpy().ravel(), ref_carry.ravel(), 0) <= tol
