@@ -210,6 +210,33 @@ int32_t launch_gemm_bf16_cat(pssa_b200_ctx* ctx, const void* x16, const void* w1
                              size_t ldo, int c1, int c2, int c3, void* side_a = nullptr, size_t ld_side_a = 0, void* side_b = nullptr,
                              size_t ld_side_b = 0);
 
+// step_decode.cu: one token per row through every block and the vocabulary head in one cooperative launch (bf16 mode)
+struct StepLaunch {
+    int rows, d, s, k, cap, nc, off_b, off_q, off_gate, off_act;
+    size_t depth;
+    unsigned vocab;
+    float ssm_scale, head_scale, tau;
+    const float* embed;
+    const uint32_t *ids, *slots;     // [rows]
+    const void* unembed;
+    size_t carry_stride;
+    float *feat_a, *feat_b, *proj, *y, *qpart, *ssq, *inv;  // qpart [rows, d / 8, k], ssq [rows, d / 16], inv [rows]
+    float* logits;                   // [rows, vocab] or null
+    void *w, *z, *act;               // bf16: weight rows (pitch 3 cap), MLP operands (pitches d + 64, 2d + 64)
+    void* barrier;                   // 8 bytes, zero before the first launch
+    struct Block {
+        const void *wcat, *wqh, *vp, *w1, *w2;
+        const float *rates, *gamma, *beta, *keys_t, *norm_sq;
+        float* state;
+        float res_scale;
+        int count;
+    };
+    const Block* blocks;
+};
+bool step_shape_ok(size_t depth, size_t d, size_t s, size_t k, size_t cap, size_t rank);
+int32_t launch_decode_step(pssa_b200_ctx* ctx, const StepLaunch& p);
+int32_t launch_keys_by_quad(pssa_b200_ctx* ctx, const float* keys, float* out, int cap, int k);
+
 // elementwise.cu
 int32_t launch_embed_norm(pssa_b200_ctx* ctx, const float* embed, const uint32_t* ids, const float* feats, const float* gamma,
                           const float* beta, float* x_norm, void* x_bf16, size_t rows, int d, bool exact, size_t vocab);

@@ -142,6 +142,7 @@ void pssa_b200_model_destroy(pssa_b200_model* m) {
     cudaFree(m->sampler.recent), cudaFree(m->sampler.count), cudaFree(m->sampler.rng), cudaFree(m->sampler.ids);
     cudaFree(m->sampler.status), cudaFree(m->sampler.head_slot), cudaFree(m->sampler.probs), cudaFree(m->sampler.conf);
     cudaFree(m->chunks.off), cudaFree(m->chunks.len), cudaFree(m->chunks.records), cudaFree(m->chunks.carry_in);
+    cudaFree(m->step.keys_t), cudaFree(m->step.barrier), cudaFree(m->step.scratch);
     for (auto& b : m->blocks) {
         for (int id : kBlockTensors) cudaFree(b.w[id]);
         cudaFree(b.rates);
@@ -252,7 +253,7 @@ int32_t pssa_b200_model_set_bank(pssa_b200_model* m, int32_t layer, const float*
     b.write_head = write_head;
     b.vsplit_dirty = true;
     b.vp_dirty = true;
-    b.ksplit_dirty = true;
+    b.ksplit_dirty = b.keys_t_dirty = true;
     if (confidence) b.confidence.assign(confidence, confidence + m->cap);
     if (last_seen_step) b.last_seen.assign(last_seen_step, last_seen_step + m->cap);
     PSSA_CUDA(ctx, cudaStreamSynchronize(st));

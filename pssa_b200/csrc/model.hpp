@@ -47,6 +47,7 @@ struct DeviceBlock {
     bool vsplit_dirty = true;
     bool vp_dirty = true;
     bool ksplit_dirty = true;
+    bool keys_t_dirty = true;     // step.keys_t of this block
 };
 
 struct Workspace {
@@ -137,5 +138,13 @@ struct pssa_b200_model {
         float* records = nullptr;   // [capacity][d + d*s]  (local mode; the sharded mode uses sp.send)
         float* carry_in = nullptr;  // [capacity][d*s]
     } chunks;
+    // decode step in one kernel (step_decode.cu): the banks' keys by quads [depth][k * cap], the barrier word and the step's own
+    // scratch, sized for `rows` streams
+    struct Step {
+        float* keys_t = nullptr;
+        void* barrier = nullptr;
+        float* scratch = nullptr;
+        size_t rows = 0;
+    } step;
     std::vector<bool> tensor_set;  // [depth * T_COUNT + id] upload bookkeeping
 };

@@ -523,6 +523,75 @@ int32_t head_rows(pssa_b200_model* m, const float* feats, size_t n_heads, bool w
     return PSSA_B200_OK;
 }
 
+// One token per lane, every lane present and in row order, in the bf16 mode: the whole step is one kernel (step_decode.cu).
+// The choice follows the shape of the step and the model's options, never the number of lanes: a stream's bits are the same
+// alone and in a batch.
+bool step_model_ok(const pssa_b200_model* m) {
+    return m->precision == PSSA_B200_PRECISION_BF16 && m->loops == 1 && step_shape_ok(m->depth, m->d, m->s, m->k, m->cap, m->rank) &&
+           1.0f / m->cfg.tau_mem < 3.0e38f;
+}
+bool decode_step_fused(const pssa_b200_model* m, size_t rows, size_t lanes, const uint32_t* h_off, const uint32_t* h_len) {
+    if (rows != lanes || rows > 65536 || m->sp.active || m->obs.enabled || !step_model_ok(m)) return false;
+    for (auto& b : m->blocks)
+        if (b.count == 0 || (m->top_k != 0 && m->top_k < b.count)) return false;
+    for (size_t l = 0; l < lanes; ++l)
+        if (h_len[l] != 1 || h_off[l] != l) return false;
+    return true;
+}
+
+// What a decode step keeps: called by every forward pass of a model that can take it, so that the first step of a stream
+// that has just read its prompt does not stop for allocations.
+int32_t ensure_step(pssa_b200_model* m, size_t rows) {
+    pssa_b200_ctx* ctx = m->ctx;
+    auto& st = m->step;
+    int32_t rc;
+    if (!st.keys_t) {
+        PSSA_CUDA(ctx, cudaMalloc((void**)&st.keys_t, m->depth * m->k * m->cap * sizeof(float)));
+        PSSA_CUDA(ctx, cudaMalloc(&st.barrier, 256));
+        PSSA_CUDA(ctx, cudaMemsetAsync(st.barrier, 0, 256, ctx->stream));
+    }
+    if (rows > st.rows) {
+        PSSA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        cudaFree(st.scratch);
+        st.scratch = nullptr, st.rows = 0;
+        PSSA_CUDA(ctx, cudaMalloc((void**)&st.scratch, rows * (m->d / 8 * m->k + m->d / 16 + 1) * sizeof(float)));
+        st.rows = rows;
+    }
+    for (size_t l = 0; l < m->depth; ++l) {
+        DeviceBlock& b = m->blocks[l];
+        if (!b.keys_t_dirty) continue;
+        if ((rc = launch_keys_by_quad(ctx, b.w[T_BANK_KEYS], st.keys_t + l * m->k * m->cap, (int)m->cap, (int)m->k))) return rc;
+        b.keys_t_dirty = false;
+    }
+    return PSSA_B200_OK;
+}
+
+// logits [rows, vocab] (null: not wanted); ids is a device array
+int32_t run_decode_step(pssa_b200_model* m, size_t rows, const uint32_t* ids, float* logits) {
+    pssa_b200_ctx* ctx = m->ctx;
+    Workspace& ws = m->ws;
+    auto& st = m->step;
+    int32_t rc;
+    if ((rc = refresh_bf16(m)) || (rc = ensure_step(m, rows))) return rc;
+    StepLaunch::Block blocks[64];
+    const size_t ds = m->d * m->s;
+    for (size_t l = 0; l < m->depth; ++l) {
+        DeviceBlock& b = m->blocks[l];
+        blocks[l] = {b.wcat_bf16, b.wqh_bf16, b.vpsplit_bf16, b.w1cat_bf16, b.w2cat_bf16, b.rates, b.w[T_NORM_GAMMA], b.w[T_NORM_BETA],
+                     st.keys_t + l * m->k * m->cap, b.w[T_BANK_NORM_SQ], m->state + l * ds, l == 0 ? 1.0f : m->residual_scales[l - 1], (int)b.count};
+    }
+    StepLaunch p{};
+    p.rows = (int)rows, p.d = (int)m->d, p.s = (int)m->s, p.k = (int)m->k, p.cap = (int)m->cap, p.nc = (int)m->ncat;
+    p.off_b = (int)m->off_b, p.off_q = (int)m->off_q, p.off_gate = (int)m->off_gate, p.off_act = (int)m->off_act;
+    p.depth = m->depth, p.vocab = (unsigned)m->v;
+    p.ssm_scale = 1.0f / std::sqrt((float)m->s), p.head_scale = 1.0f / std::sqrt((float)m->d), p.tau = m->cfg.tau_mem;
+    p.embed = m->embed, p.ids = ids, p.slots = ws.lane_slot, p.unembed = m->unembed_bf16, p.carry_stride = m->depth * ds;
+    p.feat_a = ws.feat_a, p.feat_b = ws.feat_b, p.proj = ws.proj, p.y = ws.y;
+    p.qpart = st.scratch, p.ssq = p.qpart + st.rows * (m->d / 8 * m->k), p.inv = p.ssq + st.rows * (m->d / 16);
+    p.logits = logits, p.w = ws.w_split, p.z = ws.z_bf16, p.act = ws.act_bf16, p.barrier = st.barrier, p.blocks = blocks;
+    return launch_decode_step(ctx, p);
+}
+
 // Shared driver: lanes described on the host; processes them in passes of at most max_rows rows.
 // per-stream sampler state (history window and generator), allocated on first use; generators start from seed 1337 like
 // the reference engine's (src/inference.rs:70-73)
@@ -600,9 +669,17 @@ int32_t run_lanes(pssa_b200_model* m, const uint64_t* ids, const uint32_t* offse
         PSSA_CUDA(ctx, cudaMemcpyAsync(ws.lane_slot, h_slot.data(), n_lanes * 4, cudaMemcpyHostToDevice, st));
         if (!h_last.empty()) PSSA_CUDA(ctx, cudaMemcpyAsync(ws.last_rows, h_last.data(), h_last.size() * 4, cudaMemcpyHostToDevice, st));
         float* feats = nullptr;
-        if ((rc = forward_rows(m, rows, n_lanes, h_off.data(), h_len.data(), &feats, h_last.size()))) return rc;
-        if (!h_last.empty() && (logits || greedy || sampling)) {
-            if ((rc = head_rows(m, feats, h_last.size(), greedy != nullptr && !sampling))) return rc;
+        const bool step = decode_step_fused(m, rows, n_lanes, h_off.data(), h_len.data()), want_head = logits || greedy || sampling;
+        if (step) {
+            if ((rc = run_decode_step(m, rows, ws.ids, want_head && !h_last.empty() ? ws.logits : nullptr))) return rc;
+        } else {
+            if (step_model_ok(m) && (rc = ensure_step(m, std::min<size_t>(m->max_streams, 1024)))) return rc;
+            if ((rc = forward_rows(m, rows, n_lanes, h_off.data(), h_len.data(), &feats, h_last.size()))) return rc;
+        }
+        if (!h_last.empty() && want_head) {
+            const bool want_greedy = greedy != nullptr && !sampling;
+            if (!step && (rc = head_rows(m, feats, h_last.size(), want_greedy))) return rc;
+            if (step && want_greedy && (rc = launch_greedy(ctx, ws.logits, ws.greedy, rows, (int)m->v))) return rc;
             std::vector<uint32_t> g(h_last.size()), g_status(h_last.size(), 0);
             std::vector<float> g_conf;
             if (sampling) {
@@ -721,7 +798,6 @@ int32_t pssa_b200_model_prefill_batch_dev(pssa_b200_model* m, const uint32_t* id
     if ((rc = ensure_workspace(m, span, n_lanes))) return rc;
     Workspace& ws = m->ws;
     cudaStream_t st = ctx->stream;
-    PSSA_CUDA(ctx, cudaMemcpyAsync(ws.ids, ids_dev, span * 4, cudaMemcpyDeviceToDevice, st));
     // The lane description is uploaded only when it differs from what the workspace already holds. A repeated call with
     // the same layout (a decode loop) then consists of kernel launches and device-to-device copies only, so the caller can
     // capture it in a CUDA graph on the context's stream.
@@ -734,6 +810,17 @@ int32_t pssa_b200_model_prefill_batch_dev(pssa_b200_model* m, const uint32_t* id
         lay.ws_base = ws.base, lay.off = h_off, lay.len = h_len, lay.slot = h_slot;
     }
     float* feats = nullptr;
+    if (m->sp.world <= 1 && decode_step_fused(m, span, n_lanes, h_off.data(), h_len.data())) {
+        float* out = logits_dev ? logits_dev : ws.logits;
+        if ((rc = run_decode_step(m, span, ids_dev, logits_dev || greedy_dev ? out : nullptr))) return rc;
+        if (greedy_dev) {
+            if ((rc = launch_greedy(ctx, out, ws.greedy, span, (int)m->v))) return rc;
+            PSSA_CUDA(ctx, cudaMemcpyAsync(greedy_dev, ws.greedy, span * 4, cudaMemcpyDeviceToDevice, st));
+        }
+        return PSSA_B200_OK;
+    }
+    if (step_model_ok(m) && (rc = ensure_step(m, std::min<size_t>(m->max_streams, 1024)))) return rc;
+    PSSA_CUDA(ctx, cudaMemcpyAsync(ws.ids, ids_dev, span * 4, cudaMemcpyDeviceToDevice, st));
     m->sp.active = m->sp.world > 1;
     rc = forward_rows(m, span, n_lanes, h_off.data(), h_len.data(), &feats, h_last.size());
     m->sp.active = false;
@@ -904,7 +991,7 @@ int32_t pssa_b200_model_insert_memory(pssa_b200_model* m, uint32_t index, float 
         PSSA_CUDA(ctx, cudaMemcpyAsync(&slot, slot_dev, 8, cudaMemcpyDeviceToHost, st));
         PSSA_CUDA(ctx, cudaStreamSynchronize(st));
         b.count = meta_back[0], b.write_head = meta_back[1];
-        if (slot >= 0) b.ksplit_dirty = b.vsplit_dirty = b.vp_dirty = true;  // the derived copies of keys and values are stale
+        if (slot >= 0) b.ksplit_dirty = b.keys_t_dirty = b.vsplit_dirty = b.vp_dirty = true;  // the derived copies of keys and values are stale
         if (slots_out) slots_out[l] = slot;
     }
     return PSSA_B200_OK;
