@@ -222,7 +222,7 @@ struct StepLaunch {
     size_t carry_stride;
     float *feat_a, *feat_b, *proj, *y, *qpart, *ssq, *inv;  // qpart [rows, d / 8, k], ssq [rows, d / 16], inv [rows]
     float* logits;                   // [rows, vocab] or null
-    void *w, *z, *act;               // bf16: weight rows (pitch 3 cap), MLP operands (pitches d + 64, 2d + 64)
+    void *x, *w, *z, *act;           // bf16: rows [rows, d], weight rows (pitch 3 cap), MLP operands (pitches d + 64, 2d + 64)
     void* barrier;                   // 8 bytes, zero before the first launch
     struct Block {
         const void *wcat, *wqh, *vp, *w1, *w2;

@@ -588,7 +588,7 @@ int32_t run_decode_step(pssa_b200_model* m, size_t rows, const uint32_t* ids, fl
     p.embed = m->embed, p.ids = ids, p.slots = ws.lane_slot, p.unembed = m->unembed_bf16, p.carry_stride = m->depth * ds;
     p.feat_a = ws.feat_a, p.feat_b = ws.feat_b, p.proj = ws.proj, p.y = ws.y;
     p.qpart = st.scratch, p.ssq = p.qpart + st.rows * (m->d / 8 * m->k), p.inv = p.ssq + st.rows * (m->d / 16);
-    p.logits = logits, p.w = ws.w_split, p.z = ws.z_bf16, p.act = ws.act_bf16, p.barrier = st.barrier, p.blocks = blocks;
+    p.logits = logits, p.x = ws.x_bf16, p.w = ws.w_split, p.z = ws.z_bf16, p.act = ws.act_bf16, p.barrier = st.barrier, p.blocks = blocks;
     return launch_decode_step(ctx, p);
 }
 

@@ -131,7 +131,7 @@ struct StepArgs {
     const __nv_bfloat16* unembed;
     size_t carry_stride;
     float *feat_a, *feat_b, *proj, *y, *qpart, *ssq, *inv, *logits;
-    __nv_bfloat16 *w, *z, *act;
+    __nv_bfloat16 *x, *w, *z, *act;  // x: the normalised rows, at the end the features (many-rows kernel)
     unsigned long long* barrier;
     int* status;
     StepBlock block[kMaxDepth];
@@ -246,121 +246,105 @@ __device__ __forceinline__ void small_product(const Weights& w, const X& x, int 
     }
 }
 
-// ---- more rows: tiles of 64 rows x (WC * MT * 16) columns, the warps WC x (8 / WC) over columns and rows. Both operands of a tile
-// come into shared memory in quarters of K (two segments each), as many of them in flight as fit; a row pitch that is an odd
-// multiple of 64 bytes keeps the 16-byte fragment reads conflict free. Everything is in functions of its own: inlined into
-// one kernel the stages' registers spill, and with the shared memory in use there is no L1 to spill to.
-struct Quarters {
-    int first[5], pitch;
-    __device__ __forceinline__ explicit Quarters(int k) {
-        int widest = 0, n;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) segment(k, 2 * q, first[q], n);
-        first[4] = k >> 5;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) widest = max(widest, first[q + 1] - first[q]);
-        pitch = (widest | 1) * 64;
-    }
-};
+// ---- more rows: tiles of 64 rows x (WC * MT * 16) columns, the warps WC x (8 / WC) over columns and rows. Both operands come into
+// shared memory a segment of K at a time; the segments of a CTA's tiles form one stream, as much of it in flight as fits (a
+// segment arrives from L2 in about a microsecond and is used up in a quarter of one), so a tile's first segments are on
+// their way during the epilogue before it. A row pitch that is an odd multiple of 64 bytes keeps the 16-byte fragment reads
+// conflict free.
 __device__ __forceinline__ void cp16(char* dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
 }
-struct PutBf16 {
-    const __nv_bfloat16* x;
-    size_t ld;
-    __device__ __forceinline__ void put(char* dst, int row, int k) const { cp16(dst, x + (size_t)row * ld + k); }
-};
-template <class Rows>
-struct PutRows {
-    Rows x;
-    __device__ __forceinline__ void put(char* dst, int row, int k) const { *reinterpret_cast<uint4*>(dst) = x.get(row, k); }
-};
-template <int WC, int MT, class Put, class Pre, class Epi>
-__device__ __forceinline__ void large_product(const Weights& w, const Put& put, int rows, char* sm, Pre&& pre, Epi&& epi) {
+__device__ __forceinline__ void wait_pending(int n) {  // at most n copy groups still in flight
+    switch (n) {
+        case 0: asm volatile("cp.async.wait_group 0;" ::: "memory"); break;
+        case 1: asm volatile("cp.async.wait_group 1;" ::: "memory"); break;
+        case 2: asm volatile("cp.async.wait_group 2;" ::: "memory"); break;
+        case 3: asm volatile("cp.async.wait_group 3;" ::: "memory"); break;
+        case 4: asm volatile("cp.async.wait_group 4;" ::: "memory"); break;
+        case 5: asm volatile("cp.async.wait_group 5;" ::: "memory"); break;
+        case 6: asm volatile("cp.async.wait_group 6;" ::: "memory"); break;
+        default: asm volatile("cp.async.wait_group 7;" ::: "memory"); break;
+    }
+}
+template <int WC, int MT, class Epi>
+__device__ __forceinline__ void large_product(const Weights& w, const RowsBf16& x, int rows, char* sm, Epi&& epi) {
     constexpr int WR = kWarps / WC, NT = 8 / WR, COLS = WC * MT * 16;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int wr = warp % WR, wc = warp / WR;
     const int ct = (w.n + COLS - 1) / COLS, rt = (rows + 63) / 64;
-    const Quarters qs(w.k);
-    const int buf = (64 + COLS) * qs.pitch, nbuf = min(4, kTileBytes / buf);
-    const int per = (ct * rt + gridDim.x - 1) / gridDim.x, last = min(ct * rt, (int)(blockIdx.x + 1) * per);
-    for (int task = blockIdx.x * per; task < last; ++task) {
-        const int r0 = task / ct * 64, c0 = task % ct * COLS, n = min(64, rows - r0);
-        auto load = [&](int q) {
-            char* dst = sm + q % nbuf * buf;
-            // a warp takes a row at a time, a lane 16 bytes of it: no division per piece
-            int k0 = qs.first[0], k1 = qs.first[1];
-            if (q == 1) k0 = qs.first[1], k1 = qs.first[2];
-            if (q == 2) k0 = qs.first[2], k1 = qs.first[3];
-            if (q == 3) k0 = qs.first[3], k1 = qs.first[4];
-            for (int c = lane; c < (k1 - k0) * 4; c += 32) {
-                const __nv_bfloat16* src = w.w + k0 * 32 + c * 8;
-                char* to = dst + 64 * qs.pitch + c * 16;
-#pragma unroll 4
-                for (int r = warp; r < COLS; r += kWarps) cp16(to + r * qs.pitch, src + (size_t)min(c0 + r, w.n - 1) * w.ld);
-                to = dst + c * 16;
-#pragma unroll 4
-                for (int r = warp; r < 64; r += kWarps) put.put(to + r * qs.pitch, r0 + min(r, n - 1), k0 * 32 + c * 8);
-            }
-            asm volatile("cp.async.commit_group;" ::: "memory");
-        };
-        pre(r0, n, task % ct == 0);
-        for (int q = 0; q < 4; ++q) {
-            if (q < nbuf) load(q);
-            else asm volatile("cp.async.commit_group;" ::: "memory");
-        }
-        float tot[2][MT][NT][4];
+    const int pitch = (((w.k >> 5) + 7) / 8 | 1) * 64, buf = (64 + COLS) * pitch, nbuf = min(8, kTileBytes / buf);
+    // a CTA's tiles lie one after another on the same rows as far as there are columns
+    const int per = (ct * rt + gridDim.x - 1) / gridDim.x, task0 = blockIdx.x * per, tasks = min(ct * rt, task0 + per) - task0;
+    if (tasks <= 0) return;
+    const int stream = tasks * 8;
+    auto load = [&](int j) {
+        if (j < stream) {
+            const int task = task0 + (j >> 3), r0 = task / ct * 64, c0 = task % ct * COLS;
+            int first, count;
+            segment(w.k, j & 7, first, count);
+            char* const dst = sm + j % nbuf * buf;
+            // eight lanes take the 16-byte pieces of a row (a piece of up to 8 x 64 bytes), four rows to a warp
+            for (int c = lane & 7; c < count * 4; c += 8) {
+                const __nv_bfloat16* ws = w.w + first * 32 + c * 8;
+                const __nv_bfloat16* xs = x.x + first * 32 + c * 8;
+                char* const to = dst + c * 16;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            if (q == 0) asm volatile("cp.async.wait_group 3;" ::: "memory");
-            if (q == 1) asm volatile("cp.async.wait_group 2;" ::: "memory");
-            if (q == 2) {
-                if (nbuf >= 3) asm volatile("cp.async.wait_group 1;" ::: "memory");
-                else asm volatile("cp.async.wait_group 0;" ::: "memory");
-            }
-            if (q == 3) asm volatile("cp.async.wait_group 0;" ::: "memory");
-            __syncthreads();
-            const char* src = sm + q % nbuf * buf;
-            const char* xb = src + (wr * NT * 8 + g) * qs.pitch + t * 16;
-            const char* wb = src + (64 + wc * MT * 16 + g) * qs.pitch + t * 16;
-#pragma unroll
-            for (int half = 0; half < 2; ++half) {  // the quarter's two segments
-                float acc[MT][NT][4];
-#pragma unroll
-                for (int m = 0; m < MT; ++m)
-#pragma unroll
-                    for (int nt = 0; nt < NT; ++nt) acc[m][nt][0] = acc[m][nt][1] = acc[m][nt][2] = acc[m][nt][3] = 0.0f;
-                int first, count;
-                segment(w.k, 2 * q + half, first, count);
-                first -= qs.first[q];
-#pragma unroll 2
-                for (int kb = first; kb < first + count; ++kb) {
-                    uint4 a[MT][2], b[NT];
-#pragma unroll
-                    for (int m = 0; m < MT; ++m) {
-                        a[m][0] = *reinterpret_cast<const uint4*>(wb + m * 16 * qs.pitch + kb * 64);
-                        a[m][1] = *reinterpret_cast<const uint4*>(wb + (m * 16 + 8) * qs.pitch + kb * 64);
-                    }
-#pragma unroll
-                    for (int nt = 0; nt < NT; ++nt) b[nt] = *reinterpret_cast<const uint4*>(xb + nt * 8 * qs.pitch + kb * 64);
-#pragma unroll
-                    for (int m = 0; m < MT; ++m)
-#pragma unroll
-                        for (int nt = 0; nt < NT; ++nt) mma_step(acc[m][nt], a[m][0], a[m][1], b[nt]);
+                for (int i = 0; i < 64 / 32; ++i) {
+                    const int r = i * 32 + warp * 4 + (lane >> 3);
+                    cp16(to + r * pitch, xs + (size_t)min(r0 + r, rows - 1) * x.ld);
                 }
 #pragma unroll
-                for (int m = 0; m < MT; ++m)
-#pragma unroll
-                    for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-                        for (int e = 0; e < 4; ++e)
-                            tot[q >> 1][m][nt][e] = (q & 1) == 0 && half == 0 ? acc[m][nt][e] : tot[q >> 1][m][nt][e] + acc[m][nt][e];
-            }
-            if (q + nbuf < 4) {  // this quarter's buffer is free for one that is still to come
-                __syncthreads();
-                load(q + nbuf);
+                for (int i = 0; i < COLS / 32; ++i) {
+                    const int r = i * 32 + warp * 4 + (lane >> 3);
+                    cp16(to + (64 + r) * pitch, ws + (size_t)min(c0 + r, w.n - 1) * w.ld);
+                }
             }
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    for (int j = 0; j < nbuf - 1; ++j) load(j);
+    float tot[2][MT][NT][4];
+    for (int task = task0; task < task0 + tasks; ++task) {
+        const int j0 = (task - task0) * 8;
+#pragma unroll
+        for (int sg = 0; sg < 8; ++sg) {
+            wait_pending(nbuf - 2);
+            __syncthreads();  // segment j0 + sg has landed; every warp is done with the one before, whose buffer comes next
+            load(j0 + sg + nbuf - 1);
+            const char* src = sm + (j0 + sg) % nbuf * buf;
+            const char* xb = src + (wr * NT * 8 + g) * pitch + t * 16;
+            const char* wb = src + (64 + wc * MT * 16 + g) * pitch + t * 16;
+            float acc[MT][NT][4];
+#pragma unroll
+            for (int m = 0; m < MT; ++m)
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt) acc[m][nt][0] = acc[m][nt][1] = acc[m][nt][2] = acc[m][nt][3] = 0.0f;
+            int first, count;
+            segment(w.k, sg, first, count);
+#pragma unroll 2
+            for (int kb = 0; kb < count; ++kb) {
+                uint4 a[MT][2], b[NT];
+#pragma unroll
+                for (int m = 0; m < MT; ++m) {
+                    a[m][0] = *reinterpret_cast<const uint4*>(wb + m * 16 * pitch + kb * 64);
+                    a[m][1] = *reinterpret_cast<const uint4*>(wb + (m * 16 + 8) * pitch + kb * 64);
+                }
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt) b[nt] = *reinterpret_cast<const uint4*>(xb + nt * 8 * pitch + kb * 64);
+#pragma unroll
+                for (int m = 0; m < MT; ++m)
+#pragma unroll
+                    for (int nt = 0; nt < NT; ++nt) mma_step(acc[m][nt], a[m][0], a[m][1], b[nt]);
+            }
+#pragma unroll
+            for (int m = 0; m < MT; ++m)
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        tot[sg >> 2][m][nt][e] = (sg & 3) == 0 ? acc[m][nt][e] : tot[sg >> 2][m][nt][e] + acc[m][nt][e];
+        }
+        const int r0 = task / ct * 64, c0 = task % ct * COLS;
 #pragma unroll
         for (int m = 0; m < MT; ++m)
 #pragma unroll
@@ -372,8 +356,15 @@ __device__ __forceinline__ void large_product(const Weights& w, const Put& put, 
                 epi(c, r, v[0], v[2]);      // columns c and c + 8 of row r
                 epi(c, r + 1, v[1], v[3]);  // and of row r + 1
             }
-        __syncthreads();  // the buffers and what `pre` prepared are free again
     }
+    wait_pending(0);
+    __syncthreads();
+}
+// fewer than a tile per SM: tiles of 32 columns, otherwise 64
+template <class Epi>
+__device__ __forceinline__ void large_product(const Weights& w, const RowsBf16& x, int rows, char* sm, bool narrow, Epi&& epi) {
+    if (narrow) large_product<1, 2>(w, x, rows, sm, epi);
+    else large_product<2, 2>(w, x, rows, sm, epi);
 }
 
 // 1 / rms of rows [r0, r0 + n) into inv_s, and into memory for the SSM stage
@@ -634,14 +625,11 @@ __device__ __forceinline__ void store_hidden(const StepArgs& a, int col, int row
     if (col >= 2 * a.d || row >= a.rows) return;
     a.act[(size_t)row * (2 * a.d + 64) + col] = __float2bfloat16_rn(v / (1.0f + __expf(-v)));
 }
-// returns the new feature's square (0 outside)
-__device__ __forceinline__ float store_features(const StepArgs& a, const float* in, float* out, float scale, int col, int row, float v) {
+__device__ __forceinline__ float new_feature(const StepArgs& a, const float* in, float scale, int col, int row, float v) {
     if (col >= a.d || row >= a.rows) return 0.0f;
     const unsigned short zb = __ldcg(reinterpret_cast<const unsigned short*>(a.z + (size_t)row * (a.d + 64) + col));
-    float f = __fadd_rn(v, __bfloat162float(__ushort_as_bfloat16(zb)));
-    if (in) f = fmaf(scale, f, ld_f(in + (size_t)row * a.d + col));
-    out[(size_t)row * a.d + col] = f;
-    return __fmul_rn(f, f);
+    const float f = __fadd_rn(v, __bfloat162float(__ushort_as_bfloat16(zb)));
+    return in ? fmaf(scale, f, ld_f(in + (size_t)row * a.d + col)) : f;
 }
 __device__ __forceinline__ void store_logit(const StepArgs& a, int col, int row, float v) {
     if (col < (int)a.vocab && row < a.rows) a.logits[(size_t)row * a.vocab + col] = __fmul_rn(v, a.head_scale);
@@ -664,76 +652,112 @@ __device__ __forceinline__ void check_ids(const StepArgs& a) {
             if (a.ids[r] >= a.vocab) atomicExch(a.status, PSSA_B200_ERR_TOKEN);
 }
 
-// ---- the stages of the many-rows kernel, each with registers of its own
-__device__ __noinline__ void large_xside(const StepArgs& a, const StepBlock& b, const Features f, float* inv_s, char* sm) {
-    RowsNorm x{f, b.gamma, b.beta, inv_s, 0};
-    large_product<2, 2>({b.wcat, (size_t)a.d, a.nc, a.d}, PutRows<RowsNorm&>{x}, a.rows, sm,
-                        [&](int r0, int n, bool first) { x.row0 = r0, row_scales(a, f, r0, n, inv_s, first); },
-                        [&](int c, int r, float v0, float v1) { store_xside(a, c, r, v0), store_xside(a, c + 8, r, v1); });
+// ---- many rows: the same stages with 64-row tiles, and the normalised rows formed once, in a stage of their own
+__device__ __forceinline__ void norm_stage(const StepArgs& a, const StepBlock& b, const Features& f) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tiles = a.d / 16;
+    for (int r = warp * gridDim.x + blockIdx.x; r < a.rows; r += gridDim.x * kWarps) {
+        const float* e = f.row(r);
+        float sum = 0.0f;
+        if (f.ids) {
+            for (int i = lane * 4; i < a.d; i += 128) {
+                const float4 v = __ldg(reinterpret_cast<const float4*>(e + i));
+                sum = fmaf(v.x, v.x, sum), sum = fmaf(v.y, v.y, sum), sum = fmaf(v.z, v.z, sum), sum = fmaf(v.w, v.w, sum);
+            }
+        } else {
+            for (int i = lane; i < tiles; i += 32) sum += ld_f(a.ssq + (size_t)r * tiles + i);
+        }
+#pragma unroll
+        for (int m = 16; m > 0; m >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, m);
+        const float inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(sum, (float)a.d), 1e-5f)));
+        if (lane == 0) a.inv[r] = inv;
+#pragma unroll 2
+        for (int i = lane * 8; i < a.d; i += 256) {
+            const float4 u = ld_f4(e + i), v = ld_f4(e + i + 4);
+            const float4 gu = __ldg(reinterpret_cast<const float4*>(b.gamma + i)), gv = __ldg(reinterpret_cast<const float4*>(b.gamma + i + 4));
+            const float4 tu = __ldg(reinterpret_cast<const float4*>(b.beta + i)), tv = __ldg(reinterpret_cast<const float4*>(b.beta + i + 4));
+            *reinterpret_cast<uint4*>(a.x + (size_t)r * a.d + i) =
+                make_uint4(pack_bf16(norm1(u.x, inv, gu.x, tu.x), norm1(u.y, inv, gu.y, tu.y)), pack_bf16(norm1(u.z, inv, gu.z, tu.z), norm1(u.w, inv, gu.w, tu.w)),
+                           pack_bf16(norm1(v.x, inv, gv.x, tv.x), norm1(v.y, inv, gv.y, tv.y)), pack_bf16(norm1(v.z, inv, gv.z, tv.z), norm1(v.w, inv, gv.w, tv.w)));
+        }
+    }
 }
-template <int NV>
-__device__ __noinline__ void large_ssm(const StepArgs& a, const StepBlock& b, const Features f) {
-    SsmAhead<NV, 3> sa;
-    ssm_request(a, b, sa);
-    ssm_stage(a, f, sa, b.state);
-}
-__device__ __noinline__ void large_read(const StepArgs& a, const StepBlock& b, float* sm, float* keys) {
-    read_stage(a, b, sm, request_keys(a, b, keys) ? keys : nullptr);
-}
-__device__ __noinline__ void large_gated(const StepArgs& a, const StepBlock& b, char* sm) {
-    large_product<1, 2>({b.vp, (size_t)3 * a.cap, a.d, a.cap}, PutBf16{a.w, (size_t)3 * a.cap}, a.rows, sm, [](int, int, bool) {},
-                        [&](int c, int r, float v0, float v1) { store_gated(a, c, r, v0), store_gated(a, c + 8, r, v1); });
-}
-__device__ __noinline__ void large_hidden(const StepArgs& a, const StepBlock& b, char* sm) {
-    large_product<2, 2>({b.w1, (size_t)a.d + 64, 2 * a.d, a.d + 64}, PutBf16{a.z, (size_t)a.d + 64}, a.rows, sm, [](int, int, bool) {},
-                        [&](int c, int r, float v0, float v1) { store_hidden(a, c, r, v0), store_hidden(a, c + 8, r, v1); });
-}
-__device__ __noinline__ void large_features(const StepArgs& a, const StepBlock& b, const float* in, float* out, char* sm) {
-    large_product<1, 2>({b.w2, (size_t)2 * a.d + 64, a.d, 2 * a.d + 64}, PutBf16{a.act, (size_t)2 * a.d + 64}, a.rows, sm, [](int, int, bool) {},
-                        [&](int c, int r, float v0, float v1) {
-        // and the sum of squares of each 16 of them: pair c, c + 8 first, then over the eight c
-        float q = __fadd_rn(store_features(a, in, out, b.res_scale, c, r, v0), store_features(a, in, out, b.res_scale, c + 8, r, v1));
-        q = __fadd_rn(q, __shfl_xor_sync(0xffffffffu, q, 4));
-        q = __fadd_rn(q, __shfl_xor_sync(0xffffffffu, q, 8));
-        q = __fadd_rn(q, __shfl_xor_sync(0xffffffffu, q, 16));
-        if ((threadIdx.x & 31) < 4 && r < a.rows && c < a.d) a.ssq[(size_t)r * (a.d / 16) + c / 16] = q;
-    });
-}
-__device__ __noinline__ void large_head(const StepArgs& a, const float* in, char* sm) {
-    large_product<2, 2>({a.unembed, (size_t)a.d, (int)a.vocab, a.d}, PutRows<RowsF32>{RowsF32{in, (size_t)a.d}}, a.rows, sm, [](int, int, bool) {},
-                        [&](int c, int r, float v0, float v1) { store_logit(a, c, r, v0), store_logit(a, c + 8, r, v1); });
+// Weights of this block's later products and the next block's first one, on their way to L2 during the SSM stage: a product's
+// tiles are few and would wait for HBM otherwise
+__device__ __forceinline__ void prefetch_weights(const StepArgs& a, int l) {
+    const size_t d = a.d;
+    const int thread = blockIdx.x * kThreads + threadIdx.x, threads = gridDim.x * kThreads;
+    auto lines = [&](const __nv_bfloat16* w, size_t n) {
+        for (size_t i = (size_t)thread * 64; i < n; i += (size_t)threads * 64) asm volatile("prefetch.global.L2 [%0];" ::"l"(w + i));
+    };
+    const StepBlock& b = a.block[l];
+    lines(b.w1, 2 * d * (d + 64));
+    lines(b.w2, d * (2 * d + 64));
+    for (int i = thread; i < a.d * (a.cap / 64); i += threads)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(b.vp + (size_t)(i / (a.cap / 64)) * 3 * a.cap + i % (a.cap / 64) * 64));
+    if (l + 1 < a.depth) lines(a.block[l + 1].wcat, (size_t)a.nc * d);
 }
 
 template <int NV>
 __global__ void __launch_bounds__(kThreads, 1) step_large_kernel(const __grid_constant__ StepArgs a) {
     extern __shared__ __align__(128) float step_smem[];
-    float* inv_s = step_smem;  // [64] row scales, then the stages' own
-    char* sm = reinterpret_cast<char*>(step_smem + 64);
+    char* sm = reinterpret_cast<char*>(step_smem);
     Barrier bar{a.barrier, a.status, 0, false};
     bar.init();
     check_ids(a);
     prefetch_vectors(a, 0);
+    const int d = a.d, tiles = d / 16, rt = (a.rows + 63) / 64;
+    const bool narrow = (d / 32) * rt <= (int)gridDim.x;  // tiles of 64 columns would leave half of the SMs without one
     const float* in = nullptr;
     for (int l = 0; l < a.depth; ++l) {
         const StepBlock& b = a.block[l];
         float* out = in == a.feat_a ? a.feat_b : a.feat_a;
-        const Features f{a.embed, l == 0 ? a.ids : nullptr, in, a.d, a.vocab};
-        large_xside(a, b, f, inv_s, sm);
+        const Features f{a.embed, l == 0 ? a.ids : nullptr, in, d, a.vocab};
+        norm_stage(a, b, f);
         bar.wait();
-        large_ssm<NV>(a, b, f);
+        large_product({b.wcat, (size_t)d, a.nc, d}, RowsBf16{a.x, (size_t)d}, a.rows, sm, narrow,
+                      [&](int c, int r, float v0, float v1) { store_xside(a, c, r, v0), store_xside(a, c + 8, r, v1); });
         bar.wait();
-        large_read(a, b, reinterpret_cast<float*>(sm), reinterpret_cast<float*>(sm) + 448);
+        prefetch_weights(a, l);
+        {
+            SsmAhead<NV, 3> sa;
+            ssm_request(a, b, sa);
+            ssm_stage(a, f, sa, b.state);
+        }
         bar.wait();
-        large_gated(a, b, sm);
+        {
+            float* const keys = reinterpret_cast<float*>(sm) + 448;
+            const bool staged = request_keys(a, b, keys);
+            read_stage(a, b, reinterpret_cast<float*>(sm), staged ? keys : nullptr);
+        }
+        bar.wait();
+        large_product({b.vp, (size_t)3 * a.cap, d, a.cap}, RowsBf16{a.w, (size_t)3 * a.cap}, a.rows, sm, narrow,
+                      [&](int c, int r, float v0, float v1) { store_gated(a, c, r, v0), store_gated(a, c + 8, r, v1); });
         prefetch_vectors(a, l + 1);
         bar.wait();
-        large_hidden(a, b, sm);
+        large_product({b.w1, (size_t)d + 64, 2 * d, d + 64}, RowsBf16{a.z, (size_t)d + 64}, a.rows, sm, narrow,
+                      [&](int c, int r, float v0, float v1) { store_hidden(a, c, r, v0), store_hidden(a, c + 8, r, v1); });
         bar.wait();
-        large_features(a, b, in, out, sm);
+        large_product({b.w2, (size_t)2 * d + 64, d, 2 * d + 64}, RowsBf16{a.act, (size_t)2 * d + 64}, a.rows, sm, narrow,
+                      [&](int c, int r, float v0, float v1) {
+            // and the sum of squares of each 16 of them: pair c, c + 8 first, then over the eight c
+            const float f0 = new_feature(a, in, b.res_scale, c, r, v0), f1 = new_feature(a, in, b.res_scale, c + 8, r, v1);
+            const bool live = r < a.rows && c < d;
+            if (live) {
+                out[(size_t)r * d + c] = f0, out[(size_t)r * d + c + 8] = f1;
+                if (l + 1 == a.depth) a.x[(size_t)r * d + c] = __float2bfloat16_rn(f0), a.x[(size_t)r * d + c + 8] = __float2bfloat16_rn(f1);
+            }
+            float q = __fadd_rn(__fmul_rn(f0, f0), __fmul_rn(f1, f1));
+            q = __fadd_rn(q, __shfl_xor_sync(0xffffffffu, q, 4));
+            q = __fadd_rn(q, __shfl_xor_sync(0xffffffffu, q, 8));
+            q = __fadd_rn(q, __shfl_xor_sync(0xffffffffu, q, 16));
+            if ((threadIdx.x & 31) < 4 && live) a.ssq[(size_t)r * tiles + c / 16] = q;
+        });
         in = out;
         bar.wait();
     }
-    if (a.logits) large_head(a, in, sm);
+    if (a.logits)
+        large_product<2, 2>({a.unembed, (size_t)d, (int)a.vocab, d}, RowsBf16{a.x, (size_t)d}, a.rows, sm,
+                            [&](int c, int r, float v0, float v1) { store_logit(a, c, r, v0), store_logit(a, c + 8, r, v1); });
 }
 
 // Up to kSmallRows rows, NT 8-row tiles of them: the stages are inlined, because the weights and carries that a stage asks for before
@@ -781,7 +805,9 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(const __grid_constant
         ahead(w2);
         bar.wait();
         small_product<NT>(w2, xa, a.rows, ah, sm, [&](int c, int r, float v) {
-            float q = store_features(a, in, out, b.res_scale, c, r, v);
+            const float fv = new_feature(a, in, b.res_scale, c, r, v);
+            if (r < a.rows) out[(size_t)r * d + c] = fv;
+            float q = __fmul_rn(fv, fv);
             q = __fadd_rn(q, __shfl_xor_sync(0xffffffffu, q, 8));
             q = __fadd_rn(q, __shfl_xor_sync(0xffffffffu, q, 1));
             q = __fadd_rn(q, __shfl_xor_sync(0xffffffffu, q, 2));
@@ -830,7 +856,7 @@ int32_t launch_decode_step(pssa_b200_ctx* ctx, const StepLaunch& p) {
     a.ssm_scale = p.ssm_scale, a.head_scale = p.head_scale, a.tau = p.tau;
     a.embed = p.embed, a.ids = p.ids, a.slots = p.slots, a.unembed = (const __nv_bfloat16*)p.unembed, a.carry_stride = p.carry_stride;
     a.feat_a = p.feat_a, a.feat_b = p.feat_b, a.proj = p.proj, a.y = p.y, a.qpart = p.qpart, a.ssq = p.ssq, a.inv = p.inv, a.logits = p.logits;
-    a.w = (__nv_bfloat16*)p.w, a.z = (__nv_bfloat16*)p.z, a.act = (__nv_bfloat16*)p.act, a.barrier = (unsigned long long*)p.barrier;
+    a.x = (__nv_bfloat16*)p.x, a.w = (__nv_bfloat16*)p.w, a.z = (__nv_bfloat16*)p.z, a.act = (__nv_bfloat16*)p.act, a.barrier = (unsigned long long*)p.barrier;
     a.status = ctx->status_dev;
     for (size_t l = 0; l < p.depth; ++l) {
         const StepLaunch::Block& s = p.blocks[l];
