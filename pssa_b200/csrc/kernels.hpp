@@ -233,6 +233,7 @@ struct StepLaunch {
     };
     const Block* blocks;
 };
+bool step_rows_ok(size_t rows);
 bool step_shape_ok(size_t depth, size_t d, size_t s, size_t k, size_t cap, size_t rank);
 int32_t launch_decode_step(pssa_b200_ctx* ctx, const StepLaunch& p);
 int32_t launch_keys_by_quad(pssa_b200_ctx* ctx, const float* keys, float* out, int cap, int k);

@@ -524,14 +524,14 @@ int32_t head_rows(pssa_b200_model* m, const float* feats, size_t n_heads, bool w
 }
 
 // One token per lane, every lane present and in row order, in the bf16 mode: the whole step is one kernel (step_decode.cu).
-// The choice follows the shape of the step and the model's options, never the number of lanes: a stream's bits are the same
-// alone and in a batch.
+// Up to 128 lanes (step_rows_ok) every sum has one order whatever the number of lanes: a stream's bits are the same alone and
+// in any such batch, and the same in any larger one.
 bool step_model_ok(const pssa_b200_model* m) {
     return m->precision == PSSA_B200_PRECISION_BF16 && m->loops == 1 && step_shape_ok(m->depth, m->d, m->s, m->k, m->cap, m->rank) &&
            1.0f / m->cfg.tau_mem < 3.0e38f;
 }
 bool decode_step_fused(const pssa_b200_model* m, size_t rows, size_t lanes, const uint32_t* h_off, const uint32_t* h_len) {
-    if (rows != lanes || rows > 65536 || m->sp.active || m->obs.enabled || !step_model_ok(m)) return false;
+    if (rows != lanes || !step_rows_ok(rows) || m->sp.active || m->obs.enabled || !step_model_ok(m)) return false;
     for (auto& b : m->blocks)
         if (b.count == 0 || (m->top_k != 0 && m->top_k < b.count)) return false;
     for (size_t l = 0; l < lanes; ++l)
@@ -673,7 +673,7 @@ int32_t run_lanes(pssa_b200_model* m, const uint64_t* ids, const uint32_t* offse
         if (step) {
             if ((rc = run_decode_step(m, rows, ws.ids, want_head && !h_last.empty() ? ws.logits : nullptr))) return rc;
         } else {
-            if (step_model_ok(m) && (rc = ensure_step(m, std::min<size_t>(m->max_streams, 1024)))) return rc;
+            if (step_model_ok(m) && (rc = ensure_step(m, std::min<size_t>(m->max_streams, 128)))) return rc;
             if ((rc = forward_rows(m, rows, n_lanes, h_off.data(), h_len.data(), &feats, h_last.size()))) return rc;
         }
         if (!h_last.empty() && want_head) {
@@ -819,7 +819,7 @@ int32_t pssa_b200_model_prefill_batch_dev(pssa_b200_model* m, const uint32_t* id
         }
         return PSSA_B200_OK;
     }
-    if (step_model_ok(m) && (rc = ensure_step(m, std::min<size_t>(m->max_streams, 1024)))) return rc;
+    if (step_model_ok(m) && (rc = ensure_step(m, std::min<size_t>(m->max_streams, 128)))) return rc;
     PSSA_CUDA(ctx, cudaMemcpyAsync(ws.ids, ids_dev, span * 4, cudaMemcpyDeviceToDevice, st));
     m->sp.active = m->sp.world > 1;
     rc = forward_rows(m, span, n_lanes, h_off.data(), h_len.data(), &feats, h_last.size());

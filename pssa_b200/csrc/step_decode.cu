@@ -39,6 +39,8 @@ constexpr int kWarps = 8;
 constexpr int kMaxSegKb = 8;         // 32-wide k steps of a segment whose weights are requested ahead: K <= 2048
 constexpr int kMaxDepth = 32;        // blocks whose pointers fit in the kernel's parameters
 constexpr int kSmallRows = 32;       // rows up to which a warp takes a segment of K
+constexpr int kStepRows = 128;       // rows up to which this kernel is the faster way: 12 blocks, d 768, us per step at 1 / 32 / 128 rows
+                                     // 840 -> 260 / 960 -> 540 / 1060 -> 1090; at 256 the separate kernels' tensor-core products win (1130, 1840)
 constexpr int kKeyQuads = 8192;      // the bank's keys are staged in shared memory (128 KB) up to here
 constexpr int kTileBytes = 212 * 1024;
 constexpr int kPitch = 20;           // floats per row of a partial tile: the fragment stores of a warp hit 32 banks
@@ -101,11 +103,16 @@ struct Barrier {
         if (threadIdx.x == 0) target = look(count) / gridDim.x * gridDim.x;
         dead = false;
     }
-    __device__ __forceinline__ void wait() {
+    // arrive, then what does not depend on the other CTAs (the next stage's weights), then wait
+    __device__ __forceinline__ void arrive() {
         __syncthreads();
         if (threadIdx.x == 0) {
             target += gridDim.x;
             asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(count) : "memory");
+        }
+    }
+    __device__ __forceinline__ void wait() {
+        if (threadIdx.x == 0) {
             unsigned polls = 0;
             while (!dead && look(count) < target)
                 if (++polls > (1u << 20)) atomicExch(status, PSSA_B200_ERR_TIMEOUT), dead = true;
@@ -713,9 +720,11 @@ __global__ void __launch_bounds__(kThreads, 1) step_large_kernel(const __grid_co
         float* out = in == a.feat_a ? a.feat_b : a.feat_a;
         const Features f{a.embed, l == 0 ? a.ids : nullptr, in, d, a.vocab};
         norm_stage(a, b, f);
+        bar.arrive();
         bar.wait();
         large_product({b.wcat, (size_t)d, a.nc, d}, RowsBf16{a.x, (size_t)d}, a.rows, sm, narrow,
                       [&](int c, int r, float v0, float v1) { store_xside(a, c, r, v0), store_xside(a, c + 8, r, v1); });
+        bar.arrive();
         bar.wait();
         prefetch_weights(a, l);
         {
@@ -723,19 +732,23 @@ __global__ void __launch_bounds__(kThreads, 1) step_large_kernel(const __grid_co
             ssm_request(a, b, sa);
             ssm_stage(a, f, sa, b.state);
         }
+        bar.arrive();
         bar.wait();
         {
             float* const keys = reinterpret_cast<float*>(sm) + 448;
             const bool staged = request_keys(a, b, keys);
             read_stage(a, b, reinterpret_cast<float*>(sm), staged ? keys : nullptr);
         }
+        bar.arrive();
         bar.wait();
         large_product({b.vp, (size_t)3 * a.cap, d, a.cap}, RowsBf16{a.w, (size_t)3 * a.cap}, a.rows, sm, narrow,
                       [&](int c, int r, float v0, float v1) { store_gated(a, c, r, v0), store_gated(a, c + 8, r, v1); });
         prefetch_vectors(a, l + 1);
+        bar.arrive();
         bar.wait();
         large_product({b.w1, (size_t)d + 64, 2 * d, d + 64}, RowsBf16{a.z, (size_t)d + 64}, a.rows, sm, narrow,
                       [&](int c, int r, float v0, float v1) { store_hidden(a, c, r, v0), store_hidden(a, c + 8, r, v1); });
+        bar.arrive();
         bar.wait();
         large_product({b.w2, (size_t)2 * d + 64, d, 2 * d + 64}, RowsBf16{a.act, (size_t)2 * d + 64}, a.rows, sm, narrow,
                       [&](int c, int r, float v0, float v1) {
@@ -753,6 +766,7 @@ __global__ void __launch_bounds__(kThreads, 1) step_large_kernel(const __grid_co
             if ((threadIdx.x & 31) < 4 && live) a.ssq[(size_t)r * tiles + c / 16] = q;
         });
         in = out;
+        bar.arrive();
         bar.wait();
     }
     if (a.logits)
@@ -787,21 +801,26 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(const __grid_constant
             w2{b.w2, (size_t)2 * d + 64, d, 2 * d + 64};
         row_scales(a, f, 0, a.rows, inv_s, blockIdx.x == 0);
         small_product<NT>(wcat, RowsNorm{f, b.gamma, b.beta, inv_s, 0}, a.rows, ah, sm, [&](int c, int r, float v) { store_xside(a, c, r, v); });
+        bar.arrive();
         SsmAhead<NV, 2> sa;
         ssm_request(a, b, sa);
         const bool keys_here = request_keys(a, b, keys_s);
         bar.wait();
         ssm_stage(a, f, sa, b.state);
+        bar.arrive();
         ahead(vp);
         bar.wait();
         read_stage(a, b, sm, keys_here ? keys_s : nullptr);
+        bar.arrive();
         bar.wait();
         const RowsBf16 xw{a.w, (size_t)3 * a.cap}, xz{a.z, (size_t)d + 64}, xa{a.act, (size_t)2 * d + 64};
         small_product<NT>(vp, xw, a.rows, ah, sm, [&](int c, int r, float v) { store_gated(a, c, r, v); });
+        bar.arrive();
         ahead(w1);
         prefetch_vectors(a, l + 1);
         bar.wait();
         small_product<NT>(w1, xz, a.rows, ah, sm, [&](int c, int r, float v) { store_hidden(a, c, r, v); });
+        bar.arrive();
         ahead(w2);
         bar.wait();
         small_product<NT>(w2, xa, a.rows, ah, sm, [&](int c, int r, float v) {
@@ -815,6 +834,7 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(const __grid_constant
             if (c % 16 == 0 && r < a.rows) a.ssq[(size_t)r * tiles + c / 16] = q;
         });
         in = out;
+        bar.arrive();
         if (l + 1 < a.depth) ahead({a.block[l + 1].wcat, (size_t)d, a.nc, d});
         else if (a.logits) ahead({a.unembed, (size_t)d, (int)a.vocab, d});
         bar.wait();
@@ -843,6 +863,8 @@ int32_t launch_keys_by_quad(pssa_b200_ctx* ctx, const float* keys, float* out, i
     keys_by_quad_kernel<<<(n + 255) / 256, 256, 0, ctx->stream>>>(keys, out, cap, k);
     return after_launch(ctx, "keys_by_quad_kernel");
 }
+
+bool step_rows_ok(size_t rows) { return rows <= kStepRows; }
 
 bool step_shape_ok(size_t depth, size_t d, size_t s, size_t k, size_t cap, size_t rank) {
     return depth <= kMaxDepth && d % 32 == 0 && 2 * d + 64 <= 1664 && (s == 16 || s == 32 || s == 64) && (k == 64 || k == 128) && cap % 64 == 0 &&
