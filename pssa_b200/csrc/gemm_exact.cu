@@ -103,16 +103,174 @@ __global__ void __launch_bounds__(256) gemm_xwt_exact_kernel(const float* __rest
     }
 }
 
+// ---- tiled form for K == 8 or K >= 16. What bounded the kernel above was its fold (five shuffles for every output of a warp) and,
+// with few rows, one round trip to HBM per 32 columns of W. Here
+//   * the fold is a butterfly that halves a lane's outputs at every level: the additions pair the same sums as the reference's
+//     (a + b and b + a are the same number), so RT * CT outputs cost RT * CT - 1 shuffles and end one to a lane;
+//   * with few rows (AHEAD > 0) a warp requests AHEAD steps of its W rows at once;
+//   * several products of one X (the six x-side projections) are one launch.
+constexpr int kMaxParts = 6;
+struct ExactPart {
+    const float* w;
+    float* out;
+    int n, tile0, epi;  // columns, first column tile
+};
+struct ExactParts {
+    ExactPart p[kMaxParts];
+    int count, tiles;
+};
+template <int RT, int CT, int AHEAD>
+__global__ void __launch_bounds__(256) gemm_xwt_exact_tiled_kernel(const float* __restrict__ x, const __grid_constant__ ExactParts parts, size_t M,
+                                                                   int K, size_t ldo, float alpha) {
+    pdl_trigger();
+    pdl_wait();
+    constexpr int NO = RT * CT;
+    const int lane = threadIdx.x & 31;
+    const size_t row_tiles = (M + RT - 1) / RT, job = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (job >= row_tiles * parts.tiles) return;
+    const int ct = (int)(job % parts.tiles);
+    const size_t row0 = job / parts.tiles * RT;
+    int pi = 0;
+#pragma unroll
+    for (int i = 1; i < kMaxParts; ++i)
+        if (i < parts.count && ct >= parts.p[i].tile0) pi = i;
+    const ExactPart part = parts.p[pi];
+    const int col0 = (ct - part.tile0) * CT;
+    const float* xr[RT];
+    const float* wc[CT];
+#pragma unroll
+    for (int r = 0; r < RT; ++r) xr[r] = x + (row0 + r < M ? row0 + r : M - 1) * (size_t)K + lane;
+#pragma unroll
+    for (int c = 0; c < CT; ++c) wc[c] = part.w + (size_t)min(col0 + c, part.n - 1) * K + lane;
+    float acc[NO];
+#pragma unroll
+    for (int o = 0; o < NO; ++o) acc[o] = 0.0f;
+    const int steps = K >> 5;
+    if constexpr (AHEAD > 0) {
+        for (int s0 = 0; s0 < steps; s0 += AHEAD) {
+            float wb[AHEAD][CT];
+#pragma unroll
+            for (int s = 0; s < AHEAD; ++s)
+#pragma unroll
+                for (int c = 0; c < CT; ++c) wb[s][c] = s0 + s < steps ? __ldg(wc[c] + (s0 + s) * 32) : 0.0f;
+#pragma unroll
+            for (int s = 0; s < AHEAD; ++s)
+                if (s0 + s < steps) {
+                    float xa[RT];
+#pragma unroll
+                    for (int r = 0; r < RT; ++r) xa[r] = __ldg(xr[r] + (s0 + s) * 32);
+#pragma unroll
+                    for (int r = 0; r < RT; ++r)
+#pragma unroll
+                        for (int c = 0; c < CT; ++c) acc[r * CT + c] = fmaf(xa[r], wb[s][c], acc[r * CT + c]);
+                }
+        }
+    } else {
+#pragma unroll 2
+        for (int s = 0; s < steps; ++s) {
+            float xa[RT], wb[CT];
+#pragma unroll
+            for (int r = 0; r < RT; ++r) xa[r] = __ldg(xr[r] + s * 32);
+#pragma unroll
+            for (int c = 0; c < CT; ++c) wb[c] = __ldg(wc[c] + s * 32);
+#pragma unroll
+            for (int r = 0; r < RT; ++r)
+#pragma unroll
+                for (int c = 0; c < CT; ++c) acc[r * CT + c] = fmaf(xa[r], wb[c], acc[r * CT + c]);
+        }
+    }
+    int i = steps << 5;
+    for (; i + 8 <= K; i += 8)  // remaining whole vectors go to accumulator 0 (lanes 0..7)
+        if (lane < 8) {
+#pragma unroll
+            for (int r = 0; r < RT; ++r)
+#pragma unroll
+                for (int c = 0; c < CT; ++c) acc[r * CT + c] = fmaf(__ldg(xr[r] + i), __ldg(wc[c] + i), acc[r * CT + c]);
+        }
+    // acc0+acc1 / acc2+acc3 (distance 8), their sum (16), low + high half (4), the two horizontal adds (1, 2)
+    int mine = 0;  // which output ends in this lane (its first, where a lane keeps several)
+#pragma unroll
+    for (int level = 0; level < 5; ++level) {
+        constexpr int kDist[5] = {8, 16, 4, 1, 2};
+        const int m = kDist[level];
+        if (NO >> level > 1) {
+            const int half = (NO >> level) / 2;
+            const bool up = (lane & m) != 0;
+#pragma unroll
+            for (int o = 0; o < half; ++o) {
+                const float send = up ? acc[o] : acc[o + half], keep = up ? acc[o + half] : acc[o];
+                acc[o] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, send, m));
+            }
+            if (up) mine += half;
+        } else {
+            acc[0] = __fadd_rn(acc[0], __shfl_xor_sync(0xffffffffu, acc[0], m));
+        }
+    }
+    constexpr int OWN = NO >= 32 ? NO / 32 : 1;
+    // with fewer than 32 outputs the lanes that differ in the last levels hold the same one: one of them stores
+    constexpr int kDup = NO >= 32 ? 0 : NO == 16 ? 2 : NO == 8 ? 3 : NO == 4 ? 7 : 31;
+    if (NO < 32 && (lane & kDup)) return;
+#pragma unroll
+    for (int o = 0; o < OWN; ++o) {
+        const int r = (mine + o) / CT, c = (mine + o) % CT;
+        if (row0 + r >= M || col0 + c >= part.n) continue;
+        float sum = acc[o];
+        const float *xs = x + (row0 + r) * (size_t)K, *ws = part.w + (size_t)(col0 + c) * K;
+        for (int t = i; t < K; ++t) sum = __fadd_rn(sum, __fmul_rn(xs[t], ws[t]));
+        float* dst = part.out + (row0 + r) * ldo + col0 + c;
+        *dst = apply_epilogue(part.epi, sum, alpha, part.epi == EPI_ADD_OUT ? *dst : 0.0f);
+    }
+}
+
+template <int RT, int CT, int AHEAD>
+int32_t launch_tiled(pssa_b200_ctx* ctx, const float* x, ExactParts& parts, size_t M, size_t K, size_t ldo, float alpha) {
+    parts.tiles = 0;
+    for (int i = 0; i < parts.count; ++i) parts.p[i].tile0 = parts.tiles, parts.tiles += (parts.p[i].n + CT - 1) / CT;
+    const size_t jobs = (M + RT - 1) / RT * parts.tiles, blocks = (jobs + 7) / 8;
+    if (blocks > 0x7fffffffull) return fail(ctx, PSSA_B200_ERR_SHAPE, "B200 GEMM grid (%zu, 1) exceeds grid limits; refusing launch", blocks);
+    PSSA_CUDA(ctx, launch_dependent(gemm_xwt_exact_tiled_kernel<RT, CT, AHEAD>, dim3((unsigned)blocks), dim3(256), 0, ctx->stream, x, parts, M, (int)K, ldo, alpha));
+    return after_launch(ctx, "gemm_xwt_exact_kernel");
+}
+int32_t launch_parts(pssa_b200_ctx* ctx, const float* x, ExactParts& parts, size_t M, size_t K, size_t ldo, float alpha) {
+    size_t n = 0;
+    for (int i = 0; i < parts.count; ++i) n += parts.p[i].n;
+    // few rows: every row in one warp, two columns of W a warp, so that W's rows are spread over the most warps; otherwise 8 x 8
+    // tiles (four multiply-adds a load) while they give every SM its eight warps, 8 x 4 below
+    if (M <= 4) return launch_tiled<4, 2, 24>(ctx, x, parts, M, K, ldo, alpha);
+    if (M <= 16) return launch_tiled<16, 2, 24>(ctx, x, parts, M, K, ldo, alpha);
+    if ((M + 7) / 8 * ((n + 7) / 8) >= (size_t)ctx->sm_count * 8) return launch_tiled<8, 8, 0>(ctx, x, parts, M, K, ldo, alpha);
+    return launch_tiled<8, 4, 0>(ctx, x, parts, M, K, ldo, alpha);
+}
+
 }  // namespace
 
 int32_t launch_gemm_exact(pssa_b200_ctx* ctx, const float* x, const float* w, float* out, size_t M, size_t N, size_t K,
                           size_t ldo, int epi, float alpha) {
+    if (K == 8 || K >= 16) {
+        ExactParts parts{};
+        parts.count = 1, parts.p[0] = {w, out, (int)N, 0, epi};
+        return launch_parts(ctx, x, parts, M, K, ldo, alpha);
+    }
     size_t bx = (M + 4 * RT - 1) / (4 * RT), by = (N + 2 * CT - 1) / (2 * CT);
     if (bx > 0x7fffffffull || by > 65535)
         return fail(ctx, PSSA_B200_ERR_SHAPE, "B200 GEMM grid (%zu, %zu) exceeds grid limits; refusing launch", bx, by);
     gemm_xwt_exact_kernel<<<dim3((unsigned)bx, (unsigned)by), 256, 0, ctx->stream>>>(x, w, out, M, (int)N, (int)K, ldo, epi,
                                                                                    alpha);
     return after_launch(ctx, "gemm_xwt_exact_kernel");
+}
+
+int32_t launch_gemm_exact_many(pssa_b200_ctx* ctx, const float* x, const ExactProduct* products, int count, size_t M, size_t K, size_t ldo) {
+    if (count > kMaxParts || !(K == 8 || K >= 16)) {
+        for (int i = 0; i < count; ++i) {
+            const int32_t rc = launch_gemm_exact(ctx, x, products[i].w, products[i].out, M, products[i].n, K, ldo, products[i].epi, 1.0f);
+            if (rc) return rc;
+        }
+        return PSSA_B200_OK;
+    }
+    ExactParts parts{};
+    parts.count = count;
+    for (int i = 0; i < count; ++i) parts.p[i] = {products[i].w, products[i].out, (int)products[i].n, 0, products[i].epi};
+    return launch_parts(ctx, x, parts, M, K, ldo, 1.0f);
 }
 
 }  // namespace pssa

@@ -183,6 +183,15 @@ int32_t launch_consolidate(pssa_b200_ctx* ctx, float* up_fast, float* up_slow, s
 int32_t launch_gemm_exact(pssa_b200_ctx* ctx, const float* x, const float* w, float* out, size_t M, size_t N, size_t K,
                           size_t ldo, int epi, float alpha);
 
+// the same for several W of one X in one launch
+struct ExactProduct {
+    const float* w;
+    float* out;
+    size_t n;
+    int epi;
+};
+int32_t launch_gemm_exact_many(pssa_b200_ctx* ctx, const float* x, const ExactProduct* products, int count, size_t M, size_t K, size_t ldo);
+
 // gemm_tcgen05.cu: one warp waits `polls` polls on an mbarrier nobody arrives at and records the expiry (self-test)
 int32_t launch_wait_expiry_selftest(pssa_b200_ctx* ctx, unsigned polls);
 // gemm_tcgen05.cu: bf16 operands [rows, K] row-major, fp32 accumulate in TMEM; out fp32 [M, ldo] and/or bf16 [M, N]

@@ -328,12 +328,10 @@ int32_t forward_rows(pssa_b200_model* m, size_t rows, size_t lanes, const uint32
             return rc;
         // stage 2: x-side projections (src/gpu_batch.rs:477-536 plus the query/gate/adapter rows that read x_norm)
         if (exact) {
-            struct P { int id; size_t off, n; int epi; };
-            P ps[] = {{T_W_DELTA, m->off_delta, m->d, EPI_SOFTPLUS}, {T_W_B, m->off_b, m->s, EPI_NONE},
-                      {T_W_C, m->off_c, m->s, EPI_NONE},            {T_W_QX, m->off_q, m->k, EPI_NONE},
-                      {T_W_GATE, m->off_gate, m->d, EPI_SIGMOID},   {T_AD_DOWN, m->off_act, m->rank, EPI_SILU}};
-            for (auto& p : ps)
-                if ((rc = launch_gemm_exact(ctx, v.x_norm, b.w[p.id], v.proj + p.off, nr, p.n, m->d, nc, p.epi, 1.0f))) return rc;
+            const ExactProduct ps[] = {{b.w[T_W_DELTA], v.proj + m->off_delta, m->d, EPI_SOFTPLUS}, {b.w[T_W_B], v.proj + m->off_b, m->s, EPI_NONE},
+                                       {b.w[T_W_C], v.proj + m->off_c, m->s, EPI_NONE},             {b.w[T_W_QX], v.proj + m->off_q, m->k, EPI_NONE},
+                                       {b.w[T_W_GATE], v.proj + m->off_gate, m->d, EPI_SIGMOID},    {b.w[T_AD_DOWN], v.proj + m->off_act, m->rank, EPI_SILU}};
+            if ((rc = launch_gemm_exact_many(ctx, v.x_norm, ps, 6, nr, m->d, nc))) return rc;
         } else {
             // the adapter activations (last column range) also go, as bf16, into the extra K block of both MLP operands
             if ((rc = launch_gemm_bf16_cat(ctx, v.x_bf16, b.wcat_bf16, v.proj, nr, nc, m->d, nc, (int)m->off_b, (int)m->off_gate,
