@@ -21,7 +21,7 @@
 namespace pssa {
 namespace {
 
-constexpr int kSampleThreads = 256;
+constexpr int kSampleThreads = 1024;  // a row's passes over the vocabulary are one CTA's: its loads in flight are what bounds them
 constexpr int kRecent = 64;
 
 __device__ __forceinline__ int order_key(float v) {  // monotone signed key of f32::total_cmp
@@ -39,10 +39,25 @@ __device__ __forceinline__ unsigned long long block_max_u64(unsigned long long v
     __syncthreads();  // scratch may still be read from the previous call
     if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = v;
     __syncthreads();
-    unsigned long long r = scratch[0];
+    unsigned long long r = scratch[threadIdx.x & 31];
 #pragma unroll
-    for (int w = 1; w < kSampleThreads / 32; ++w) r = scratch[w] > r ? scratch[w] : r;
+    for (int m = 16; m > 0; m >>= 1) {
+        unsigned long long o = __shfl_xor_sync(0xffffffffu, r, m);
+        r = o > r ? o : r;
+    }
     return r;
+}
+// block-wide sum in a fixed tree; every thread gets the result
+__device__ __forceinline__ float block_sum(float v, float* scratch) {
+#pragma unroll
+    for (int m = 16; m > 0; m >>= 1) v += __shfl_xor_sync(0xffffffffu, v, m);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = v;
+    __syncthreads();
+    v = scratch[threadIdx.x & 31];
+#pragma unroll
+    for (int m = 16; m > 0; m >>= 1) v += __shfl_xor_sync(0xffffffffu, v, m);
+    return v;
 }
 
 __global__ void __launch_bounds__(kSampleThreads) sample_kernel(SampleParams p) {
@@ -91,14 +106,11 @@ __global__ void __launch_bounds__(kSampleThreads) sample_kernel(SampleParams p) 
         mxr = s_raw_max;
         float part = 0.0f;
         for (int i = tid; i < v; i += kSampleThreads) part += expf(__fsub_rn(lg[i], mxr));
-        s_part[tid] = part;
-        __syncthreads();
+        float sum = block_sum(part, s_part);
         if (tid == 0) {
-            float sum = 0.0f;
             if (p.exact) {
+                sum = 0.0f;
                 for (int i = 0; i < v; ++i) sum = __fadd_rn(sum, expf(__fsub_rn(lg[i], mxr)));  // the reference's order
-            } else {
-                for (int t = 0; t < kSampleThreads; ++t) sum += s_part[t];
             }
             s_raw_sum = sum;
         }
@@ -154,19 +166,17 @@ __global__ void __launch_bounds__(kSampleThreads) sample_kernel(SampleParams p) 
         pr[i] = e;
         part += e;
     }
-    s_part[tid] = part;
-    __syncthreads();
-    if (tid == 0) {
-        float sum = 0.0f;
-        if (p.exact) {
+    float sum = block_sum(part, s_part);
+    if (p.exact) {
+        __syncthreads();
+        if (tid == 0) {
+            sum = 0.0f;
             for (int i = 1; i < v; ++i) sum = __fadd_rn(sum, pr[i]);  // the reference's order
-        } else {
-            for (int t = 0; t < kSampleThreads; ++t) sum += s_part[t];
+            s_part[0] = sum;
         }
-        s_part[0] = sum;
+        __syncthreads();
+        sum = s_part[0];
     }
-    __syncthreads();
-    const float sum = s_part[0];
     if (!isfinite(sum) || sum <= 0.0f) {
         if (tid == 0) p.ids_out[row] = 0xffffffffu, p.status_out[row] = 2;
         return;

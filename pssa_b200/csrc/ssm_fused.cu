@@ -776,12 +776,14 @@ __global__ void __launch_bounds__(kWideWarps * 32) ssm_wide_kernel(SsmParams p) 
 // Decode step: every lane advances by one token, so the launch is one pass over the carries (2 * d * s * 4 bytes per
 // lane in and out) and nothing else matters. A thread owns four consecutive states of one channel: rates, carry in and
 // carry out are 16-byte accesses that a warp makes over a contiguous 512 bytes; y is finished by a shuffle tree over the
-// TPC threads of the channel. Same arithmetic as the fast mode of the tiled kernel (ex2.approx, fused multiply-adds).
-template <int TPC>
+// TPC threads of the channel. Same arithmetic as the fast mode of the tiled kernel (ex2.approx, fused multiply-adds), or as the
+// exact one: then the products h * C wait in shared memory for one thread per channel to add them in order.
+template <int TPC, bool EXACT>
 __global__ void __launch_bounds__(256) ssm_step_kernel(SsmParams p) {
     pdl_trigger();  // the next kernel in the stream may start its prologue now ...
     pdl_wait();     // ... and this one, if launched as a dependent, waits here for its own predecessor
     constexpr int CPB = 256 / TPC;  // channels per CTA
+    __shared__ float prod[EXACT ? CPB * (4 * TPC + 1) : 1];
     const int tid = threadIdx.x;
     const int q = tid % TPC, c = tid / TPC;
     const int ncb = (p.d + CPB - 1) / CPB;
@@ -806,30 +808,46 @@ __global__ void __launch_bounds__(256) ssm_step_kernel(SsmParams p) {
         const float4 c4 = __ldg(reinterpret_cast<const float4*>(p.c_proj + row * ldbc + q * 4));
         const float dl = __ldg(p.delta + row * ldd + i);
         const float w = dl * __ldg(p.x_norm + row * d + i);
-        const float k = dl * 1.4426950408889634f;
         float4 h;
-        h.x = fmaf(ex2_approx(k * a4.x), h4.x, w * b4.x);
-        h.y = fmaf(ex2_approx(k * a4.y), h4.y, w * b4.y);
-        h.z = fmaf(ex2_approx(k * a4.z), h4.z, w * b4.z);
-        h.w = fmaf(ex2_approx(k * a4.w), h4.w, w * b4.w);
-        yp = fmaf(h.x, c4.x, fmaf(h.y, c4.y, fmaf(h.z, c4.z, h.w * c4.w)));
+        if constexpr (EXACT) {
+            const float xv = __ldg(p.x_norm + row * d + i);
+            h.x = __fadd_rn(__fmul_rn(exp_exact(__fmul_rn(dl, a4.x)), h4.x), __fmul_rn(__fmul_rn(dl, b4.x), xv));
+            h.y = __fadd_rn(__fmul_rn(exp_exact(__fmul_rn(dl, a4.y)), h4.y), __fmul_rn(__fmul_rn(dl, b4.y), xv));
+            h.z = __fadd_rn(__fmul_rn(exp_exact(__fmul_rn(dl, a4.z)), h4.z), __fmul_rn(__fmul_rn(dl, b4.z), xv));
+            h.w = __fadd_rn(__fmul_rn(exp_exact(__fmul_rn(dl, a4.w)), h4.w), __fmul_rn(__fmul_rn(dl, b4.w), xv));
+            float* pr = prod + c * (4 * TPC + 1) + q * 4;
+            pr[0] = __fmul_rn(h.x, c4.x), pr[1] = __fmul_rn(h.y, c4.y), pr[2] = __fmul_rn(h.z, c4.z), pr[3] = __fmul_rn(h.w, c4.w);
+        } else {
+            const float k = dl * 1.4426950408889634f;
+            h.x = fmaf(ex2_approx(k * a4.x), h4.x, w * b4.x);
+            h.y = fmaf(ex2_approx(k * a4.y), h4.y, w * b4.y);
+            h.z = fmaf(ex2_approx(k * a4.z), h4.z, w * b4.z);
+            h.w = fmaf(ex2_approx(k * a4.w), h4.w, w * b4.w);
+            yp = fmaf(h.x, c4.x, fmaf(h.y, c4.y, fmaf(h.z, c4.z, h.w * c4.w)));
+        }
         if (carry) *reinterpret_cast<float4*>(carry + so) = h;
     }
+    if constexpr (EXACT) {
+        __syncthreads();
+        if (q == 0 && i < d)
+            for (int j = 0; j < s; ++j) yp = __fadd_rn(yp, prod[c * (4 * TPC + 1) + j]);
+    } else {
 #pragma unroll
-    for (int m = 1; m < TPC; m <<= 1) yp += __shfl_xor_sync(0xffffffffu, yp, m);
+        for (int m = 1; m < TPC; m <<= 1) yp += __shfl_xor_sync(0xffffffffu, yp, m);
+    }
     if (q == 0 && i < d) {
         p.y[row * d + i] = yp;
         if (p.y_bf16) reinterpret_cast<__nv_bfloat16*>(p.y_bf16)[row * d + i] = __float2bfloat16_rn(yp);
     }
 }
 
-template <int TPC>
+template <int TPC, bool EXACT>
 int32_t launch_step(pssa_b200_ctx* ctx, const SsmParams& p) {
     constexpr int CPB = 256 / TPC;
     size_t blocks = (size_t)((p.d + CPB - 1) / CPB) * p.lanes;
     if (blocks > 0x7fffffffull)
         return fail(ctx, PSSA_B200_ERR_SHAPE, "B200 SSM grid (%zu, 1) exceeds grid limits; refusing launch", blocks);
-    PSSA_CUDA(ctx, launch_dependent(ssm_step_kernel<TPC>, dim3((unsigned)blocks), dim3(256), 0, ctx->stream, p));
+    PSSA_CUDA(ctx, launch_dependent(ssm_step_kernel<TPC, EXACT>, dim3((unsigned)blocks), dim3(256), 0, ctx->stream, p));
     return after_launch(ctx, "ssm_step_kernel");
 }
 
@@ -1023,12 +1041,13 @@ int32_t launch_ssm_fused(pssa_b200_ctx* ctx, const SsmParams& p, bool exact) {
         if (rc != PSSA_B200_OK) return rc;
     }
     const bool tape = p.states || p.bar_a || p.bar_b;
-    if (p.single_token && !exact && !tape && p.aligned && s <= 128 && (reinterpret_cast<uintptr_t>(p.rates) & 15) == 0 &&
+    if (p.single_token && !tape && (!exact || s <= 64) && p.aligned && s <= 128 && (reinterpret_cast<uintptr_t>(p.rates) & 15) == 0 &&
         (reinterpret_cast<uintptr_t>(p.carry) & 15) == 0 && ((p.carry_stride ? p.carry_stride : (size_t)p.d * s) & 3) == 0) {
-        if (s <= 16) return launch_step<4>(ctx, p);
-        if (s <= 32) return launch_step<8>(ctx, p);
-        if (s <= 64) return launch_step<16>(ctx, p);
-        return launch_step<32>(ctx, p);
+        // (above 64 states the exact mode sums y over shuffled groups: the tiled kernel's order stays)
+        if (s <= 16) return exact ? launch_step<4, true>(ctx, p) : launch_step<4, false>(ctx, p);
+        if (s <= 32) return exact ? launch_step<8, true>(ctx, p) : launch_step<8, false>(ctx, p);
+        if (s <= 64) return exact ? launch_step<16, true>(ctx, p) : launch_step<16, false>(ctx, p);
+        return launch_step<32, false>(ctx, p);
     }
     if (ssm_wide_ok(p)) {
         // Channels in flight: lanes counted by their share of the longest one. With 64 states, up to one channel per scheduler
