@@ -55,25 +55,23 @@ __global__ void __launch_bounds__(256) embed_norm_kernel(const float* __restrict
     }
     float sum;
     if (EXACT) {
-        // the squares by all lanes, 128 at a time; the sum itself is one chain of additions in lane 0's registers
-        // (a multiply and a scalar shared-memory read inside the chain made it 14 us at 768 elements)
+        // one chain of additions, as in the reference; the elements come 32 at a time, as vectors, ahead of it
+        // (a scalar shared-memory read and a multiply inside the chain made it 12 us at 768 elements)
         __syncwarp();
         sum = 0.0f;
         int i0 = 0;
-        for (; i0 + 128 <= d; i0 += 128) {
-            float sq[4];
+        if ((d & 3) == 0)
+            for (; i0 + 32 <= d; i0 += 32) {
+                float4 e[8];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const float e = buf[i0 + u * 32 + lane];
-                sq[u] = __fmul_rn(e, e);
+                for (int u = 0; u < 8; ++u) e[u] = *reinterpret_cast<const float4*>(buf + i0 + u * 4);
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    sum = __fadd_rn(sum, __fmul_rn(e[u].x, e[u].x)), sum = __fadd_rn(sum, __fmul_rn(e[u].y, e[u].y));
+                    sum = __fadd_rn(sum, __fmul_rn(e[u].z, e[u].z)), sum = __fadd_rn(sum, __fmul_rn(e[u].w, e[u].w));
+                }
             }
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-#pragma unroll
-                for (int j = 0; j < 32; ++j) sum = __fadd_rn(sum, __shfl_sync(0xffffffffu, sq[u], j));
-        }
         for (; i0 < d; ++i0) sum = __fadd_rn(sum, __fmul_rn(buf[i0], buf[i0]));
-        sum = __shfl_sync(0xffffffffu, sum, 0);
     } else {
         sum = part;
 #pragma unroll
@@ -108,16 +106,16 @@ __global__ void __launch_bounds__(256) embed_norm_kernel(const float* __restrict
 // One thread owns one channel for ROWS_PER_CTA consecutive rows: its 16 up-projection weights stay in registers,
 // the 16 adapter activations of a row are one address for the whole CTA (broadcast), and y / g / m_proj / z are
 // read and written as coalesced rows.
-constexpr int kCombineRows = 16;
+constexpr int kCombineRows = 16;  // 4 up to 256 rows, where 16 would leave a few CTAs with four trips to memory each
 template <int RANK>
 __global__ void __launch_bounds__(256) combine_zraw_kernel(const float* __restrict__ y, const float* __restrict__ g,
                                                            size_t ldg, const float* __restrict__ m_proj,
                                                            const float* __restrict__ act, size_t ldact,
                                                            const float* __restrict__ u_eff, float* __restrict__ z_raw,
                                                            __nv_bfloat16* __restrict__ z_bf16, size_t rows, int d, int rank,
-                                                           float ssm_scale) {
+                                                           float ssm_scale, int per) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t row0 = (size_t)blockIdx.y * kCombineRows;
+    const size_t row0 = (size_t)blockIdx.y * per;
     if (i >= d) return;
     float u[RANK > 0 ? RANK : 1];
     if (RANK > 0) {
@@ -125,7 +123,7 @@ __global__ void __launch_bounds__(256) combine_zraw_kernel(const float* __restri
         for (int r = 0; r < RANK; ++r) u[r] = __ldg(u_eff + (size_t)i * RANK + r);
     }
     // rows in groups of four: all global loads of a group are issued before any arithmetic
-    for (int r0 = 0; r0 < kCombineRows; r0 += 4) {
+    for (int r0 = 0; r0 < per; r0 += 4) {
         float yv[4], gv[4], mv[4];
         size_t rowv[4];
 #pragma unroll
@@ -360,7 +358,8 @@ int32_t launch_embed_norm(pssa_b200_ctx* ctx, const float* embed, const uint32_t
 int32_t launch_combine_zraw(pssa_b200_ctx* ctx, const float* y, const float* g, size_t ldg, const float* m_proj, const float* act,
                             size_t ldact, const float* u_eff, float* z_raw, void* z_bf16, size_t rows, int d, int rank,
                             float ssm_scale) {
-    dim3 grid((unsigned)((d + 255) / 256), (unsigned)((rows + kCombineRows - 1) / kCombineRows));
+    const int per = rows <= 256 ? 4 : kCombineRows;
+    dim3 grid((unsigned)((d + 255) / 256), (unsigned)((rows + per - 1) / per));
     if (grid.y > 65535) {
         // very long passes: fall back to several launches of at most 65535 row groups
         size_t step = (size_t)65535 * kCombineRows;
@@ -374,10 +373,10 @@ int32_t launch_combine_zraw(pssa_b200_ctx* ctx, const float* y, const float* g, 
     }
     if (rank == 16)
         combine_zraw_kernel<16><<<grid, 256, 0, ctx->stream>>>(y, g, ldg, m_proj, act, ldact, u_eff, z_raw, (__nv_bfloat16*)z_bf16,
-                                                             rows, d, rank, ssm_scale);
+                                                             rows, d, rank, ssm_scale, per);
     else
         combine_zraw_kernel<0><<<grid, 256, 0, ctx->stream>>>(y, g, ldg, m_proj, act, ldact, u_eff, z_raw, (__nv_bfloat16*)z_bf16,
-                                                            rows, d, rank, ssm_scale);
+                                                            rows, d, rank, ssm_scale, per);
     return after_launch(ctx, "combine_zraw_kernel");
 }
 

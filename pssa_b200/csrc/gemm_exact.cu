@@ -107,9 +107,10 @@ __global__ void __launch_bounds__(256) gemm_xwt_exact_kernel(const float* __rest
 // with few rows, one round trip to HBM per 32 columns of W. Here
 //   * the fold is a butterfly that halves a lane's outputs at every level: the additions pair the same sums as the reference's
 //     (a + b and b + a are the same number), so RT * CT outputs cost RT * CT - 1 shuffles and end one to a lane;
-//   * with few rows (AHEAD > 0) a warp requests AHEAD steps of its W rows at once;
+//   * with few rows (AHEAD > 0) a warp requests AHEAD steps of its W rows at once and X is staged in shared memory;
 //   * several products of one X (the six x-side projections) are one launch.
 constexpr int kMaxParts = 6;
+constexpr int kMaxStagedX = 200 * 1024;
 struct ExactPart {
     const float* w;
     float* out;
@@ -122,12 +123,16 @@ struct ExactParts {
 template <int RT, int CT, int AHEAD>
 __global__ void __launch_bounds__(256) gemm_xwt_exact_tiled_kernel(const float* __restrict__ x, const __grid_constant__ ExactParts parts, size_t M,
                                                                    int K, size_t ldo, float alpha) {
-    pdl_trigger();
-    pdl_wait();
+    extern __shared__ __align__(16) float sm_x[];  // AHEAD > 0: [RT][K], the only row tile
     constexpr int NO = RT * CT;
     const int lane = threadIdx.x & 31;
-    const size_t row_tiles = (M + RT - 1) / RT, job = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (job >= row_tiles * parts.tiles) return;
+    const size_t row_tiles = (M + RT - 1) / RT, job0 = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5), jobs = row_tiles * parts.tiles;
+    const size_t job = job0 < jobs ? job0 : jobs - 1;
+    if (AHEAD == 0) {
+        pdl_trigger();
+        pdl_wait();
+        if (job0 >= jobs) return;
+    }
     const int ct = (int)(job % parts.tiles);
     const size_t row0 = job / parts.tiles * RT;
     int pi = 0;
@@ -147,6 +152,23 @@ __global__ void __launch_bounds__(256) gemm_xwt_exact_tiled_kernel(const float* 
     for (int o = 0; o < NO; ++o) acc[o] = 0.0f;
     const int steps = K >> 5;
     if constexpr (AHEAD > 0) {
+        // W towards L2 before the wait (a prefetch reads nothing), X whole into shared memory: one trip to memory each
+#pragma unroll
+        for (int c = 0; c < CT; ++c)
+            for (int k = lane * 32; k < K; k += 1024) asm volatile("prefetch.global.L2 [%0];" ::"l"(wc[c] - lane + k));
+        pdl_trigger();
+        pdl_wait();
+        if ((K & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
+            const int q = K >> 2, rows = M < RT ? (int)M : RT;
+            for (int r = 0; r < rows; ++r)
+                for (int k = threadIdx.x; k < q; k += 256)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(sm_x + r * K + k * 4)), "l"(x + (size_t)r * K + k * 4));
+            asm volatile("cp.async.commit_group;\n cp.async.wait_group 0;" ::: "memory");
+        } else {
+            for (int idx = threadIdx.x; idx < (int)(M < RT ? M : RT) * K; idx += 256) sm_x[idx] = x[idx];
+        }
+        __syncthreads();
+        if (job0 >= jobs) return;
         for (int s0 = 0; s0 < steps; s0 += AHEAD) {
             float wb[AHEAD][CT];
 #pragma unroll
@@ -158,7 +180,7 @@ __global__ void __launch_bounds__(256) gemm_xwt_exact_tiled_kernel(const float* 
                 if (s0 + s < steps) {
                     float xa[RT];
 #pragma unroll
-                    for (int r = 0; r < RT; ++r) xa[r] = __ldg(xr[r] + (s0 + s) * 32);
+                    for (int r = 0; r < RT; ++r) xa[r] = sm_x[(r < (int)M ? r : (int)M - 1) * K + (s0 + s) * 32 + lane];
 #pragma unroll
                     for (int r = 0; r < RT; ++r)
 #pragma unroll
@@ -228,7 +250,13 @@ int32_t launch_tiled(pssa_b200_ctx* ctx, const float* x, ExactParts& parts, size
     for (int i = 0; i < parts.count; ++i) parts.p[i].tile0 = parts.tiles, parts.tiles += (parts.p[i].n + CT - 1) / CT;
     const size_t jobs = (M + RT - 1) / RT * parts.tiles, blocks = (jobs + 7) / 8;
     if (blocks > 0x7fffffffull) return fail(ctx, PSSA_B200_ERR_SHAPE, "B200 GEMM grid (%zu, 1) exceeds grid limits; refusing launch", blocks);
-    PSSA_CUDA(ctx, launch_dependent(gemm_xwt_exact_tiled_kernel<RT, CT, AHEAD>, dim3((unsigned)blocks), dim3(256), 0, ctx->stream, x, parts, M, (int)K, ldo, alpha));
+    const size_t smem = AHEAD ? (size_t)RT * K * sizeof(float) : 0;
+    static PerDeviceOnce attr_set;
+    if (smem > 48 * 1024 && attr_set.need(ctx->device)) {
+        PSSA_CUDA(ctx, cudaFuncSetAttribute(gemm_xwt_exact_tiled_kernel<RT, CT, AHEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxStagedX));
+        attr_set.done(ctx->device);
+    }
+    PSSA_CUDA(ctx, launch_dependent(gemm_xwt_exact_tiled_kernel<RT, CT, AHEAD>, dim3((unsigned)blocks), dim3(256), smem, ctx->stream, x, parts, M, (int)K, ldo, alpha));
     return after_launch(ctx, "gemm_xwt_exact_kernel");
 }
 int32_t launch_parts(pssa_b200_ctx* ctx, const float* x, ExactParts& parts, size_t M, size_t K, size_t ldo, float alpha) {
@@ -236,8 +264,8 @@ int32_t launch_parts(pssa_b200_ctx* ctx, const float* x, ExactParts& parts, size
     for (int i = 0; i < parts.count; ++i) n += parts.p[i].n;
     // few rows: every row in one warp, two columns of W a warp, so that W's rows are spread over the most warps; otherwise 8 x 8
     // tiles (four multiply-adds a load) while they give every SM its eight warps, 8 x 4 below
-    if (M <= 4) return launch_tiled<4, 2, 24>(ctx, x, parts, M, K, ldo, alpha);
-    if (M <= 16) return launch_tiled<16, 2, 24>(ctx, x, parts, M, K, ldo, alpha);
+    if (M <= 4 && 4 * K * 4 <= kMaxStagedX) return launch_tiled<4, 2, 24>(ctx, x, parts, M, K, ldo, alpha);
+    if (M <= 16 && 16 * K * 4 <= kMaxStagedX) return launch_tiled<16, 2, 24>(ctx, x, parts, M, K, ldo, alpha);
     if ((M + 7) / 8 * ((n + 7) / 8) >= (size_t)ctx->sm_count * 8) return launch_tiled<8, 8, 0>(ctx, x, parts, M, K, ldo, alpha);
     return launch_tiled<8, 4, 0>(ctx, x, parts, M, K, ldo, alpha);
 }

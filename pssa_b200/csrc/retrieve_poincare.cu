@@ -915,46 +915,59 @@ __global__ void __launch_bounds__(256) softmax_topk_kernel(RetrieveParams p) {
 }
 
 // ------------------------------------------------------------------ C: dense value read m = W x V
-// Up to kMixRows rows: four rows x one column a thread, the rows' weights in shared memory as one quad per slot and sixteen slots
+// Up to kMixRows rows: four rows x one column a thread, the rows' weights in shared memory as one quad per slot and 32 slots
 // of the column in flight. The 64 x 64 tiles below leave a dozen CTAs with two barriers per 32 slots; the order of a sum
 // is the same, slots ascending.
 constexpr int kMixRows = 1024;
 template <bool EXACT>
 __global__ void __launch_bounds__(128) value_mix_rows_kernel(RetrieveParams p) {
+    {   // the column tile on its way to L2, all of it at once: with hundreds of MB of fp32 weights a step every block's bank comes
+        // from HBM, and sixteen slots in flight a thread are 32 round trips (16 rows of 768 columns, 512 slots: 55 us). Before the
+        // wait: a prefetch reads nothing
+        const int c0 = blockIdx.y * 128 + (threadIdx.x & 3) * 32;
+        if (c0 < p.dv)
+            for (int s = threadIdx.x >> 2; s < p.count; s += 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.values + (size_t)s * p.dv + c0));
+    }
+    pdl_trigger();
+    pdl_wait();
     extern __shared__ __align__(16) float4 mix_w[];
     const size_t q0 = (size_t)blockIdx.x * 4;
     const int col = blockIdx.y * 128 + threadIdx.x, count = p.count;
+    // padded to whole batches with weight zero: the sums start at +0, so adding +-0 to one leaves its bits
+    constexpr int U = 32;
+    const int padded = (count + 2 * U - 1) / (2 * U) * (2 * U);
     for (int r = 0; r < 4; ++r)
-        for (int s = threadIdx.x; s < count; s += 128)
-            reinterpret_cast<float*>(mix_w)[s * 4 + r] = q0 + r < p.rows ? p.weights[(q0 + r) * p.cap + s] : 0.0f;
+        for (int s = threadIdx.x; s < padded; s += 128)
+            reinterpret_cast<float*>(mix_w)[s * 4 + r] = q0 + r < p.rows && s < count ? p.weights[(q0 + r) * p.cap + s] : 0.0f;
     __syncthreads();
     if (col >= p.dv) return;
     const float* v = p.values + col;
     float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    auto step = [&](float x, const float4& w) {
-        if (EXACT) {
-            acc[0] = __fadd_rn(acc[0], __fmul_rn(w.x, x)), acc[1] = __fadd_rn(acc[1], __fmul_rn(w.y, x));
-            acc[2] = __fadd_rn(acc[2], __fmul_rn(w.z, x)), acc[3] = __fadd_rn(acc[3], __fmul_rn(w.w, x));
-        } else {
-            acc[0] = fmaf(w.x, x, acc[0]), acc[1] = fmaf(w.y, x, acc[1]), acc[2] = fmaf(w.z, x, acc[2]), acc[3] = fmaf(w.w, x, acc[3]);
-        }
-    };
-    constexpr int U = 16;
     float ring[2][U];
     auto fetch = [&](float (&b)[U], int s0) {
 #pragma unroll
         for (int u = 0; u < U; ++u) b[u] = s0 + u < count ? __ldg(v + (size_t)(s0 + u) * p.dv) : 0.0f;
     };
+    auto batch = [&](const float (&b)[U], int s0) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const float4 w = mix_w[s0 + u];
+            const float x = b[u];
+            if (EXACT) {
+                acc[0] = __fadd_rn(acc[0], __fmul_rn(w.x, x)), acc[1] = __fadd_rn(acc[1], __fmul_rn(w.y, x));
+                acc[2] = __fadd_rn(acc[2], __fmul_rn(w.z, x)), acc[3] = __fadd_rn(acc[3], __fmul_rn(w.w, x));
+            } else {
+                acc[0] = fmaf(w.x, x, acc[0]), acc[1] = fmaf(w.y, x, acc[1]), acc[2] = fmaf(w.z, x, acc[2]), acc[3] = fmaf(w.w, x, acc[3]);
+            }
+        }
+    };
     fetch(ring[0], 0);
-    for (int s0 = 0; s0 < count; s0 += 2 * U) {
+#pragma unroll 1
+    for (int s0 = 0; s0 < padded; s0 += 2 * U) {
         fetch(ring[1], s0 + U);
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-            if (s0 + u < count) step(ring[0][u], mix_w[s0 + u]);
+        batch(ring[0], s0);
         fetch(ring[0], s0 + 2 * U);
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-            if (s0 + U + u < count) step(ring[1][u], mix_w[s0 + U + u]);
+        batch(ring[1], s0 + U);
     }
 #pragma unroll
     for (int r = 0; r < 4; ++r)
@@ -1140,8 +1153,8 @@ int32_t launch_memory_read(pssa_b200_ctx* ctx, const RetrieveParams& p, bool exa
         dim3 grid((unsigned)qblocks, (unsigned)((p.dv + 63) / 64));
         if (p.rows <= kMixRows && p.count <= 2048) {
             const dim3 small((unsigned)((p.rows + 3) / 4), (unsigned)((p.dv + 127) / 128));
-            if (exact) value_mix_rows_kernel<true><<<small, 128, (size_t)p.count * 16, ctx->stream>>>(p);
-            else value_mix_rows_kernel<false><<<small, 128, (size_t)p.count * 16, ctx->stream>>>(p);
+            const size_t smem = (size_t)((p.count + 63) / 64 * 64) * 16;
+            PSSA_CUDA(ctx, launch_dependent(exact ? value_mix_rows_kernel<true> : value_mix_rows_kernel<false>, small, dim3(128), smem, ctx->stream, p));
         } else if (exact)
             value_mix_kernel<true><<<grid, 256, 0, ctx->stream>>>(p);
         else

@@ -117,18 +117,25 @@ __global__ void __launch_bounds__(kSampleThreads) sample_kernel(SampleParams p) 
         __syncthreads();
     }
     if (tid == 0) s_pen_n = 0;
-    // 2. repetition penalty, in the order the ids were generated
-    if (tid == 0 && p.repetition_penalty > 1.0f && p.recent_ids) {
-        const unsigned n = min(p.recent_count[slot], (unsigned)kRecent);
-        const unsigned* ids = p.recent_ids + slot * kRecent;
-        for (unsigned g = 0; g < n; ++g) {
-            const unsigned id = ids[g];
-            if (id < (unsigned)v) {
-                bool known = false;  // remember the unpenalised value once per id (for the raw confidence)
-                for (unsigned q = 0; q < g && !known; ++q) known = ids[q] == id;
-                if (!known) s_pen_id[s_pen_n] = id, s_pen_orig[s_pen_n] = lg[id], ++s_pen_n;
-                lg[id] = lg[id] > 0.0f ? __fdiv_rn(lg[id], p.repetition_penalty) : __fmul_rn(lg[id], p.repetition_penalty);
-            }
+    // 2. repetition penalty, once for every time an id occurs among the generated ones: a thread per first occurrence (64 ids
+    // one after another by one thread are 64 trips to L2 and 2000 comparisons)
+    __shared__ unsigned s_recent[kRecent];
+    const unsigned n_recent = p.repetition_penalty > 1.0f && p.recent_ids ? min(p.recent_count[slot], (unsigned)kRecent) : 0u;
+    if (tid < (int)n_recent) s_recent[tid] = p.recent_ids[slot * kRecent + tid];
+    __syncthreads();
+    if (tid < (int)n_recent && s_recent[tid] < (unsigned)v) {
+        const unsigned id = s_recent[tid];
+        int before = 0, times = 0;
+        for (unsigned q = 0; q < n_recent; ++q) {
+            before += s_recent[q] == id && q < (unsigned)tid;
+            times += s_recent[q] == id;
+        }
+        if (before == 0) {
+            float x = lg[id];
+            const unsigned at = atomicAdd(&s_pen_n, 1u);  // the unpenalised value, for the raw confidence
+            s_pen_id[at] = id, s_pen_orig[at] = x;
+            for (int t = 0; t < times; ++t) x = x > 0.0f ? __fdiv_rn(x, p.repetition_penalty) : __fmul_rn(x, p.repetition_penalty);
+            lg[id] = x;
         }
     }
     __syncthreads();

@@ -19,6 +19,7 @@
 // Arithmetic is multiply-then-add with separate roundings (no FMA contraction), which is what the
 // reference's scalar recurrence does (src/gpu_batch.rs:564-567); with a single chunk the states are
 // therefore bit-identical to the ordered CPU recurrence.
+#include <cstdlib>
 #include "bounds.hpp"
 #include "context.hpp"
 #include "kernels.hpp"
@@ -227,6 +228,47 @@ __global__ void __launch_bounds__(128, MAPS ? 4 : 7)
         VecIO<V>::store_keep(last + it.lane * g.stride + (size_t)it.cv * V, cb);
 }
 
+// Single pass for few channels (states only): U rows of both inputs stay in flight in registers at all times -- a row's slot is
+// refilled as soon as it is consumed -- so a tenth of the usual threads keep HBM busy and no time chunks, which read the
+// inputs twice, are needed.
+constexpr int kDeepRows = 16;
+__global__ void __launch_bounds__(64) scan_states_deep(const float* a, const float* b, const float* __restrict__ h0,
+                                                       float* h, float* __restrict__ last, ScanGeom g) {
+    constexpr int U = kDeepRows;
+    const size_t gid = (size_t)blockIdx.x * 64 + threadIdx.x;
+    if (gid >= g.total) return;
+    const Item it = decode(g, gid);
+    const size_t base = it.lane * g.len * g.stride + (size_t)it.cv * 4, co = it.lane * g.stride + (size_t)it.cv * 4;
+    const float *pa = a + base, *pb = b + base;
+    float* po = h + base;
+    float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    if (h0 != nullptr) VecIO<4>::load_keep(h0 + co, c);
+    float av[U][4], bv[U][4];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+        if ((size_t)u < g.len) {
+            VecIO<4>::load(pa, av[u]);
+            VecIO<4>::load(pb, bv[u]);
+            pa += g.stride, pb += g.stride;
+        }
+    for (size_t t = 0; t < g.len; t += U) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (t + u >= g.len) break;
+#pragma unroll
+            for (int v = 0; v < 4; ++v) c[v] = __fadd_rn(__fmul_rn(av[u][v], c[v]), bv[u][v]);
+            VecIO<4>::store(po, c);
+            po += g.stride;
+            if (t + u + U < g.len) {
+                VecIO<4>::load(pa, av[u]);
+                VecIO<4>::load(pb, bv[u]);
+                pa += g.stride, pb += g.stride;
+            }
+        }
+    }
+    if (last != nullptr) VecIO<4>::store_keep(last + co, c);
+}
+
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 // Split time only when channels alone leave SMs idle. Target: one resident wave of 128-thread CTAs.
@@ -252,6 +294,18 @@ int32_t run_scan(pssa_b200_ctx* ctx, const float* a, const float* b, const float
     g.chunk_len = (unsigned)((len + g.n_chunks - 1) / g.n_chunks);
     g.n_chunks = (unsigned)((len + g.chunk_len - 1) / g.chunk_len);
     g.total = lanes * g.n_chunks * g.cvecs;
+    if constexpr (V == 4 && !MAPS) {
+        const size_t items = lanes * g.cvecs;
+        static const char* e = getenv("DEEP");
+        const size_t lo = e ? atoi(e) : 8192;
+        // (h may be b itself: a row is read before it is written, by the same thread)
+        if (forced_chunks <= 0 && items >= lo && items < 49152 && len >= 4 * kDeepRows) {
+            g.n_chunks = 1, g.chunk_len = (unsigned)len, g.total = items;
+            scan_states_deep<<<(unsigned)((items + 63) / 64), 64, 0, ctx->stream>>>(a, b, h0, out_b, last, g);
+            return after_launch(ctx, "scan_states_deep");
+        }
+        if (forced_chunks <= 0 && e && items >= 49152) g.n_chunks = 1, g.chunk_len = (unsigned)len, g.total = items;
+    }
     constexpr int U = MAPS ? 4 : 4;
     const int threads = 128;
     size_t blocks = (g.total + threads - 1) / threads;
