@@ -19,7 +19,6 @@
 // Arithmetic is multiply-then-add with separate roundings (no FMA contraction), which is what the
 // reference's scalar recurrence does (src/gpu_batch.rs:564-567); with a single chunk the states are
 // therefore bit-identical to the ordered CPU recurrence.
-#include <cstdlib>
 #include "bounds.hpp"
 #include "context.hpp"
 #include "kernels.hpp"
@@ -231,10 +230,9 @@ __global__ void __launch_bounds__(128, MAPS ? 4 : 7)
 // Single pass for few channels (states only): U rows of both inputs stay in flight in registers at all times -- a row's slot is
 // refilled as soon as it is consumed -- so a tenth of the usual threads keep HBM busy and no time chunks, which read the
 // inputs twice, are needed.
-constexpr int kDeepRows = 16;
+template <int U>
 __global__ void __launch_bounds__(64) scan_states_deep(const float* a, const float* b, const float* __restrict__ h0,
                                                        float* h, float* __restrict__ last, ScanGeom g) {
-    constexpr int U = kDeepRows;
     const size_t gid = (size_t)blockIdx.x * 64 + threadIdx.x;
     if (gid >= g.total) return;
     const Item it = decode(g, gid);
@@ -296,15 +294,17 @@ int32_t run_scan(pssa_b200_ctx* ctx, const float* a, const float* b, const float
     g.total = lanes * g.n_chunks * g.cvecs;
     if constexpr (V == 4 && !MAPS) {
         const size_t items = lanes * g.cvecs;
-        static const char* e = getenv("DEEP");
-        const size_t lo = e ? atoi(e) : 8192;
-        // (h may be b itself: a row is read before it is written, by the same thread)
-        if (forced_chunks <= 0 && items >= lo && items < 49152 && len >= 4 * kDeepRows) {
+        // Thousands of channel vectors: at 49152 the ordinary pass fills HBM without chunks, below 5120 even 24 rows a thread
+        // do not. Us, chunks against this pass: 12288 vectors x 8191 rows 1275 -> 825, 24576 x 4096 1273 -> 755,
+        // 36864 x 2048 960 -> 572, 8192 x 4096 437 -> 357.
+        if (forced_chunks <= 0 && items >= 5120 && items < 49152 && len >= 64) {
             g.n_chunks = 1, g.chunk_len = (unsigned)len, g.total = items;
-            scan_states_deep<<<(unsigned)((items + 63) / 64), 64, 0, ctx->stream>>>(a, b, h0, out_b, last, g);
+            const unsigned blocks = (unsigned)((items + 63) / 64);
+            if (items < 20480) scan_states_deep<24><<<blocks, 64, 0, ctx->stream>>>(a, b, h0, out_b, last, g);
+            else scan_states_deep<16><<<blocks, 64, 0, ctx->stream>>>(a, b, h0, out_b, last, g);
             return after_launch(ctx, "scan_states_deep");
         }
-        if (forced_chunks <= 0 && e && items >= 49152) g.n_chunks = 1, g.chunk_len = (unsigned)len, g.total = items;
+        if (forced_chunks <= 0 && items >= 49152) g.n_chunks = 1, g.chunk_len = (unsigned)len, g.total = items;
     }
     constexpr int U = MAPS ? 4 : 4;
     const int threads = 128;
