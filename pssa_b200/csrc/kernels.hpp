@@ -52,6 +52,9 @@ struct SsmParams {
 int32_t launch_ssm_fused(pssa_b200_ctx* ctx, const SsmParams& p, bool exact);
 // into how many consecutive time chunks each lane of this call is best cut (1 = a single pass); needs max_len and rows
 size_t ssm_time_chunks(const pssa_b200_ctx* ctx, const SsmParams& p, bool exact);
+constexpr int kMaxTimeChunks = 37;
+// a call with sum_delta set: true = every word of the maps is written, false = the end states must be zero beforehand
+bool ssm_writes_maps(const SsmParams& p, bool exact);
 // 16-byte staging and stores need 16-byte aligned bases and row pitches / widths that are multiples of 4 floats
 inline bool ssm_vector_ok(const SsmParams& p) {
     auto al = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };

@@ -6,6 +6,7 @@
 
 #include "bounds.hpp"
 #include "context.hpp"
+#include "host_io.hpp"
 #include "device_math.cuh"
 #include "kernels.hpp"
 #include "model.hpp"
@@ -341,9 +342,7 @@ int32_t pssa_b200_model_get_state(pssa_b200_model* m, uint32_t stream, float* ou
     if (stream >= m->max_streams || len != n)
         return fail(m->ctx, PSSA_B200_ERR_SHAPE, "recurrent state: stream %u of %u, length %zu, expected %zu", stream, m->max_streams, len, n);
     PSSA_CUDA(m->ctx, cudaSetDevice(m->ctx->device));
-    PSSA_CUDA(m->ctx, cudaMemcpyAsync(out, m->state + (size_t)stream * n, n * 4, cudaMemcpyDeviceToHost, m->ctx->stream));
-    PSSA_CUDA(m->ctx, cudaStreamSynchronize(m->ctx->stream));
-    return PSSA_B200_OK;
+    return copy_to_host(m->ctx, out, m->state + (size_t)stream * n, n * 4);
 }
 
 int32_t pssa_b200_model_set_state(pssa_b200_model* m, uint32_t stream, const float* data, size_t len) {

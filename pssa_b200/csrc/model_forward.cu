@@ -348,12 +348,12 @@ int32_t forward_rows(pssa_b200_model* m, size_t rows, size_t lanes, const uint32
             // pass 1: every chunk's affine map (sum of delta, end state from a zero carry), one record per virtual lane
             const size_t rec = (size_t)d + ds;
             float* records = m->sp.active ? m->sp.send : m->chunks.records;
-            PSSA_CUDA(ctx, cudaMemsetAsync(records, 0, vlanes * rec * sizeof(float), ctx->stream));
             SsmParams ag = sp;
             ag.offsets = m->chunks.off, ag.lengths = m->chunks.len, ag.lanes = (int)vlanes, ag.max_len = chunk_len, ag.tiled = 1;
             ag.carry = records + d, ag.carry_stride = rec, ag.lane_slots = nullptr;
             ag.sum_delta = records, ag.sum_delta_stride = rec;
             ag.y_bf16 = nullptr, ag.single_token = 0;  // y of this pass is scratch: the real pass below overwrites it
+            if (!ssm_writes_maps(ag, exact)) PSSA_CUDA(ctx, cudaMemsetAsync(records, 0, vlanes * rec * sizeof(float), ctx->stream));
             if ((rc = launch_ssm_fused(ctx, ag, exact))) return rc;
             const float* gathered = records;
             int world = 1, rank = 0;
@@ -1116,7 +1116,7 @@ int32_t pssa_b200_model_reserve(pssa_b200_model* m, size_t rows, size_t lanes) {
     PSSA_CUDA(ctx, cudaSetDevice(ctx->device));
     int32_t rc;
     if ((rc = ensure_workspace(m, std::min(rows, m->max_rows), lanes))) return rc;
-    if ((rc = ensure_chunks(m, lanes * 16))) return rc;  // the most time chunks a lane is ever cut into
+    if ((rc = ensure_chunks(m, std::max(lanes * 16, std::min<size_t>(lanes, 16) * kMaxTimeChunks)))) return rc;  // the most time chunks lanes are ever cut into
     return ensure_sampler(m, lanes);
 }
 

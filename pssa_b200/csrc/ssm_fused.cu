@@ -133,7 +133,9 @@ __device__ __forceinline__ f32x2 exp2_approx2(f32x2 x) {
     return pack2(ex2_approx(x0), ex2_approx(x1));
 }
 
-template <int ST, int G, bool EXACT, bool TAPE, int THR = kThreads, int CPT = 1>
+// MAPS: the first of the two passes over time chunks. It leaves every chunk's affine map at `sum_delta` (sum of delta, then the
+// end state from a zero carry) and no y: what would form and store it, a third of the instructions, is not in it.
+template <int ST, int G, bool EXACT, bool TAPE, int THR = kThreads, int CPT = 1, bool MAPS = false>
 __global__ void __launch_bounds__(THR, (ST <= 16 && !TAPE && !EXACT) ? ((THR > 256 || CPT > 1) ? 2 : kMinCtasFast) : 1) ssm_fused_kernel(SsmParams p) {
     // CPT channels per thread (fast mode without tape only): a token's B and C rows are loaded once for both channels and
     // the two recurrences are independent instruction streams, so a warp-token of twice the work takes fewer than twice
@@ -169,8 +171,8 @@ __global__ void __launch_bounds__(THR, (ST <= 16 && !TAPE && !EXACT) ? ((THR > 2
     const int j0 = g * ST;
     const size_t ldd = p.ld_delta ? p.ld_delta : (size_t)d;
     const size_t ldbc = p.ld_bc ? p.ld_bc : (size_t)s;
-    float* carry = p.carry ? p.carry + (size_t)(p.lane_slots ? p.lane_slots[lane] : lane) * (p.carry_stride ? p.carry_stride : ds)
-                           : nullptr;
+    float* carry = p.carry && !MAPS ? p.carry + (size_t)(p.lane_slots ? p.lane_slots[lane] : lane) * (p.carry_stride ? p.carry_stride : ds)
+                                    : nullptr;
 
     float A[ST], h[ST];
     float A1[CPT > 1 ? ST : 1], h1[CPT > 1 ? ST : 1];  // the second channel of a two-channel thread
@@ -206,6 +208,8 @@ __global__ void __launch_bounds__(THR, (ST <= 16 && !TAPE && !EXACT) ? ((THR > 2
     };
     load_state(A, h, i, valid);
     if constexpr (CPT > 1) load_state(A1, h1, i1, valid1);
+    float sum_t = 0.0f, sum_t1 = 0.0f;  // MAPS: delta summed over the tile, and over the chunk in f64
+    double sum_d = 0.0, sum_d1 = 0.0;
 
     const int ntiles = (len + kTileTokens - 1) / kTileTokens;
 
@@ -297,7 +301,8 @@ __global__ void __launch_bounds__(THR, (ST <= 16 && !TAPE && !EXACT) ? ((THR > 2
 #pragma unroll
             for (int q = 0; q < ST / 4; ++q) {
                 float4 vb = *reinterpret_cast<const float4*>(db + tt * SP + q * 4);
-                float4 vc = *reinterpret_cast<const float4*>(dc + tt * SP + q * 4);
+                float4 vc = make_float4(0.f, 0.f, 0.f, 0.f);
+                if constexpr (!MAPS) vc = *reinterpret_cast<const float4*>(dc + tt * SP + q * 4);
                 bj[q * 4] = vb.x, bj[q * 4 + 1] = vb.y, bj[q * 4 + 2] = vb.z, bj[q * 4 + 3] = vb.w;
                 cj[q * 4] = vc.x, cj[q * 4 + 1] = vc.y, cj[q * 4 + 2] = vc.z, cj[q * 4 + 3] = vc.w;
             }
@@ -324,18 +329,19 @@ __global__ void __launch_bounds__(THR, (ST <= 16 && !TAPE && !EXACT) ? ((THR > 2
                     const f32x2 b2 = pack2(bj[jj], bj[jj + 1]), c2 = pack2(cj[jj], cj[jj + 1]);
                     // one pair of exponentials in eight goes to the FMA pipe (the benchmark's launch: 960 us with none, 925 with
                     // one, 1039 with two, whose extra issue slots cost more than the XU pipe gains)
-                    const bool poly = ST == 16 && G == 4 && !TAPE && jj == 0;
+                    // (the map pass, which has no y to form, takes two)
+                    const bool poly = ST == 16 && G == 4 && !TAPE && (jj == 0 || (MAPS && jj == 8));
                     const f32x2 arg = mul2(dl2, pack2(A[jj], A[jj + 1]));
                     const f32x2 a2 = poly ? exp2_poly2(arg) : exp2_approx2(arg);
                     f32x2 h2 = fma2(a2, pack2(h[jj], h[jj + 1]), mul2(w2, b2));
                     unpack2(h2, h[jj], h[jj + 1]);
-                    y2 = fma2(h2, c2, y2);
+                    if constexpr (!MAPS) y2 = fma2(h2, c2, y2);
                     if (TAPE) unpack2(a2, av[jj], av[jj + 1]), bv[jj] = dl * bj[jj], bv[jj + 1] = dl * bj[jj + 1];
                     if constexpr (CPT > 1) {
                         const f32x2 argb = mul2(dlb2, pack2(A1[jj], A1[jj + 1]));
                         f32x2 hb2 = fma2(poly ? exp2_poly2(argb) : exp2_approx2(argb), pack2(h1[jj], h1[jj + 1]), mul2(wb2, b2));
                         unpack2(hb2, h1[jj], h1[jj + 1]);
-                        yb2 = fma2(hb2, c2, yb2);
+                        if constexpr (!MAPS) yb2 = fma2(hb2, c2, yb2);
                     }
                 }
                 float y_lo, y_hi;
@@ -345,6 +351,10 @@ __global__ void __launch_bounds__(THR, (ST <= 16 && !TAPE && !EXACT) ? ((THR > 2
                     unpack2(yb2, y_lo, y_hi);
                     ypb = y_lo + y_hi;
                 }
+            }
+            if constexpr (MAPS) {
+                sum_t += dl, sum_t1 += dlb;
+                return;
             }
 #pragma unroll
             for (int m = LPG; m < 32; m <<= 1) yp += __shfl_xor_sync(0xffffffffu, yp, m);
@@ -372,6 +382,10 @@ __global__ void __launch_bounds__(THR, (ST <= 16 && !TAPE && !EXACT) ? ((THR > 2
             for (int tt = 0; tt < kTileTokens; ++tt) token(tt);
         } else {
             for (int tt = 0; tt < nt; ++tt) token(tt);
+        }
+        if constexpr (MAPS) {
+            sum_d += (double)sum_t, sum_d1 += (double)sum_t1, sum_t = sum_t1 = 0.0f;
+            continue;
         }
         __syncthreads();
         // write the tile's y rows out together: 16-byte stores instead of one predicated scalar store per token
@@ -405,6 +419,19 @@ __global__ void __launch_bounds__(THR, (ST <= 16 && !TAPE && !EXACT) ? ((THR > 2
         }
     }
     cp_async_wait<0>();
+    if constexpr (MAPS) {
+        float* rec = p.sum_delta + (size_t)lane * p.sum_delta_stride;
+        auto store_map = [&](const float* hv, int ch, bool ok_ch, double sum) {
+            if (g == 0 && ok_ch) rec[ch] = (float)sum;
+#pragma unroll
+            for (int q = 0; q < ST / 4; ++q)
+                if (ok_ch && j0 + q * 4 < s)
+                    *(reinterpret_cast<float4*>(rec + d + (size_t)ch * s + j0) + q) = make_float4(hv[q * 4], hv[q * 4 + 1], hv[q * 4 + 2], hv[q * 4 + 3]);
+        };
+        store_map(h, i, valid, sum_d);
+        if constexpr (CPT > 1) store_map(h1, i1, valid1, sum_d1);
+        return;
+    }
     if (carry && len > 0) {
         auto store_state = [&](const float* hv, int ch, bool ok_ch) {
             if (vec_state) {
@@ -882,6 +909,8 @@ __global__ void __launch_bounds__(256) seqpar_fold_kernel(const float* __restric
                                                           float* __restrict__ state, size_t state_stride,
                                                           const uint32_t* __restrict__ lane_slots, float* __restrict__ carry_in,
                                                           int d, int s) {
+    pdl_trigger();
+    pdl_wait();
     const size_t ds = (size_t)d * s;
     const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = blockIdx.y;
@@ -890,13 +919,14 @@ __global__ void __launch_bounds__(256) seqpar_fold_kernel(const float* __restric
     float* st = state + (size_t)(lane_slots ? lane_slots[lane] : lane) * state_stride;
     const float a = rates[e];
     float h = st[e];
-    // the records are independent of h: four of them are requested (and their decay factors formed) before the
+    // the records are independent of h: twelve of them are requested (and their decay factors formed) before the
     // dependent multiply-adds, so the walk is not one memory round trip per record
+    constexpr int U = 12;
     const int n = world * chunks;
-    for (int j0 = 0; j0 < n; j0 += 4) {
-        float pk[4], add[4];
+    for (int j0 = 0; j0 < n; j0 += U) {
+        float pk[U], add[U];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < U; ++u) {
             const int j = j0 + u;
             if (j < n) {
                 const int k = j / chunks, c = j - k * chunks;
@@ -906,7 +936,7 @@ __global__ void __launch_bounds__(256) seqpar_fold_kernel(const float* __restric
             }
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < U; ++u) {
             const int j = j0 + u;
             if (j < n) {
                 const int k = j / chunks, c = j - k * chunks;
@@ -918,14 +948,14 @@ __global__ void __launch_bounds__(256) seqpar_fold_kernel(const float* __restric
     st[e] = h;
 }
 
-template <int ST, int G, bool EXACT, bool TAPE, int THR = kThreads, int CPT = 1>
+template <int ST, int G, bool EXACT, bool TAPE, int THR = kThreads, int CPT = 1, bool MAPS = false>
 int32_t launch_cfg(pssa_b200_ctx* ctx, const SsmParams& p) {
     constexpr int kThreads = THR;
     constexpr int CH = kThreads / G * CPT;
     constexpr int SP = (ST + 4) * G;
     constexpr int kTileTokens = kTileTokensFor<G>;
     size_t smem = (size_t)kStages * kTileTokens * (2 * CH + 2 * SP) * sizeof(float);
-    auto kern = ssm_fused_kernel<ST, G, EXACT, TAPE, THR, CPT>;
+    auto kern = ssm_fused_kernel<ST, G, EXACT, TAPE, THR, CPT, MAPS>;
     static PerDeviceOnce attr_set;  // per instantiation and per device
     if (smem > 48 * 1024 && attr_set.need(ctx->device)) {
         PSSA_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -936,7 +966,7 @@ int32_t launch_cfg(pssa_b200_ctx* ctx, const SsmParams& p) {
     if (blocks > 0x7fffffffull)
         return fail(ctx, PSSA_B200_ERR_SHAPE, "B200 SSM grid (%zu, 1) exceeds grid limits; refusing launch", blocks);
     PSSA_CUDA(ctx, launch_dependent(kern, dim3((unsigned)blocks), dim3(kThreads), smem, ctx->stream, p));
-    return after_launch(ctx, "ssm_fused_kernel");
+    return after_launch(ctx, MAPS ? "ssm_fused_kernel[chunk maps]" : "ssm_fused_kernel");
 }
 
 template <int LPC, int SPL, int TT, bool EXACT, bool TAPE>
@@ -1014,23 +1044,38 @@ int32_t launch_seqpar_fold(pssa_b200_ctx* ctx, const float* gathered, size_t rec
     const size_t ds = (size_t)d * s;
     dim3 grid((unsigned)((ds + 255) / 256), (unsigned)lanes);
     if (lanes < 1 || lanes > 65535) return fail(ctx, PSSA_B200_ERR_SHAPE, "chunk fold: %d lanes outside 1..65535", lanes);
-    seqpar_fold_kernel<<<grid, 256, 0, ctx->stream>>>(gathered, rec, world, rank, chunks, rank_stride, rates, state, state_stride,
-                                                     lane_slots, carry_in, d, s);
+    PSSA_CUDA(ctx, launch_dependent(seqpar_fold_kernel, grid, dim3(256), 0, ctx->stream, gathered, rec, world, rank, chunks, rank_stride, rates, state,
+                                    state_stride, lane_slots, carry_in, d, s));
     return after_launch(ctx, "seqpar_fold_kernel");
 }
 
 size_t ssm_time_chunks(const pssa_b200_ctx* ctx, const SsmParams& p, bool exact) {
-    const size_t longest = (size_t)p.max_len, ctas = (size_t)p.lanes * ((p.d + 63) / 64);
+    const size_t longest = (size_t)p.max_len, ctas = (size_t)p.lanes * ((p.d + 63) / 64), schedulers = 4 * (size_t)ctx->sm_count;
     // Two passes pay every exponential twice. Where the few-lanes kernel applies they are the faster way only for a long
-    // sequence that leaves it under one and a half channels a scheduler (us, d 768, 64 states, one sequence: 2048 tokens 94
-    // in one pass, about 90 in two; 8192 tokens 357 and 326).
-    if (ssm_wide_ok(p) && (p.s < 64 || longest < (exact ? 4096 : 2048) || 2 * p.rows * (size_t)p.d > 3 * longest * 4 * (size_t)ctx->sm_count)) return 1;
+    // sequence that leaves it at few channels a scheduler.
+    if (ssm_wide_ok(p)) {
+        if (exact || p.s < 64) {
+            if (!exact || longest < 4096 || 2 * p.rows * (size_t)p.d > 3 * longest * schedulers) return 1;
+        } else {
+            // CTAs of 64 channels, three to an SM. Us per pass of the 12-block model, few lanes against this: 1 lane of 1024 tokens
+            // 1888 and 2047, 2048 2825 -> 2550, 8192 7749 -> 5050; 2 lanes of 2048 3149 and 3543, 4096 4880 and 5355.
+            const size_t n = std::min<size_t>({(size_t)kMaxTimeChunks, 3 * (size_t)ctx->sm_count / std::max<size_t>(1, ctas), longest / 64});
+            return longest >= 2048 && n >= 30 ? n : 1;
+        }
+    }
     if (ctas > (size_t)ctx->sm_count) return 1;
-    return std::min({(size_t)16, std::max<size_t>(1, 4 * (size_t)ctx->sm_count / ctas), std::max<size_t>(1, longest / 128)});
+    return std::min({(size_t)16, std::max<size_t>(1, schedulers / ctas), std::max<size_t>(1, longest / 128)});
+}
+
+bool ssm_writes_maps(const SsmParams& p, bool exact) {
+    return p.sum_delta && !exact && p.s > 32 && p.s <= 64 && p.aligned && p.offsets && p.lengths && (reinterpret_cast<uintptr_t>(p.rates) & 15) == 0 &&
+           (reinterpret_cast<uintptr_t>(p.sum_delta) & 15) == 0 && p.sum_delta_stride % 4 == 0 && p.carry == p.sum_delta + p.d &&
+           p.carry_stride == p.sum_delta_stride;
 }
 
 int32_t launch_ssm_fused(pssa_b200_ctx* ctx, const SsmParams& p, bool exact) {
     const int s = p.s;
+    if (ssm_writes_maps(p, exact)) return launch_cfg<16, 4, false, false, 128, 2, true>(ctx, p);
     if (p.sum_delta) {
         if (!p.offsets || !p.lengths) return fail(ctx, PSSA_B200_ERR_INVALID_ARGUMENT, "B200 SSM: sum_delta needs lane offsets and lengths");
         if (p.lanes > 65535) return fail(ctx, PSSA_B200_ERR_SHAPE, "B200 SSM: sum_delta supports at most 65535 lanes; refusing launch");
