@@ -21,7 +21,9 @@
 namespace pssa {
 namespace {
 
-constexpr int kSampleThreads = 1024;  // a row's passes over the vocabulary are one CTA's: its loads in flight are what bounds them
+// A row's passes over the vocabulary are one CTA's, bounded by its loads in flight: 256 -> 1024 threads, and the sums as trees.
+// 16 rows of 16384 ids with 64 recent ones: 167 -> 62 us.
+constexpr int kSampleThreads = 1024;
 constexpr int kRecent = 64;
 
 __device__ __forceinline__ int order_key(float v) {  // monotone signed key of f32::total_cmp

@@ -31,6 +31,19 @@ def test_exact_gemm_is_dot_slice_bit_for_bit(gpu, k):
     assert np.array_equal(bits(got), bits(O.gemm_xwt(x, w)))
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 33, 768), (4, 5, 40), (5, 2, 24), (16, 31, 777), (17, 36, 96), (130, 77, 200), (700, 260, 64)])
+def test_exact_gemm_tiles_are_dot_slice_bit_for_bit(gpu, m, n, k):
+    """Row counts on both sides of every tile shape of the exact product, and the read-modify-write epilogue."""
+    from pssa_b200 import _native as N
+    rng = np.random.default_rng(m + n)
+    x, w = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((n, k)).astype(np.float32)
+    got = gpu.dispatch_gemm(x, w, m, n, k, 1).reshape(m, n)
+    want = O.gemm_xwt(x, w)
+    assert np.array_equal(bits(got), bits(want))
+    gpu.dispatch_gemm_into(x, w, m, n, k, 1, got.reshape(-1), epilogue=N.EPI_ADD_OUT)
+    assert np.array_equal(bits(got), bits(want + want))
+
+
 def test_batch_folds_into_rows_and_bad_lengths_leave_output_untouched(gpu):
     # tests/backend.rs:9-82
     import pssa_b200

@@ -36,6 +36,17 @@ def test_states_single_chunk_is_bit_identical_to_the_ordered_recurrence(gpu, T, 
     assert np.array_equal(last.view(np.uint32), ref[:, -1].view(np.uint32))
 
 
+@pytest.mark.parametrize("lanes,T,stride", [(1, 64, 20480), (1, 97, 20484), (3, 71, 27300), (2, 65, 40964), (1, 66, 196604), (1, 65, 196608)])
+def test_thousands_of_channels_take_one_pass(gpu, lanes, T, stride):
+    """Channel counts on both sides of the deep single pass and of its two row depths: one pass, so the bits are the recurrence's."""
+    a, b, h0 = make(lanes, T, stride, T + stride)
+    gpu.set_scan_chunks(0)
+    h, last = gpu.scan_states(a, b, h0, want_last=True)
+    ref = O.scan_states(a, b, h0)
+    assert np.array_equal(h.view(np.uint32), ref.view(np.uint32))
+    assert np.array_equal(last.view(np.uint32), ref[:, -1].view(np.uint32))
+
+
 @pytest.mark.parametrize("chunks", [2, 3, 7, 64])
 @pytest.mark.parametrize("T,stride", [(2, 4), (33, 5), (257, 12), (1024, 64), (4096, 8)])
 def test_states_chunked_passes_match_within_tolerance(gpu, chunks, T, stride):
