@@ -548,6 +548,20 @@ int32_t check_shape(pssa_b200_ctx* ctx, const void* a, const void* b, size_t M, 
     return PSSA_B200_OK;
 }
 
+// The block schedule's products with 64- and 128-wide tiles: one epilogue family and one output set per instantiation here too. The
+// run-time-mode kernel these sizes used carries every family, and with one or two tiles a CTA the fetch of that code was a
+// good part of the launch.
+template <int BN, int STAGES>
+int32_t launch_mid(pssa_b200_ctx* ctx, const void* a, const void* b, const GemmEpilogue& e, bool only32, bool only16) {
+    if (e.epi == -1 && only32) return launch_tile<BN, STAGES, -1, 1>(ctx, a, b, e);
+    if (e.epi == EPI_GATE && only16) return launch_tile<BN, STAGES, EPI_GATE, 2>(ctx, a, b, e);
+    if (e.epi == EPI_SILU && only16) return launch_tile<BN, STAGES, EPI_SILU, 2>(ctx, a, b, e);
+    if (e.epi == EPI_RESIDUAL && only32) return launch_tile<BN, STAGES, EPI_RESIDUAL, 1>(ctx, a, b, e);
+    if (e.epi == EPI_ADD_OUT && only32 && e.n_pairs == 0) return launch_tile<BN, STAGES, EPI_ADD_OUT, 1>(ctx, a, b, e);
+    if (e.epi == EPI_SCALE && only32) return launch_tile<BN, STAGES, EPI_SCALE, 1>(ctx, a, b, e);
+    return launch_tile<BN, STAGES>(ctx, a, b, e);
+}
+
 int32_t dispatch(pssa_b200_ctx* ctx, const void* a, const void* b, GemmEpilogue& e) {
     e.status = ctx->status_dev;
     // widest tile that still gives every SM work: 256 columns halve the shared-memory operand traffic per flop,
@@ -567,10 +581,12 @@ int32_t dispatch(pssa_b200_ctx* ctx, const void* a, const void* b, GemmEpilogue&
         if (e.epi == EPI_RESIDUAL && only32) return launch_tile<32, 10, EPI_RESIDUAL, 1, 4>(ctx, a, b, e);
         return launch_tile<32, 10, kRuntimeMode, 0, 4>(ctx, a, b, e);
     }
-    if (e.N <= 64 || m_tiles * ((e.N + 127) / 128) < ctx->sm_count / 2)
-        return (e.epi == EPI_ADD_OUT && e.out && !e.out16 && e.n_pairs == 0) ? launch_tile<64, 7, EPI_ADD_OUT, 1>(ctx, a, b, e)
-                                                                            : launch_tile<64, 7>(ctx, a, b, e);
-    if (e.N <= 128 || m_tiles * ((e.N + 255) / 256) < ctx->sm_count) return launch_tile<128, 5>(ctx, a, b, e);
+    if (e.N <= 64 || m_tiles * ((e.N + 127) / 128) < ctx->sm_count / 2) return launch_mid<64, 7>(ctx, a, b, e, only32, only16);
+    // 128-wide tiles below one tile an SM, and up to four waves where they end sooner: 8192 rows of a 768-wide product are 192
+    // tiles of 256 columns, two rounds of which the second is a third full, or 384 of 128, three rounds of half the length
+    const long long t256 = m_tiles * ((e.N + 255) / 256), t128 = m_tiles * ((e.N + 127) / 128), sms = ctx->sm_count;
+    const bool shorter = e.n_pairs <= 1 && t256 <= 4 * sms && ((t128 + sms - 1) / sms) * 13 < ((t256 + sms - 1) / sms) * 20;
+    if (e.N <= 128 || t256 < sms || shorter) return launch_mid<128, 5>(ctx, a, b, e, only32, only16);
     // Four 48 KB stages: with three, the issuing thread of the K = 768 products spent 56 % of its cycles waiting for
     // operands (cycle counters around its two waits, 32 x 2048-token lanes) and 40 % with four (its loop 8-14 % shorter);
     // what then limits these products is the epilogue (its warps wait for an accumulator 9 % of the time). The gated
