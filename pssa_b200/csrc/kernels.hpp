@@ -222,7 +222,8 @@ int32_t launch_gemm_bf16_cat(pssa_b200_ctx* ctx, const void* x16, const void* w1
                              size_t ldo, int c1, int c2, int c3, void* side_a = nullptr, size_t ld_side_a = 0, void* side_b = nullptr,
                              size_t ld_side_b = 0);
 
-// step_decode.cu: one token per row through every block and the vocabulary head in one cooperative launch (bf16 mode)
+// step_decode.cu, step_schedule.cu: one token per row through every block and the vocabulary head (bf16 mode), in one cooperative
+// launch or, for many rows, in a launch per stage. A row's bits do not depend on the number of rows.
 struct StepLaunch {
     int rows, d, s, k, cap, nc, off_b, off_q, off_gate, off_act;
     size_t depth;
@@ -245,9 +246,9 @@ struct StepLaunch {
     };
     const Block* blocks;
 };
-bool step_rows_ok(size_t rows);
 bool step_shape_ok(size_t depth, size_t d, size_t s, size_t k, size_t cap, size_t rank);
 int32_t launch_decode_step(pssa_b200_ctx* ctx, const StepLaunch& p);
+int32_t launch_step_schedule(pssa_b200_ctx* ctx, const StepLaunch& p);
 int32_t launch_keys_by_quad(pssa_b200_ctx* ctx, const float* keys, float* out, int cap, int k);
 
 // elementwise.cu

@@ -53,7 +53,7 @@ struct DeviceBlock {
 struct Workspace {
     size_t rows = 0, lanes = 0;
     uint32_t *ids = nullptr, *lane_off = nullptr, *lane_len = nullptr, *lane_slot = nullptr, *last_rows = nullptr,
-             *greedy = nullptr;
+             *greedy = nullptr, *row_slot = nullptr;  // row_slot: stream of each row of a decode step
     float* feat_c = nullptr;  // Ouro passes only: a block's input features, kept for its depth residual
     float *feat_a = nullptr, *feat_b = nullptr, *x_norm = nullptr, *proj = nullptr, *y = nullptr, *weights = nullptr,
           *m_val = nullptr, *m_proj = nullptr, *z = nullptr, *mlp_act = nullptr, *last_feat = nullptr, *logits = nullptr;
@@ -139,7 +139,7 @@ struct pssa_b200_model {
         float* carry_in = nullptr;  // [capacity][d*s]
     } chunks;
     // decode step in one kernel (step_decode.cu): the banks' keys by quads [depth][k * cap], the barrier word and the step's own
-    // scratch, sized for `rows` streams
+    // scratch, sized for `rows` streams of one pass
     struct Step {
         float* keys_t = nullptr;
         void* barrier = nullptr;

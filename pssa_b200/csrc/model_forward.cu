@@ -32,7 +32,7 @@ int32_t ensure_workspace(pssa_b200_model* m, size_t rows, size_t lanes) {
     const size_t d = m->d, f = sizeof(float);
     Carver c;
     size_t o_ids = c.take(rows * 4), o_off = c.take(lanes * 4), o_len = c.take(lanes * 4), o_slot = c.take(lanes * 4),
-           o_last = c.take(lanes * 4), o_greedy = c.take(lanes * 4);
+           o_last = c.take(lanes * 4), o_greedy = c.take(lanes * 4), o_rslot = c.take(lanes * 4);
     size_t o_fc = c.take(m->loops > 1 ? rows * d * f : 0);
     size_t o_fa = c.take(rows * d * f), o_fb = c.take(rows * d * f), o_xn = c.take(rows * d * f),
            o_proj = c.take(rows * m->ncat * f), o_y = c.take(rows * d * f), o_w = c.take(rows * m->cap * f),
@@ -56,6 +56,7 @@ int32_t ensure_workspace(pssa_b200_model* m, size_t rows, size_t lanes) {
     char* b = ws.base;
     ws.ids = (uint32_t*)(b + o_ids), ws.lane_off = (uint32_t*)(b + o_off), ws.lane_len = (uint32_t*)(b + o_len);
     ws.lane_slot = (uint32_t*)(b + o_slot), ws.last_rows = (uint32_t*)(b + o_last), ws.greedy = (uint32_t*)(b + o_greedy);
+    ws.row_slot = (uint32_t*)(b + o_rslot);
     ws.feat_c = m->loops > 1 ? (float*)(b + o_fc) : nullptr;
     ws.feat_a = (float*)(b + o_fa), ws.feat_b = (float*)(b + o_fb), ws.x_norm = (float*)(b + o_xn);
     ws.proj = (float*)(b + o_proj), ws.y = (float*)(b + o_y), ws.weights = (float*)(b + o_w), ws.m_val = (float*)(b + o_mv);
@@ -521,28 +522,30 @@ int32_t head_rows(pssa_b200_model* m, const float* feats, size_t n_heads, bool w
     return PSSA_B200_OK;
 }
 
-// One token per lane, every lane present and in row order, in the bf16 mode: the whole step is one kernel (step_decode.cu).
-// Up to 128 lanes (step_rows_ok) every sum has one order whatever the number of lanes: a stream's bits are the same alone and
-// in any such batch, and the same in any larger one.
+// A decode step of the bf16 mode -- no lane longer than one token -- is its own schedule (step_decode.cu, step_schedule.cu). What
+// selects it are the model and the lanes' lengths, never their number: a stream's bits are the same alone, in any batch,
+// beside idle lanes and in a shard of the batch on another GPU. (The observer wants rows that this schedule never forms.)
 bool step_model_ok(const pssa_b200_model* m) {
     return m->precision == PSSA_B200_PRECISION_BF16 && m->loops == 1 && step_shape_ok(m->depth, m->d, m->s, m->k, m->cap, m->rank) &&
            1.0f / m->cfg.tau_mem < 3.0e38f;
 }
-bool decode_step_fused(const pssa_b200_model* m, size_t rows, size_t lanes, const uint32_t* h_off, const uint32_t* h_len) {
-    if (rows != lanes || !step_rows_ok(rows) || m->sp.active || m->obs.enabled || !step_model_ok(m)) return false;
+bool is_decode_step(const pssa_b200_model* m, size_t lanes, const uint32_t* h_len) {
+    if (m->sp.active || m->obs.enabled || !step_model_ok(m)) return false;
     for (auto& b : m->blocks)
         if (b.count == 0 || (m->top_k != 0 && m->top_k < b.count)) return false;
     for (size_t l = 0; l < lanes; ++l)
-        if (h_len[l] != 1 || h_off[l] != l) return false;
+        if (h_len[l] > 1) return false;
     return true;
 }
 
-// What a decode step keeps: called by every forward pass of a model that can take it, so that the first step of a stream
-// that has just read its prompt does not stop for allocations.
+// What a decode step keeps, and the scratch of up to kStepSlice rows of it: called by every forward pass of a model that can take
+// it, so that the first step of a stream that has just read its prompt does not stop for allocations.
+constexpr size_t kStepSlice = 2048;
 int32_t ensure_step(pssa_b200_model* m, size_t rows) {
     pssa_b200_ctx* ctx = m->ctx;
     auto& st = m->step;
     int32_t rc;
+    rows = std::min(rows, kStepSlice);
     if (!st.keys_t) {
         PSSA_CUDA(ctx, cudaMalloc((void**)&st.keys_t, m->depth * m->k * m->cap * sizeof(float)));
         PSSA_CUDA(ctx, cudaMalloc(&st.barrier, 256));
@@ -564,7 +567,7 @@ int32_t ensure_step(pssa_b200_model* m, size_t rows) {
     return PSSA_B200_OK;
 }
 
-// logits [rows, vocab] (null: not wanted); ids is a device array
+// logits [rows, vocab] (null: not wanted); ids [rows] is a device array, ws.row_slot [rows] holds the rows' streams
 int32_t run_decode_step(pssa_b200_model* m, size_t rows, const uint32_t* ids, float* logits) {
     pssa_b200_ctx* ctx = m->ctx;
     Workspace& ws = m->ws;
@@ -579,15 +582,20 @@ int32_t run_decode_step(pssa_b200_model* m, size_t rows, const uint32_t* ids, fl
                      st.keys_t + l * m->k * m->cap, b.w[T_BANK_NORM_SQ], m->state + l * ds, l == 0 ? 1.0f : m->residual_scales[l - 1], (int)b.count};
     }
     StepLaunch p{};
-    p.rows = (int)rows, p.d = (int)m->d, p.s = (int)m->s, p.k = (int)m->k, p.cap = (int)m->cap, p.nc = (int)m->ncat;
+    p.d = (int)m->d, p.s = (int)m->s, p.k = (int)m->k, p.cap = (int)m->cap, p.nc = (int)m->ncat;
     p.off_b = (int)m->off_b, p.off_q = (int)m->off_q, p.off_gate = (int)m->off_gate, p.off_act = (int)m->off_act;
     p.depth = m->depth, p.vocab = (unsigned)m->v;
     p.ssm_scale = 1.0f / std::sqrt((float)m->s), p.head_scale = 1.0f / std::sqrt((float)m->d), p.tau = m->cfg.tau_mem;
-    p.embed = m->embed, p.ids = ids, p.slots = ws.lane_slot, p.unembed = m->unembed_bf16, p.carry_stride = m->depth * ds;
+    p.embed = m->embed, p.unembed = m->unembed_bf16, p.carry_stride = m->depth * ds;
     p.feat_a = ws.feat_a, p.feat_b = ws.feat_b, p.proj = ws.proj, p.y = ws.y;
     p.qpart = st.scratch, p.ssq = p.qpart + st.rows * (m->d / 8 * m->k), p.inv = p.ssq + st.rows * (m->d / 16);
-    p.logits = logits, p.x = ws.x_bf16, p.w = ws.w_split, p.z = ws.z_bf16, p.act = ws.act_bf16, p.barrier = st.barrier, p.blocks = blocks;
-    return launch_decode_step(ctx, p);
+    p.x = ws.x_bf16, p.w = ws.w_split, p.z = ws.z_bf16, p.act = ws.act_bf16, p.barrier = st.barrier, p.blocks = blocks;
+    for (size_t r0 = 0; r0 < rows; r0 += kStepSlice) {  // rows share nothing: slices keep the scratch small
+        p.rows = (int)std::min(kStepSlice, rows - r0), p.ids = ids + r0, p.slots = ws.row_slot + r0;
+        p.logits = logits ? logits + r0 * m->v : nullptr;
+        if ((rc = launch_decode_step(ctx, p))) return rc;
+    }
+    return PSSA_B200_OK;
 }
 
 // Shared driver: lanes described on the host; processes them in passes of at most max_rows rows.
@@ -635,7 +643,7 @@ int32_t run_lanes(pssa_b200_model* m, const uint64_t* ids, const uint32_t* offse
     // window of tokens per lane per pass
     size_t window = std::max<size_t>(1, m->max_rows / n_lanes);
     if (window > max_len) window = max_len;
-    std::vector<uint32_t> h_ids, h_off(n_lanes), h_len(n_lanes), h_slot(n_lanes), h_last;
+    std::vector<uint32_t> h_ids, h_off(n_lanes), h_len(n_lanes), h_slot(n_lanes), h_row_slot, h_last;
     int32_t rc;
     for (size_t t0 = 0; t0 < max_len; t0 += window) {
         if (cancelled && cancelled(cancel_arg)) return fail(ctx, PSSA_B200_ERR_CANCELLED, "prefill cancelled after %zu tokens", t0);
@@ -662,15 +670,19 @@ int32_t run_lanes(pssa_b200_model* m, const uint64_t* ids, const uint32_t* offse
         cudaStream_t st = ctx->stream;
         m->dev_layout.ws_base = nullptr;  // the cached layout of the device-resident entry no longer holds
         PSSA_CUDA(ctx, cudaMemcpyAsync(ws.ids, h_ids.data(), rows * 4, cudaMemcpyHostToDevice, st));
-        PSSA_CUDA(ctx, cudaMemcpyAsync(ws.lane_off, h_off.data(), n_lanes * 4, cudaMemcpyHostToDevice, st));
-        PSSA_CUDA(ctx, cudaMemcpyAsync(ws.lane_len, h_len.data(), n_lanes * 4, cudaMemcpyHostToDevice, st));
-        PSSA_CUDA(ctx, cudaMemcpyAsync(ws.lane_slot, h_slot.data(), n_lanes * 4, cudaMemcpyHostToDevice, st));
-        if (!h_last.empty()) PSSA_CUDA(ctx, cudaMemcpyAsync(ws.last_rows, h_last.data(), h_last.size() * 4, cudaMemcpyHostToDevice, st));
         float* feats = nullptr;
-        const bool step = decode_step_fused(m, rows, n_lanes, h_off.data(), h_len.data()), want_head = logits || greedy || sampling;
+        const bool step = is_decode_step(m, n_lanes, h_len.data()), want_head = logits || greedy || sampling;
         if (step) {
+            h_row_slot.clear();
+            for (size_t l = 0; l < n_lanes; ++l)
+                if (h_len[l]) h_row_slot.push_back(h_slot[l]);
+            PSSA_CUDA(ctx, cudaMemcpyAsync(ws.row_slot, h_row_slot.data(), rows * 4, cudaMemcpyHostToDevice, st));
             if ((rc = run_decode_step(m, rows, ws.ids, want_head && !h_last.empty() ? ws.logits : nullptr))) return rc;
         } else {
+            PSSA_CUDA(ctx, cudaMemcpyAsync(ws.lane_off, h_off.data(), n_lanes * 4, cudaMemcpyHostToDevice, st));
+            PSSA_CUDA(ctx, cudaMemcpyAsync(ws.lane_len, h_len.data(), n_lanes * 4, cudaMemcpyHostToDevice, st));
+            PSSA_CUDA(ctx, cudaMemcpyAsync(ws.lane_slot, h_slot.data(), n_lanes * 4, cudaMemcpyHostToDevice, st));
+            if (!h_last.empty()) PSSA_CUDA(ctx, cudaMemcpyAsync(ws.last_rows, h_last.data(), h_last.size() * 4, cudaMemcpyHostToDevice, st));
             if (step_model_ok(m) && (rc = ensure_step(m, std::min<size_t>(m->max_streams, 128)))) return rc;
             if ((rc = forward_rows(m, rows, n_lanes, h_off.data(), h_len.data(), &feats, h_last.size()))) return rc;
         }
@@ -767,7 +779,7 @@ int32_t pssa_b200_model_prefill_batch_dev(pssa_b200_model* m, const uint32_t* id
     pssa_b200_ctx* ctx = m->ctx;
     if (n_lanes == 0 || n_lanes > 0x7fffffff) return fail(ctx, PSSA_B200_ERR_SHAPE, "prefill_batch: lane count must be in 1..2^31-1");
     std::vector<bool> seen(m->max_streams, false);
-    std::vector<uint32_t> h_off(n_lanes), h_len(n_lanes), h_slot(n_lanes), h_last;
+    std::vector<uint32_t> h_off(n_lanes), h_len(n_lanes), h_slot(n_lanes), h_row_slot, h_last;
     std::vector<size_t> head_lane;
     size_t rows = 0, span = 0;
     for (size_t l = 0; l < n_lanes; ++l) {
@@ -780,6 +792,7 @@ int32_t pssa_b200_model_prefill_batch_dev(pssa_b200_model* m, const uint32_t* id
         span = std::max(span, (size_t)offsets[l] + lengths[l]);
         if (lengths[l] > 0) {
             h_last.push_back(offsets[l] + lengths[l] - 1);
+            h_row_slot.push_back(slot);
             head_lane.push_back(l);
         }
     }
@@ -793,7 +806,8 @@ int32_t pssa_b200_model_prefill_batch_dev(pssa_b200_model* m, const uint32_t* id
         return fail(ctx, PSSA_B200_ERR_SHAPE, "prefill_batch_dev: %zu token rows exceed one pass of %zu rows (set_max_rows)", span, m->max_rows);
     PSSA_CUDA(ctx, cudaSetDevice(ctx->device));
     int32_t rc;
-    if ((rc = ensure_workspace(m, span, n_lanes))) return rc;
+    const bool step = m->sp.world <= 1 && is_decode_step(m, n_lanes, h_len.data());
+    if ((rc = ensure_workspace(m, step ? std::max(span, rows) : span, n_lanes))) return rc;
     Workspace& ws = m->ws;
     cudaStream_t st = ctx->stream;
     // The lane description is uploaded only when it differs from what the workspace already holds. A repeated call with
@@ -805,16 +819,43 @@ int32_t pssa_b200_model_prefill_batch_dev(pssa_b200_model* m, const uint32_t* id
         PSSA_CUDA(ctx, cudaMemcpyAsync(ws.lane_len, h_len.data(), n_lanes * 4, cudaMemcpyHostToDevice, st));
         PSSA_CUDA(ctx, cudaMemcpyAsync(ws.lane_slot, h_slot.data(), n_lanes * 4, cudaMemcpyHostToDevice, st));
         PSSA_CUDA(ctx, cudaMemcpyAsync(ws.last_rows, h_last.data(), h_last.size() * 4, cudaMemcpyHostToDevice, st));
+        PSSA_CUDA(ctx, cudaMemcpyAsync(ws.row_slot, h_row_slot.data(), h_row_slot.size() * 4, cudaMemcpyHostToDevice, st));
         lay.ws_base = ws.base, lay.off = h_off, lay.len = h_len, lay.slot = h_slot;
     }
     float* feats = nullptr;
-    if (m->sp.world <= 1 && decode_step_fused(m, span, n_lanes, h_off.data(), h_len.data())) {
-        float* out = logits_dev ? logits_dev : ws.logits;
-        if ((rc = run_decode_step(m, span, ids_dev, logits_dev || greedy_dev ? out : nullptr))) return rc;
-        if (greedy_dev) {
-            if ((rc = launch_greedy(ctx, out, ws.greedy, span, (int)m->v))) return rc;
-            PSSA_CUDA(ctx, cudaMemcpyAsync(greedy_dev, ws.greedy, span * 4, cudaMemcpyDeviceToDevice, st));
+    // logits and greedy ids of the rows in ws.logits, to the places of their lanes: contiguous runs of non-empty lanes in one copy
+    auto rows_to_lanes = [&]() -> int32_t {
+        size_t i = 0;
+        while (i < head_lane.size()) {
+            size_t j = i;
+            while (j + 1 < head_lane.size() && head_lane[j + 1] == head_lane[j] + 1) ++j;
+            if (logits_dev)
+                PSSA_CUDA(ctx, cudaMemcpyAsync(logits_dev + head_lane[i] * m->v, ws.logits + i * m->v, (j - i + 1) * m->v * 4,
+                                               cudaMemcpyDeviceToDevice, st));
+            if (greedy_dev)
+                PSSA_CUDA(ctx, cudaMemcpyAsync(greedy_dev + head_lane[i], ws.greedy + i, (j - i + 1) * 4, cudaMemcpyDeviceToDevice, st));
+            i = j + 1;
         }
+        return PSSA_B200_OK;
+    };
+    if (step) {
+        // a row per non-empty lane, in lane order; ids that do not lie that way are brought together
+        const uint32_t* ids = ids_dev;
+        bool in_order = true;
+        for (size_t i = 0; i < rows; ++i) in_order = in_order && h_last[i] == i;
+        if (!in_order) {
+            for (size_t i = 0, j; i < rows; i = j) {
+                for (j = i + 1; j < rows && h_last[j] == h_last[j - 1] + 1; ++j) {}
+                PSSA_CUDA(ctx, cudaMemcpyAsync(ws.ids + i, ids_dev + h_last[i], (j - i) * 4, cudaMemcpyDeviceToDevice, st));
+            }
+            ids = ws.ids;
+        }
+        const bool whole = rows == n_lanes && logits_dev;  // rows are lanes: no copy
+        float* out = whole ? logits_dev : ws.logits;
+        if ((rc = run_decode_step(m, rows, ids, logits_dev || greedy_dev ? out : nullptr))) return rc;
+        if (greedy_dev && (rc = launch_greedy(ctx, out, ws.greedy, rows, (int)m->v))) return rc;
+        if (!whole) return rows_to_lanes();
+        if (greedy_dev) PSSA_CUDA(ctx, cudaMemcpyAsync(greedy_dev, ws.greedy, rows * 4, cudaMemcpyDeviceToDevice, st));
         return PSSA_B200_OK;
     }
     if (step_model_ok(m) && (rc = ensure_step(m, std::min<size_t>(m->max_streams, 128)))) return rc;
@@ -825,17 +866,7 @@ int32_t pssa_b200_model_prefill_batch_dev(pssa_b200_model* m, const uint32_t* id
     if (rc) return rc;
     if (logits_dev || greedy_dev) {
         if ((rc = head_rows(m, feats, h_last.size(), greedy_dev != nullptr))) return rc;
-        size_t i = 0;
-        while (i < head_lane.size()) {  // contiguous runs of non-empty lanes go out in one copy
-            size_t j = i;
-            while (j + 1 < head_lane.size() && head_lane[j + 1] == head_lane[j] + 1) ++j;
-            if (logits_dev)
-                PSSA_CUDA(ctx, cudaMemcpyAsync(logits_dev + head_lane[i] * m->v, ws.logits + i * m->v, (j - i + 1) * m->v * 4,
-                                               cudaMemcpyDeviceToDevice, st));
-            if (greedy_dev)
-                PSSA_CUDA(ctx, cudaMemcpyAsync(greedy_dev + head_lane[i], ws.greedy + i, (j - i + 1) * 4, cudaMemcpyDeviceToDevice, st));
-            i = j + 1;
-        }
+        return rows_to_lanes();
     }
     return PSSA_B200_OK;
 }
