@@ -538,8 +538,7 @@ bool is_decode_step(const pssa_b200_model* m, size_t lanes, const uint32_t* h_le
     return true;
 }
 
-// What a decode step keeps, and the scratch of up to kStepSlice rows of it: called by every forward pass of a model that can take
-// it, so that the first step of a stream that has just read its prompt does not stop for allocations.
+// What a decode step keeps, and the scratch of up to kStepSlice rows of it: allocated by the first step, or by `reserve`
 constexpr size_t kStepSlice = 2048;
 int32_t ensure_step(pssa_b200_model* m, size_t rows) {
     pssa_b200_ctx* ctx = m->ctx;
@@ -683,7 +682,6 @@ int32_t run_lanes(pssa_b200_model* m, const uint64_t* ids, const uint32_t* offse
             PSSA_CUDA(ctx, cudaMemcpyAsync(ws.lane_len, h_len.data(), n_lanes * 4, cudaMemcpyHostToDevice, st));
             PSSA_CUDA(ctx, cudaMemcpyAsync(ws.lane_slot, h_slot.data(), n_lanes * 4, cudaMemcpyHostToDevice, st));
             if (!h_last.empty()) PSSA_CUDA(ctx, cudaMemcpyAsync(ws.last_rows, h_last.data(), h_last.size() * 4, cudaMemcpyHostToDevice, st));
-            if (step_model_ok(m) && (rc = ensure_step(m, std::min<size_t>(m->max_streams, 128)))) return rc;
             if ((rc = forward_rows(m, rows, n_lanes, h_off.data(), h_len.data(), &feats, h_last.size()))) return rc;
         }
         if (!h_last.empty() && want_head) {
@@ -858,7 +856,6 @@ int32_t pssa_b200_model_prefill_batch_dev(pssa_b200_model* m, const uint32_t* id
         if (greedy_dev) PSSA_CUDA(ctx, cudaMemcpyAsync(greedy_dev, ws.greedy, rows * 4, cudaMemcpyDeviceToDevice, st));
         return PSSA_B200_OK;
     }
-    if (step_model_ok(m) && (rc = ensure_step(m, std::min<size_t>(m->max_streams, 128)))) return rc;
     PSSA_CUDA(ctx, cudaMemcpyAsync(ws.ids, ids_dev, span * 4, cudaMemcpyDeviceToDevice, st));
     m->sp.active = m->sp.world > 1;
     rc = forward_rows(m, span, n_lanes, h_off.data(), h_len.data(), &feats, h_last.size());
@@ -1148,6 +1145,7 @@ int32_t pssa_b200_model_reserve(pssa_b200_model* m, size_t rows, size_t lanes) {
     int32_t rc;
     if ((rc = ensure_workspace(m, std::min(rows, m->max_rows), lanes))) return rc;
     if ((rc = ensure_chunks(m, std::max(lanes * 16, std::min<size_t>(lanes, 16) * kMaxTimeChunks)))) return rc;  // the most time chunks lanes are ever cut into
+    if (step_model_ok(m) && (rc = ensure_step(m, std::min(rows, lanes)))) return rc;
     return ensure_sampler(m, lanes);
 }
 

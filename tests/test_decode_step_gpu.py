@@ -108,3 +108,40 @@ def test_more_rows_than_one_slice(gpu):
         big.copy_recurrent_state_from(st, i)
         assert np.array_equal(big.decode_step(ids[i:i + 1], [i])[0], full[i]), i
     big.close(), exact.close()
+
+
+def test_the_step_allocates_in_the_first_step_or_in_reserve(gpu):
+    """A model that only reads prompts keeps no scratch of the decode step; a reserved one allocates nothing in its first steps."""
+    import pssa_b200
+    import torch
+    streams, d = 512, 768  # 12 MB of scratch: more than the allocator's granularity
+    om = O.Model.new(1, 64, d, 16, 64, 64, tau_mem=0.1, seed=9)
+    fill_synthetic(om, 9, 1.0)
+    rng = np.random.default_rng(9)
+    prompts = [rng.integers(1, 64, 2) for _ in range(streams)]
+    ids = rng.integers(1, 64, streams)
+
+    def model():
+        m = pssa_b200.PSSAModel(gpu, 1, 64, d, 16, 64, 64, tau_mem=0.1, streams=streams, precision=0)
+        upload(om, m)
+        return m
+
+    def free():
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+
+    first = model()  # loads the kernels, whose code takes memory too
+    first.prefill_batch(prompts)
+    first.decode_step(ids), first.decode_step(ids[:1], [0])
+    plain = model()
+    plain.prefill_batch(prompts)
+    before = free()
+    plain.decode_step(ids)
+    assert before - free() >= streams * (d // 8 * 64) * 4
+    reserved = model()
+    reserved.reserve(2 * streams, streams)
+    before = free()
+    reserved.decode_step(ids), reserved.decode_step(ids[:1], [0])
+    reserved.prefill_batch(prompts)
+    assert free() == before
+    first.close(), plain.close(), reserved.close()
