@@ -107,13 +107,19 @@ __device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
-// 2^x for a pair of x <= 0 on the FMA pipe: x = n + f with |f| <= 1/2 by adding and taking off 1.5 * 2^23, 2^f by a degree-5
+// to [-126, 128], where 2^128 is infinity; a NaN stays one
+__device__ __forceinline__ float clamp_exp2(float x) {
+    float y;
+    asm("max.NaN.f32 %0, %1, 0fC2FC0000;\n\tmin.NaN.f32 %0, %0, 0f43000000;" : "=f"(y) : "f"(x));
+    return y;
+}
+// 2^x for a pair of x on the FMA pipe: x = n + f with |f| <= 1/2 by adding and taking off 1.5 * 2^23, 2^f by a degree-5
 // polynomial with p(0) = 1 (least largest relative error under that constraint, fitted by linear programming: 2^-22.5 after
 // fp32 rounding, mean -2e-8), n added to the exponent. Below 2^-126 the result stays at that size instead of going to zero.
 __device__ __forceinline__ f32x2 exp2_poly2(f32x2 x) {
     float x0, x1;
     unpack2(x, x0, x1);
-    x = pack2(fmaxf(x0, -126.0f), fmaxf(x1, -126.0f));
+    x = pack2(clamp_exp2(x0), clamp_exp2(x1));
     const f32x2 t = add2(x, pack2(12582912.0f, 12582912.0f));
     const f32x2 f = fma2(add2(t, pack2(-12582912.0f, -12582912.0f)), pack2(-1.0f, -1.0f), x);
     f32x2 r = pack2(0.001326472731307149f, 0.001326472731307149f);
@@ -125,7 +131,8 @@ __device__ __forceinline__ f32x2 exp2_poly2(f32x2 x) {
     float t0, t1, r0, r1;
     unpack2(t, t0, t1);
     unpack2(r, r0, r1);
-    return pack2(__int_as_float(__float_as_int(r0) + (__float_as_int(t0) << 23)), __int_as_float(__float_as_int(r1) + (__float_as_int(t1) << 23)));
+    r = pack2(__int_as_float(__float_as_int(r0) + (__float_as_int(t0) << 23)), __int_as_float(__float_as_int(r1) + (__float_as_int(t1) << 23)));
+    return fma2(x, pack2(0.0f, 0.0f), r);  // a NaN, which the additions to the exponent turn into a number, is one again
 }
 __device__ __forceinline__ f32x2 exp2_approx2(f32x2 x) {
     float x0, x1;

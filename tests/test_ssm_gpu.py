@@ -151,3 +151,44 @@ def test_shape_and_lane_errors(gpu):
     with pytest.raises(pssa_b200.B200Error) as e:
         gpu.ssm_forward_dev(z, z, z, z, z, None, z, np.array([0, 3], np.uint32), np.array([3, 2], np.uint32), 4, 8, 4)
     assert e.value.status == 2 and "outside 4 rows" in str(e.value)
+
+
+def test_edge_values_of_the_decay_reach_every_state(gpu):
+    """Rates and deltas outside the model's (a NaN, infinities, positive rates up to and past overflow), in the states whose exponential
+    is the polynomial (0 and 1 of every 16) and in their neighbours, through the kernel of many states that has it (48 of them)."""
+    import torch
+    d, s, T = 64, 48, 2
+    rng = np.random.default_rng(4)
+    rates = -rng.uniform(0.01, 0.7, (d, s)).astype(np.float32)
+    delta = np.full((T, d), 1.0, np.float32)
+    delta[1] = 0.5
+    edge = [np.nan, np.inf, -np.inf, 88.5, 89.5, 127.0, 200.0, 1e30, -1e30, 0.5, 0.0, -87.0, -103.0]
+    for i, v in enumerate(edge):
+        rates[i, [0, 1, 2, 3, 16, 17, 47]] = v
+    delta[0, 20], delta[0, 21], delta[0, 22], delta[0, 23] = np.nan, 0.0, -200.0, np.inf
+    rates[21, [0, 5]], rates[23, [0, 5]] = np.inf, 0.0
+    b, c = rng.normal(0, 1, (T, s)).astype(np.float32), rng.normal(0, 1, (T, s)).astype(np.float32)
+    x, h0 = rng.normal(0, 1, (T, d)).astype(np.float32), rng.normal(0, 1, (d, s)).astype(np.float32)
+    want = h0.astype(np.float64)
+    size = np.abs(want)  # of the terms: they can cancel
+    with np.errstate(all="ignore"):
+        for t in range(T):
+            a = np.exp((delta[t][:, None].astype(np.float64) * rates)).astype(np.float32).astype(np.float64)
+            u = (delta[t] * x[t]).astype(np.float64)[:, None] * b[t]
+            want, size = a * want + u, a * size + np.abs(u)
+            want = want.astype(np.float32).astype(np.float64)
+    carry = torch.from_numpy(h0.copy()).cuda()
+    y = torch.zeros(T, d, device="cuda")
+    dev = [torch.from_numpy(v).cuda() for v in (delta, b, c, x, rates)]
+    torch.cuda.synchronize()
+    gpu.ssm_forward_dev(*dev, carry, y, None, None, T, d, s)
+    gpu.synchronize()
+    got = carry.cpu().numpy()
+    assert np.array_equal(np.isnan(got), np.isnan(want))
+    assert np.array_equal(np.isinf(got), np.isinf(want))
+    fin = np.isfinite(want)
+    assert np.array_equal(np.sign(got[np.isinf(want)]), np.sign(want[np.isinf(want)]))
+    # the argument carries three roundings of 2^-24 of at most 128, the exponential 2^-22; below 2^-126 a decay may stay there
+    assert np.max(np.abs(got[fin] - want[fin]) / np.maximum(size[fin], 1e-30)) <= 2 * (3 * 128 * 2.0 ** -24 + 2.0 ** -22)  # two tokens
+    with np.errstate(all="ignore"):
+        assert np.array_equal(np.isnan(y.cpu().numpy()[1]), np.isnan((want * c[1]).sum(1)))
