@@ -1109,13 +1109,13 @@ int32_t launch_ssm_fused(pssa_b200_ctx* ctx, const SsmParams& p, bool exact) {
         // 344 and 402: the two lines below are fits of both. With 32 and 16 states this one is ahead at every size
         // (384 x 32: 1 lane 226 -> 40, 64 lanes 369 -> 336; 192 x 16: 106 -> 40, 137 -> 104), and in the exact mode
         // (64 states, 1 lane 1600 -> 107, 32 lanes 1742 -> 1604). The tape's stores decide where it is asked for: whole lines
-        // here, 4-byte pieces there. The lane splits sum y in different orders, so for calls of under 64 tokens a lane
-        // (decode loops start with those) the split follows the shape alone and a stream sees the same bits alone and in a
-        // batch; the exact mode's order is always the same.
+        // here, 4-byte pieces there. The lane splits sum y in different orders, so for calls of under 256 tokens a lane
+        // (from there on time chunks depend on the lanes too) the split follows the shape alone and a stream sees the same bits
+        // alone and in a batch; the exact mode's order is always the same.
         const size_t longest = p.max_len ? (size_t)p.max_len : (p.lengths ? 1 : p.rows);
         const int lanes = (int)std::max<size_t>(1, p.max_len || !p.lengths ? p.rows / std::max<size_t>(1, longest) : (size_t)p.lanes);
         const size_t channels = (size_t)lanes * p.d, schedulers = 4 * (size_t)ctx->sm_count;
-        const bool by_shape = !exact && longest < 64;
+        const bool by_shape = !exact && longest < 256;
         if (s == 16) return channels <= 4 * schedulers && !by_shape ? launch_wide<8, 2, 32>(ctx, p, exact) : launch_wide<4, 4, 16>(ctx, p, exact);
         if (s == 32) return channels <= 2 * schedulers && !by_shape ? launch_wide<16, 2, 32>(ctx, p, exact) : launch_wide<8, 4, 32>(ctx, p, exact);
         if (channels <= (exact ? 2 : 1) * schedulers && !by_shape) return launch_wide<32, 2, 32>(ctx, p, exact);

@@ -181,6 +181,34 @@ def test_a_stream_decodes_the_same_alone_and_inside_a_large_batch(gpu):
     big.close(), small.close()
 
 
+@pytest.mark.parametrize("d,s", [(192, 64), (384, 32), (320, 16)])
+def test_a_prompt_below_256_tokens_has_the_same_bits_alone_and_in_any_batch(gpu, d, s):
+    """Prompts of 64 to 255 tokens: logits and carries of the first lanes of a batch of 80 (more channels than any lane split of the
+    SSM takes in one wave), of 13, 5 and 2, and of each prompt alone."""
+    import pssa_b200
+    om = O.Model.new(2, 257, d, s, 64, 128, tau_mem=0.1, seed=s)
+    fill_synthetic(om, s)
+    gm = pssa_b200.PSSAModel(gpu, 2, 257, d, s, 64, 128, tau_mem=0.1, streams=80, precision=0)
+    upload(om, gm)
+    rng = np.random.default_rng(s)
+    prompts = [rng.integers(1, 257, n) for n in [255, 64, 100] + [int(x) for x in rng.integers(1, 256, 77)]]
+
+    def run(n):
+        gm.reset_recurrent_state()
+        logits = gm.prefill_batch(prompts[:n])[0]
+        return logits, [gm.copy_recurrent_state_to(i) for i in range(min(n, 5))]
+
+    logits, state = run(80)
+    for n in (13, 5, 2, 1):
+        lg, st = run(n)
+        assert np.array_equal(lg, logits[:n]), n
+        assert all(np.array_equal(a, b) for a, b in zip(st, state)), n
+    for i in (1, 2):
+        gm.reset_recurrent_state()
+        assert np.array_equal(gm.prefill_batch(prompts[i:i + 1])[0][0], logits[i]), i
+    gm.close()
+
+
 def test_closing_the_context_first_closes_its_models():
     """A model holds a pointer into its context; closing the context must retire the model rather than
     leave it to free device memory through a dead context later."""
