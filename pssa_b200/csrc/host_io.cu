@@ -202,6 +202,9 @@ int32_t scatter(pssa_b200_ctx* ctx, const char* src, size_t bytes, const std::ve
                 }
             upto[i] = spans.size();
         }
+        // The kernels in front of the first piece may take long: only this thread waits for them, and the helpers stay free for
+        // other contexts until there is something to copy.
+        PSSA_CUDA(ctx, cudaEventSynchronize(ctx->io_events[0]));
         CopyPool& pool = copy_pool();
         std::unique_lock<std::mutex> mine(pool.busy, std::try_to_lock);
         if (!mine.owns_lock()) {
