@@ -509,14 +509,15 @@ int32_t head_rows(pssa_b200_model* m, const float* feats, size_t n_heads, bool w
     Workspace& ws = m->ws;
     int32_t rc;
     const bool exact = m->precision == PSSA_B200_PRECISION_FP32_EXACT;
-    // the last rows of the lanes; the tensor-core head takes them as bf16 straight from the gather (in place of the z staging buffer)
-    if ((rc = launch_gather_rows(ctx, feats, ws.last_rows, exact ? ws.last_feat : nullptr, n_heads, (int)m->d, 0, exact ? nullptr : ws.z_bf16)))
+    // the last rows of the lanes; the tensor-core head takes them as bf16 straight from the gather, in place of the normalised rows
+    // (not in the MLP operands, whose pad columns meet weights of zero and must stay finite)
+    if ((rc = launch_gather_rows(ctx, feats, ws.last_rows, exact ? ws.last_feat : nullptr, n_heads, (int)m->d, 0, exact ? nullptr : ws.x_bf16)))
         return rc;
     const float scale = 1.0f / std::sqrt((float)m->d);
     if (exact) {
         if ((rc = launch_gemm_exact(ctx, ws.last_feat, m->unembed, ws.logits, n_heads, m->v, m->d, m->v, EPI_SCALE, scale))) return rc;
     } else {
-        if ((rc = launch_gemm_bf16(ctx, ws.z_bf16, m->unembed_bf16, ws.logits, nullptr, n_heads, m->v, m->d, m->v, EPI_SCALE, scale))) return rc;
+        if ((rc = launch_gemm_bf16(ctx, ws.x_bf16, m->unembed_bf16, ws.logits, nullptr, n_heads, m->v, m->d, m->v, EPI_SCALE, scale))) return rc;
     }
     if (want_greedy && (rc = launch_greedy(ctx, ws.logits, ws.greedy, n_heads, (int)m->v))) return rc;
     return PSSA_B200_OK;
@@ -919,8 +920,8 @@ int32_t pssa_b200_model_score(pssa_b200_model* m, uint32_t stream, const uint64_
             if (exact) {
                 if ((rc = launch_gemm_exact(ctx, feats + r0 * m->d, m->unembed, sc.logits, nr, m->v, m->d, m->v, EPI_SCALE, scale))) return rc;
             } else {
-                if ((rc = launch_to_bf16(ctx, feats + r0 * m->d, ws.z_bf16, nr * m->d))) return rc;
-                if ((rc = launch_gemm_bf16(ctx, ws.z_bf16, m->unembed_bf16, sc.logits, nullptr, nr, m->v, m->d, m->v, EPI_SCALE, scale))) return rc;
+                if ((rc = launch_to_bf16(ctx, feats + r0 * m->d, ws.x_bf16, nr * m->d))) return rc;
+                if ((rc = launch_gemm_bf16(ctx, ws.x_bf16, m->unembed_bf16, sc.logits, nullptr, nr, m->v, m->d, m->v, EPI_SCALE, scale))) return rc;
             }
             if ((rc = launch_cross_entropy(ctx, sc.logits, sc.targets + r0, sc.loss + r0, nr, (int)m->v))) return rc;
             if (logits_out)

@@ -209,6 +209,35 @@ def test_a_prompt_below_256_tokens_has_the_same_bits_alone_and_in_any_batch(gpu,
     gm.close()
 
 
+def test_a_non_finite_stream_leaves_nothing_behind(gpu):
+    """One stream whose carry has overflowed: its logits are not finite, and every later pass of the others (prefill, step, score) is
+    what it would have been without it."""
+    import pssa_b200
+    om = O.Model.new(2, 257, 192, 64, 64, 128, tau_mem=0.1, seed=6)
+    fill_synthetic(om, 6)
+    gm = pssa_b200.PSSAModel(gpu, 2, 257, 192, 64, 64, 128, tau_mem=0.1, streams=3, precision=0)
+    upload(om, gm)
+    rng = np.random.default_rng(6)
+    prompts = [rng.integers(1, 200, n) for n in (90, 40, 70)]
+    ids = rng.integers(1, 200, 80)
+
+    def clean():
+        gm.reset_recurrent_state()
+        out = [gm.prefill_batch(prompts)[0], gm.decode_step([5, 6, 7]), gm.decode_step(list(range(1, 4)))]
+        gm.reset_recurrent_state()
+        return out + [np.float32(gm.score(ids[:-1], ids[1:])[0])]
+
+    want = clean()
+    gm.reset_recurrent_state()
+    gm.copy_recurrent_state_from(np.full_like(gm.copy_recurrent_state_to(1), np.inf), 1)
+    assert not np.isfinite(gm.prefill_batch(prompts)[0][1]).any()
+    assert not np.isfinite(gm.decode_step([5, 6, 7])[1]).any()
+    got = clean()
+    for g, w in zip(got, want):
+        assert np.array_equal(g, w)
+    gm.close()
+
+
 def test_closing_the_context_first_closes_its_models():
     """A model holds a pointer into its context; closing the context must retire the model rather than
     leave it to free device memory through a dead context later."""
