@@ -583,7 +583,9 @@ int32_t dispatch(pssa_b200_ctx* ctx, const void* a, const void* b, GemmEpilogue&
     }
     if (e.N <= 64 || m_tiles * ((e.N + 127) / 128) < ctx->sm_count / 2) return launch_mid<64, 7>(ctx, a, b, e, only32, only16);
     // 128-wide tiles below one tile an SM, and up to four waves where they end sooner: 8192 rows of a 768-wide product are 192
-    // tiles of 256 columns, two rounds of which the second is a third full, or 384 of 128, three rounds of half the length
+    // tiles of 256 columns, two rounds of which the second is a third full, or 384 of 128, three rounds of shorter ones. A round of
+    // 128-wide tiles takes 0.53, 0.68, 0.74, 0.69 of one of 256-wide ones at K = 512, 768, 832, 1600 (4.9 / 9.2, 6.1 / 9.0, 6.5 / 8.8,
+    // 11.0 / 16.0 us, plain epilogue): 13 to 20
     const long long t256 = m_tiles * ((e.N + 255) / 256), t128 = m_tiles * ((e.N + 127) / 128), sms = ctx->sm_count;
     const bool shorter = e.n_pairs <= 1 && t256 <= 4 * sms && ((t128 + sms - 1) / sms) * 13 < ((t256 + sms - 1) / sms) * 20;
     if (e.N <= 128 || t256 < sms || shorter) return launch_mid<128, 5>(ctx, a, b, e, only32, only16);

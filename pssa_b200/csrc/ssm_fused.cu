@@ -64,7 +64,7 @@ __device__ __forceinline__ float ex2_approx(float x) {
 // error on |r| <= ln 2 / 2, fitted by linear programming: 2^-28.3), n added to the exponent. For the decays of the
 // recurrence (-0.08 < x <= 0) 97 % of the results are the correctly rounded ones (largest error 0.57 ulp), which is what the
 // reference's host libm returns, so its states are met in far more bits than with a 1 to 2 ulp exp; and the XU pipe is not
-// used. Results near or below the smallest normal number, and overflow, are left to expf.
+// used. Below -1 90 % are, and the largest error is 1.0 ulp. Results near or below the smallest normal number, and overflow, are left to expf.
 __device__ __forceinline__ float exp_exact(float x) {
     const float t = fmaf(x, 1.4426950408889634f, 12582912.0f);  // 1.5 * 2^23: the integer part ends up in the low bits
     const float n = t - 12582912.0f;
@@ -334,9 +334,9 @@ __global__ void __launch_bounds__(THR, (ST <= 16 && !TAPE && !EXACT) ? ((THR > 2
 #pragma unroll
                 for (int jj = 0; jj < ST; jj += 2) {
                     const f32x2 b2 = pack2(bj[jj], bj[jj + 1]), c2 = pack2(cj[jj], cj[jj + 1]);
-                    // one pair of exponentials in eight goes to the FMA pipe (the benchmark's launch: 960 us with none, 925 with
-                    // one, 1039 with two, whose extra issue slots cost more than the XU pipe gains)
-                    // (the map pass, which has no y to form, takes two)
+                    // one pair of exponentials in eight goes to the FMA pipe (the benchmark's launch: 976 us with none, 952 with
+                    // one, 1059 with two, whose extra issue slots cost more than the XU pipe gains)
+                    // (the map pass, which has no y to form, takes two: 109 -> 105 us for 8192 tokens)
                     const bool poly = ST == 16 && G == 4 && !TAPE && (jj == 0 || (MAPS && jj == 8));
                     const f32x2 arg = mul2(dl2, pack2(A[jj], A[jj + 1]));
                     const f32x2 a2 = poly ? exp2_poly2(arg) : exp2_approx2(arg);
@@ -469,7 +469,7 @@ __global__ void __launch_bounds__(THR, (ST <= 16 && !TAPE && !EXACT) ? ((THR > 2
 //   * few lanes leave a warp alone on its scheduler, so everything has to overlap inside it: see the token loop.
 //   * a tile's tail is padded with delta = 0, which leaves the state as it is (exp(0) = 1, input 0).
 // What bounds it: alone, a token's dependent instructions (about 85 cycles, 32 of them exponentials); with many warps the
-// shared-memory pipe (0.7 of its wavefronts) before the XU pipe (0.55).
+// shared-memory pipe (0.67 of its wavefronts at 8 lanes of 768 channels) and the XU pipe (0.62) side by side.
 constexpr int kWideStages = 3;
 constexpr int kWideWarps = 4;
 template <int LPC, int SPL, int TT, bool EXACT>

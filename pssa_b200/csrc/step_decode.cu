@@ -57,7 +57,7 @@ __device__ __forceinline__ void mma_step(float (&d)[4], const uint4& lo, const u
 
 // ---- grid barrier on one 64-bit arrival count that is never reset: a launch finds it between k and k + 1 times the grid size
 // (no CTA passes the first barrier before all have read it), so barrier i of the launch is over at (k + i + 1) * grid. One
-// word to arrive at and to poll: 2400 cycles, 900 of them the release. A CTA that waits too long records the expiry and no
+// word to arrive at and to poll: 2430 cycles (1.3 us), 2950 with a store to publish, of which 820 are the release. A CTA that waits too long records the expiry and no
 // longer waits.
 struct Barrier {
     unsigned long long* count;

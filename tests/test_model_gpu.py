@@ -209,6 +209,41 @@ def test_a_prompt_below_256_tokens_has_the_same_bits_alone_and_in_any_batch(gpu,
     gm.close()
 
 
+def test_time_chunks_that_hold_no_token_leave_the_carry_as_it_is(gpu):
+    """A long prompt cut into 37 time chunks beside prompts of 7, 36 and 1 tokens, most of whose chunks are empty: carries and logits
+    against the same prompts read in windows too short to be cut. (A chunk's decay is one exponential where the recurrence multiplies
+    68 of them, each good to 2^-22 and its argument to 2^-23 of at most 8.)"""
+    import pssa_b200
+    om = O.Model.new(1, 257, 192, 64, 64, 128, tau_mem=0.1, seed=8)
+    fill_synthetic(om, 8)
+    gm = pssa_b200.PSSAModel(gpu, 1, 257, 192, 64, 64, 128, tau_mem=0.1, streams=4, precision=0)
+    upload(om, gm)
+    rng = np.random.default_rng(8)
+    prompts = [rng.integers(1, 257, n) for n in (2500, 7, 36, 1)]
+    start = rng.standard_normal((4, gm.recurrent_state_len())).astype(np.float32)
+
+    def run(lanes):
+        for i in range(4):
+            gm.copy_recurrent_state_from(start[i], i)
+        gpu.profile_begin()
+        logits = gm.prefill_batch([prompts[i] for i in lanes], streams=lanes)[0]
+        return logits, [gm.copy_recurrent_state_to(i) for i in lanes], gpu.profile_end()
+
+    gm.set_max_rows(4 * 1000)
+    want, want_state, rows = run([0, 1, 2, 3])
+    assert not any("chunk maps" in k for k in rows)
+    gm.set_max_rows(65536)
+    for lanes in ([0, 1, 2, 3], [3, 0]):
+        logits, state, rows = run(lanes)
+        assert any("chunk maps" in k for k in rows)
+        for got, i in zip(state, lanes):
+            ref = want_state[i].reshape(192, 64)
+            scale = np.maximum(np.abs(ref), np.abs(start[i].reshape(192, 64))).max(1, keepdims=True)
+            assert np.max(np.abs(got.reshape(192, 64) - ref) / scale) <= 68 * (2.0 ** -22 + 8 * 2.0 ** -23), i
+        assert scale_err(logits, want[lanes]) <= 1e-2  # bf16 operands behind the recurrence
+    gm.close()
+
+
 def test_a_non_finite_stream_leaves_nothing_behind(gpu):
     """One stream whose carry has overflowed: its logits are not finite, and every later pass of the others (prefill, step, score) is
     what it would have been without it."""
