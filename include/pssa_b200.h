@@ -147,7 +147,8 @@ int32_t pssa_b200_scan_states_noalloc_dev(pssa_b200_ctx* ctx, const float* a, co
  * reference's own GPU kernel (src/cuda/stages.ptx:21-22), in some of the states a polynomial as good -- with fused
  * multiply-adds. EXACT: an exp of at most 1 ulp (0.57 for the small arguments of a decay) and
  * separately rounded multiply/add in the order of the CPU reference (src/pssa.rs:1131-1144). Rates and deltas may be any
- * numbers: a NaN or an infinity reaches the states that it is part of, and no others. */
+ * numbers: a NaN or an infinity reaches the states that it is part of, and no others (an infinite rate at a delta of 0 gives a
+ * NaN or leaves the state as it is, which of them the kernel of the shape decides). */
 #define PSSA_B200_SSM_EXACT 1u
 
 /*

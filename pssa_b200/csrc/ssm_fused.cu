@@ -26,6 +26,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cfloat>
 
 #include "bounds.hpp"
 #include "context.hpp"
@@ -539,6 +540,11 @@ __global__ void __launch_bounds__(kWideWarps * 32) ssm_wide_kernel(SsmParams p) 
 #pragma unroll
         for (int v = 0; v < V; ++v) A[q * V + v] = reinterpret_cast<const float*>(&a)[v], h[q * V + v] = reinterpret_cast<const float*>(&hv)[v];
     }
+    // an infinite rate (times log2 e, in the fast mode) would make a NaN of the padding's delta 0: the largest finite one does the
+    // same for any other delta
+    constexpr float kRateMax = EXACT ? FLT_MAX : FLT_MAX / 1.45f;
+#pragma unroll
+    for (int q = 0; q < SPL; ++q) A[q] = fabsf(A[q]) > kRateMax ? copysignf(kRateMax, A[q]) : A[q];
     auto put = [&](float* base, int t, int q, const float* v) {  // one piece of a tape row
         vec o;
 #pragma unroll

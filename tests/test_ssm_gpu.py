@@ -153,20 +153,24 @@ def test_shape_and_lane_errors(gpu):
     assert e.value.status == 2 and "outside 4 rows" in str(e.value)
 
 
-def test_edge_values_of_the_decay_reach_every_state(gpu):
+@pytest.mark.parametrize("exact", [False, True])
+@pytest.mark.parametrize("s", [48, 64, 32, 16])
+def test_edge_values_of_the_decay_reach_every_state(gpu, s, exact):
     """Rates and deltas outside the model's (a NaN, infinities, positive rates up to and past overflow), in the states whose exponential
-    is the polynomial (0 and 1 of every 16) and in their neighbours, through the kernel of many states that has it (48 of them)."""
+    is the polynomial (0 and 1 of every 16 in the kernel that 48 states take) and in their neighbours, and in the few-lanes kernel
+    (16, 32, 64 states), whose tiles are padded with tokens of delta 0. There an infinite rate at a delta of 0 leaves a state as it
+    is, elsewhere it is a NaN: that one pair is left out."""
     import torch
-    d, s, T = 64, 48, 2
+    d, T = 64, 2
     rng = np.random.default_rng(4)
     rates = -rng.uniform(0.01, 0.7, (d, s)).astype(np.float32)
     delta = np.full((T, d), 1.0, np.float32)
     delta[1] = 0.5
     edge = [np.nan, np.inf, -np.inf, 88.5, 89.5, 127.0, 200.0, 1e30, -1e30, 0.5, 0.0, -87.0, -103.0]
     for i, v in enumerate(edge):
-        rates[i, [0, 1, 2, 3, 16, 17, 47]] = v
+        rates[i, [0, 1, 2, 3, s // 3, s // 3 + 1, s - 1]] = v
     delta[0, 20], delta[0, 21], delta[0, 22], delta[0, 23] = np.nan, 0.0, -200.0, np.inf
-    rates[21, [0, 5]], rates[23, [0, 5]] = np.inf, 0.0
+    rates[21, [0, 5]], rates[23, [0, 5]] = np.inf if s == 48 else 0.1, 0.0
     b, c = rng.normal(0, 1, (T, s)).astype(np.float32), rng.normal(0, 1, (T, s)).astype(np.float32)
     x, h0 = rng.normal(0, 1, (T, d)).astype(np.float32), rng.normal(0, 1, (d, s)).astype(np.float32)
     want = h0.astype(np.float64)
@@ -181,7 +185,7 @@ def test_edge_values_of_the_decay_reach_every_state(gpu):
     y = torch.zeros(T, d, device="cuda")
     dev = [torch.from_numpy(v).cuda() for v in (delta, b, c, x, rates)]
     torch.cuda.synchronize()
-    gpu.ssm_forward_dev(*dev, carry, y, None, None, T, d, s)
+    gpu.ssm_forward_dev(*dev, carry, y, None, None, T, d, s, exact=exact)
     gpu.synchronize()
     got = carry.cpu().numpy()
     assert np.array_equal(np.isnan(got), np.isnan(want))
