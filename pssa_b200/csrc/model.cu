@@ -95,6 +95,8 @@ int32_t pssa_b200_model_create(pssa_b200_ctx* ctx, const pssa_b200_config* cfg, 
     guard(dev_alloc(ctx, (void**)&m->unembed, m->v * m->d * 4, true));
     guard(dev_alloc(ctx, &m->unembed_bf16, m->v * m->d * 2, true));
     guard(dev_alloc(ctx, (void**)&m->state, (size_t)max_streams * m->depth * m->d * m->s * 4, true));
+    const bool step = step_shape_ok(m->depth, m->d, m->s, m->k, m->cap, m->rank);
+    if (step) guard(dev_alloc(ctx, &m->step_barrier, 256, true));
     for (auto& b : m->blocks) {
         for (int id : kBlockTensors) guard(dev_alloc(ctx, (void**)&b.w[id], tensor_len(m, id) * 4, true));
         guard(dev_alloc(ctx, (void**)&b.rates, m->d * m->s * 4, true));
@@ -110,6 +112,7 @@ int32_t pssa_b200_model_create(pssa_b200_ctx* ctx, const pssa_b200_config* cfg, 
         guard(dev_alloc(ctx, (void**)&b.vp, m->cap * m->d * sizeof(float), true));
         guard(dev_alloc(ctx, &b.ksplit_bf16, m->cap * 3 * m->k * 2, true));
         guard(dev_alloc(ctx, (void**)&b.kstat, m->cap * sizeof(float2), true));
+        if (step) guard(dev_alloc(ctx, (void**)&b.keys_t, m->cap * m->k * 4, true));
         b.host_up.assign(m->d * m->rank, 0.0f);
         b.host_cons.assign(m->d * m->rank, 0.0f);
         b.confidence.assign(m->cap, 1.0f);
@@ -143,7 +146,7 @@ void pssa_b200_model_destroy(pssa_b200_model* m) {
     cudaFree(m->sampler.recent), cudaFree(m->sampler.count), cudaFree(m->sampler.rng), cudaFree(m->sampler.ids);
     cudaFree(m->sampler.status), cudaFree(m->sampler.head_slot), cudaFree(m->sampler.probs), cudaFree(m->sampler.conf);
     cudaFree(m->chunks.off), cudaFree(m->chunks.len), cudaFree(m->chunks.records), cudaFree(m->chunks.carry_in);
-    cudaFree(m->step.keys_t), cudaFree(m->step.barrier), cudaFree(m->step.scratch);
+    cudaFree(m->step_barrier);
     for (auto& b : m->blocks) {
         for (int id : kBlockTensors) cudaFree(b.w[id]);
         cudaFree(b.rates);
@@ -158,6 +161,7 @@ void pssa_b200_model_destroy(pssa_b200_model* m) {
         cudaFree(b.vpsplit_bf16);
         cudaFree(b.vp);
         cudaFree(b.ksplit_bf16);
+        cudaFree(b.keys_t);
         cudaFree(b.kstat);
     }
     free_workspace(m->ws);

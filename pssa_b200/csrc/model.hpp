@@ -37,6 +37,7 @@ struct DeviceBlock {
     float* w1u = nullptr;
     void* vsplit_bf16 = nullptr;  // bank values transposed, three bf16 pieces [d, 3*cap] (tensor-core value read)
     void* ksplit_bf16 = nullptr;  // bank keys as three bf16 pieces [cap, 3*k] and (|k|^2, 1/(1-|k|^2)) per slot
+    float* keys_t = nullptr;      // the keys by quads [k / 4][cap] (decode step); null where the model's shape has no such step
     float2* kstat = nullptr;      //   (tensor-core distances); rebuilt together with vsplit_bf16
     // bf16 mode: W_proj (sum_s w_s v_s) = sum_s w_s (W_proj v_s), so the bank's values are carried through the memory
     // projection once per upload: vp = V W_proj^T [cap, d] fp32, vpsplit_bf16 = its transpose as bf16 pieces [d, 3*cap]
@@ -47,7 +48,7 @@ struct DeviceBlock {
     bool vsplit_dirty = true;
     bool vp_dirty = true;
     bool ksplit_dirty = true;
-    bool keys_t_dirty = true;     // step.keys_t of this block
+    bool keys_t_dirty = true;
 };
 
 struct Workspace {
@@ -62,6 +63,8 @@ struct Workspace {
     float2* q_stat = nullptr;    // [rows] (|p|^2, 1/(1-|p|^2))
     uint32_t* fixup = nullptr;   // [8] rows the fused top-k read recomputed over every slot, per lane group
     // z_bf16 is [rows, d + 64] and act_bf16 [rows, 2d + 64] when the adapter rides in the MLP products (rank 16)
+    float* step = nullptr;       // decode step: query partials, sums of squares and row scales of up to step_rows rows
+    size_t step_rows = 0;
     char* base = nullptr;
     size_t bytes = 0;
 };
@@ -138,13 +141,6 @@ struct pssa_b200_model {
         float* records = nullptr;   // [capacity][d + d*s]  (local mode; the sharded mode uses sp.send)
         float* carry_in = nullptr;  // [capacity][d*s]
     } chunks;
-    // decode step in one kernel (step_decode.cu): the banks' keys by quads [depth][k * cap], the barrier word and the step's own
-    // scratch, sized for `rows` streams of one pass
-    struct Step {
-        float* keys_t = nullptr;
-        void* barrier = nullptr;
-        float* scratch = nullptr;
-        size_t rows = 0;
-    } step;
+    void* step_barrier = nullptr;  // grid barrier of the decode step in one kernel (step_decode.cu)
     std::vector<bool> tensor_set;  // [depth * T_COUNT + id] upload bookkeeping
 };

@@ -22,6 +22,8 @@ struct Carver {
     }
 };
 
+constexpr size_t kStepSlice = 2048;  // rows of a decode step at a time, at most
+
 // one allocation carved into the per-row activation buffers; grows when a larger pass is requested
 int32_t ensure_workspace(pssa_b200_model* m, size_t rows, size_t lanes) {
     Workspace& ws = m->ws;
@@ -41,6 +43,8 @@ int32_t ensure_workspace(pssa_b200_model* m, size_t rows, size_t lanes) {
     size_t o_xb = c.take(rows * d * 2), o_yb = c.take(rows * d * 2), o_mb = c.take(rows * d * 2), o_zb = c.take(rows * (d + 64) * 2),
            o_ab = c.take(rows * (2 * d + 64) * 2), o_wsp = c.take(rows * 3 * m->cap * 2), o_qsp = c.take(rows * 3 * m->k * 2),
            o_qst = c.take(rows * sizeof(float2)), o_fix = c.take(8 * 4);  // counters of the one-kernel top-k read, one per lane group
+    const size_t step_rows = m->step_barrier ? std::min(lanes, kStepSlice) : 0;  // a decode step's rows are lanes
+    size_t o_step = c.take(step_rows * (d / 8 * m->k + d / 16 + 1) * f);
     size_t total = c.take(0);
     PSSA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     if (ws.base) cudaFree(ws.base);
@@ -57,6 +61,7 @@ int32_t ensure_workspace(pssa_b200_model* m, size_t rows, size_t lanes) {
     ws.ids = (uint32_t*)(b + o_ids), ws.lane_off = (uint32_t*)(b + o_off), ws.lane_len = (uint32_t*)(b + o_len);
     ws.lane_slot = (uint32_t*)(b + o_slot), ws.last_rows = (uint32_t*)(b + o_last), ws.greedy = (uint32_t*)(b + o_greedy);
     ws.row_slot = (uint32_t*)(b + o_rslot);
+    ws.step = (float*)(b + o_step), ws.step_rows = step_rows;
     ws.feat_c = m->loops > 1 ? (float*)(b + o_fc) : nullptr;
     ws.feat_a = (float*)(b + o_fa), ws.feat_b = (float*)(b + o_fb), ws.x_norm = (float*)(b + o_xn);
     ws.proj = (float*)(b + o_proj), ws.y = (float*)(b + o_y), ws.weights = (float*)(b + o_w), ws.m_val = (float*)(b + o_mv);
@@ -539,47 +544,23 @@ bool is_decode_step(const pssa_b200_model* m, size_t lanes, const uint32_t* h_le
     return true;
 }
 
-// What a decode step keeps, and the scratch of up to kStepSlice rows of it: allocated by the first step, or by `reserve`
-constexpr size_t kStepSlice = 2048;
-int32_t ensure_step(pssa_b200_model* m, size_t rows) {
-    pssa_b200_ctx* ctx = m->ctx;
-    auto& st = m->step;
-    int32_t rc;
-    rows = std::min(rows, kStepSlice);
-    if (!st.keys_t) {
-        PSSA_CUDA(ctx, cudaMalloc((void**)&st.keys_t, m->depth * m->k * m->cap * sizeof(float)));
-        PSSA_CUDA(ctx, cudaMalloc(&st.barrier, 256));
-        PSSA_CUDA(ctx, cudaMemsetAsync(st.barrier, 0, 256, ctx->stream));
-    }
-    if (rows > st.rows) {
-        PSSA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-        cudaFree(st.scratch);
-        st.scratch = nullptr, st.rows = 0;
-        PSSA_CUDA(ctx, cudaMalloc((void**)&st.scratch, rows * (m->d / 8 * m->k + m->d / 16 + 1) * sizeof(float)));
-        st.rows = rows;
-    }
-    for (size_t l = 0; l < m->depth; ++l) {
-        DeviceBlock& b = m->blocks[l];
-        if (!b.keys_t_dirty) continue;
-        if ((rc = launch_keys_by_quad(ctx, b.w[T_BANK_KEYS], st.keys_t + l * m->k * m->cap, (int)m->cap, (int)m->k))) return rc;
-        b.keys_t_dirty = false;
-    }
-    return PSSA_B200_OK;
-}
-
 // logits [rows, vocab] (null: not wanted); ids [rows] is a device array, ws.row_slot [rows] holds the rows' streams
 int32_t run_decode_step(pssa_b200_model* m, size_t rows, const uint32_t* ids, float* logits) {
     pssa_b200_ctx* ctx = m->ctx;
     Workspace& ws = m->ws;
-    auto& st = m->step;
     int32_t rc;
-    if ((rc = refresh_bf16(m)) || (rc = ensure_step(m, rows))) return rc;
+    if ((rc = refresh_bf16(m))) return rc;
+    for (auto& b : m->blocks) {
+        if (!b.keys_t_dirty) continue;
+        if ((rc = launch_keys_by_quad(ctx, b.w[T_BANK_KEYS], b.keys_t, (int)m->cap, (int)m->k))) return rc;
+        b.keys_t_dirty = false;
+    }
     StepLaunch::Block blocks[64];
     const size_t ds = m->d * m->s;
     for (size_t l = 0; l < m->depth; ++l) {
         DeviceBlock& b = m->blocks[l];
         blocks[l] = {b.wcat_bf16, b.wqh_bf16, b.vpsplit_bf16, b.w1cat_bf16, b.w2cat_bf16, b.rates, b.w[T_NORM_GAMMA], b.w[T_NORM_BETA],
-                     st.keys_t + l * m->k * m->cap, b.w[T_BANK_NORM_SQ], m->state + l * ds, l == 0 ? 1.0f : m->residual_scales[l - 1], (int)b.count};
+                     b.keys_t, b.w[T_BANK_NORM_SQ], m->state + l * ds, l == 0 ? 1.0f : m->residual_scales[l - 1], (int)b.count};
     }
     StepLaunch p{};
     p.d = (int)m->d, p.s = (int)m->s, p.k = (int)m->k, p.cap = (int)m->cap, p.nc = (int)m->ncat;
@@ -588,8 +569,8 @@ int32_t run_decode_step(pssa_b200_model* m, size_t rows, const uint32_t* ids, fl
     p.ssm_scale = 1.0f / std::sqrt((float)m->s), p.head_scale = 1.0f / std::sqrt((float)m->d), p.tau = m->cfg.tau_mem;
     p.embed = m->embed, p.unembed = m->unembed_bf16, p.carry_stride = m->depth * ds;
     p.feat_a = ws.feat_a, p.feat_b = ws.feat_b, p.proj = ws.proj, p.y = ws.y;
-    p.qpart = st.scratch, p.ssq = p.qpart + st.rows * (m->d / 8 * m->k), p.inv = p.ssq + st.rows * (m->d / 16);
-    p.x = ws.x_bf16, p.w = ws.w_split, p.z = ws.z_bf16, p.act = ws.act_bf16, p.barrier = st.barrier, p.blocks = blocks;
+    p.qpart = ws.step, p.ssq = p.qpart + ws.step_rows * (m->d / 8 * m->k), p.inv = p.ssq + ws.step_rows * (m->d / 16);
+    p.x = ws.x_bf16, p.w = ws.w_split, p.z = ws.z_bf16, p.act = ws.act_bf16, p.barrier = m->step_barrier, p.blocks = blocks;
     for (size_t r0 = 0; r0 < rows; r0 += kStepSlice) {  // rows share nothing: slices keep the scratch small
         p.rows = (int)std::min(kStepSlice, rows - r0), p.ids = ids + r0, p.slots = ws.row_slot + r0;
         p.logits = logits ? logits + r0 * m->v : nullptr;
@@ -1146,7 +1127,6 @@ int32_t pssa_b200_model_reserve(pssa_b200_model* m, size_t rows, size_t lanes) {
     int32_t rc;
     if ((rc = ensure_workspace(m, std::min(rows, m->max_rows), lanes))) return rc;
     if ((rc = ensure_chunks(m, std::max(lanes * 16, std::min<size_t>(lanes, 16) * kMaxTimeChunks)))) return rc;  // the most time chunks lanes are ever cut into
-    if (step_model_ok(m) && (rc = ensure_step(m, std::min(rows, lanes)))) return rc;
     return ensure_sampler(m, lanes);
 }
 
