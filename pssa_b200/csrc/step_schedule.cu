@@ -23,6 +23,11 @@ using namespace tc;
 constexpr int kEpiWarps = 16;  // four per TMEM lane quadrant
 constexpr int kReadRows = 4;  // rows of a CTA of the memory read: a key is loaded once for them
 
+// A block of the 12-block, d 768 model at 256 streams, us a launch under a profiler: norm 7, x-side 13, SSM 25 (100 MB of carries, 16 at
+// the copy rate), read 14, gated value read 10, MLP up 12, MLP down 16; the step 1107, as the block schedule that it replaces above
+// 128 streams (1124), and 864 / 935 at 64 / 128 streams where the one kernel's 64-row mma.sync tiles took 959 / 1088. A launch of a
+// few hundred rows is prologue, first trip to memory and epilogue: nothing is busy.
+
 // The block's output rows; q sums of squares of 16 columns go to the next norm, at the last block the bf16 rows to the head.
 struct PutFeature {
     static constexpr bool kReads = true;
@@ -96,9 +101,9 @@ __device__ __forceinline__ Run run_of(int k, int r) {
     return {f0 * 32, (c0 + c1 + 1) / 2, c0, c1};
 }
 
-// One 128 x BN tile per CTA: x [rows, .] times w [n, .]^T over the first k of K. Warp 0 loads, warp 1 issues: an MMA this small waits
-// some 190 cycles for the one before it in its accumulator (950 cycles a box of 64 in K order, three quarters of the launch), so the four
-// runs of K take turns. Warps 2 to 17: of a quadrant's four, two add up half of the segments for half of the columns each way,
+// One 128 x BN tile per CTA: x [rows, .] times w [n, .]^T over the first k of K. Warp 0 loads, warp 1 issues: the four runs of K take
+// turns, so that MMAs next to each other go to different accumulators (cycles for four boxes of 64, stamps in the issuing warp: 3800
+// in K order, 2850 in turns, 2115 with an elected lane; the arrival of the boxes from L2, 38 B a cycle, is what is left). Warps 2 to 17: of a quadrant's four, two add up half of the segments for half of the columns each way,
 // then each stores a quarter of the rows. What is read for an output is requested before the accumulators are waited for.
 template <int BN, int STAGES, class Put>
 __device__ __forceinline__ void product_tile(const CUtensorMap& map_x, const CUtensorMap& map_w, int n, int k, const Put& put) {
@@ -283,6 +288,8 @@ __global__ void __launch_bounds__(kThreads) step_norm_kernel(const __grid_consta
     if (ids) check_ids(a);
     norm_stage(a, b, Features{a.embed, ids, in, a.d, a.vocab});
 }
+// CTAs to an SM: with few states two of 128 registers instead of one with three rows in flight a warp (32 states, 4 blocks of d 384,
+// 256 / 512 streams: 256 -> 247, 305 -> 284 us a step), with 64 the rows' carries need the registers
 constexpr int ssm_ctas(int nv) { return nv > 2 ? 1 : 2; }
 template <int NV>
 __global__ void __launch_bounds__(kThreads, ssm_ctas(NV)) step_ssm_kernel(const __grid_constant__ StepCommon a, const __grid_constant__ StepBlock b,
