@@ -25,8 +25,11 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <math_constants.h>
+
 #include <algorithm>
 #include <cfloat>
+#include <type_traits>
 
 #include "bounds.hpp"
 #include "context.hpp"
@@ -135,6 +138,16 @@ __device__ __forceinline__ f32x2 exp2_poly2(f32x2 x) {
     r = pack2(__int_as_float(__float_as_int(r0) + (__float_as_int(t0) << 23)), __int_as_float(__float_as_int(r1) + (__float_as_int(t1) << 23)));
     return fma2(x, pack2(0.0f, 0.0f), r);  // a NaN, which the additions to the exponent turn into a number, is one again
 }
+// 2^x for a pair of x in [-0.4, 0]: no range reduction, a degree-4 polynomial with p(0) = 1 (least largest relative error under that
+// constraint, fitted by linear programming: 2^-23.4 after fp32 rounding, rms 2^-25.0; ex2.approx has 2^-22.9 and 2^-24.6 there).
+constexpr float kSmallArg = 0.4f;
+__device__ __forceinline__ f32x2 exp2_small2(f32x2 x) {
+    f32x2 r = pack2(0.008396584540605545f, 0.008396584540605545f);
+    r = fma2(r, x, pack2(0.05509750917553902f, 0.05509750917553902f));
+    r = fma2(r, x, pack2(0.24017220735549927f, 0.24017220735549927f));
+    r = fma2(r, x, pack2(0.6931449174880981f, 0.6931449174880981f));
+    return fma2(r, x, pack2(1.0f, 1.0f));
+}
 __device__ __forceinline__ f32x2 exp2_approx2(f32x2 x) {
     float x0, x1;
     unpack2(x, x0, x1);
@@ -144,7 +157,7 @@ __device__ __forceinline__ f32x2 exp2_approx2(f32x2 x) {
 // MAPS: the first of the two passes over time chunks. It leaves every chunk's affine map at `sum_delta` (sum of delta, then the
 // end state from a zero carry) and no y: what would form and store it, a third of the instructions, is not in it.
 template <int ST, int G, bool EXACT, bool TAPE, int THR = kThreads, int CPT = 1, bool MAPS = false>
-__global__ void __launch_bounds__(THR, (ST <= 16 && !TAPE && !EXACT) ? ((THR > 256 || CPT > 1) ? 2 : kMinCtasFast) : 1) ssm_fused_kernel(SsmParams p) {
+__global__ void __launch_bounds__(THR, (ST <= 16 && !TAPE && !EXACT) ? (CPT > 1 ? 3 : THR > 256 ? 2 : kMinCtasFast) : 1) ssm_fused_kernel(SsmParams p) {
     // CPT channels per thread (fast mode without tape only): a token's B and C rows are loaded once for both channels and
     // the two recurrences are independent instruction streams, so a warp-token of twice the work takes fewer than twice
     // the instructions.
@@ -155,8 +168,8 @@ __global__ void __launch_bounds__(THR, (ST <= 16 && !TAPE && !EXACT) ? ((THR > 2
     constexpr int CH = kThreads / G * CPT;  // channels per CTA
     constexpr int kTileTokens = kTileTokensFor<G>;
     constexpr int LPG = 32 / G;       // lanes of a warp that share one state group
-    constexpr int SG = ST + 4;        // shared-memory pitch of a state group (bank spreading)
-    constexpr int SP = SG * G;        // floats per token row of B / C in shared memory
+    constexpr int SP = ST * G;        // floats per token row of B / C in shared memory
+    constexpr int QS = 4 * G;         // a thread's states lie in pieces of four, this far apart
     extern __shared__ __align__(16) float smem[];
     float* sm_delta = smem;                                   // [kStages][kTileTokens][CH]
     float* sm_x = sm_delta + kStages * kTileTokens * CH;      // [kStages][kTileTokens][CH]
@@ -176,7 +189,7 @@ __global__ void __launch_bounds__(THR, (ST <= 16 && !TAPE && !EXACT) ? ((THR > 2
     const int len = p.lengths ? (int)p.lengths[lane] : (int)p.rows;
     const int d = p.d, s = p.s;
     const size_t ds = (size_t)d * s;
-    const int j0 = g * ST;
+    const int j0 = g * 4;
     const size_t ldd = p.ld_delta ? p.ld_delta : (size_t)d;
     const size_t ldbc = p.ld_bc ? p.ld_bc : (size_t)s;
     float* carry = p.carry && !MAPS ? p.carry + (size_t)(p.lane_slots ? p.lane_slots[lane] : lane) * (p.carry_stride ? p.carry_stride : ds)
@@ -186,17 +199,16 @@ __global__ void __launch_bounds__(THR, (ST <= 16 && !TAPE && !EXACT) ? ((THR > 2
     float A1[CPT > 1 ? ST : 1], h1[CPT > 1 ? ST : 1];  // the second channel of a two-channel thread
     const int i1 = i + 1;
     const bool valid1 = CPT > 1 && i1 < p.d;
-    // a thread's states are contiguous in `rates` and in the carry: 16-byte accesses when the layout allows (decode
-    // steps are one token long, so this load and the store at the end are most of their traffic)
+    // pieces of four states: 16-byte accesses when the layout allows
     const bool vec_state = p.aligned && (s & 3) == 0 && (reinterpret_cast<uintptr_t>(p.rates) & 15) == 0 &&
                            (reinterpret_cast<uintptr_t>(carry) & 15) == 0;
     auto load_state = [&](float* Av, float* hv, int ch, bool ok_ch) {
         if (vec_state) {
 #pragma unroll
             for (int q = 0; q < ST / 4; ++q) {
-                const bool ok = ok_ch && (j0 + q * 4) < s;
-                const float4 r4 = ok ? __ldg(reinterpret_cast<const float4*>(p.rates + (size_t)ch * s + j0) + q) : make_float4(0.f, 0.f, 0.f, 0.f);
-                const float4 h4 = (ok && carry) ? *(reinterpret_cast<const float4*>(carry + (size_t)ch * s + j0) + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+                const bool ok = ok_ch && (j0 + q * QS) < s;
+                const float4 r4 = ok ? __ldg(reinterpret_cast<const float4*>(p.rates + (size_t)ch * s + j0 + q * QS)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                const float4 h4 = (ok && carry) ? *(reinterpret_cast<const float4*>(carry + (size_t)ch * s + j0 + q * QS)) : make_float4(0.f, 0.f, 0.f, 0.f);
                 Av[q * 4] = r4.x, Av[q * 4 + 1] = r4.y, Av[q * 4 + 2] = r4.z, Av[q * 4 + 3] = r4.w;
                 hv[q * 4] = h4.x, hv[q * 4 + 1] = h4.y, hv[q * 4 + 2] = h4.z, hv[q * 4 + 3] = h4.w;
             }
@@ -207,15 +219,33 @@ __global__ void __launch_bounds__(THR, (ST <= 16 && !TAPE && !EXACT) ? ((THR > 2
         } else {
 #pragma unroll
             for (int jj = 0; jj < ST; ++jj) {
-                bool ok = ok_ch && (j0 + jj) < s;
-                float rate = ok ? __ldg(p.rates + (size_t)ch * s + j0 + jj) : 0.0f;
+                const int j = j0 + jj / 4 * QS + jj % 4;
+                bool ok = ok_ch && j < s;
+                float rate = ok ? __ldg(p.rates + (size_t)ch * s + j) : 0.0f;
                 Av[jj] = EXACT ? rate : rate * 1.4426950408889634f;
-                hv[jj] = (ok && carry) ? carry[(size_t)ch * s + j0 + jj] : 0.0f;
+                hv[jj] = (ok && carry) ? carry[(size_t)ch * s + j] : 0.0f;
             }
         }
     };
     load_state(A, h, i, valid);
     if constexpr (CPT > 1) load_state(A1, h1, i1, valid1);
+    // Small arguments. A slow state's delta * A is near zero, and there the exponential is four packed multiply-adds without a range
+    // reduction, cheap enough to share the exponentials between the XU and the FMA pipe. Two of a thread's eight pairs (three in the map
+    // pass, which forms no y) take that way in every tile whose arguments allow it; a thread's states are interleaved with the other
+    // groups' so that its last pieces come from the slow end of a table of ascending timescales. Us a launch at 32 x 2048, 24 x 2048, 16 x
+    // 2048 and 1 x 8192 tokens (d 768), with one general polynomial pair in eight before: 945 -> 889, 697 -> 619, 539 -> 474, 115 -> 107;
+    // the map pass of 8192 tokens 104 -> 86. The apply pass with 0 / 1 / 3 / 4 pairs: 960 / 922 / 894 / 944.
+    // amax: the largest |rate| of those states; infinite if one is positive or NaN
+    constexpr bool HAS_SMALL = ST == 16 && G == 4 && !TAPE && !EXACT;
+    constexpr int kSmallFrom = ST - (MAPS ? 6 : 4);
+    float amax = 0.0f;
+    if constexpr (HAS_SMALL) {
+#pragma unroll
+        for (int jj = kSmallFrom; jj < ST; ++jj) {
+            amax = A[jj] <= 0.0f ? fmaxf(amax, -A[jj]) : CUDART_INF_F;
+            if constexpr (CPT > 1) amax = A1[jj] <= 0.0f ? fmaxf(amax, -A1[jj]) : CUDART_INF_F;
+        }
+    }
     float sum_t = 0.0f, sum_t1 = 0.0f;  // MAPS: delta summed over the tile, and over the chunk in f64
     double sum_d = 0.0, sum_d1 = 0.0;
 
@@ -248,7 +278,7 @@ __global__ void __launch_bounds__(THR, (ST <= 16 && !TAPE && !EXACT) ? ((THR > 2
                 for (int idx = tid; idx < nt * SQ; idx += kThreads) {
                     int tt = idx / SQ, q = idx % SQ;
                     int j = q * 4;
-                    int dst = tt * SP + (j / ST) * SG + j % ST;
+                    int dst = tt * SP + j;
                     size_t gro = (row0 + t0 + tt) * ldbc + j;
                     if (j < s) {
                         cp_async16(db + dst, p.b_proj + gro);
@@ -268,7 +298,7 @@ __global__ void __launch_bounds__(THR, (ST <= 16 && !TAPE && !EXACT) ? ((THR > 2
                 }
                 for (int idx = tid; idx < nt * ST * G; idx += kThreads) {
                     int tt = idx / (ST * G), j = idx % (ST * G);
-                    int dst = tt * SP + (j / ST) * SG + j % ST;
+                    int dst = tt * SP + j;
                     size_t gro = (row0 + t0 + tt) * ldbc + j;
                     db[dst] = j < s ? __ldg(p.b_proj + gro) : 0.0f;
                     dc[dst] = j < s ? __ldg(p.c_proj + gro) : 0.0f;
@@ -292,9 +322,11 @@ __global__ void __launch_bounds__(THR, (ST <= 16 && !TAPE && !EXACT) ? ((THR > 2
         const int nt = min(kTileTokens, len - t0);
         float* dd = sm_delta + st * kTileTokens * CH;
         const float* dx = sm_x + st * kTileTokens * CH;
-        const float* db = sm_b + st * kTileTokens * SP + g * SG;
-        const float* dc = sm_c + st * kTileTokens * SP + g * SG;
-        auto token = [&](int tt) {
+        const float* db = sm_b + st * kTileTokens * SP + j0;
+        const float* dc = sm_c + st * kTileTokens * SP + j0;
+        // one token's recurrence; yp, ypb: this thread's part of y
+        auto token = [&](int tt, auto small_args, float& yp, float& ypb) {
+            constexpr bool SMALL = decltype(small_args)::value;
             float dl, xv, dlb = 0.0f, xvb = 0.0f;
             if constexpr (CPT > 1) {  // both channels' values with one 8-byte load each
                 const float2 d2 = *reinterpret_cast<const float2*>(dd + tt * CH + 2 * c);
@@ -308,13 +340,13 @@ __global__ void __launch_bounds__(THR, (ST <= 16 && !TAPE && !EXACT) ? ((THR > 2
             float bj[ST], cj[ST];
 #pragma unroll
             for (int q = 0; q < ST / 4; ++q) {
-                float4 vb = *reinterpret_cast<const float4*>(db + tt * SP + q * 4);
+                float4 vb = *reinterpret_cast<const float4*>(db + tt * SP + q * QS);
                 float4 vc = make_float4(0.f, 0.f, 0.f, 0.f);
-                if constexpr (!MAPS) vc = *reinterpret_cast<const float4*>(dc + tt * SP + q * 4);
+                if constexpr (!MAPS) vc = *reinterpret_cast<const float4*>(dc + tt * SP + q * QS);
                 bj[q * 4] = vb.x, bj[q * 4 + 1] = vb.y, bj[q * 4 + 2] = vb.z, bj[q * 4 + 3] = vb.w;
                 cj[q * 4] = vc.x, cj[q * 4 + 1] = vc.y, cj[q * 4 + 2] = vc.z, cj[q * 4 + 3] = vc.w;
             }
-            float yp = 0.0f, ypb = 0.0f;
+            yp = 0.0f, ypb = 0.0f;
             float av[TAPE ? ST : 1], bv[TAPE ? ST : 1];
             if (EXACT) {
 #pragma unroll
@@ -338,16 +370,15 @@ __global__ void __launch_bounds__(THR, (ST <= 16 && !TAPE && !EXACT) ? ((THR > 2
                     // one pair of exponentials in eight goes to the FMA pipe (the benchmark's launch: 976 us with none, 952 with
                     // one, 1059 with two, whose extra issue slots cost more than the XU pipe gains)
                     // (the map pass, which has no y to form, takes two: 109 -> 105 us for 8192 tokens)
-                    const bool poly = ST == 16 && G == 4 && !TAPE && (jj == 0 || (MAPS && jj == 8));
-                    const f32x2 arg = mul2(dl2, pack2(A[jj], A[jj + 1]));
-                    const f32x2 a2 = poly ? exp2_poly2(arg) : exp2_approx2(arg);
+                    const bool poly = !SMALL && ST == 16 && G == 4 && !TAPE && (jj == 0 || (MAPS && jj == 8));
+                    auto exp2_of = [&](f32x2 x) { return SMALL && jj >= kSmallFrom ? exp2_small2(x) : poly ? exp2_poly2(x) : exp2_approx2(x); };
+                    const f32x2 a2 = exp2_of(mul2(dl2, pack2(A[jj], A[jj + 1])));
                     f32x2 h2 = fma2(a2, pack2(h[jj], h[jj + 1]), mul2(w2, b2));
                     unpack2(h2, h[jj], h[jj + 1]);
                     if constexpr (!MAPS) y2 = fma2(h2, c2, y2);
                     if (TAPE) unpack2(a2, av[jj], av[jj + 1]), bv[jj] = dl * bj[jj], bv[jj + 1] = dl * bj[jj + 1];
                     if constexpr (CPT > 1) {
-                        const f32x2 argb = mul2(dlb2, pack2(A1[jj], A1[jj + 1]));
-                        f32x2 hb2 = fma2(poly ? exp2_poly2(argb) : exp2_approx2(argb), pack2(h1[jj], h1[jj + 1]), mul2(wb2, b2));
+                        f32x2 hb2 = fma2(exp2_of(mul2(dlb2, pack2(A1[jj], A1[jj + 1]))), pack2(h1[jj], h1[jj + 1]), mul2(wb2, b2));
                         unpack2(hb2, h1[jj], h1[jj + 1]);
                         if constexpr (!MAPS) yb2 = fma2(hb2, c2, yb2);
                     }
@@ -360,24 +391,13 @@ __global__ void __launch_bounds__(THR, (ST <= 16 && !TAPE && !EXACT) ? ((THR > 2
                     ypb = y_lo + y_hi;
                 }
             }
-            if constexpr (MAPS) {
-                sum_t += dl, sum_t1 += dlb;
-                return;
-            }
-#pragma unroll
-            for (int m = LPG; m < 32; m <<= 1) yp += __shfl_xor_sync(0xffffffffu, yp, m);
-            if constexpr (CPT > 1) {
-#pragma unroll
-                for (int m = LPG; m < 32; m <<= 1) ypb += __shfl_xor_sync(0xffffffffu, ypb, m);
-                if (g == 0) *reinterpret_cast<float2*>(dd + tt * CH + 2 * c) = make_float2(yp, ypb);
-            } else {
-                if (g == 0) dd[tt * CH + c] = yp;  // every reader of this delta slot sits in this warp and has read it
-            }
+            if constexpr (MAPS) sum_t += dl, sum_t1 += dlb;
             if (TAPE) {
 #pragma unroll
                 for (int jj = 0; jj < ST; ++jj) {
-                    if (valid && j0 + jj < s) {
-                        size_t o = row * ds + (size_t)i * s + j0 + jj;
+                    const int j = j0 + jj / 4 * QS + jj % 4;
+                    if (valid && j < s) {
+                        size_t o = row * ds + (size_t)i * s + j;
                         if (p.states) p.states[o] = h[jj];
                         if (p.bar_a) p.bar_a[o] = av[jj];
                         if (p.bar_b) p.bar_b[o] = bv[jj];
@@ -385,12 +405,80 @@ __global__ void __launch_bounds__(THR, (ST <= 16 && !TAPE && !EXACT) ? ((THR > 2
                 }
             }
         };
-        if (nt == kTileTokens) {
+        // y of one token: a shuffle tree over the G groups. (Every reader of the delta slot it goes to sits in this warp and has read it.)
+        auto finish = [&](int tt, float yp, float ypb) {
+            if constexpr (MAPS) return;
+#pragma unroll
+            for (int m = LPG; m < 32; m <<= 1) yp += __shfl_xor_sync(0xffffffffu, yp, m);
+            if constexpr (CPT > 1) {
+#pragma unroll
+                for (int m = LPG; m < 32; m <<= 1) ypb += __shfl_xor_sync(0xffffffffu, ypb, m);
+                if (g == 0) *reinterpret_cast<float2*>(dd + tt * CH + 2 * c) = make_float2(yp, ypb);
+            } else {
+                if (g == 0) dd[tt * CH + c] = yp;
+            }
+        };
+        // The same sums for four tokens over four groups at once, each group ending with its token: three shuffles instead of eight and one
+        // store instead of four, and the tokens' operand loads are not held up behind one another's stores.
+        auto sum_four = [&](const float* v) {
+            const bool odd = g & 1, high = g & 2;
+            const float r0 = (odd ? v[1] : v[0]) + __shfl_xor_sync(0xffffffffu, odd ? v[0] : v[1], LPG);
+            const float r1 = (odd ? v[3] : v[2]) + __shfl_xor_sync(0xffffffffu, odd ? v[2] : v[3], LPG);
+            return (high ? r1 : r0) + __shfl_xor_sync(0xffffffffu, high ? r0 : r1, 2 * LPG);
+        };
+        const std::false_type any{};
+        auto tile = [&](auto small_args) {
+            int tt = 0;
+            if (G == 4 && (decltype(small_args)::value || nt == kTileTokens)) {
+#pragma unroll 1
+                for (int t4 = 0; t4 < kTileTokens; t4 += 4) {
+                    float yv[4], yw[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) token(t4 + u, small_args, yv[u], yw[u]);
+                    if constexpr (MAPS) continue;
+                    const float y = sum_four(yv);
+                    if constexpr (CPT > 1) {
+                        *reinterpret_cast<float2*>(dd + (t4 + g) * CH + 2 * c) = make_float2(y, sum_four(yw));
+                    } else {
+                        dd[(t4 + g) * CH + c] = y;
+                    }
+                }
+                return;
+            } else if (nt == kTileTokens) {
 #pragma unroll 4
-            for (int tt = 0; tt < kTileTokens; ++tt) token(tt);
-        } else {
-            for (int tt = 0; tt < nt; ++tt) token(tt);
+                for (; tt < kTileTokens; ++tt) {
+                    float yp, ypb;
+                    token(tt, small_args, yp, ypb);
+                    finish(tt, yp, ypb);
+                }
+            }
+            for (; tt < nt; ++tt) {
+                float yp, ypb;
+                token(tt, any, yp, ypb);
+                finish(tt, yp, ypb);
+            }
+        };
+        bool small = HAS_SMALL && nt == kTileTokens;
+        if constexpr (HAS_SMALL) {
+            // largest delta of the warp's channels over the tile, each group of lanes looking at its share of the tokens: bit
+            // patterns compare like the numbers, and negative deltas and NaNs lie above all others
+            unsigned top = 0;
+#pragma unroll
+            for (int t = 0; t < kTileTokens / G; ++t) {
+                const float* dp = dd + (t * G + g) * CH + CPT * c;
+                if constexpr (CPT > 1) {
+                    const uint2 v = *reinterpret_cast<const uint2*>(dp);
+                    top = max(top, max(v.x, v.y));
+                } else {
+                    top = max(top, *reinterpret_cast<const unsigned*>(dp));
+                }
+            }
+#pragma unroll
+            for (int m = LPG; m < 32; m <<= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, m));
+            small = __all_sync(0xffffffffu, small && __uint_as_float(top) * amax <= kSmallArg && top < 0x80000000u);
         }
+        if (HAS_SMALL && small) tile(std::integral_constant<bool, HAS_SMALL>{});
+        else tile(any);
         if constexpr (MAPS) {
             sum_d += (double)sum_t, sum_d1 += (double)sum_t1, sum_t = sum_t1 = 0.0f;
             continue;
@@ -433,8 +521,8 @@ __global__ void __launch_bounds__(THR, (ST <= 16 && !TAPE && !EXACT) ? ((THR > 2
             if (g == 0 && ok_ch) rec[ch] = (float)sum;
 #pragma unroll
             for (int q = 0; q < ST / 4; ++q)
-                if (ok_ch && j0 + q * 4 < s)
-                    *(reinterpret_cast<float4*>(rec + d + (size_t)ch * s + j0) + q) = make_float4(hv[q * 4], hv[q * 4 + 1], hv[q * 4 + 2], hv[q * 4 + 3]);
+                if (ok_ch && j0 + q * QS < s)
+                    *reinterpret_cast<float4*>(rec + d + (size_t)ch * s + j0 + q * QS) = make_float4(hv[q * 4], hv[q * 4 + 1], hv[q * 4 + 2], hv[q * 4 + 3]);
         };
         store_map(h, i, valid, sum_d);
         if constexpr (CPT > 1) store_map(h1, i1, valid1, sum_d1);
@@ -445,12 +533,14 @@ __global__ void __launch_bounds__(THR, (ST <= 16 && !TAPE && !EXACT) ? ((THR > 2
             if (vec_state) {
 #pragma unroll
                 for (int q = 0; q < ST / 4; ++q)
-                    if (ok_ch && j0 + q * 4 < s)
-                        *(reinterpret_cast<float4*>(carry + (size_t)ch * s + j0) + q) = make_float4(hv[q * 4], hv[q * 4 + 1], hv[q * 4 + 2], hv[q * 4 + 3]);
+                    if (ok_ch && j0 + q * QS < s)
+                        *reinterpret_cast<float4*>(carry + (size_t)ch * s + j0 + q * QS) = make_float4(hv[q * 4], hv[q * 4 + 1], hv[q * 4 + 2], hv[q * 4 + 3]);
             } else {
 #pragma unroll
-                for (int jj = 0; jj < ST; ++jj)
-                    if (ok_ch && j0 + jj < s) carry[(size_t)ch * s + j0 + jj] = hv[jj];
+                for (int jj = 0; jj < ST; ++jj) {
+                    const int j = j0 + jj / 4 * QS + jj % 4;
+                    if (ok_ch && j < s) carry[(size_t)ch * s + j] = hv[jj];
+                }
             }
         };
         store_state(h, i, valid);
@@ -965,7 +1055,7 @@ template <int ST, int G, bool EXACT, bool TAPE, int THR = kThreads, int CPT = 1,
 int32_t launch_cfg(pssa_b200_ctx* ctx, const SsmParams& p) {
     constexpr int kThreads = THR;
     constexpr int CH = kThreads / G * CPT;
-    constexpr int SP = (ST + 4) * G;
+    constexpr int SP = ST * G;
     constexpr int kTileTokens = kTileTokensFor<G>;
     size_t smem = (size_t)kStages * kTileTokens * (2 * CH + 2 * SP) * sizeof(float);
     auto kern = ssm_fused_kernel<ST, G, EXACT, TAPE, THR, CPT, MAPS>;
@@ -1127,7 +1217,7 @@ int32_t launch_ssm_fused(pssa_b200_ctx* ctx, const SsmParams& p, bool exact) {
         if (channels <= (exact ? 2 : 1) * schedulers && !by_shape) return launch_wide<32, 2, 32>(ctx, p, exact);
         if (channels <= 4 * schedulers) return launch_wide<16, 4, 32>(ctx, p, exact);
         const double wide_us = 13.8 * (double)channels / (double)schedulers;
-        const double tiled_us = 66.0 + 70.0 * (double)tiled_shape(ctx, p.d, lanes).busiest;
+        const double tiled_us = 60.0 + 64.5 * (double)tiled_shape(ctx, p.d, lanes).busiest;
         if (exact || tape || by_shape || wide_us < tiled_us) return launch_wide<16, 4, 16>(ctx, p, exact);
     }
     if (exact) {

@@ -196,3 +196,43 @@ def test_edge_values_of_the_decay_reach_every_state(gpu, s, exact):
     assert np.max(np.abs(got[fin] - want[fin]) / np.maximum(size[fin], 1e-30)) <= 2 * (3 * 128 * 2.0 ** -24 + 2.0 ** -22)  # two tokens
     with np.errstate(all="ignore"):
         assert np.array_equal(np.isnan(y.cpu().numpy()[1]), np.isnan((want * c[1]).sum(1)))
+
+
+# (lanes, d): two channels a thread, 352 and 256 threads a CTA (one, 16 and 48 lanes of 768 channels); whole tiles, a tail, ragged states
+@pytest.mark.parametrize("lanes,d,s,T", [(1, 68, 48, 101), (16, 768, 36, 64), (48, 768, 48, 35)])
+def test_small_argument_tiles_and_their_borders(gpu, lanes, d, s, T):
+    """Tiles whose exponents allow the polynomial of small arguments beside tiles that do not: a delta at, past and far past its
+    limit, negative, infinite and NaN deltas, rates of zero, of the other sign and NaN among the states it serves."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(d + s)
+    f = lambda *sh: torch.randn(*sh, device="cuda", generator=g)  # noqa: E731
+    rows = lanes * T
+    delta = torch.rand(rows, d, device="cuda", generator=g)
+    rates = -torch.exp(torch.empty(d, s, device="cuda").uniform_(-5.0, -1.4, generator=g))  # all below 0.4 / log2(e) = 0.277
+    rates[4, 33], rates[5, 34], rates[6, 33], rates[7, 35] = 0.0, 0.02, float("nan"), 0.277
+    t = T - 1 if T < 64 else 40  # in the tail or in the second tile; the first whole tile stays small
+    for ch, v in ((8, 0.4 / 1.4427 / 0.25), (9, 3.0), (10, -1.0), (11, float("inf")), (12, float("nan")), (13, 60.0)):
+        delta[t, ch] = v
+    bp, cp, x, h0 = f(rows, s), f(rows, s), f(rows, d), f(lanes, d * s)
+    off, ln = (np.arange(lanes) * T).astype(np.uint32), np.full(lanes, T, np.uint32)
+    carry, y = h0.clone(), torch.zeros(rows, d, device="cuda")
+    gpu.set_stream(torch.cuda.current_stream())
+    gpu.ssm_forward_dev(delta, bp, cp, x, rates, carry, y, off, ln, rows, d, s)
+    torch.cuda.synchronize()
+    gpu.set_stream(None)
+    q = lambda a, w: a.double().reshape(lanes, T, w)  # noqa: E731
+    dl, b, c, xv, want = q(delta, d), q(bp, s), q(cp, s), q(x, d), h0.double().reshape(lanes, d, s)
+    size = want.abs()  # of the terms: they can cancel
+    for i in range(T):
+        a = torch.exp(dl[:, i, :, None] * rates.double())
+        u = (dl[:, i] * xv[:, i])[:, :, None] * b[:, i, None, :]
+        want, size = a * want + u, a * size + u.abs()
+        got, ref, mag = q(y, d)[:, i], (want * c[:, i, None, :]).sum(2), (size * c[:, i, None, :].abs()).sum(2)
+        assert torch.equal(torch.isnan(got), torch.isnan(ref))
+        # a token: the argument's two roundings (2^-24 of at most 60 * 0.25 / ln 2 = 22) and the exponential's 2^-22; sums 2^-24 each
+        fin = torch.isfinite(ref)
+        assert float(((got - ref).abs() / mag)[fin].max()) <= (i + 1) * 2.0 ** -22 + (2 * 22 + s) * 2.0 ** -24
+    got, want, size = carry.double().reshape(lanes, d, s), want, size
+    assert torch.equal(torch.isnan(got), torch.isnan(want))
+    fin = torch.isfinite(want)
+    assert float(((got - want).abs() / size)[fin].max()) <= T * 2.0 ** -22 + 2 * 22 * 2.0 ** -24
