@@ -1006,8 +1006,11 @@ __global__ void __launch_bounds__(256) sum_delta_kernel(const float* __restrict_
     }
 }
 
-// One thread per (lane, channel, state): walks the shard maps of every rank and time chunk in time order.
-__global__ void __launch_bounds__(256) seqpar_fold_kernel(const float* __restrict__ gathered, size_t rec, int world, int rank,
+// One thread per (lane, channel, state): walks the shard maps of every rank and time chunk in time order. The records do not depend
+// on h, so a batch of them is always on its way while the batch before goes through its dependent multiply-adds: what is left
+// is a few trips to L2, where the map pass has just left the records (37 chunks of 768 x 64 states: 31 -> 12 us, of which about 5 are
+// the launch; before, a division per record and loads that waited for the batch before them).
+__global__ void __launch_bounds__(128) seqpar_fold_kernel(const float* __restrict__ gathered, size_t rec, int world, int rank,
                                                           int chunks, size_t rank_stride, const float* __restrict__ rates,
                                                           float* __restrict__ state, size_t state_stride,
                                                           const uint32_t* __restrict__ lane_slots, float* __restrict__ carry_in,
@@ -1018,34 +1021,34 @@ __global__ void __launch_bounds__(256) seqpar_fold_kernel(const float* __restric
     const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = blockIdx.y;
     if (e >= ds) return;
-    const int i = (int)(e / s);
+    const int i = (int)((unsigned)e / (unsigned)s);
     float* st = state + (size_t)(lane_slots ? lane_slots[lane] : lane) * state_stride;
     const float a = rates[e];
     float h = st[e];
-    // the records are independent of h: twelve of them are requested (and their decay factors formed) before the
-    // dependent multiply-adds, so the walk is not one memory round trip per record
-    constexpr int U = 12;
-    const int n = world * chunks;
-    for (int j0 = 0; j0 < n; j0 += U) {
-        float pk[U], add[U];
+    constexpr int U = 10;
+    for (int k = 0; k < world; ++k) {
+        const float* r = gathered + (size_t)k * rank_stride + (size_t)lane * chunks * rec;
+        float* out = k == rank ? carry_in + (size_t)lane * chunks * ds + e : nullptr;
+        float sum[U], add[U];
+        auto request = [&](int left) {
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int j = j0 + u;
-            if (j < n) {
-                const int k = j / chunks, c = j - k * chunks;
-                const float* r = gathered + (size_t)k * rank_stride + ((size_t)lane * chunks + c) * rec;
-                pk[u] = exp_exact(__fmul_rn(a, __ldg(r + i)));
-                add[u] = __ldg(r + d + e);
-            }
-        }
+            for (int u = 0; u < U; ++u)
+                if (u < left) sum[u] = __ldcg(r + i), add[u] = __ldcg(r + d + e), r += rec;
+        };
+        request(chunks);
+        for (int c = 0; c < chunks; c += U) {
+            float pk[U], ad[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int j = j0 + u;
-            if (j < n) {
-                const int k = j / chunks, c = j - k * chunks;
-                if (k == rank) carry_in[((size_t)lane * chunks + c) * ds + e] = h;
-                h = __fadd_rn(__fmul_rn(pk[u], h), add[u]);
-            }
+            for (int u = 0; u < U; ++u) pk[u] = sum[u], ad[u] = add[u];
+            request(chunks - c - U);
+#pragma unroll
+            for (int u = 0; u < U; ++u) pk[u] = u < chunks - c ? exp_exact(__fmul_rn(a, pk[u])) : 0.0f;
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (u < chunks - c) {
+                    if (out) *out = h, out += ds;
+                    h = __fadd_rn(__fmul_rn(pk[u], h), ad[u]);
+                }
         }
     }
     st[e] = h;
@@ -1145,9 +1148,9 @@ int32_t launch_seqpar_fold(pssa_b200_ctx* ctx, const float* gathered, size_t rec
                            size_t rank_stride, const float* rates, float* state, size_t state_stride, const uint32_t* lane_slots,
                            float* carry_in, int d, int s) {
     const size_t ds = (size_t)d * s;
-    dim3 grid((unsigned)((ds + 255) / 256), (unsigned)lanes);
+    dim3 grid((unsigned)((ds + 127) / 128), (unsigned)lanes);
     if (lanes < 1 || lanes > 65535) return fail(ctx, PSSA_B200_ERR_SHAPE, "chunk fold: %d lanes outside 1..65535", lanes);
-    PSSA_CUDA(ctx, launch_dependent(seqpar_fold_kernel, grid, dim3(256), 0, ctx->stream, gathered, rec, world, rank, chunks, rank_stride, rates, state,
+    PSSA_CUDA(ctx, launch_dependent(seqpar_fold_kernel, grid, dim3(128), 0, ctx->stream, gathered, rec, world, rank, chunks, rank_stride, rates, state,
                                     state_stride, lane_slots, carry_in, d, s));
     return after_launch(ctx, "seqpar_fold_kernel");
 }
