@@ -1071,7 +1071,8 @@ int32_t launch_cfg(pssa_b200_ctx* ctx, const SsmParams& p) {
     size_t blocks = (size_t)ncb * p.lanes;
     if (blocks > 0x7fffffffull)
         return fail(ctx, PSSA_B200_ERR_SHAPE, "B200 SSM grid (%zu, 1) exceeds grid limits; refusing launch", blocks);
-    PSSA_CUDA(ctx, launch_dependent(kern, dim3((unsigned)blocks), dim3(kThreads), smem, ctx->stream, p));
+    static PerDeviceCount resident;
+    PSSA_CUDA(ctx, launch_spread(resident, ctx->device, ctx->sm_count, kern, dim3((unsigned)blocks), dim3(kThreads), smem, ctx->stream, p));
     return after_launch(ctx, MAPS ? "ssm_fused_kernel[chunk maps]" : "ssm_fused_kernel");
 }
 
@@ -1088,7 +1089,8 @@ int32_t launch_wide_cfg(pssa_b200_ctx* ctx, const SsmParams& p) {
     const size_t blocks = (size_t)((p.d + CH - 1) / CH) * p.lanes;
     if (blocks > 0x7fffffffull)
         return fail(ctx, PSSA_B200_ERR_SHAPE, "B200 SSM grid (%zu, 1) exceeds grid limits; refusing launch", blocks);
-    PSSA_CUDA(ctx, launch_dependent(kern, dim3((unsigned)blocks), dim3(kWideWarps * 32), smem, ctx->stream, p));
+    static PerDeviceCount resident;
+    PSSA_CUDA(ctx, launch_spread(resident, ctx->device, ctx->sm_count, kern, dim3((unsigned)blocks), dim3(kWideWarps * 32), smem, ctx->stream, p));
     return after_launch(ctx, "ssm_fused_kernel[few lanes]");
 }
 template <int LPC, int SPL, int TT>
@@ -1163,10 +1165,13 @@ size_t ssm_time_chunks(const pssa_b200_ctx* ctx, const SsmParams& p, bool exact)
         if (exact || p.s < 64) {
             if (!exact || longest < 4096 || 2 * p.rows * (size_t)p.d > 3 * longest * schedulers) return 1;
         } else {
-            // CTAs of 64 channels, three to an SM. Us per pass of the 12-block model, few lanes against this: 1 lane of 1024 tokens
-            // 1888 and 2047, 2048 2825 -> 2550, 8192 7749 -> 5050; 2 lanes of 2048 3149 and 3543, 4096 4880 and 5355.
+            // CTAs of 64 channels, three to an SM. Us per pass of the 12-block model (d 768), few lanes against this: 1 lane of 512
+            // tokens 1231 and 1339, 1024 1508 -> 1476, 2048 2210 -> 1961, 8192 6246 -> 4288; 2 lanes of 2048 2825 and 2842, 4096
+            // 4789 -> 4364; 3 lanes of 8192 9968 and 10726. One block of d 192: 1 lane of 1024 105 -> 103, 4096 213 -> 129, 4 lanes 300 -> 226,
+            // 8 lanes 418 -> 378.
             const size_t n = std::min<size_t>({(size_t)kMaxTimeChunks, 3 * (size_t)ctx->sm_count / std::max<size_t>(1, ctas), longest / 64});
-            return longest >= 2048 && n >= 30 ? n : 1;
+            const size_t channels = (size_t)p.lanes * p.d;
+            return channels <= 3 * schedulers && longest >= (2 * channels <= 3 * schedulers ? 1024u : 2560u) ? n : 1;
         }
     }
     if (ctas > (size_t)ctx->sm_count) return 1;
