@@ -136,12 +136,13 @@ inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 bl
 // An early dependent start places CTAs on whichever SMs the predecessor frees first, as many as fit: a grid that does not fill the
 // machine then crowds on some SMs and leaves others empty (the fused SSM of 16 lanes of 1024 tokens at d 768: 635 us a launch in a
 // stream where it takes 435 evenly spread). So a long kernel of several small CTAs to an SM starts early only when the fullest
-// SM is as full either way. `resident`: the kernel's CTAs to an SM, asked for once per device.
+// SM is as full either way, or holds at least 1 / `slack` of what fits, where that many hide its latency. `resident`: the kernel's
+// CTAs to an SM, asked for once per device.
 struct PerDeviceCount {
     std::atomic<int> n[64]{};
 };
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_spread(PerDeviceCount& resident, int device, int sm_count, void (*kernel)(KArgs...), dim3 grid, dim3 block,
+inline cudaError_t launch_spread(PerDeviceCount& resident, int slack, int device, int sm_count, void (*kernel)(KArgs...), dim3 grid, dim3 block,
                                  size_t smem, cudaStream_t stream, Args... args) {
     const bool known = device >= 0 && device < 64;
     int per_sm = known ? resident.n[device].load(std::memory_order_relaxed) : 0;
@@ -151,7 +152,7 @@ inline cudaError_t launch_spread(PerDeviceCount& resident, int device, int sm_co
         if (known) resident.n[device].store(per_sm, std::memory_order_relaxed);
     }
     const size_t blocks = (size_t)grid.x * grid.y * grid.z, even = (blocks + sm_count - 1) / sm_count;
-    if (even >= (size_t)per_sm) return launch_dependent(kernel, grid, block, smem, stream, args...);
+    if (even * slack >= (size_t)per_sm) return launch_dependent(kernel, grid, block, smem, stream, args...);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid, cfg.blockDim = block, cfg.dynamicSmemBytes = smem, cfg.stream = stream;
     return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);

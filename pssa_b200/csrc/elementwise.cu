@@ -349,9 +349,13 @@ int32_t launch_embed_norm(pssa_b200_ctx* ctx, const float* embed, const uint32_t
     if (exact)
         PSSA_CUDA(ctx, launch_dependent(embed_norm_kernel<true>, dim3(blocks), dim3(256), smem, ctx->stream, embed, ids, feats, gamma, beta,
                                         x_norm, (__nv_bfloat16*)x_bf16, rows, d, (uint32_t)vocab, ctx->status_dev));
-    else
-        PSSA_CUDA(ctx, launch_dependent(embed_norm_kernel<false>, dim3(blocks), dim3(256), smem, ctx->stream, embed, ids, feats, gamma, beta,
-                                        x_norm, (__nv_bfloat16*)x_bf16, rows, d, (uint32_t)vocab, ctx->status_dev));
+    else {
+        // a few hundred rows started early would share a handful of SMs (512 rows of the 12-block model: 1226 -> 1202 us a pass); with
+        // half of the machine's CTAs or more the early start is worth its latency (8192 rows: 3433 us against 3443)
+        static PerDeviceCount resident;
+        PSSA_CUDA(ctx, launch_spread(resident, 2, ctx->device, ctx->sm_count, embed_norm_kernel<false>, dim3(blocks), dim3(256), smem, ctx->stream,
+                                     embed, ids, feats, gamma, beta, x_norm, (__nv_bfloat16*)x_bf16, rows, d, (uint32_t)vocab, ctx->status_dev));
+    }
     return after_launch(ctx, "embed_norm_kernel");
 }
 

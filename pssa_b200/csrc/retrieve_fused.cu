@@ -1152,7 +1152,15 @@ int32_t launch_retrieve_all_fused(pssa_b200_ctx* ctx, const RetrieveParams& p) {
             PSSA_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             attr[which].done(ctx->device);
         }
-        PSSA_CUDA(ctx, launch_dependent(kernel, dim3(grid), dim3(kThreads), smem, ctx->stream, map_b, q));
+        // An early start hides this launch's latency, but from about 64 tiles up it costs more than that somewhere in the chain of
+        // dependent launches (a pass of the 12-block model, early against in order: 512 rows 1226 and 1258 us, 4096 2448 and 2454, 8192
+        // 3958 and 3925, 16384 7093 and 6959, 65536 21570 and 21019; breaking the chain at the products instead gives the same, both
+        // together no more)
+        if (tiles < 64) {
+            PSSA_CUDA(ctx, launch_dependent(kernel, dim3(grid), dim3(kThreads), smem, ctx->stream, map_b, q));
+        } else {
+            kernel<<<grid, kThreads, smem, ctx->stream>>>(map_b, q);
+        }
         return PSSA_B200_OK;
     };
     rc = p.dk == 64 ? go(retrieve_topk_fused_kernel<64, 9, true>, 0) : go(retrieve_topk_fused_kernel<128, 9, true>, 1);

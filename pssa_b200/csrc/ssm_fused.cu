@@ -1072,7 +1072,7 @@ int32_t launch_cfg(pssa_b200_ctx* ctx, const SsmParams& p) {
     if (blocks > 0x7fffffffull)
         return fail(ctx, PSSA_B200_ERR_SHAPE, "B200 SSM grid (%zu, 1) exceeds grid limits; refusing launch", blocks);
     static PerDeviceCount resident;
-    PSSA_CUDA(ctx, launch_spread(resident, ctx->device, ctx->sm_count, kern, dim3((unsigned)blocks), dim3(kThreads), smem, ctx->stream, p));
+    PSSA_CUDA(ctx, launch_spread(resident, 1, ctx->device, ctx->sm_count, kern, dim3((unsigned)blocks), dim3(kThreads), smem, ctx->stream, p));
     return after_launch(ctx, MAPS ? "ssm_fused_kernel[chunk maps]" : "ssm_fused_kernel");
 }
 
@@ -1090,7 +1090,7 @@ int32_t launch_wide_cfg(pssa_b200_ctx* ctx, const SsmParams& p) {
     if (blocks > 0x7fffffffull)
         return fail(ctx, PSSA_B200_ERR_SHAPE, "B200 SSM grid (%zu, 1) exceeds grid limits; refusing launch", blocks);
     static PerDeviceCount resident;
-    PSSA_CUDA(ctx, launch_spread(resident, ctx->device, ctx->sm_count, kern, dim3((unsigned)blocks), dim3(kWideWarps * 32), smem, ctx->stream, p));
+    PSSA_CUDA(ctx, launch_spread(resident, 1, ctx->device, ctx->sm_count, kern, dim3((unsigned)blocks), dim3(kWideWarps * 32), smem, ctx->stream, p));
     return after_launch(ctx, "ssm_fused_kernel[few lanes]");
 }
 template <int LPC, int SPL, int TT>
