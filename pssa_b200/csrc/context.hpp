@@ -136,7 +136,7 @@ inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 bl
 // An early dependent start places CTAs on whichever SMs the predecessor frees first, as many as fit: a grid that does not fill the
 // machine then crowds on some SMs and leaves others empty (the fused SSM of 16 lanes of 1024 tokens at d 768: 635 us a launch in a
 // stream where it takes 435 evenly spread). So a long kernel of several small CTAs to an SM starts early only when the fullest
-// SM is as full either way, or holds at least 1 / `slack` of what fits, where that many hide its latency. `resident`: the kernel's
+// SM is as full either way, or holds at least 1 / `slack` of what fits, where that many hide its latency (0: never). `resident`: the kernel's
 // CTAs to an SM, asked for once per device.
 struct PerDeviceCount {
     std::atomic<int> n[64]{};

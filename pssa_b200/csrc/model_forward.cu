@@ -157,6 +157,22 @@ int32_t dense(pssa_b200_model* m, const float* x32, const void* x16, const float
     return launch_gemm_bf16(m->ctx, x16, w16, out, out_bf16, rows, n, k, ldo, epi, alpha);
 }
 
+// Lanes in the order the SSM stage takes them: longest first, so that the CTAs of long lanes start first and are spread over the SMs
+// (everything else is per row, and the head's rows are listed apart). Not for explicit lane groups,
+// which are ranges of rows, nor in the sequence-parallel mode, whose record order all ranks share.
+void longest_first(const pssa_b200_model* m, std::vector<uint32_t>& off, std::vector<uint32_t>& len, std::vector<uint32_t>& slot) {
+    if (m->lane_groups > 1 || m->sp.world > 1) return;
+    auto longer = [&](uint32_t a, uint32_t b) { return len[a] > len[b]; };
+    std::vector<uint32_t> order(len.size());
+    for (size_t l = 0; l < order.size(); ++l) order[l] = (uint32_t)l;
+    if (std::is_sorted(order.begin(), order.end(), longer)) return;
+    std::stable_sort(order.begin(), order.end(), longer);
+    for (auto* v : {&off, &len, &slot}) {
+        const std::vector<uint32_t> was = *v;
+        for (size_t l = 0; l < order.size(); ++l) (*v)[l] = was[order[l]];
+    }
+}
+
 // One pass: `rows` packed token rows of `lanes` lanes already described in the workspace (ids, lane_off, lane_len,
 // lane_slot, last_rows). Leaves the final features of every row in ws.feat_a or feat_b (returned).
 int32_t forward_rows(pssa_b200_model* m, size_t rows, size_t lanes, const uint32_t* h_off, const uint32_t* h_len, float** feats_out,
@@ -183,6 +199,7 @@ int32_t forward_rows(pssa_b200_model* m, size_t rows, size_t lanes, const uint32
     ssm.ld_delta = nc, ssm.ld_bc = nc, ssm.lane_slots = ws.lane_slot, ssm.carry_stride = m->depth * m->loops * ds;
     ssm.aligned = ssm_vector_ok(ssm);
     ssm.single_token = single_token, ssm.max_len = (int)max_len;
+    ssm.ragged = lanes > 1 && 8 * rows < 7 * lanes * max_len && std::is_sorted(h_len, h_len + lanes, [](uint32_t a, uint32_t b) { return a > b; });
     // Time chunks. The SSM kernels parallelise over lanes x channels only; one long sequence can leave most of the machine
     // idle, so each lane can be cut into `n_chunks` consecutive time chunks that run as independent "virtual lanes" in two
     // passes: chunk maps from a zero carry, a fold of the maps in time order, then the real pass with each chunk's
@@ -624,7 +641,7 @@ int32_t run_lanes(pssa_b200_model* m, const uint64_t* ids, const uint32_t* offse
     // window of tokens per lane per pass
     size_t window = std::max<size_t>(1, m->max_rows / n_lanes);
     if (window > max_len) window = max_len;
-    std::vector<uint32_t> h_ids, h_off(n_lanes), h_len(n_lanes), h_slot(n_lanes), h_row_slot, h_last;
+    std::vector<uint32_t> h_ids, h_off(n_lanes), h_len(n_lanes), h_slot(n_lanes), h_row_slot, h_last, s_off, s_len, s_slot;
     int32_t rc;
     for (size_t t0 = 0; t0 < max_len; t0 += window) {
         if (cancelled && cancelled(cancel_arg)) return fail(ctx, PSSA_B200_ERR_CANCELLED, "prefill cancelled after %zu tokens", t0);
@@ -660,11 +677,13 @@ int32_t run_lanes(pssa_b200_model* m, const uint64_t* ids, const uint32_t* offse
             PSSA_CUDA(ctx, cudaMemcpyAsync(ws.row_slot, h_row_slot.data(), rows * 4, cudaMemcpyHostToDevice, st));
             if ((rc = run_decode_step(m, rows, ws.ids, want_head && !h_last.empty() ? ws.logits : nullptr))) return rc;
         } else {
-            PSSA_CUDA(ctx, cudaMemcpyAsync(ws.lane_off, h_off.data(), n_lanes * 4, cudaMemcpyHostToDevice, st));
-            PSSA_CUDA(ctx, cudaMemcpyAsync(ws.lane_len, h_len.data(), n_lanes * 4, cudaMemcpyHostToDevice, st));
-            PSSA_CUDA(ctx, cudaMemcpyAsync(ws.lane_slot, h_slot.data(), n_lanes * 4, cudaMemcpyHostToDevice, st));
+            s_off = h_off, s_len = h_len, s_slot = h_slot;
+            longest_first(m, s_off, s_len, s_slot);
+            PSSA_CUDA(ctx, cudaMemcpyAsync(ws.lane_off, s_off.data(), n_lanes * 4, cudaMemcpyHostToDevice, st));
+            PSSA_CUDA(ctx, cudaMemcpyAsync(ws.lane_len, s_len.data(), n_lanes * 4, cudaMemcpyHostToDevice, st));
+            PSSA_CUDA(ctx, cudaMemcpyAsync(ws.lane_slot, s_slot.data(), n_lanes * 4, cudaMemcpyHostToDevice, st));
             if (!h_last.empty()) PSSA_CUDA(ctx, cudaMemcpyAsync(ws.last_rows, h_last.data(), h_last.size() * 4, cudaMemcpyHostToDevice, st));
-            if ((rc = forward_rows(m, rows, n_lanes, h_off.data(), h_len.data(), &feats, h_last.size()))) return rc;
+            if ((rc = forward_rows(m, rows, n_lanes, s_off.data(), s_len.data(), &feats, h_last.size()))) return rc;
         }
         if (!h_last.empty() && want_head) {
             const bool want_greedy = greedy != nullptr && !sampling;
@@ -760,6 +779,7 @@ int32_t pssa_b200_model_prefill_batch_dev(pssa_b200_model* m, const uint32_t* id
     if (n_lanes == 0 || n_lanes > 0x7fffffff) return fail(ctx, PSSA_B200_ERR_SHAPE, "prefill_batch: lane count must be in 1..2^31-1");
     std::vector<bool> seen(m->max_streams, false);
     std::vector<uint32_t> h_off(n_lanes), h_len(n_lanes), h_slot(n_lanes), h_row_slot, h_last;
+    std::vector<uint32_t> s_off, s_len, s_slot;  // the lanes as the SSM stage takes them
     std::vector<size_t> head_lane;
     size_t rows = 0, span = 0;
     for (size_t l = 0; l < n_lanes; ++l) {
@@ -793,11 +813,13 @@ int32_t pssa_b200_model_prefill_batch_dev(pssa_b200_model* m, const uint32_t* id
     // The lane description is uploaded only when it differs from what the workspace already holds. A repeated call with
     // the same layout (a decode loop) then consists of kernel launches and device-to-device copies only, so the caller can
     // capture it in a CUDA graph on the context's stream.
+    s_off = h_off, s_len = h_len, s_slot = h_slot;
+    longest_first(m, s_off, s_len, s_slot);
     auto& lay = m->dev_layout;
     if (lay.ws_base != ws.base || lay.off != h_off || lay.len != h_len || lay.slot != h_slot) {
-        PSSA_CUDA(ctx, cudaMemcpyAsync(ws.lane_off, h_off.data(), n_lanes * 4, cudaMemcpyHostToDevice, st));
-        PSSA_CUDA(ctx, cudaMemcpyAsync(ws.lane_len, h_len.data(), n_lanes * 4, cudaMemcpyHostToDevice, st));
-        PSSA_CUDA(ctx, cudaMemcpyAsync(ws.lane_slot, h_slot.data(), n_lanes * 4, cudaMemcpyHostToDevice, st));
+        PSSA_CUDA(ctx, cudaMemcpyAsync(ws.lane_off, s_off.data(), n_lanes * 4, cudaMemcpyHostToDevice, st));
+        PSSA_CUDA(ctx, cudaMemcpyAsync(ws.lane_len, s_len.data(), n_lanes * 4, cudaMemcpyHostToDevice, st));
+        PSSA_CUDA(ctx, cudaMemcpyAsync(ws.lane_slot, s_slot.data(), n_lanes * 4, cudaMemcpyHostToDevice, st));
         PSSA_CUDA(ctx, cudaMemcpyAsync(ws.last_rows, h_last.data(), h_last.size() * 4, cudaMemcpyHostToDevice, st));
         PSSA_CUDA(ctx, cudaMemcpyAsync(ws.row_slot, h_row_slot.data(), h_row_slot.size() * 4, cudaMemcpyHostToDevice, st));
         lay.ws_base = ws.base, lay.off = h_off, lay.len = h_len, lay.slot = h_slot;
@@ -840,7 +862,7 @@ int32_t pssa_b200_model_prefill_batch_dev(pssa_b200_model* m, const uint32_t* id
     }
     PSSA_CUDA(ctx, cudaMemcpyAsync(ws.ids, ids_dev, span * 4, cudaMemcpyDeviceToDevice, st));
     m->sp.active = m->sp.world > 1;
-    rc = forward_rows(m, span, n_lanes, h_off.data(), h_len.data(), &feats, h_last.size());
+    rc = forward_rows(m, span, n_lanes, s_off.data(), s_len.data(), &feats, h_last.size());
     m->sp.active = false;
     if (rc) return rc;
     if (logits_dev || greedy_dev) {
@@ -1079,6 +1101,7 @@ int32_t pssa_b200_model_set_seqpar(pssa_b200_model* m, uint32_t rank, uint32_t w
     PSSA_CUDA(ctx, cudaSetDevice(ctx->device));
     PSSA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     m->sp = pssa_b200_model::SeqPar{};
+    m->dev_layout.ws_base = nullptr;  // ranks keep the caller's order of lanes
     if (world <= 1 || !exchange) return PSSA_B200_OK;
     if (rank >= world) return fail(ctx, PSSA_B200_ERR_INVALID_ARGUMENT, "sequence-parallel rank %u outside world of %u", rank, world);
     if (!send_dev || !recv_dev || capacity == 0)

@@ -154,6 +154,16 @@ __device__ __forceinline__ f32x2 exp2_approx2(f32x2 x) {
     return pack2(ex2_approx(x0), ex2_approx(x1));
 }
 
+// Which CTA of the lanes x channel blocks this one is. CTAs go to the SMs in rounds; lanes of different lengths come longest first, and
+// every second round runs backwards, so that an SM with a long lane's CTA of one round gets a shorter one's of the next (seven
+// prompts of 33 to 1501 tokens at d 768: 157 us a launch in the caller's order and with early starts, 143 in this).
+__device__ __forceinline__ unsigned ssm_cta(unsigned per_round) {
+    const unsigned b = blockIdx.x;
+    if (per_round == 0) return b;
+    const unsigned round = b / per_round, first = round * per_round;
+    return (round & 1) && first + per_round <= gridDim.x ? first + (per_round - 1 - (b - first)) : b;
+}
+
 // MAPS: the first of the two passes over time chunks. It leaves every chunk's affine map at `sum_delta` (sum of delta, then the
 // end state from a zero carry) and no y: what would form and store it, a third of the instructions, is not in it.
 template <int ST, int G, bool EXACT, bool TAPE, int THR = kThreads, int CPT = 1, bool MAPS = false>
@@ -181,8 +191,9 @@ __global__ void __launch_bounds__(THR, (ST <= 16 && !TAPE && !EXACT) ? (CPT > 1 
     const int g = lane_id / LPG;
     const int c = (tid >> 5) * LPG + lane_id % LPG;
     const int ncb = (p.d + CH - 1) / CH;
-    const int lane = blockIdx.x / ncb;
-    const int i0 = (blockIdx.x % ncb) * CH;
+    const unsigned cta = ssm_cta(p.ragged);
+    const int lane = cta / ncb;
+    const int i0 = (cta % ncb) * CH;
     const int i = i0 + CPT * c;  // a two-channel thread owns the adjacent channels CPT * c and CPT * c + 1
     const bool valid = i < p.d;
     const size_t row0 = p.offsets ? p.offsets[lane] : 0;
@@ -608,8 +619,9 @@ __global__ void __launch_bounds__(kWideWarps * 32) ssm_wide_kernel(SsmParams p) 
     const int jl = lane_id / CPW, cw = lane_id % CPW;
     const int c = wid * CPW + cw;
     const int ncb = (p.d + CH - 1) / CH;
-    const int lane = blockIdx.x / ncb;
-    const int i0 = (blockIdx.x % ncb) * CH;
+    const unsigned cta = ssm_cta(p.ragged);
+    const int lane = cta / ncb;
+    const int i0 = (cta % ncb) * CH;
     const int i = i0 + c;
     const bool valid = i < p.d;
     const size_t row0 = p.offsets ? p.offsets[lane] : 0;
@@ -1072,7 +1084,10 @@ int32_t launch_cfg(pssa_b200_ctx* ctx, const SsmParams& p) {
     if (blocks > 0x7fffffffull)
         return fail(ctx, PSSA_B200_ERR_SHAPE, "B200 SSM grid (%zu, 1) exceeds grid limits; refusing launch", blocks);
     static PerDeviceCount resident;
-    PSSA_CUDA(ctx, launch_spread(resident, 1, ctx->device, ctx->sm_count, kern, dim3((unsigned)blocks), dim3(kThreads), smem, ctx->stream, p));
+    SsmParams q = p;
+    q.ragged = p.ragged ? ctx->sm_count : 0;
+    PSSA_CUDA(ctx, launch_spread(resident, p.ragged ? 0 : 1, ctx->device, ctx->sm_count, kern, dim3((unsigned)blocks), dim3(kThreads), smem,
+                                 ctx->stream, q));
     return after_launch(ctx, MAPS ? "ssm_fused_kernel[chunk maps]" : "ssm_fused_kernel");
 }
 
@@ -1090,7 +1105,10 @@ int32_t launch_wide_cfg(pssa_b200_ctx* ctx, const SsmParams& p) {
     if (blocks > 0x7fffffffull)
         return fail(ctx, PSSA_B200_ERR_SHAPE, "B200 SSM grid (%zu, 1) exceeds grid limits; refusing launch", blocks);
     static PerDeviceCount resident;
-    PSSA_CUDA(ctx, launch_spread(resident, 1, ctx->device, ctx->sm_count, kern, dim3((unsigned)blocks), dim3(kWideWarps * 32), smem, ctx->stream, p));
+    SsmParams q = p;
+    q.ragged = p.ragged ? ctx->sm_count : 0;
+    PSSA_CUDA(ctx, launch_spread(resident, p.ragged ? 0 : 1, ctx->device, ctx->sm_count, kern, dim3((unsigned)blocks), dim3(kWideWarps * 32), smem,
+                                 ctx->stream, q));
     return after_launch(ctx, "ssm_fused_kernel[few lanes]");
 }
 template <int LPC, int SPL, int TT>
@@ -1223,7 +1241,8 @@ int32_t launch_ssm_fused(pssa_b200_ctx* ctx, const SsmParams& p, bool exact) {
         if (s == 16) return channels <= 4 * schedulers && !by_shape ? launch_wide<8, 2, 32>(ctx, p, exact) : launch_wide<4, 4, 16>(ctx, p, exact);
         if (s == 32) return channels <= 2 * schedulers && !by_shape ? launch_wide<16, 2, 32>(ctx, p, exact) : launch_wide<8, 4, 32>(ctx, p, exact);
         if (channels <= (exact ? 2 : 1) * schedulers && !by_shape) return launch_wide<32, 2, 32>(ctx, p, exact);
-        if (channels <= 4 * schedulers) return launch_wide<16, 4, 32>(ctx, p, exact);
+        // (resident CTAs count every lane, however short)
+        if (channels <= 4 * schedulers && (size_t)p.lanes * p.d <= 4 * schedulers) return launch_wide<16, 4, 32>(ctx, p, exact);
         const double wide_us = 13.8 * (double)channels / (double)schedulers;
         const double tiled_us = 60.0 + 64.5 * (double)tiled_shape(ctx, p.d, lanes).busiest;
         if (exact || tape || by_shape || wide_us < tiled_us) return launch_wide<16, 4, 16>(ctx, p, exact);

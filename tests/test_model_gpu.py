@@ -209,6 +209,45 @@ def test_a_prompt_below_256_tokens_has_the_same_bits_alone_and_in_any_batch(gpu,
     gm.close()
 
 
+@pytest.mark.parametrize("lengths", [(40, 300, 0, 1, 290, 33, 300, 2), (700, 20, 1500, 300), (3, 1), (255,) * 3 + (1,) * 200])
+def test_the_order_of_ragged_lanes_does_not_matter(gpu, lengths):
+    """Lanes are taken longest first inside: a lane's logits and carry are those of the same call in another order, bit for bit,
+    through host and device arrays, where the rows also lie in another order than the lanes."""
+    import torch
+    import pssa_b200
+    n = len(lengths)
+    om = O.Model.new(2, 257, 768, 64, 64, 128, tau_mem=0.1, seed=3)
+    fill_synthetic(om, 3)
+    gm = pssa_b200.PSSAModel(gpu, 2, 257, 768, 64, 64, 128, tau_mem=0.1, streams=n, precision=0)
+    upload(om, gm)
+    rng = np.random.default_rng(n)
+    prompts = [rng.integers(1, 257, k).astype(np.uint64) for k in lengths]
+
+    def run(order, dev):
+        gm.reset_recurrent_state()
+        live = [i for i in order if lengths[i]]
+        if not dev:
+            out = gm.prefill_batch([prompts[i] for i in order], streams=order)[0]
+        else:
+            rows = np.cumsum([0] + [lengths[i] for i in sorted(order)])
+            ids = torch.from_numpy(np.concatenate([prompts[i] for i in sorted(order)]).astype(np.int32)).cuda()
+            out = torch.zeros(n, 257, device="cuda")
+            torch.cuda.synchronize()
+            gm.prefill_batch_dev(ids, [rows[i] for i in order], [lengths[i] for i in order], order, out)
+            gpu.synchronize()
+            out = out.cpu().numpy()
+        return {i: out[order.index(i)] for i in live}, [gm.copy_recurrent_state_to(i) for i in (0, 1, n - 1)]
+
+    first = sorted(range(n), key=lambda i: -lengths[i])
+    want, state = run(first, False)
+    for order in (list(range(n)), first[::-1]):
+        for dev in (False, True):
+            got, st = run(order, dev)
+            assert all(np.array_equal(got[i], want[i]) for i in want), (order, dev)
+            assert all(np.array_equal(a, b) for a, b in zip(st, state)), (order, dev)
+    gm.close()
+
+
 def test_time_chunks_that_hold_no_token_leave_the_carry_as_it_is(gpu):
     """A long prompt cut into 37 time chunks beside prompts of 7, 36 and 1 tokens, most of whose chunks are empty: carries and logits
     against the same prompts read in windows too short to be cut. (A chunk's decay is one exponential where the recurrence multiplies
