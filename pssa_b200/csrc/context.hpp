@@ -23,6 +23,8 @@ struct pssa_b200_ctx {
     char *io = nullptr, *pinned = nullptr;
     size_t io_bytes = 0, pinned_bytes = 0;
     std::vector<cudaEvent_t> io_events;
+    cudaEvent_t staged_ev = nullptr;  // behind the last copy out of `pinned` that nobody has waited for yet
+    bool staged = false;
     std::string error;
     std::string label;
     uint64_t launches = 0;

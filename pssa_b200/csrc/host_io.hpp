@@ -49,8 +49,15 @@ class HostCall {
 
 // device -> host through the context's pinned buffer, in stream order; waits for the stream
 int32_t copy_to_host(pssa_b200_ctx* ctx, void* dst, const void* src_dev, size_t bytes);
-// pinned host memory of the context, at least `bytes`, valid until the next call; waits for the stream when it has to grow
+// host -> device through the context's pinned buffer; waits for the stream
+int32_t copy_to_device(pssa_b200_ctx* ctx, void* dst_dev, const void* src, size_t bytes);
+// outputs from here on are copied by several threads
+constexpr size_t kThreadsFrom = (size_t)1 << 20;
+// pinned host memory of the context, at least `bytes`, valid until the next call; waits for the stream when it has to grow, and for
+// a copy that pinned_send left behind
 int32_t pinned_reserve(pssa_b200_ctx* ctx, size_t bytes);
+// enqueues the copy of `bytes` at `off` of the pinned buffer to the device and returns
+int32_t pinned_send(pssa_b200_ctx* ctx, void* dst_dev, size_t off, size_t bytes);
 void host_io_create();  // once per context
 void host_io_destroy(pssa_b200_ctx* ctx);
 

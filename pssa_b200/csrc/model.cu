@@ -144,7 +144,7 @@ void pssa_b200_model_destroy(pssa_b200_model* m) {
     cudaFree(m->obs.q_pnc), cudaFree(m->obs.buf);
     cudaFree(m->score.logits), cudaFree(m->score.targets), cudaFree(m->score.loss);
     cudaFree(m->sampler.recent), cudaFree(m->sampler.count), cudaFree(m->sampler.rng), cudaFree(m->sampler.ids);
-    cudaFree(m->sampler.status), cudaFree(m->sampler.head_slot), cudaFree(m->sampler.probs), cudaFree(m->sampler.conf);
+    cudaFree(m->sampler.status), cudaFree(m->sampler.probs), cudaFree(m->sampler.conf);
     cudaFree(m->chunks.off), cudaFree(m->chunks.len), cudaFree(m->chunks.records), cudaFree(m->chunks.carry_in);
     cudaFree(m->step_barrier);
     for (auto& b : m->blocks) {
@@ -355,9 +355,7 @@ int32_t pssa_b200_model_set_state(pssa_b200_model* m, uint32_t stream, const flo
     if (stream >= m->max_streams || len != n)
         return fail(m->ctx, PSSA_B200_ERR_SHAPE, "recurrent state: stream %u of %u, length %zu, expected %zu", stream, m->max_streams, len, n);
     PSSA_CUDA(m->ctx, cudaSetDevice(m->ctx->device));
-    PSSA_CUDA(m->ctx, cudaMemcpyAsync(m->state + (size_t)stream * n, data, n * 4, cudaMemcpyHostToDevice, m->ctx->stream));
-    PSSA_CUDA(m->ctx, cudaStreamSynchronize(m->ctx->stream));
-    return PSSA_B200_OK;
+    return copy_to_device(m->ctx, m->state + (size_t)stream * n, data, n * 4);
 }
 
 }  // extern "C"

@@ -54,7 +54,8 @@ struct DeviceBlock {
 struct Workspace {
     size_t rows = 0, lanes = 0;
     uint32_t *ids = nullptr, *lane_off = nullptr, *lane_len = nullptr, *lane_slot = nullptr, *last_rows = nullptr,
-             *greedy = nullptr, *row_slot = nullptr;  // row_slot: stream of each row of a decode step
+             *greedy = nullptr, *row_slot = nullptr,  // row_slot: stream of each row of a decode step
+             *head_slot = nullptr;                    // stream of each row the head emits
     float* feat_c = nullptr;  // Ouro passes only: a block's input features, kept for its depth residual
     float *feat_a = nullptr, *feat_b = nullptr, *x_norm = nullptr, *proj = nullptr, *y = nullptr, *weights = nullptr,
           *m_val = nullptr, *m_proj = nullptr, *z = nullptr, *mlp_act = nullptr, *last_feat = nullptr, *logits = nullptr;
@@ -128,7 +129,7 @@ struct pssa_b200_model {
         unsigned* recent = nullptr;            // [max_streams][64]
         unsigned* count = nullptr;             // [max_streams]
         unsigned long long* rng = nullptr;     // [max_streams]
-        unsigned *ids = nullptr, *status = nullptr, *head_slot = nullptr;  // [lanes capacity]
+        unsigned *ids = nullptr, *status = nullptr;  // [lanes capacity]
         float* probs = nullptr;                // [lanes capacity][vocab]
         float* conf = nullptr;                 // [lanes capacity]
         size_t lanes = 0;

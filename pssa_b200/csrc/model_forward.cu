@@ -6,6 +6,7 @@
 #include "bounds.hpp"
 #include "context.hpp"
 #include "device_math.cuh"
+#include "host_io.hpp"
 #include "kernels.hpp"
 #include "model.hpp"
 
@@ -33,8 +34,9 @@ int32_t ensure_workspace(pssa_b200_model* m, size_t rows, size_t lanes) {
     lanes = std::max(lanes, ws.lanes);
     const size_t d = m->d, f = sizeof(float);
     Carver c;
-    size_t o_ids = c.take(rows * 4), o_off = c.take(lanes * 4), o_len = c.take(lanes * 4), o_slot = c.take(lanes * 4),
-           o_last = c.take(lanes * 4), o_greedy = c.take(lanes * 4), o_rslot = c.take(lanes * 4);
+    // a call's description side by side, the ids last: the host entry points send it in one copy (send_description)
+    size_t o_off = c.take(lanes * 4), o_len = c.take(lanes * 4), o_slot = c.take(lanes * 4), o_last = c.take(lanes * 4),
+           o_rslot = c.take(lanes * 4), o_hslot = c.take(lanes * 4), o_ids = c.take(rows * 4), o_greedy = c.take(lanes * 4);
     size_t o_fc = c.take(m->loops > 1 ? rows * d * f : 0);
     size_t o_fa = c.take(rows * d * f), o_fb = c.take(rows * d * f), o_xn = c.take(rows * d * f),
            o_proj = c.take(rows * m->ncat * f), o_y = c.take(rows * d * f), o_w = c.take(rows * m->cap * f),
@@ -60,7 +62,7 @@ int32_t ensure_workspace(pssa_b200_model* m, size_t rows, size_t lanes) {
     char* b = ws.base;
     ws.ids = (uint32_t*)(b + o_ids), ws.lane_off = (uint32_t*)(b + o_off), ws.lane_len = (uint32_t*)(b + o_len);
     ws.lane_slot = (uint32_t*)(b + o_slot), ws.last_rows = (uint32_t*)(b + o_last), ws.greedy = (uint32_t*)(b + o_greedy);
-    ws.row_slot = (uint32_t*)(b + o_rslot);
+    ws.row_slot = (uint32_t*)(b + o_rslot), ws.head_slot = (uint32_t*)(b + o_hslot);
     ws.step = (float*)(b + o_step), ws.step_rows = step_rows;
     ws.feat_c = m->loops > 1 ? (float*)(b + o_fc) : nullptr;
     ws.feat_a = (float*)(b + o_fa), ws.feat_b = (float*)(b + o_fb), ws.x_norm = (float*)(b + o_xn);
@@ -613,16 +615,37 @@ int32_t ensure_sampler(pssa_b200_model* m, size_t lanes) {
     }
     if (lanes > sm.lanes) {
         PSSA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-        cudaFree(sm.ids), cudaFree(sm.status), cudaFree(sm.head_slot), cudaFree(sm.probs), cudaFree(sm.conf);
-        sm.ids = sm.status = sm.head_slot = nullptr, sm.probs = sm.conf = nullptr, sm.lanes = 0;
+        cudaFree(sm.ids), cudaFree(sm.status), cudaFree(sm.probs), cudaFree(sm.conf);
+        sm.ids = sm.status = nullptr, sm.probs = sm.conf = nullptr, sm.lanes = 0;
         PSSA_CUDA(ctx, cudaMalloc((void**)&sm.ids, lanes * 4));
         PSSA_CUDA(ctx, cudaMalloc((void**)&sm.status, lanes * 4));
-        PSSA_CUDA(ctx, cudaMalloc((void**)&sm.head_slot, lanes * 4));
         PSSA_CUDA(ctx, cudaMalloc((void**)&sm.probs, lanes * m->v * sizeof(float)));
         PSSA_CUDA(ctx, cudaMalloc((void**)&sm.conf, lanes * sizeof(float)));
         sm.lanes = lanes;
     }
     return PSSA_B200_OK;
+}
+
+// What the device has to know of a host call -- lanes, rows of the heads, ids -- in one copy out of pinned memory. (Five or six copies
+// from pageable memory at 4 to 5 us of this thread's time each before.) With `also`, that many words go to `also_dev` too.
+int32_t send_description(pssa_b200_model* m, const std::vector<uint32_t>& ids, const std::vector<uint32_t>& off, const std::vector<uint32_t>& len,
+                         const std::vector<uint32_t>& slot, const std::vector<uint32_t>& last, const std::vector<uint32_t>& row_slot,
+                         const std::vector<uint32_t>& head_slot, const std::vector<uint32_t>* also = nullptr, void* also_dev = nullptr) {
+    Workspace& ws = m->ws;
+    const size_t bytes = ((const char*)ws.ids - (const char*)ws.lane_off) + ids.size() * 4, more = also ? also->size() * 4 : 0;
+    int32_t rc = pinned_reserve(m->ctx, bytes + more);
+    if (rc) return rc;
+    char* const h = m->ctx->pinned;
+    auto put = [&](const uint32_t* dev, const std::vector<uint32_t>& v) {
+        if (!v.empty()) std::memcpy(h + ((const char*)dev - (const char*)ws.lane_off), v.data(), v.size() * 4);
+    };
+    put(ws.lane_off, off), put(ws.lane_len, len), put(ws.lane_slot, slot), put(ws.last_rows, last);
+    put(ws.row_slot, row_slot), put(ws.head_slot, head_slot), put(ws.ids, ids);
+    if (more) {
+        std::memcpy(h + bytes, also->data(), more);
+        if ((rc = pinned_send(m->ctx, also_dev, bytes, more))) return rc;
+    }
+    return pinned_send(m->ctx, ws.lane_off, 0, bytes);
 }
 
 int32_t run_lanes(pssa_b200_model* m, const uint64_t* ids, const uint32_t* offsets, const uint32_t* lengths, const uint32_t* streams,
@@ -641,7 +664,7 @@ int32_t run_lanes(pssa_b200_model* m, const uint64_t* ids, const uint32_t* offse
     // window of tokens per lane per pass
     size_t window = std::max<size_t>(1, m->max_rows / n_lanes);
     if (window > max_len) window = max_len;
-    std::vector<uint32_t> h_ids, h_off(n_lanes), h_len(n_lanes), h_slot(n_lanes), h_row_slot, h_last, s_off, s_len, s_slot;
+    std::vector<uint32_t> h_ids, h_off(n_lanes), h_len(n_lanes), h_slot(n_lanes), h_row_slot, h_last, s_off, s_len, s_slot, head_slot;
     int32_t rc;
     for (size_t t0 = 0; t0 < max_len; t0 += window) {
         if (cancelled && cancelled(cancel_arg)) return fail(ctx, PSSA_B200_ERR_CANCELLED, "prefill cancelled after %zu tokens", t0);
@@ -667,77 +690,67 @@ int32_t run_lanes(pssa_b200_model* m, const uint64_t* ids, const uint32_t* offse
         Workspace& ws = m->ws;
         cudaStream_t st = ctx->stream;
         m->dev_layout.ws_base = nullptr;  // the cached layout of the device-resident entry no longer holds
-        PSSA_CUDA(ctx, cudaMemcpyAsync(ws.ids, h_ids.data(), rows * 4, cudaMemcpyHostToDevice, st));
         float* feats = nullptr;
         const bool step = is_decode_step(m, n_lanes, h_len.data()), want_head = logits || greedy || sampling;
-        if (step) {
-            h_row_slot.clear();
+        h_row_slot.clear(), head_slot.clear();
+        if (step)
             for (size_t l = 0; l < n_lanes; ++l)
                 if (h_len[l]) h_row_slot.push_back(h_slot[l]);
-            PSSA_CUDA(ctx, cudaMemcpyAsync(ws.row_slot, h_row_slot.data(), rows * 4, cudaMemcpyHostToDevice, st));
+        for (size_t l : head_lane) head_slot.push_back(h_slot[l]);
+        s_off = h_off, s_len = h_len, s_slot = h_slot;
+        longest_first(m, s_off, s_len, s_slot);
+        if ((rc = send_description(m, h_ids, s_off, s_len, s_slot, h_last, h_row_slot, head_slot))) return rc;
+        if (step) {
             if ((rc = run_decode_step(m, rows, ws.ids, want_head && !h_last.empty() ? ws.logits : nullptr))) return rc;
         } else {
-            s_off = h_off, s_len = h_len, s_slot = h_slot;
-            longest_first(m, s_off, s_len, s_slot);
-            PSSA_CUDA(ctx, cudaMemcpyAsync(ws.lane_off, s_off.data(), n_lanes * 4, cudaMemcpyHostToDevice, st));
-            PSSA_CUDA(ctx, cudaMemcpyAsync(ws.lane_len, s_len.data(), n_lanes * 4, cudaMemcpyHostToDevice, st));
-            PSSA_CUDA(ctx, cudaMemcpyAsync(ws.lane_slot, s_slot.data(), n_lanes * 4, cudaMemcpyHostToDevice, st));
-            if (!h_last.empty()) PSSA_CUDA(ctx, cudaMemcpyAsync(ws.last_rows, h_last.data(), h_last.size() * 4, cudaMemcpyHostToDevice, st));
             if ((rc = forward_rows(m, rows, n_lanes, s_off.data(), s_len.data(), &feats, h_last.size()))) return rc;
         }
         if (!h_last.empty() && want_head) {
             const bool want_greedy = greedy != nullptr && !sampling;
             if (!step && (rc = head_rows(m, feats, h_last.size(), want_greedy))) return rc;
             if (step && want_greedy && (rc = launch_greedy(ctx, ws.logits, ws.greedy, rows, (int)m->v))) return rc;
-            std::vector<uint32_t> g(h_last.size()), g_status(h_last.size(), 0);
-            std::vector<float> g_conf;
+            const size_t nh = h_last.size();
             if (sampling) {
                 // sample on the device from the logits the head just wrote; only ids come back
                 if ((rc = ensure_sampler(m, n_lanes))) return rc;
-                std::vector<uint32_t> head_slot(h_last.size());
-                for (size_t i = 0; i < head_lane.size(); ++i) head_slot[i] = h_slot[head_lane[i]];
-                PSSA_CUDA(ctx, cudaMemcpyAsync(m->sampler.head_slot, head_slot.data(), head_slot.size() * 4, cudaMemcpyHostToDevice, st));
-                PSSA_CUDA(ctx, cudaStreamSynchronize(st));  // head_slot is a local vector
                 SampleParams sp{};
-                sp.logits = ws.logits, sp.probs = m->sampler.probs, sp.rows = h_last.size(), sp.vocab = (int)m->v;
+                sp.logits = ws.logits, sp.probs = m->sampler.probs, sp.rows = nh, sp.vocab = (int)m->v;
                 sp.top_k = (int)std::min<size_t>(sampling->top_k, m->v);
                 sp.temperature = sampling->temperature, sp.top_p = sampling->top_p, sp.repetition_penalty = sampling->repetition_penalty;
                 sp.recent_ids = m->sampler.recent, sp.recent_count = m->sampler.count, sp.rng_state = m->sampler.rng;
                 sp.ids_out = m->sampler.ids, sp.status_out = m->sampler.status, sp.exact = (sample_flags & PSSA_B200_SAMPLE_EXACT) != 0;
-                sp.slots = m->sampler.head_slot, sp.confidence_out = confidence ? m->sampler.conf : nullptr;
+                sp.slots = ws.head_slot, sp.confidence_out = confidence ? m->sampler.conf : nullptr;
                 if ((rc = launch_sample(ctx, sp))) return rc;
-                if ((rc = launch_push_recent(ctx, m->sampler.ids, m->sampler.head_slot, m->sampler.recent, m->sampler.count, h_last.size())))
-                    return rc;
-                PSSA_CUDA(ctx, cudaMemcpyAsync(g.data(), m->sampler.ids, g.size() * 4, cudaMemcpyDeviceToHost, st));
-                PSSA_CUDA(ctx, cudaMemcpyAsync(g_status.data(), m->sampler.status, g.size() * 4, cudaMemcpyDeviceToHost, st));
-                if (confidence) {
-                    g_conf.resize(g.size());
-                    PSSA_CUDA(ctx, cudaMemcpyAsync(g_conf.data(), m->sampler.conf, g.size() * 4, cudaMemcpyDeviceToHost, st));
-                }
-            } else if (greedy) {
-                PSSA_CUDA(ctx, cudaMemcpyAsync(g.data(), ws.greedy, g.size() * 4, cudaMemcpyDeviceToHost, st));
+                if ((rc = launch_push_recent(ctx, m->sampler.ids, ws.head_slot, m->sampler.recent, m->sampler.count, nh))) return rc;
             }
-            if (logits) {
-                // contiguous runs of lanes are copied in one transfer
-                size_t i = 0;
-                while (i < head_lane.size()) {
-                    size_t j = i;
-                    while (j + 1 < head_lane.size() && head_lane[j + 1] == head_lane[j] + 1) ++j;
-                    PSSA_CUDA(ctx, cudaMemcpyAsync(logits + head_lane[i] * m->v, ws.logits + i * m->v, (j - i + 1) * m->v * 4,
-                                                   cudaMemcpyDeviceToHost, st));
-                    i = j + 1;
-                }
-            }
+            // results through pinned memory: ids, sampler status, confidences, then the logits unless there are many
+            const size_t row = m->v * 4, o_conf = 2 * nh * 4, o_logits = 3 * nh * 4;
+            const bool together = logits && nh * row < kThreadsFrom;
+            if ((rc = pinned_reserve(ctx, o_logits + (together ? nh * row : 0)))) return rc;
+            char* const h = ctx->pinned;
+            if (greedy) PSSA_CUDA(ctx, cudaMemcpyAsync(h, sampling ? m->sampler.ids : ws.greedy, nh * 4, cudaMemcpyDeviceToHost, st));
+            if (sampling) PSSA_CUDA(ctx, cudaMemcpyAsync(h + nh * 4, m->sampler.status, nh * 4, cudaMemcpyDeviceToHost, st));
+            if (sampling && confidence) PSSA_CUDA(ctx, cudaMemcpyAsync(h + o_conf, m->sampler.conf, nh * 4, cudaMemcpyDeviceToHost, st));
+            if (together) PSSA_CUDA(ctx, cudaMemcpyAsync(h + o_logits, ws.logits, nh * row, cudaMemcpyDeviceToHost, st));
             PSSA_CUDA(ctx, cudaStreamSynchronize(st));
+            if (together)
+                for (size_t i = 0; i < nh; ++i) std::memcpy(logits + head_lane[i] * m->v, h + o_logits + i * row, row);
+            const std::vector<uint32_t> got((const uint32_t*)h, (const uint32_t*)(h + o_logits));
+            if (logits && !together)
+                for (size_t i = 0, j; i < nh; i = j) {  // contiguous runs of lanes in one transfer
+                    for (j = i + 1; j < nh && head_lane[j] == head_lane[j - 1] + 1; ++j) {}
+                    if ((rc = copy_to_host(ctx, logits + head_lane[i] * m->v, ws.logits + i * m->v, (j - i) * row))) return rc;
+                }
             if (greedy)
-                for (size_t i = 0; i < head_lane.size(); ++i) {
-                    if (g[i] == 0xffffffffu) {  // src/inference.rs:111-113, 146-147, 153-154
-                        const char* why = g_status[i] == 2 ? "invalid sampling probability mass"
-                                          : g_status[i] == 3 ? "no valid generation candidates" : "model emitted non-finite logits";
+                for (size_t i = 0; i < nh; ++i) {
+                    if (got[i] == 0xffffffffu) {  // src/inference.rs:111-113, 146-147, 153-154
+                        const unsigned status = sampling ? got[nh + i] : 0;
+                        const char* why = status == 2 ? "invalid sampling probability mass"
+                                          : status == 3 ? "no valid generation candidates" : "model emitted non-finite logits";
                         return fail(ctx, PSSA_B200_ERR_INVALID_ARGUMENT, "%s", why);
                     }
-                    greedy[head_lane[i]] = g[i];
-                    if (confidence && !g_conf.empty()) confidence[head_lane[i]] = g_conf[i];
+                    greedy[head_lane[i]] = got[i];
+                    if (sampling && confidence) std::memcpy(&confidence[head_lane[i]], &got[2 * nh + i], 4);
                 }
         } else if (final_pass || cancelled) {
             PSSA_CUDA(ctx, cudaStreamSynchronize(st));
@@ -908,14 +921,10 @@ int32_t pssa_b200_model_score(pssa_b200_model* m, uint32_t stream, const uint64_
         for (size_t t = 0; t < rows; ++t) h_ids[t] = (uint32_t)ids[t0 + t], h_tgt[t] = (uint32_t)targets[t0 + t];
         if ((rc = ensure_workspace(m, rows, 1))) return rc;
         Workspace& ws = m->ws;
-        const uint32_t off = 0, len = (uint32_t)rows, slot = stream;
+        const uint32_t off = 0, len = (uint32_t)rows;
         m->dev_layout.ws_base = nullptr;
-        PSSA_CUDA(ctx, cudaMemcpyAsync(ws.ids, h_ids.data(), rows * 4, cudaMemcpyHostToDevice, st));
-        PSSA_CUDA(ctx, cudaMemcpyAsync(sc.targets, h_tgt.data(), rows * 4, cudaMemcpyHostToDevice, st));
-        PSSA_CUDA(ctx, cudaMemcpyAsync(ws.lane_off, &off, 4, cudaMemcpyHostToDevice, st));
-        PSSA_CUDA(ctx, cudaMemcpyAsync(ws.lane_len, &len, 4, cudaMemcpyHostToDevice, st));
-        PSSA_CUDA(ctx, cudaMemcpyAsync(ws.lane_slot, &slot, 4, cudaMemcpyHostToDevice, st));
-        PSSA_CUDA(ctx, cudaStreamSynchronize(st));  // the three scalars above live on this stack frame
+        h_ids.resize(rows), h_tgt.resize(rows);
+        if ((rc = send_description(m, h_ids, {off}, {len}, {stream}, {}, {}, {}, &h_tgt, sc.targets))) return rc;
         float* feats = nullptr;
         if ((rc = forward_rows(m, rows, 1, &off, &len, &feats))) return rc;
         for (size_t r0 = 0; r0 < rows; r0 += tile) {
@@ -930,8 +939,7 @@ int32_t pssa_b200_model_score(pssa_b200_model* m, uint32_t stream, const uint64_
             if (logits_out)
                 PSSA_CUDA(ctx, cudaMemcpyAsync(logits_out + (t0 + r0) * m->v, sc.logits, nr * m->v * sizeof(float), cudaMemcpyDeviceToHost, st));
         }
-        PSSA_CUDA(ctx, cudaMemcpyAsync(h_loss.data(), sc.loss, rows * 4, cudaMemcpyDeviceToHost, st));
-        PSSA_CUDA(ctx, cudaStreamSynchronize(st));
+        if ((rc = copy_to_host(ctx, h_loss.data(), sc.loss, rows * 4))) return rc;
         for (size_t t = 0; t < rows; ++t) {
             if (!std::isfinite(h_loss[t])) return fail(ctx, PSSA_B200_ERR_INVALID_ARGUMENT, "model emitted non-finite logits at token %zu", t0 + t);
             total += (double)h_loss[t];
