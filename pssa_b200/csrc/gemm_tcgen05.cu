@@ -112,7 +112,8 @@ constexpr int kRuntimeMode = -100;
 // PAIR: the kernel runs as clusters of two CTAs on 256 x BN tiles (cta_group::2): each CTA keeps its own 128 rows of A,
 // loads only its half of the B tile (32 KB instead of 48 KB per K block and CTA at BN = 256) and drains its own 128
 // accumulator rows; the even CTA issues the MMAs for both and its barriers count both CTAs' operand bytes.
-template <int BN, int STAGES, int MODE, int OUTS, int EW, bool PAIR>
+// PART: M is not a multiple of 32, so the last band of rows is handled row by row (see there).
+template <int BN, int STAGES, int MODE, int OUTS, int EW, bool PAIR, bool PART>
 __global__ void __launch_bounds__(64 + 32 * EW, 1) gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
                                                                             const __grid_constant__ CUtensorMap map_b,
                                                                             GemmEpilogue e) {
@@ -274,7 +275,14 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1) gemm_bf16_tcgen05_kernel(cons
             tcgen05_fence_after();
             const uint32_t taddr = tmem_base + buf * BN + half * HALF_COLS + ((uint32_t)(quad * 32) << 16);
             const int rbase = m0 + quad * 32;
-            const bool rows_in = rbase + 32 <= e.M;  // whole 32-row band inside the matrix
+            const int rows_left = e.M - rbase;
+            // A last band of fewer than 32 rows takes the vector path too, row by row: the scalar path below is a round trip to memory
+            // for every row group, 3 us a launch and more for wide tiles (us per pass of the 12-block model: 24 tokens 1125 -> 923, 7 x 333
+            // 1948 -> 1686, 13 x 1001 5777 -> 5390). The narrow tiles always test the rows (0.5 % of 64 whole ones); the 256-wide
+            // ones, where the tests cost 1 % of 65536 rows, in an instantiation of their own.
+            constexpr bool kPartRows = PART;
+            const bool rows_in = rows_left >= 32 || (kPartRows && rows_left > 0);
+            auto row_ok = [&](int i) { return !kPartRows || rsub + i * 4 < rows_left; };
             bool released = false;
             // EPI_GATE with row factors: the eight rows a lane stores are the same for every chunk of the tile
             // (kept in registers by the instantiation that carries only this family; the run-time one loads them where used)
@@ -286,6 +294,7 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1) gemm_bf16_tcgen05_kernel(cons
             }
 #pragma unroll 1
             for (int c0 = 0; c0 < HALF_COLS; c0 += 32) {
+                if (kPartRows && rows_left <= 0) break;  // a band below the matrix
                 const int col0 = n0 + c0;
                 // Chunks that lie inside the matrix take the 16-byte path without per-element bounds checks; so does the
                 // matrix's last, partial chunk when N is a multiple of 4 (a lane's column quad is then all in or all out)
@@ -300,7 +309,7 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1) gemm_bf16_tcgen05_kernel(cons
                 if (prefetch) {
 #pragma unroll
                     for (int i = 0; i < 8; ++i) {
-                        if (!lane_in) break;
+                        if (!lane_in || !row_ok(i)) break;
                         const size_t ro = (size_t)(rbase + rsub + i * 4);
                         if (epi == EPI_RESIDUAL && e.add_is_bf16)
                             // kept as raw bits: converting here would wait for the load before the TMEM read is issued
@@ -316,7 +325,7 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1) gemm_bf16_tcgen05_kernel(cons
                     // per row group inside the store loop
 #pragma unroll
                     for (int i = 0; i < 8; ++i)
-                        if (lane_in) pre_add[i] = *reinterpret_cast<const float4*>(out32 + (size_t)(rbase + rsub + i * 4) * e.ldo + col0 + cq);
+                        if (lane_in && row_ok(i)) pre_add[i] = *reinterpret_cast<const float4*>(out32 + (size_t)(rbase + rsub + i * 4) * e.ldo + col0 + cq);
                 }
                 float v[32];
                 if (col0 < e.N) tcgen05_ld_32x32(taddr + (uint32_t)c0, v);  // warp-uniform
@@ -388,7 +397,7 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1) gemm_bf16_tcgen05_kernel(cons
                     for (int i = 0; i < 8; ++i) {
                         const int sr = i * 4 + rsub;  // staged row; its column quads are swizzled with (row & 7)
                         float4 val = *reinterpret_cast<const float4*>(stg + sr * STG_PITCH + ((((cq >> 2) ^ (sr & 7))) << 2));
-                        if (!lane_in) break;
+                        if (!lane_in || !row_ok(i)) break;
                         {
                             if (epi == EPI_ADD_OUT && gp) {
                                 const float4 pv = pre_add[i];
@@ -468,7 +477,7 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1) gemm_bf16_tcgen05_kernel(cons
                 }
                 __syncwarp();
             }
-            if (!released) {  // this warp's column half lies entirely outside the matrix
+            if (!released) {  // this warp's column half or its band lies entirely outside the matrix
                 tcgen05_fence_before();
                 __syncwarp();
                 if (lane == 0) {
@@ -490,7 +499,7 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1) gemm_bf16_tcgen05_kernel(cons
 }
 
 // ---- host side --------------------------------------------------------------------------------
-template <int BN, int STAGES, int MODE = kRuntimeMode, int OUTS = 0, int EW = EPI_WARPS, bool PAIR = false>
+template <int BN, int STAGES, int MODE = kRuntimeMode, int OUTS = 0, int EW = EPI_WARPS, bool PAIR = false, bool PART = (BN <= 128)>
 int32_t launch_tile(pssa_b200_ctx* ctx, const void* a, const void* b, const GemmEpilogue& e) {
     CUtensorMap map_a, map_b;
     int32_t rc;
@@ -498,7 +507,7 @@ int32_t launch_tile(pssa_b200_ctx* ctx, const void* a, const void* b, const Gemm
     if ((rc = make_map(ctx, &map_a, a, e.M, e.K, BM))) return rc;
     if ((rc = make_map(ctx, &map_b, b, e.N, e.K, B_ROWS))) return rc;
     size_t smem = 1024 + (size_t)STAGES * (BM * BK * 2 + B_ROWS * BK * 2) + (2 * STAGES + 4) * 8 + 16 + EW * 32 * STG_PITCH * 4;
-    auto kern = gemm_bf16_tcgen05_kernel<BN, STAGES, MODE, OUTS, EW, PAIR>;
+    auto kern = gemm_bf16_tcgen05_kernel<BN, STAGES, MODE, OUTS, EW, PAIR, PART>;
     static PerDeviceOnce attr;  // per instantiation and per device
     if (attr.need(ctx->device)) {
         PSSA_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -595,6 +604,8 @@ int32_t dispatch(pssa_b200_ctx* ctx, const void* a, const void* b, GemmEpilogue&
     // split value read and the distance product are bound by their epilogues already (the issuing thread waits for a
     // drained accumulator, not for operands) and measured slower with four stages (1.98 against 1.45 ms per step): three.
     if (e.epi == EPI_POINCARE && only32) return launch_tile<256, 3, EPI_POINCARE, 1, kWideEpiWarps>(ctx, a, b, e);
+    const bool part = e.M % 32 != 0;
+    if (part && e.epi == EPI_GATE && e.n_pairs > 0 && only16) return launch_tile<256, 3, EPI_GATE, 2, kWideEpiWarps, false, true>(ctx, a, b, e);
     if (e.epi == EPI_GATE && e.n_pairs > 0 && only16) return launch_tile<256, 3, EPI_GATE, 2, kWideEpiWarps>(ctx, a, b, e);
     if (e.n_pairs > 0) return (e.epi == EPI_NONE && only16) ? launch_tile<256, 4, EPI_NONE, 2>(ctx, a, b, e) : launch_tile<256, 4>(ctx, a, b, e);
     // Plain products run as CTA pairs (cta_group::2) when there are enough 256-row tiles for every pair of SMs: the
@@ -607,6 +618,9 @@ int32_t dispatch(pssa_b200_ctx* ctx, const void* a, const void* b, GemmEpilogue&
     if (pair_ok && e.epi == EPI_NONE && only32) return launch_tile<256, 6, EPI_NONE, 1, kWideEpiWarps, true>(ctx, a, b, e);
     if (pair_ok && e.epi == EPI_NONE && only16) return launch_tile<256, 6, EPI_NONE, 2, kWideEpiWarps, true>(ctx, a, b, e);
     // the block schedule's products: one epilogue family and one output set per instantiation
+    if (part && e.epi == -1 && only32) return launch_tile<256, 4, -1, 1, kWideEpiWarps, false, true>(ctx, a, b, e);
+    if (part && e.epi == EPI_RESIDUAL && only32) return launch_tile<256, 4, EPI_RESIDUAL, 1, kWideEpiWarps, false, true>(ctx, a, b, e);
+    if (part && e.epi == EPI_SILU && only16) return launch_tile<256, 4, EPI_SILU, 2, kWideEpiWarps, false, true>(ctx, a, b, e);
     if (e.epi == -1 && only32) return launch_tile<256, 4, -1, 1, kWideEpiWarps>(ctx, a, b, e);
     if (e.epi == EPI_GATE) return only16 ? launch_tile<256, 3, EPI_GATE, 2, kWideEpiWarps>(ctx, a, b, e) : launch_tile<256, 3, EPI_GATE, 0, kWideEpiWarps>(ctx, a, b, e);
     if (e.epi == EPI_RESIDUAL && only32) return launch_tile<256, 4, EPI_RESIDUAL, 1, kWideEpiWarps>(ctx, a, b, e);

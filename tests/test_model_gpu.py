@@ -248,6 +248,31 @@ def test_the_order_of_ragged_lanes_does_not_matter(gpu, lengths):
     gm.close()
 
 
+@pytest.mark.parametrize("lanes,last", [(1, 2), (1, 31), (2, 33), (6, 95), (20, 65), (78, 129), (78, 159)])
+def test_rows_of_a_partly_filled_band_have_the_bits_of_whole_ones(gpu, lanes, last):
+    """Products whose last band of 32 rows is not full, with tiles of 32 to 256 columns (2 to 19000 rows): logits and the last lane's
+    carry are those of the same call with one lane more, whose tokens fill the band."""
+    import pssa_b200
+    om = O.Model.new(1, 257, 768, 64, 64, 128, tau_mem=0.1, seed=5)
+    fill_synthetic(om, 5)
+    gm = pssa_b200.PSSAModel(gpu, 1, 257, 768, 64, 64, 128, tau_mem=0.1, streams=lanes + 2, precision=0)
+    upload(om, gm)
+    rng = np.random.default_rng(lanes + last)
+    prompts = [rng.integers(1, 257, 255 if i % 2 else 225) for i in range(lanes - 1)] + [rng.integers(1, 257, last)]
+    rows = sum(len(q) for q in prompts)
+
+    def run(more):
+        gm.reset_recurrent_state()
+        out = gm.prefill_batch(prompts + more)[0]
+        return out[:lanes], gm.copy_recurrent_state_to(lanes - 1)
+
+    got, state = run([])
+    fill = [rng.integers(1, 257, 32 - rows % 32)] if rows % 32 else [rng.integers(1, 257, 32)]
+    want, want_state = run(fill)
+    assert np.array_equal(got, want) and np.array_equal(state, want_state)
+    gm.close()
+
+
 def test_time_chunks_that_hold_no_token_leave_the_carry_as_it_is(gpu):
     """A long prompt cut into 37 time chunks beside prompts of 7, 36 and 1 tokens, most of whose chunks are empty: carries and logits
     against the same prompts read in windows too short to be cut. (A chunk's decay is one exponential where the recurrence multiplies
