@@ -109,10 +109,7 @@ __global__ void __launch_bounds__(256) gemm_xwt_exact_kernel(const float* __rest
 //     (a + b and b + a are the same number), so RT * CT outputs cost RT * CT - 1 shuffles and end one to a lane;
 //   * with few rows (AHEAD > 0) a warp requests AHEAD steps of its W rows at once and X is staged in shared memory;
 //   * several products of one X (the six x-side projections) are one launch.
-// Us, W in L2, before -> now: 16 x 768 x 768 10.3 -> 7.7, 16 x 16384 x 768 72 -> 36, 1 x 16384 x 768 39 -> 16, 512 x 592 x 192 31 -> 10,
-// 300 x 1536 x 768 74 -> 48. A scored fp32 step of 16 streams (12 blocks): 121 launches and 2.57 ms -> 61 and 0.85 ms. What is left
-// there is the launch and the warps' own instructions, not HBM: 16 x 768 x 768 7.7 us with W in L2 and 8.5 with W in HBM; with eight
-// warps on an SM a scheduler issues in 0.47 of its cycles. For many rows the shared L1 port (two loads for 2.7 to 4 fma).
+// Us, before -> now: 1 x 16384 x 768 39 -> 16. Used up to four rows, and where rows are not 16-byte aligned.
 constexpr int kMaxParts = 6;
 constexpr int kMaxStagedX = 200 * 1024;
 struct ExactPart {
@@ -124,6 +121,132 @@ struct ExactParts {
     ExactPart p[kMaxParts];
     int count, tiles;
 };
+// The partial sums of NO outputs, one of 32 per lane each, to whole outputs: acc0+acc1 / acc2+acc3 (distance 8), their sum (16), low + high
+// half (4), the two horizontal adds (1, 2). Returns the first output that this lane ends up with.
+template <int NO, int LEVEL = 0, int SIZE>
+__device__ __forceinline__ int fold_partials(float (&acc)[SIZE], int lane) {
+    if constexpr (LEVEL == 5) {
+        return 0;
+    } else {
+        constexpr int m = LEVEL == 0 ? 8 : LEVEL == 1 ? 16 : LEVEL == 2 ? 4 : LEVEL == 3 ? 1 : 2;
+        if constexpr (NO > 1) {
+            constexpr int half = NO / 2;
+            const bool up = (lane & m) != 0;
+#pragma unroll
+            for (int o = 0; o < half; ++o) {
+                const float send = up ? acc[o] : acc[o + half], keep = up ? acc[o + half] : acc[o];
+                acc[o] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, send, m));
+            }
+            return (up ? half : 0) + fold_partials<half, LEVEL + 1>(acc, lane);
+        } else {
+            acc[0] = __fadd_rn(acc[0], __shfl_xor_sync(0xffffffffu, acc[0], m));
+            return fold_partials<1, LEVEL + 1>(acc, lane);
+        }
+    }
+}
+
+// ---- many rows. The kernel below it reads every row of W once per eight rows of X, and a third of its instructions are addresses (ncu, 1000 x
+// 1536 x 768: issue slots 66 % taken, fma pipe 37 %). Here a CTA's warps share a tile of operands that comes through a cp.async ring in
+// shared memory, KB columns a stage, from pointers that only move on; the sums are the same ones in the same order. Small CTAs, three or
+// four to an SM, so that one's first loads and fold run beside another's products. Us, W in HBM, before -> now: 8 x 768 x 768 8.3 -> 5.6
+// (the launch), 16 x 768 x 1536 15.1 -> 6.8, 16 x 16384 x 768 35 -> 18, 300 x 1536 x 768 50 -> 28, 1000 x 1536 x 768 136 -> 86. What bounds
+// it: a load for four multiply-adds (8 x 16 outputs a warp: half the loads, but two warps a scheduler do not hide them: 140 us;
+// partials four to a lane with packed multiply-adds and 16-byte loads: 146).
+constexpr int kRingStages = 4;
+template <int RT, int CT, int WR, int WC, int KB>
+__global__ void __launch_bounds__(32 * WR * WC) gemm_xwt_exact_ring_kernel(const float* __restrict__ x, const __grid_constant__ ExactParts parts, size_t M,
+                                                                         int K, size_t ldo, float alpha) {
+    extern __shared__ __align__(16) float ring[];  // [stages][BR + BC][KB]
+    constexpr int NO = RT * CT, BR = RT * WR, BC = CT * WC, THR = 32 * WR * WC, Q = KB / 4;
+    constexpr int RPP = THR / Q, NX = BR / RPP, NW = BC / RPP;  // rows a pass of all threads copies, passes for X and for W
+    static_assert(BR % RPP == 0 && BC % RPP == 0, "whole passes");
+    const int tid = threadIdx.x, lane = tid & 31, wr = (tid >> 5) / WC, wc = (tid >> 5) % WC;
+    const int ct = (int)(blockIdx.x % parts.tiles);
+    const size_t row0 = (size_t)(blockIdx.x / parts.tiles) * BR;
+    int pi = 0;
+#pragma unroll
+    for (int i = 1; i < kMaxParts; ++i)
+        if (i < parts.count && ct >= parts.p[i].tile0) pi = i;
+    const ExactPart part = parts.p[pi];
+    const int col0 = (ct - part.tile0) * BC;
+    const int klen = K & ~31, blocks = (klen + KB - 1) / KB;
+    const int cr = tid / Q, ck = tid % Q * 4;  // this thread's row of a pass and its columns
+    const float *xsrc[NX], *wsrc[NW];  // rows past the end repeat the last one
+#pragma unroll
+    for (int j = 0; j < NX; ++j) xsrc[j] = x + (row0 + cr + j * RPP < M ? row0 + cr + j * RPP : M - 1) * (size_t)K + ck;
+#pragma unroll
+    for (int j = 0; j < NW; ++j) wsrc[j] = part.w + (size_t)min(col0 + cr + j * RPP, part.n - 1) * K + ck;
+    const unsigned dst = (unsigned)__cvta_generic_to_shared(ring + cr * KB + ck);
+    constexpr unsigned kStage = (BR + BC) * KB * 4;
+    auto copy = [](unsigned to, const float* from) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to), "l"(from)); };
+    auto load_x = [&](int b) {
+        if (b * KB + ck < klen)
+#pragma unroll
+            for (int j = 0; j < NX; ++j) copy(dst + (b % kRingStages) * kStage + j * RPP * KB * 4, xsrc[j] + b * KB);
+    };
+    auto load_w = [&](int b) {
+        if (b * KB + ck < klen)
+#pragma unroll
+            for (int j = 0; j < NW; ++j) copy(dst + (b % kRingStages) * kStage + (BR + j * RPP) * KB * 4, wsrc[j] + b * KB);
+    };
+    auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
+    // W towards L2 before the wait (a prefetch reads nothing: the kernel before may have written W)
+    for (int idx = tid; idx < BC * ((K + 31) / 32); idx += THR)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(part.w + (size_t)min(col0 + idx % BC, part.n - 1) * K + idx / BC * 32));
+    pdl_trigger();
+    pdl_wait();
+#pragma unroll
+    for (int b = 0; b < kRingStages - 1; ++b) load_x(b), load_w(b), commit();
+    float acc[NO];
+#pragma unroll
+    for (int o = 0; o < NO; ++o) acc[o] = 0.0f;
+    for (int b = 0; b < blocks; ++b) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kRingStages - 2) : "memory");
+        __syncthreads();  // block b has landed, and everybody is done with the stage that is filled next
+        load_x(b + kRingStages - 1), load_w(b + kRingStages - 1), commit();
+        const float* xs = ring + (b % kRingStages) * (BR + BC) * KB + wr * RT * KB + lane;
+        const float* ws = ring + (b % kRingStages) * (BR + BC) * KB + (BR + wc * CT) * KB + lane;
+#pragma unroll
+        for (int s = 0; s < KB / 32; ++s) {
+            if (b * KB + s * 32 >= klen) break;
+            float xa[RT], wb[CT];
+#pragma unroll
+            for (int r = 0; r < RT; ++r) xa[r] = xs[r * KB + s * 32];
+#pragma unroll
+            for (int c = 0; c < CT; ++c) wb[c] = ws[c * KB + s * 32];
+#pragma unroll
+            for (int r = 0; r < RT; ++r)
+#pragma unroll
+                for (int c = 0; c < CT; ++c) acc[r * CT + c] = fmaf(xa[r], wb[c], acc[r * CT + c]);
+        }
+    }
+    const size_t wrow = row0 + wr * RT;
+    const int wcol = col0 + wc * CT;
+    int i = klen;
+    for (; i + 8 <= K; i += 8)  // remaining whole vectors go to accumulator 0 (lanes 0..7)
+        if (lane < 8) {
+#pragma unroll
+            for (int r = 0; r < RT; ++r)
+#pragma unroll
+                for (int c = 0; c < CT; ++c)
+                    acc[r * CT + c] = fmaf(__ldg(x + (wrow + r < M ? wrow + r : M - 1) * (size_t)K + i + lane),
+                                           __ldg(part.w + (size_t)min(wcol + c, part.n - 1) * K + i + lane), acc[r * CT + c]);
+        }
+    const int mine = fold_partials<NO>(acc, lane);
+    constexpr int kDup = NO >= 32 ? 0 : NO == 16 ? 2 : 3;  // lanes that hold the same output
+    if (NO < 32 && (lane & kDup)) return;
+#pragma unroll
+    for (int o = 0; o < (NO >= 32 ? NO / 32 : 1); ++o) {
+        const int r = (mine + o) / CT, c = (mine + o) % CT;
+        if (wrow + r >= M || wcol + c >= part.n) continue;
+        float sum = acc[o];
+        const float *xt = x + (wrow + r) * (size_t)K, *wt = part.w + (size_t)(wcol + c) * K;
+        for (int t = i; t < K; ++t) sum = __fadd_rn(sum, __fmul_rn(xt[t], wt[t]));
+        float* dst_o = part.out + (wrow + r) * ldo + wcol + c;
+        *dst_o = apply_epilogue(part.epi, sum, alpha, part.epi == EPI_ADD_OUT ? *dst_o : 0.0f);
+    }
+}
+
 template <int RT, int CT, int AHEAD>
 __global__ void __launch_bounds__(256) gemm_xwt_exact_tiled_kernel(const float* __restrict__ x, const __grid_constant__ ExactParts parts, size_t M,
                                                                    int K, size_t ldo, float alpha) {
@@ -213,25 +336,7 @@ __global__ void __launch_bounds__(256) gemm_xwt_exact_tiled_kernel(const float* 
 #pragma unroll
                 for (int c = 0; c < CT; ++c) acc[r * CT + c] = fmaf(__ldg(xr[r] + i), __ldg(wc[c] + i), acc[r * CT + c]);
         }
-    // acc0+acc1 / acc2+acc3 (distance 8), their sum (16), low + high half (4), the two horizontal adds (1, 2)
-    int mine = 0;  // which output ends in this lane (its first, where a lane keeps several)
-#pragma unroll
-    for (int level = 0; level < 5; ++level) {
-        constexpr int kDist[5] = {8, 16, 4, 1, 2};
-        const int m = kDist[level];
-        if (NO >> level > 1) {
-            const int half = (NO >> level) / 2;
-            const bool up = (lane & m) != 0;
-#pragma unroll
-            for (int o = 0; o < half; ++o) {
-                const float send = up ? acc[o] : acc[o + half], keep = up ? acc[o + half] : acc[o];
-                acc[o] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, send, m));
-            }
-            if (up) mine += half;
-        } else {
-            acc[0] = __fadd_rn(acc[0], __shfl_xor_sync(0xffffffffu, acc[0], m));
-        }
-    }
+    const int mine = fold_partials<NO>(acc, lane);  // which output ends in this lane (its first, where a lane keeps several)
     constexpr int OWN = NO >= 32 ? NO / 32 : 1;
     // with fewer than 32 outputs the lanes that differ in the last levels hold the same one: one of them stores
     constexpr int kDup = NO >= 32 ? 0 : NO == 16 ? 2 : NO == 8 ? 3 : NO == 4 ? 7 : 31;
@@ -263,15 +368,33 @@ int32_t launch_tiled(pssa_b200_ctx* ctx, const float* x, ExactParts& parts, size
     PSSA_CUDA(ctx, launch_dependent(gemm_xwt_exact_tiled_kernel<RT, CT, AHEAD>, dim3((unsigned)blocks), dim3(256), smem, ctx->stream, x, parts, M, (int)K, ldo, alpha));
     return after_launch(ctx, "gemm_xwt_exact_kernel");
 }
+template <int RT, int CT, int WR, int WC, int KB>
+int32_t launch_ring(pssa_b200_ctx* ctx, const float* x, ExactParts& parts, size_t M, size_t K, size_t ldo, float alpha) {
+    constexpr int BR = RT * WR, BC = CT * WC;
+    parts.tiles = 0;
+    for (int i = 0; i < parts.count; ++i) parts.p[i].tile0 = parts.tiles, parts.tiles += (parts.p[i].n + BC - 1) / BC;
+    const size_t blocks = (M + BR - 1) / BR * parts.tiles;
+    if (blocks > 0x7fffffffull) return fail(ctx, PSSA_B200_ERR_SHAPE, "B200 GEMM grid (%zu, 1) exceeds grid limits; refusing launch", blocks);
+    constexpr size_t smem = (size_t)kRingStages * (BR + BC) * KB * sizeof(float);
+    auto kern = gemm_xwt_exact_ring_kernel<RT, CT, WR, WC, KB>;
+    static PerDeviceOnce attr_set;
+    if (smem > 48 * 1024 && attr_set.need(ctx->device)) {
+        PSSA_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        attr_set.done(ctx->device);
+    }
+    PSSA_CUDA(ctx, launch_dependent(kern, dim3((unsigned)blocks), dim3(32 * WR * WC), smem, ctx->stream, x, parts, M, (int)K, ldo, alpha));
+    return after_launch(ctx, "gemm_xwt_exact_kernel");
+}
 int32_t launch_parts(pssa_b200_ctx* ctx, const float* x, ExactParts& parts, size_t M, size_t K, size_t ldo, float alpha) {
-    size_t n = 0;
-    for (int i = 0; i < parts.count; ++i) n += parts.p[i].n;
-    // few rows: every row in one warp, two columns of W a warp, so that W's rows are spread over the most warps; otherwise 8 x 8
-    // tiles (four multiply-adds a load) while they give every SM its eight warps, 8 x 4 below
+    // Up to four rows a warp takes all of them and two columns of W, so that W's rows are spread over the most warps (16384 columns, 4 rows:
+    // 17.4 us; tiles of eight rows 16.3, but 8.7 to 9.5 for 1536 columns where this takes 5.5). Above, tiles of 8 rows x 16 columns where
+    // 16 x 16 would be half empty (17 rows of K = 1536: 7.3 and 11.4 us).
     if (M <= 4 && 4 * K * 4 <= kMaxStagedX) return launch_tiled<4, 2, 24>(ctx, x, parts, M, K, ldo, alpha);
-    if (M <= 16 && 16 * K * 4 <= kMaxStagedX) return launch_tiled<16, 2, 24>(ctx, x, parts, M, K, ldo, alpha);
-    if ((M + 7) / 8 * ((n + 7) / 8) >= (size_t)ctx->sm_count * 8) return launch_tiled<8, 8, 0>(ctx, x, parts, M, K, ldo, alpha);
-    return launch_tiled<8, 4, 0>(ctx, x, parts, M, K, ldo, alpha);
+    bool vec = K % 4 == 0 && K >= 32 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+    for (int i = 0; i < parts.count; ++i) vec = vec && (reinterpret_cast<uintptr_t>(parts.p[i].w) & 15) == 0;
+    if (!vec) return launch_tiled<8, 4, 0>(ctx, x, parts, M, K, ldo, alpha);
+    if (M <= 8 || (M > 16 && M <= 24)) return launch_ring<8, 4, 1, 4, 64>(ctx, x, parts, M, K, ldo, alpha);
+    return launch_ring<8, 8, 2, 2, 128>(ctx, x, parts, M, K, ldo, alpha);
 }
 
 }  // namespace

@@ -44,6 +44,20 @@ def test_exact_gemm_tiles_are_dot_slice_bit_for_bit(gpu, m, n, k):
     assert np.array_equal(bits(got), bits(want + want))
 
 
+@pytest.mark.parametrize("m,n,k", [(5, 15, 32), (8, 16, 100), (9, 17, 160), (16, 33, 36), (17, 15, 132), (24, 16, 64), (25, 31, 772),
+                                   (33, 1, 1536), (47, 19, 260), (16, 64, 520)])
+def test_exact_gemm_ring_tiles_are_dot_slice_bit_for_bit(gpu, m, n, k):
+    """Borders of the 8 x 16 and 16 x 16 tiles, of their stages of 64 and 128 columns, and every tail behind whole blocks of 32."""
+    from pssa_b200 import _native as N
+    rng = np.random.default_rng(m * n + k)
+    x, w = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((n, k)).astype(np.float32)
+    got = gpu.dispatch_gemm(x, w, m, n, k, 1).reshape(m, n)
+    want = O.gemm_xwt(x, w)
+    assert np.array_equal(bits(got), bits(want))
+    gpu.dispatch_gemm_into(x, w, m, n, k, 1, got.reshape(-1), epilogue=N.EPI_ADD_OUT)
+    assert np.array_equal(bits(got), bits(want + want))
+
+
 def test_batch_folds_into_rows_and_bad_lengths_leave_output_untouched(gpu):
     # tests/backend.rs:9-82
     import pssa_b200
