@@ -382,7 +382,11 @@ int32_t launch_ring(pssa_b200_ctx* ctx, const float* x, ExactParts& parts, size_
         PSSA_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         attr_set.done(ctx->device);
     }
-    PSSA_CUDA(ctx, launch_dependent(kern, dim3((unsigned)blocks), dim3(32 * WR * WC), smem, ctx->stream, x, parts, M, (int)K, ldo, alpha));
+    // few rows: the early start's prefetch of W is worth more than an even spread (a scored step of 16 streams 977 us, 1119 spread); 300
+    // rows, whose 64-wide query product is a CTA to every other SM: 3309 and 3139
+    static PerDeviceCount resident;
+    PSSA_CUDA(ctx, launch_spread(resident, M <= 128 ? 1 << 20 : 1, ctx->device, ctx->sm_count, kern, dim3((unsigned)blocks), dim3(32 * WR * WC),
+                                 smem, ctx->stream, x, parts, M, (int)K, ldo, alpha));
     return after_launch(ctx, "gemm_xwt_exact_kernel");
 }
 int32_t launch_parts(pssa_b200_ctx* ctx, const float* x, ExactParts& parts, size_t M, size_t K, size_t ldo, float alpha) {

@@ -184,6 +184,83 @@ __global__ void __launch_bounds__(256) poincare_distance_kernel(RetrieveParams p
     asm volatile("cp.async.wait_group 0;\n" ::);
 }
 
+// The same distances for up to kDistRows rows: 16 queries x 16 slots a CTA and one distance a thread, so that 16 rows are 32 CTAs where the
+// tiles above are 8. What bounds it is the length of its f64 chains (the norm, the projected norm, the distance), so the two norms
+// are summed by a warp of their own, the projected one beside the distances; squares, points and keys are widened once, side by
+// side. Same operations in the same order. Us, keys of 64, 512
+// slots: 16 rows 26.5 -> 10.3, 300 27.4 -> 18.5, 512 26.6 -> 22.6; 1000 rows 29.2 with the tiles above and 38 here.
+constexpr int kDistRows = 512, kDistQ = 16, kDistS = 16, kDistKey = 128;
+__global__ void __launch_bounds__(288) poincare_distance_rows_kernel(RetrieveParams p) {
+    extern __shared__ __align__(16) double dist_sm[];  // (3 dk + 1) x 16 doubles
+    __shared__ double scale[kDistQ];
+    __shared__ float qsq[kDistQ];
+    double (*const pd)[kDistQ] = reinterpret_cast<double (*)[kDistQ]>(dist_sm), (*const kd)[kDistS] = pd + p.dk;  // points and keys [dk][16]
+    double* const sq = dist_sm + 2 * p.dk * 16;  // squares [16][dk + 1]
+    const int pitch = p.dk + 1;
+    const int tid = threadIdx.x, dk = p.dk, count = p.count, row = tid >> 4, j = tid & 15;
+    const size_t q = (size_t)blockIdx.x * kDistQ + row;
+    const int slot0 = blockIdx.y * kDistS, slot = slot0 + j;
+    if (tid < 256 && slot0 + row < count)  // a prefetch reads nothing: no wait
+        for (int i = j * 32; i < dk; i += 512) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.keys + (size_t)(slot0 + row) * dk + i));
+    pdl_trigger();
+    pdl_wait();
+    float v[kDistKey / 16];
+    if (tid < 256) {
+        const float* src = p.q + q * (p.ldq ? p.ldq : (size_t)dk);
+        const float* key = p.keys + (size_t)(slot0 + row) * dk;
+#pragma unroll
+        for (int u = 0; u < kDistKey / 16; ++u) {
+            const int i = u * 16 + j;
+            if (i >= dk) break;
+            v[u] = q < p.rows ? src[i] : 0.0f;
+            sq[row * pitch + i] = __dmul_rn((double)v[u], (double)v[u]);
+            kd[i][row] = slot0 + row < count ? (double)__ldg(key + i) : 0.0;
+        }
+    }
+    __syncthreads();
+    if (tid >= 256 && tid < 256 + kDistQ && p.q_is_euclidean) {
+        // memory.rs:198-211: r = sqrt(sum q^2) in f64, sequential; p = q * min(r/(1+r), R)/r
+        const int r = tid - 256;
+        double r2 = 0.0;
+        for (int i = 0; i < dk; ++i) r2 = __dadd_rn(r2, sq[r * pitch + i]);
+        const double norm = sqrt(r2), max_radius = 1.0 - 8.0 * (double)FLT_EPSILON;
+        scale[r] = (norm == 0.0) ? 1.0 : fmin(norm / (1.0 + norm), max_radius) / norm;
+        const size_t qr = (size_t)blockIdx.x * kDistQ + r;
+        if (p.q_norm && blockIdx.y == 0 && qr < p.rows) p.q_norm[qr] = (float)fmin(norm, (double)FLT_MAX);
+    }
+    __syncthreads();
+    if (tid < 256) {
+#pragma unroll
+        for (int u = 0; u < kDistKey / 16; ++u) {
+            const int i = u * 16 + j;
+            if (i >= dk) break;
+            const float pv = p.q_is_euclidean ? (float)__dmul_rn((double)v[u], scale[row]) : v[u];
+            if (p.q_pnc && blockIdx.y == 0 && q < p.rows) p.q_pnc[q * dk + i] = pv;
+            pd[i][row] = (double)pv;
+            sq[row * pitch + i] = __dmul_rn((double)pv, (double)pv);
+        }
+    }
+    __syncthreads();
+    double acc = 0.0;
+    if (tid < 256) {
+#pragma unroll 8
+        for (int i = 0; i < dk; ++i) {
+            const double df = pd[i][row] - kd[i][j];
+            acc = fma(df, df, acc);
+        }
+    } else if (tid < 256 + kDistQ) {
+        double n2 = 0.0;
+        for (int i = 0; i < dk; ++i) n2 = __dadd_rn(n2, sq[(tid - 256) * pitch + i]);
+        qsq[tid - 256] = (n2 < 1.0 && (float)n2 == 1.0f) ? __uint_as_float(0x3f7fffffu) : (float)n2;  // memory.rs:181-188
+    }
+    __syncthreads();
+    if (tid < 256 && q < p.rows && slot < count) {
+        // memory.rs:245-262: 2*asinh(sqrt(sq/denom)); 2*asinh(z) = log1p(2u + 2*sqrt(u*u + u)), u = z^2
+        const double denom = (1.0 - (double)qsq[row]) * (1.0 - (double)__ldg(p.norm_sq + slot)), u = acc / denom;
+        p.weights[q * p.cap + slot] = (float)log1p(2.0 * u + 2.0 * sqrt(fma(u, u, u)));
+    }
+}
+
 // ------------------------------------------------------------------ A': fp32 distances (fast mode)
 // Same tiling as kernel A with the squared differences accumulated in fp32. Differences are formed first, as in the
 // reference, so near-coincident points lose nothing to cancellation: the squared distance carries a relative error of
@@ -978,6 +1055,104 @@ __global__ void __launch_bounds__(128) value_mix_rows_kernel(RetrieveParams p) {
         }
 }
 
+// The same for values whose rows start on 16 bytes: 64 columns x 4 R rows a CTA, a thread's column of R rows. The columns' values come
+// through a cp.async ring of 64 slots a stage, so that seven stages are on their way (from HBM, with hundreds of MB of fp32 weights a
+// step) while one thread's chain of additions walks the eighth. Us, 512 slots, before -> now: 16 rows of 768 columns 31 -> 16, 64
+// rows 31 -> 14, 300 44 -> 26, 1000 105 -> 65 (1200: the tiles below 70, this 84); 512 rows of 192
+// columns 28 -> 18.
+constexpr int kMixStages = 8, kMixSlots = 64;
+template <int R, bool EXACT>
+__global__ void __launch_bounds__(256) value_mix_ring_kernel(RetrieveParams p) {
+    extern __shared__ __align__(16) float mix_ring[];  // [stages][64 slots][64 columns], then the weights [slots][4][R]
+    const int tid = threadIdx.x, count = p.count, c0 = blockIdx.y * 64, cl = tid & 63, rg = tid >> 6;
+    const size_t q0 = (size_t)blockIdx.x * 4 * R;
+    const int stages = (count + kMixSlots - 1) / kMixSlots, padded = stages * kMixSlots;
+    float* const w = mix_ring + kMixStages * kMixSlots * 64;
+    for (int s = tid >> 1; s < count; s += 128) {  // to L2 before the wait: a prefetch reads nothing
+        const int c = c0 + (tid & 1) * 32;
+        if (c < p.dv) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.values + (size_t)s * p.dv + c));
+    }
+    pdl_trigger();
+    pdl_wait();
+    auto load = [&](int st) {
+        float* dst = mix_ring + (st % kMixStages) * kMixSlots * 64;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int sl = (tid >> 4) + u * 16, c = (tid & 15) * 4, slot = st * kMixSlots + sl;
+            if (c0 + c < p.dv && slot < padded)  // (past the end: the last row again, which nobody reads)
+                cp_async16(dst + sl * 64 + c, p.values + (size_t)min(slot, count - 1) * p.dv + c0 + c);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int st = 0; st < kMixStages - 1; ++st) load(st);
+#pragma unroll 1
+    for (int s = tid; s < padded; s += 256) {
+        float t[4 * R];  // all rows' weights of a slot on their way at once
+#pragma unroll
+        for (int r = 0; r < 4 * R; ++r) t[r] = q0 + r < p.rows && s < count ? p.weights[(q0 + r) * p.cap + s] : 0.0f;
+#pragma unroll
+        for (int r = 0; r < 4 * R; r += 4) *reinterpret_cast<float4*>(w + s * 4 * R + r) = make_float4(t[r], t[r + 1], t[r + 2], t[r + 3]);
+    }
+    float acc[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) acc[r] = 0.0f;
+    for (int st = 0; st < stages; ++st) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kMixStages - 2) : "memory");
+        __syncthreads();
+        load(st + kMixStages - 1);
+        const float* v = mix_ring + (st % kMixStages) * kMixSlots * 64 + cl;
+        const float* ws = w + (size_t)st * kMixSlots * 4 * R + rg * R;
+        const int n = min(kMixSlots, count - st * kMixSlots);
+        auto add = [&](int s) {
+            const float x = v[s * 64];
+            float wr[R];
+            if constexpr (R % 4 == 0) {
+#pragma unroll
+                for (int r = 0; r < R; r += 4) {
+                    const float4 q = *reinterpret_cast<const float4*>(ws + s * 4 * R + r);
+                    wr[r] = q.x, wr[r + 1] = q.y, wr[r + 2] = q.z, wr[r + 3] = q.w;
+                }
+            } else if constexpr (R == 2) {
+                const float2 q = *reinterpret_cast<const float2*>(ws + s * 4 * R);
+                wr[0] = q.x, wr[1] = q.y;
+            } else {
+#pragma unroll
+                for (int r = 0; r < R; ++r) wr[r] = ws[s * 4 * R + r];
+            }
+#pragma unroll
+            for (int r = 0; r < R; ++r) acc[r] = EXACT ? __fadd_rn(acc[r], __fmul_rn(wr[r], x)) : fmaf(wr[r], x, acc[r]);
+        };
+        if (n == kMixSlots) {
+#pragma unroll 16
+            for (int s = 0; s < kMixSlots; ++s) add(s);
+        } else {
+            for (int s = 0; s < n; ++s) add(s);
+        }
+    }
+    if (c0 + cl >= p.dv) return;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const size_t q = q0 + rg * R + r;
+        if (q >= p.rows) continue;
+        if (p.m_val) p.m_val[q * p.dv + c0 + cl] = acc[r];
+        if (p.m_bf16) reinterpret_cast<__nv_bfloat16*>(p.m_bf16)[q * p.dv + c0 + cl] = __float2bfloat16_rn(acc[r]);
+    }
+}
+template <int R>
+int32_t launch_value_mix_ring(pssa_b200_ctx* ctx, const RetrieveParams& p, bool exact) {
+    const dim3 grid((unsigned)((p.rows + 4 * R - 1) / (4 * R)), (unsigned)((p.dv + 63) / 64));
+    const size_t smem = ((size_t)kMixStages * kMixSlots * 64 + (size_t)((p.count + kMixSlots - 1) / kMixSlots * kMixSlots) * 4 * R) * sizeof(float);
+    static PerDeviceOnce attr[2];
+    auto kern = exact ? value_mix_ring_kernel<R, true> : value_mix_ring_kernel<R, false>;
+    if (attr[exact].need(ctx->device)) {
+        PSSA_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+        attr[exact].done(ctx->device);
+    }
+    PSSA_CUDA(ctx, launch_dependent(kern, grid, dim3(256), smem, ctx->stream, p));
+    return PSSA_B200_OK;
+}
+
 // 64 queries x 64 columns per CTA, 4x4 per thread, slots walked in ascending order.
 template <bool EXACT>
 __global__ void __launch_bounds__(256) value_mix_kernel(RetrieveParams p) {
@@ -1104,6 +1279,17 @@ int32_t launch_memory_read(pssa_b200_ctx* ctx, const RetrieveParams& p, bool exa
         while (qblocks * ysplit < 148 && ysplit < 8 && ysplit * 2 <= (npass ? npass : 1)) ysplit *= 2;
         PSSA_CUDA(ctx, launch_dependent(poincare_distance_f32_kernel, dim3((unsigned)qblocks, ysplit), dim3(256), smem_f, ctx->stream, p));
         if ((rc = after_launch(ctx, "poincare_distance_f32_kernel")) != PSSA_B200_OK) return rc;
+    } else if (p.rows <= kDistRows && p.dk <= kDistKey && p.count <= 65535 * kDistS) {
+        const dim3 grid((unsigned)((p.rows + kDistQ - 1) / kDistQ), (unsigned)std::max(1, (p.count + kDistS - 1) / kDistS));
+        const size_t smem = (size_t)(3 * p.dk + 1) * 16 * sizeof(double);
+        static PerDeviceOnce attr_r;
+        if (smem > 48 * 1024 && attr_r.need(ctx->device)) {
+            PSSA_CUDA(ctx, cudaFuncSetAttribute(poincare_distance_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 56 * 1024));
+            attr_r.done(ctx->device);
+        }
+        static PerDeviceCount resident;
+        PSSA_CUDA(ctx, launch_spread(resident, 1, ctx->device, ctx->sm_count, poincare_distance_rows_kernel, grid, dim3(288), smem, ctx->stream, p));
+        if ((rc = after_launch(ctx, "poincare_distance_kernel")) != PSSA_B200_OK) return rc;
     } else {
         unsigned ysplit = 1;  // few query tiles (decode): spread the slot passes over up to 8 CTAs per tile
         const unsigned npass = (unsigned)((p.count + STL - 1) / STL);
@@ -1152,7 +1338,15 @@ int32_t launch_memory_read(pssa_b200_ctx* ctx, const RetrieveParams& p, bool exa
             return rc;
     } else if (p.count > 0 && !topk) {
         dim3 grid((unsigned)qblocks, (unsigned)((p.dv + 63) / 64));
-        if (p.rows <= kMixRows && p.count <= 2048) {
+        const bool rows16 = p.dv % 4 == 0 && (reinterpret_cast<uintptr_t>(p.values) & 15) == 0 && p.count <= 1024;
+        if (p.rows <= kMixRows && rows16) {
+            // the fewest rows a thread that leave no more than a CTA to an SM (its ring takes the shared memory of one)
+            const size_t cols = (p.dv + 63) / 64;
+            auto fits = [&](size_t r) { return (p.rows + 4 * r - 1) / (4 * r) * cols <= (size_t)ctx->sm_count; };
+            rc = fits(1) ? launch_value_mix_ring<1>(ctx, p, exact) : fits(2) ? launch_value_mix_ring<2>(ctx, p, exact)
+                 : fits(4) || p.count > 640 ? launch_value_mix_ring<4>(ctx, p, exact) : launch_value_mix_ring<8>(ctx, p, exact);
+            if (rc) return rc;
+        } else if (p.rows <= kMixRows && p.count <= 2048) {
             const dim3 small((unsigned)((p.rows + 3) / 4), (unsigned)((p.dv + 127) / 128));
             const size_t smem = (size_t)((p.count + 63) / 64 * 64) * 16;
             PSSA_CUDA(ctx, launch_dependent(exact ? value_mix_rows_kernel<true> : value_mix_rows_kernel<false>, small, dim3(128), smem, ctx->stream, p));

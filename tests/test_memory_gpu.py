@@ -66,6 +66,27 @@ def test_fp32_distance_mode_stays_within_its_stated_error(gpu, rows, dk, dv, cap
     assert abs(float(w[0].sum()) - 1.0) <= 1e-5
 
 
+@pytest.mark.parametrize("rows,dk,dv,cap,count,euclid", [(1, 3, 4, 5, 1, True), (15, 64, 68, 64, 63, True), (17, 128, 192, 80, 65, False),
+                                                         (45, 64, 768, 512, 512, True), (70, 127, 64, 96, 0, True), (100, 64, 132, 700, 641, True),
+                                                         (150, 64, 768, 256, 200, True), (512, 16, 60, 64, 16, True), (513, 16, 60, 64, 17, True)])
+def test_exact_read_of_few_rows(gpu, rows, dk, dv, cap, count, euclid):
+    """The distances' 16 x 16 tiles and the value read's ring at their borders: one, two, four and eight rows a thread, columns that fill
+    no tile, one slot, and none. Projections and weights are the tiled kernels' own, the value read's order is the reference's."""
+    keys, norm_sq, values = make_bank(cap, dk, dv, rows + cap)
+    rng = np.random.default_rng(rows)
+    q = (rng.standard_normal((rows, dk)) * rng.uniform(0.05, 3.0, (rows, 1))).astype(np.float32)
+    if not euclid:
+        q = (q / np.linalg.norm(q, axis=1, keepdims=True) * rng.uniform(0, 0.9, (rows, 1))).astype(np.float32)
+    check(gpu, q, keys, norm_sq, values, count, 0.1, 0, euclid, True)
+    check(gpu, q, keys, norm_sq, values, count, 0.1, 0, euclid, False)
+    if count:  # the sum over slots in ascending order, every operation rounded
+        _, _, w, m, _ = gpu.memory_read(q, keys, norm_sq, values, count, 0.1, 0, euclid, True)
+        want = np.zeros((rows, dv), np.float32)
+        for s in range(count):
+            want = want + w[:, s:s + 1] * values[s]
+        assert np.array_equal(m.view(np.uint32), want.view(np.uint32))
+
+
 @pytest.mark.parametrize("top_k", [0, 8])
 @pytest.mark.parametrize("rows,dk,dv,cap,count", [(1, 64, 64, 64, 1), (65, 64, 64, 32, 32), (300, 64, 192, 512, 512),
                                                   (130, 64, 70, 100, 77), (17, 128, 128, 512, 300), (64, 33, 16, 64, 64)])
