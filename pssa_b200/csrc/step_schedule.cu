@@ -356,7 +356,11 @@ int32_t launch_step_schedule(pssa_b200_ctx* ctx, const StepLaunch& p) {
         const StepBlock b = step_block(p.blocks[l]);
         float* const out = in == a.feat_a ? a.feat_b : a.feat_a;
         const unsigned* const ids = l == 0 ? a.ids : nullptr;
-        PSSA_CUDA(ctx, launch_dependent(step_norm_kernel, dim3(((unsigned)a.rows + kWarps - 1) / kWarps), dim3(kThreads), 0, ctx->stream, a, b, ids, in));
+        // started early its few CTAs crowd on the SMs that the product before leaves first (256 streams of 12 blocks of d 768: 1114 -> 1074
+        // us a step, 64 871 -> 858; 128 of 4 blocks of d 384 231 -> 228); at d 192 the launch's latency is more (200 streams 66.5, 68.4)
+        const dim3 norm_grid(((unsigned)a.rows + kWarps - 1) / kWarps);
+        if (d > 256) step_norm_kernel<<<norm_grid, kThreads, 0, ctx->stream>>>(a, b, ids, in);
+        else PSSA_CUDA(ctx, launch_dependent(step_norm_kernel, norm_grid, dim3(kThreads), 0, ctx->stream, a, b, ids, in));
         if ((rc = after_launch(ctx, "step_norm_kernel"))) return rc;
         if ((rc = narrow(ctx, a, a.nc) ? product<32, 9, PutXside>(ctx, a, a.x, d, b.wcat, d, a.nc, d, "step_product_kernel[x-side]")
                                        : product<64, 7, PutXside>(ctx, a, a.x, d, b.wcat, d, a.nc, d, "step_product_kernel[x-side]")))
