@@ -225,13 +225,15 @@ int32_t launch_gemm_bf16_cat(pssa_b200_ctx* ctx, const void* x16, const void* w1
 
 // step_decode.cu, step_schedule.cu: one token per row through every block and the vocabulary head (bf16 mode), in one cooperative
 // launch or, for many rows, in a launch per stage. A row's bits do not depend on the number of rows.
+constexpr int kStepOwnRows = 32;  // as many as the one-kernel form takes
 struct StepLaunch {
     int rows, d, s, k, cap, nc, off_b, off_q, off_gate, off_act;
     size_t depth;
     unsigned vocab;
     float ssm_scale, head_scale, tau;
     const float* embed;
-    const uint32_t *ids, *slots;     // [rows]
+    const uint32_t *ids, *slots;     // [rows] on the device, or null:
+    const uint32_t *host_ids, *host_slots;  // [rows <= kStepOwnRows] host arrays that travel with the launch (one-kernel form only)
     const void* unembed;
     size_t carry_stride;
     float *feat_a, *feat_b, *proj, *y, *qpart, *ssq, *inv;  // qpart [rows, d / 8, k], ssq [rows, d / 16], inv [rows]

@@ -230,7 +230,7 @@ __device__ __forceinline__ void prefetch_vectors(const StepArgs& a, int l) {
 
 // NT 8-row tiles of rows: the stages are inlined, because the weights and carries that a stage asks for before
 // the barrier in front of it stay in registers across it.
-template <int NT, int NV>
+template <int NT, int NV, bool OWN>
 __global__ void __launch_bounds__(kThreads, 1) step_kernel(const __grid_constant__ StepArgs a) {
     extern __shared__ __align__(128) float step_smem[];
     constexpr int kShared = NT * 64 * kPitch < 448 ? 448 : NT * 64 * kPitch;
@@ -244,23 +244,23 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(const __grid_constant
         if ((int)blockIdx.x * 16 < w.n) request(w, blockIdx.x, ah);
     };
     ahead({a.block[0].wcat, (size_t)d, a.nc, d});
-    check_ids(a);
+    check_ids<OWN>(a);
     prefetch_vectors(a, 0);
     const float* in = nullptr;
     for (int l = 0; l < a.depth; ++l) {
         const StepBlock& b = a.block[l];
         float* out = in == a.feat_a ? a.feat_b : a.feat_a;
-        const Features f{a.embed, l == 0 ? a.ids : nullptr, in, d, a.vocab};
+        const Features f{a.embed, l == 0 ? ids_of<OWN>(a) : nullptr, in, d, a.vocab};
         const Weights wcat{b.wcat, (size_t)d, a.nc, d}, vp{b.vp, (size_t)3 * a.cap, d, a.cap}, w1{b.w1, (size_t)d + 64, 2 * d, d + 64},
             w2{b.w2, (size_t)2 * d + 64, d, 2 * d + 64};
         row_scales(a, f, 0, a.rows, inv_s, blockIdx.x == 0);
         small_product<NT>(wcat, RowsNorm{f, b.gamma, b.beta, inv_s, 0}, a.rows, ah, sm, [&](int c, int r, float v) { store(PutXside{a}, c, r, v); });
         bar.arrive();
         SsmAhead<NV, 2> sa;
-        ssm_request(a, b, sa);
+        ssm_request<OWN>(a, b, sa);
         const bool keys_here = request_keys(a, b, keys_s);
         bar.wait();
-        ssm_stage(a, f, sa, b.state);
+        ssm_stage<OWN>(a, f, sa, b.state);
         bar.arrive();
         ahead(vp);
         bar.wait();
@@ -293,10 +293,10 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(const __grid_constant
     small_product<NT>({a.unembed, (size_t)d, (int)a.vocab, d}, RowsF32{in, (size_t)d}, a.rows, ah, sm, [&](int c, int r, float v) { store(PutLogit{a}, c, r, v); });
 }
 
-template <int NT, int NV>
+template <int NT, int NV, bool OWN>
 int32_t launch_one_kernel(pssa_b200_ctx* ctx, StepArgs& a) {
     constexpr size_t own = 64 * 4 + (size_t)(NT * 64 * kPitch < 448 ? 448 : NT * 64 * kPitch) * 4;
-    auto kern = step_kernel<NT, NV>;
+    auto kern = step_kernel<NT, NV, OWN>;
     static PerDeviceOnce attr;
     if (attr.need(ctx->device)) {
         PSSA_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(own + kKeyQuads * 16)));
@@ -308,9 +308,9 @@ int32_t launch_one_kernel(pssa_b200_ctx* ctx, StepArgs& a) {
                                                own + (size_t)std::min(a.k / 4 * a.cap, kKeyQuads) * 16, ctx->stream));
     return after_launch(ctx, "step_kernel");
 }
-template <int NV>
+template <int NV, bool OWN>
 int32_t launch_rows(pssa_b200_ctx* ctx, StepArgs& a) {
-    return a.rows <= 8 ? launch_one_kernel<1, NV>(ctx, a) : a.rows <= 16 ? launch_one_kernel<2, NV>(ctx, a) : launch_one_kernel<4, NV>(ctx, a);
+    return a.rows <= 8 ? launch_one_kernel<1, NV, OWN>(ctx, a) : a.rows <= 16 ? launch_one_kernel<2, NV, OWN>(ctx, a) : launch_one_kernel<4, NV, OWN>(ctx, a);
 }
 
 // keys [cap, k] -> [k / 4][cap] quads: a warp's read of one quad of 32 slots is contiguous
@@ -334,13 +334,16 @@ bool step_shape_ok(size_t depth, size_t d, size_t s, size_t k, size_t cap, size_
            cap <= 4 * kThreads && rank == 16;
 }
 
+static_assert(kOneKernelRows == kStepOwnRows, "a host call's rows travel with the one kernel's launch");
+
 int32_t launch_decode_step(pssa_b200_ctx* ctx, const StepLaunch& p) {
     if (p.rows > kOneKernelRows) return launch_step_schedule(ctx, p);
     StepArgs a{};
     static_cast<StepCommon&>(a) = step_common(ctx, p);
     a.barrier = (unsigned long long*)p.barrier;
     for (size_t l = 0; l < p.depth; ++l) a.block[l] = step_block(p.blocks[l]);
-    return p.s == 16 ? launch_rows<1>(ctx, a) : p.s == 32 ? launch_rows<2>(ctx, a) : launch_rows<4>(ctx, a);
+    if (!p.ids) return p.s == 16 ? launch_rows<1, true>(ctx, a) : p.s == 32 ? launch_rows<2, true>(ctx, a) : launch_rows<4, true>(ctx, a);
+    return p.s == 16 ? launch_rows<1, false>(ctx, a) : p.s == 32 ? launch_rows<2, false>(ctx, a) : launch_rows<4, false>(ctx, a);
 }
 
 }  // namespace pssa

@@ -65,13 +65,19 @@ struct StepCommon {
     unsigned vocab;
     float ssm_scale, head_scale, tau;
     const float* embed;
-    const unsigned *ids, *slots;
+    const unsigned *ids, *slots;  // [rows]; a host call's few rows have theirs in own_ids, own_slots
     const __nv_bfloat16* unembed;
     size_t carry_stride;
     float *feat_a, *feat_b, *proj, *y, *qpart, *ssq, *inv, *logits;
     __nv_bfloat16 *x, *w, *z, *act;  // x: the normalised rows, at the end the features (where rows have a norm stage)
     int* status;
+    unsigned own_ids[kStepOwnRows], own_slots[kStepOwnRows];  // of a host call's few rows: no copy in front of the launch
 };
+// (OWN, known at compile time: a choice at run time costs the SSM stage registers it does not have, 270 -> 278 us a step)
+template <bool OWN>
+__device__ __forceinline__ const unsigned* ids_of(const StepCommon& a) { return OWN ? a.own_ids : a.ids; }
+template <bool OWN>
+__device__ __forceinline__ unsigned slot_of(const StepCommon& a, int r) { return OWN ? a.own_slots[r] : a.slots[r]; }
 
 // the features of a row: embedding row of its id (first block) or the previous block's output
 struct Features {
@@ -135,7 +141,7 @@ struct SsmAhead {
     float* carry[RING];
     int r0, r1, group;
 };
-template <int NV, int RING>
+template <bool OWN = false, int NV, int RING>
 __device__ __forceinline__ void ssm_request(const StepCommon& a, const StepBlock& b, SsmAhead<NV, RING>& q) {
     const int lane = threadIdx.x & 31, w = (threadIdx.x >> 5) * gridDim.x + blockIdx.x, groups = a.d / 8;
     const int chunks = min(a.rows, (int)gridDim.x * kWarps / groups), chunk = w / groups;
@@ -146,7 +152,7 @@ __device__ __forceinline__ void ssm_request(const StepCommon& a, const StepBlock
 #pragma unroll
     for (int u = 0; u < RING; ++u)
         if (q.r0 + u < q.r1) {
-            const float* c = q.carry[u] = b.state + (size_t)a.slots[q.r0 + u] * a.carry_stride + (size_t)i * (NV * 16) + (lane & 3) * 4;
+            const float* c = q.carry[u] = b.state + (size_t)slot_of<OWN>(a, q.r0 + u) * a.carry_stride + (size_t)i * (NV * 16) + (lane & 3) * 4;
 #pragma unroll
             for (int v = 0; v < NV; ++v) q.h[u][v] = *reinterpret_cast<const float4*>(c + v * 16);
         }
@@ -157,7 +163,7 @@ __device__ __forceinline__ void ssm_request(const StepCommon& a, const StepBlock
         if (v * 32 < a.k) q.wq[v] = __ldg(reinterpret_cast<const uint4*>(b.wqh + (size_t)(v * 32 + lane) * a.d + q.group * 8));
     q.gamma = __ldg(b.gamma + i), q.beta = __ldg(b.beta + i);
 }
-template <int NV, int RING>
+template <bool OWN = false, int NV, int RING>
 __device__ __forceinline__ void ssm_stage(const StepCommon& a, const Features& f, SsmAhead<NV, RING>& s, float* state) {
     if (s.r0 >= s.r1) return;
     constexpr int LEAD = RING > 2 ? 2 : 1;  // rows whose operands are asked for ahead
@@ -174,7 +180,7 @@ __device__ __forceinline__ void ssm_stage(const StepCommon& a, const Features& f
     };
     fetch(s.r0, in[0]);
     if (LEAD > 1 && s.r0 + 1 < s.r1) fetch(s.r0 + 1, in[1]);
-    unsigned slot = s.r0 + RING < s.r1 ? a.slots[s.r0 + RING] : 0;  // of the row whose carry is asked for next
+    unsigned slot = s.r0 + RING < s.r1 ? slot_of<OWN>(a, s.r0 + RING) : 0;  // of the row whose carry is asked for next
     for (int rb = s.r0; rb < s.r1; rb += RING) {
 #pragma unroll
         for (int u = 0; u < RING; ++u) {
@@ -197,7 +203,7 @@ __device__ __forceinline__ void ssm_stage(const StepCommon& a, const Features& f
             }
             if (r + RING < s.r1) {
                 const float* c = s.carry[u] = state + (size_t)slot * a.carry_stride + (size_t)i * (NV * 16) + q * 4;
-                if (r + RING + 1 < s.r1) slot = a.slots[r + RING + 1];
+                if (r + RING + 1 < s.r1) slot = slot_of<OWN>(a, r + RING + 1);
 #pragma unroll
                 for (int v = 0; v < NV; ++v) s.h[u][v] = *reinterpret_cast<const float4*>(c + v * 16);
             }
@@ -476,10 +482,11 @@ __device__ __forceinline__ float new_feature(const StepCommon& a, const float* i
 }
 
 // device-resident ids cannot be checked on the host: row 0 is read and the status word raised
+template <bool OWN = false>
 __device__ __forceinline__ void check_ids(const StepCommon& a) {
     if (blockIdx.x == 0)
         for (int r = threadIdx.x; r < a.rows; r += kThreads)
-            if (a.ids[r] >= a.vocab) atomicExch(a.status, PSSA_B200_ERR_TOKEN);
+            if (ids_of<OWN>(a)[r] >= a.vocab) atomicExch(a.status, PSSA_B200_ERR_TOKEN);
 }
 
 // ---- host side
@@ -492,6 +499,8 @@ inline StepCommon step_common(const pssa_b200_ctx* ctx, const StepLaunch& p) {
     a.feat_a = p.feat_a, a.feat_b = p.feat_b, a.proj = p.proj, a.y = p.y, a.qpart = p.qpart, a.ssq = p.ssq, a.inv = p.inv, a.logits = p.logits;
     a.x = (__nv_bfloat16*)p.x, a.w = (__nv_bfloat16*)p.w, a.z = (__nv_bfloat16*)p.z, a.act = (__nv_bfloat16*)p.act;
     a.status = ctx->status_dev;
+    if (!p.ids)
+        for (int r = 0; r < p.rows && r < kStepOwnRows; ++r) a.own_ids[r] = p.host_ids[r], a.own_slots[r] = p.host_slots[r];
     return a;
 }
 inline StepBlock step_block(const StepLaunch::Block& s) {
