@@ -1243,6 +1243,10 @@ int32_t launch_ssm_fused(pssa_b200_ctx* ctx, const SsmParams& p, bool exact) {
         if (channels <= (exact ? 2 : 1) * schedulers && !by_shape) return launch_wide<32, 2, 32>(ctx, p, exact);
         // (resident CTAs count every lane, however short)
         if (channels <= 4 * schedulers && (size_t)p.lanes * p.d <= 4 * schedulers) return launch_wide<16, 4, 32>(ctx, p, exact);
+        // (five CTAs of the 16 x 4 split fit an SM: a sixth would run behind them. Four channels a warp then, 8 x 8, three CTAs to an SM;
+        // 8 lanes of d 768, 1024 tokens 174 -> 148 us, but 7 lanes 142 and 148, 10 lanes 192 and 204)
+        const size_t ctas = channels / 8, sms = (size_t)ctx->sm_count;
+        if (!exact && !tape && !by_shape && !p.ragged && ctas > 5 * sms && ctas <= 6 * sms) return launch_wide<8, 8, 16>(ctx, p, exact);
         const double wide_us = 13.8 * (double)channels / (double)schedulers;
         const double tiled_us = 60.0 + 64.5 * (double)tiled_shape(ctx, p.d, lanes).busiest;
         if (exact || tape || by_shape || wide_us < tiled_us) return launch_wide<16, 4, 16>(ctx, p, exact);

@@ -48,3 +48,29 @@ def test_few_lanes_matches_the_ordered_recurrence(gpu, d, s, lengths, exact):
     assert torch.equal(c2, t[5])
     if exact:
         assert torch.equal(y, y2)
+
+
+def test_eight_lanes_of_a_wide_model_take_the_eight_by_eight_split(gpu):
+    """The split chosen where a sixth CTA of the 16 x 4 one would not fit an SM, against the recurrence in f64 (tile tails included)."""
+    import torch
+    lanes, T, d, s = 8, 277, 768, 64
+    g = torch.Generator(device="cuda").manual_seed(2)
+    f = lambda *sh: torch.randn(*sh, device="cuda", generator=g)  # noqa: E731
+    delta = torch.nn.functional.softplus(f(lanes * T, d)).contiguous()
+    rates = -torch.exp(torch.empty(d, s, device="cuda").uniform_(-5.0, -0.4, generator=g))
+    bp, cp, x, carry = f(lanes * T, s), f(lanes * T, s), f(lanes * T, d), f(lanes, d * s)
+    h = carry.double().reshape(lanes, d, s)
+    off, ln = (np.arange(lanes) * T).astype(np.uint32), np.full(lanes, T, np.uint32)
+    y = torch.zeros(lanes * T, d, device="cuda")
+    gpu.set_stream(torch.cuda.current_stream())
+    gpu.ssm_forward_dev(delta, bp, cp, x, rates, carry, y, off, ln, lanes * T, d, s)
+    torch.cuda.synchronize()
+    gpu.set_stream(None)
+    q = lambda a: a.double().reshape(lanes, T, -1)  # noqa: E731
+    dl, b, c, xv = q(delta), q(bp), q(cp), q(x)
+    want = []
+    for t in range(T):
+        h = torch.exp(dl[:, t, :, None] * rates.double()) * h + (dl[:, t] * xv[:, t])[:, :, None] * b[:, t, None, :]
+        want.append((h * c[:, t, None, :]).sum(2))
+    assert chan_err(y.cpu().numpy(), torch.stack(want, 1).reshape(lanes * T, d).cpu().numpy(), 0) <= REL_TOL
+    assert chan_err(carry.cpu().numpy().ravel(), h.cpu().numpy().ravel(), 0) <= REL_TOL
