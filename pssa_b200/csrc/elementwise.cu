@@ -40,7 +40,7 @@ __global__ void __launch_bounds__(256) embed_norm_kernel(const float* __restrict
                                        reinterpret_cast<uintptr_t>(gamma) | reinterpret_cast<uintptr_t>(beta)) & 15) == 0 &&
                      (reinterpret_cast<uintptr_t>(x_bf16) & 7) == 0;
     if (vec) {
-#pragma unroll 2
+#pragma unroll 6
         for (int i = lane * 4; i < d; i += 128) {
             const float4 v = __ldg(reinterpret_cast<const float4*>(src + i));
             *reinterpret_cast<float4*>(buf + i) = v;
@@ -79,6 +79,7 @@ __global__ void __launch_bounds__(256) embed_norm_kernel(const float* __restrict
     }
     const float inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(sum, (float)d), 1e-5f)));
     if (vec) {
+#pragma unroll 3
         for (int i = lane * 4; i < d; i += 128) {
             const float4 b4 = *reinterpret_cast<const float4*>(buf + i);
             const float4 g4 = __ldg(reinterpret_cast<const float4*>(gamma + i)), t4 = __ldg(reinterpret_cast<const float4*>(beta + i));
