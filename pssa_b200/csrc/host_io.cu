@@ -14,7 +14,6 @@ namespace {
 
 constexpr size_t kKeepDevice = (size_t)256 << 20;  // device region kept between calls, at most
 constexpr size_t kPinnedMax = (size_t)4 << 20;     // a context's pinned buffer: larger transfers go through it in windows
-constexpr size_t kPinnedMin = (size_t)256 << 10;
 constexpr size_t kPinnedKept = 4;                  // pinned buffers kept for the next context, while any context lives
 constexpr size_t kPinnedInputs = (size_t)2 << 20;  // above this the driver's own pipelined pageable copy is as fast
 constexpr size_t kPiece = (size_t)512 << 10;       // one device copy of a large transfer

@@ -53,6 +53,8 @@ int32_t copy_to_host(pssa_b200_ctx* ctx, void* dst, const void* src_dev, size_t 
 int32_t copy_to_device(pssa_b200_ctx* ctx, void* dst_dev, const void* src, size_t bytes);
 // outputs from here on are copied by several threads
 constexpr size_t kThreadsFrom = (size_t)1 << 20;
+// the pinned buffer that every context starts with: a larger one costs milliseconds to pin
+constexpr size_t kPinnedMin = (size_t)256 << 10;
 // pinned host memory of the context, at least `bytes`, valid until the next call; waits for the stream when it has to grow, and for
 // a copy that pinned_send left behind
 int32_t pinned_reserve(pssa_b200_ctx* ctx, size_t bytes);

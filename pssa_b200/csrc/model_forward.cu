@@ -706,7 +706,7 @@ int32_t run_lanes(pssa_b200_model* m, const uint64_t* ids, const uint32_t* offse
         // A step of a few streams takes its ids along with the launch and leaves logits that nothing on the device reads in pinned
         // memory itself: no copy before it and none behind (chat on the small model 56 -> 45 us a token, on the large one 306 -> 291).
         const bool own = step && rows <= kStepOwnRows && !sampling;
-        const bool direct = own && logits && !greedy && nh * row <= ((size_t)256 << 10);
+        const bool direct = own && logits && !greedy && o_logits + nh * row <= kPinnedMin;
         if (direct && (rc = pinned_reserve(ctx, o_logits + nh * row))) return rc;
         if (!own && (rc = send_description(m, h_ids, s_off, s_len, s_slot, h_last, h_row_slot, head_slot))) return rc;
         if (step) {
@@ -732,8 +732,9 @@ int32_t run_lanes(pssa_b200_model* m, const uint64_t* ids, const uint32_t* offse
                 if ((rc = launch_sample(ctx, sp))) return rc;
                 if ((rc = launch_push_recent(ctx, m->sampler.ids, ws.head_slot, m->sampler.recent, m->sampler.count, nh))) return rc;
             }
-            // results through pinned memory: ids, sampler status, confidences, then the logits unless there are many
-            const bool together = logits && nh * row < kThreadsFrom;
+            // results through pinned memory: ids, sampler status, confidences, then the logits, at once or in as many rows at a time as
+            // the smallest buffer holds (growing it in a first call would cost more than it ever gives back)
+            const bool together = logits && o_logits + nh * row <= kPinnedMin;
             if ((rc = pinned_reserve(ctx, o_logits + (together ? nh * row : 0)))) return rc;
             char* const h = ctx->pinned;
             if (greedy) PSSA_CUDA(ctx, cudaMemcpyAsync(h, sampling ? m->sampler.ids : ws.greedy, nh * 4, cudaMemcpyDeviceToHost, st));
@@ -745,9 +746,12 @@ int32_t run_lanes(pssa_b200_model* m, const uint64_t* ids, const uint32_t* offse
                 for (size_t i = 0; i < nh; ++i) std::memcpy(logits + head_lane[i] * m->v, h + o_logits + i * row, row);
             const std::vector<uint32_t> got((const uint32_t*)h, (const uint32_t*)(h + 3 * nh * 4));
             if (logits && !together)
-                for (size_t i = 0, j; i < nh; i = j) {  // contiguous runs of lanes in one transfer
-                    for (j = i + 1; j < nh && head_lane[j] == head_lane[j - 1] + 1; ++j) {}
-                    if ((rc = copy_to_host(ctx, logits + head_lane[i] * m->v, ws.logits + i * m->v, (j - i) * row))) return rc;
+                for (size_t i = 0, n; i < nh; i += n) {
+                    n = std::min(nh - i, std::max<size_t>(1, kPinnedMin / row));
+                    if ((rc = pinned_reserve(ctx, n * row))) return rc;
+                    PSSA_CUDA(ctx, cudaMemcpyAsync(ctx->pinned, ws.logits + i * m->v, n * row, cudaMemcpyDeviceToHost, st));
+                    PSSA_CUDA(ctx, cudaStreamSynchronize(st));
+                    for (size_t j = 0; j < n; ++j) std::memcpy(logits + head_lane[i + j] * m->v, ctx->pinned + j * row, row);
                 }
             if (greedy)
                 for (size_t i = 0; i < nh; ++i) {
