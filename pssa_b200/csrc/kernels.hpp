@@ -36,6 +36,7 @@ struct SsmParams {
     int d, s, lanes;
     int max_len;           // longest lane, 0 = not known: with `rows` it tells how many lanes are in flight at a time
     int tiled;             // time chunks: stay with the tiled kernel
+    int small_args;        // (set by the launch) tiles of small arguments may take their own path
     int ragged;            // lanes come longest first and differ in length: the launch spreads their CTAs evenly over the SMs
     int aligned;           // 16-byte vector staging allowed
     // row pitches in floats (0 = dense: d for delta, s for b_proj / c_proj)

@@ -469,7 +469,7 @@ __global__ void __launch_bounds__(THR, (ST <= 16 && !TAPE && !EXACT) ? (CPT > 1 
                 finish(tt, yp, ypb);
             }
         };
-        bool small = HAS_SMALL && nt == kTileTokens;
+        bool small = HAS_SMALL && p.small_args && nt == kTileTokens;
         if constexpr (HAS_SMALL) {
             // largest delta of the warp's channels over the tile, each group of lanes looking at its share of the tokens: bit
             // patterns compare like the numbers, and negative deltas and NaNs lie above all others
@@ -1086,6 +1086,9 @@ int32_t launch_cfg(pssa_b200_ctx* ctx, const SsmParams& p) {
     static PerDeviceCount resident;
     SsmParams q = p;
     q.ragged = p.ragged ? ctx->sm_count : 0;
+    // which tiles are small is a warp's verdict over its channels, whose number depends on the lanes: not for prompts of under 256
+    // tokens, whose bits are the same in any batch
+    q.small_args = p.tiled || p.max_len == 0 || p.max_len >= 256;
     PSSA_CUDA(ctx, launch_spread(resident, p.ragged ? 0 : 1, ctx->device, ctx->sm_count, kern, dim3((unsigned)blocks), dim3(kThreads), smem,
                                  ctx->stream, q));
     return after_launch(ctx, MAPS ? "ssm_fused_kernel[chunk maps]" : "ssm_fused_kernel");
@@ -1235,7 +1238,8 @@ int32_t launch_ssm_fused(pssa_b200_ctx* ctx, const SsmParams& p, bool exact) {
         // (from there on time chunks depend on the lanes too) the split follows the shape alone and a stream sees the same bits
         // alone and in a batch; the exact mode's order is always the same.
         const size_t longest = p.max_len ? (size_t)p.max_len : (p.lengths ? 1 : p.rows);
-        const int lanes = (int)std::max<size_t>(1, p.max_len || !p.lengths ? p.rows / std::max<size_t>(1, longest) : (size_t)p.lanes);
+        // (never more than there are: `rows` may count rows of no lane)
+        const int lanes = (int)std::max<size_t>(1, p.max_len || !p.lengths ? std::min<size_t>(p.rows / std::max<size_t>(1, longest), (size_t)p.lanes) : (size_t)p.lanes);
         const size_t channels = (size_t)lanes * p.d, schedulers = 4 * (size_t)ctx->sm_count;
         const bool by_shape = !exact && longest < 256;
         if (s == 16) return channels <= 4 * schedulers && !by_shape ? launch_wide<8, 2, 32>(ctx, p, exact) : launch_wide<4, 4, 16>(ctx, p, exact);

@@ -273,6 +273,23 @@ def test_rows_of_a_partly_filled_band_have_the_bits_of_whole_ones(gpu, lanes, la
     gm.close()
 
 
+def test_short_prompts_of_a_tiled_state_width_keep_their_bits_in_a_batch(gpu):
+    """48 states take the tiled SSM kernel at any number of lanes, with two channels a thread for one lane and one for 48: prompts of
+    200 tokens have the same logits and carries either way."""
+    import pssa_b200
+    om = O.Model.new(1, 257, 768, 48, 64, 128, tau_mem=0.1, seed=9)
+    fill_synthetic(om, 9)
+    gm = pssa_b200.PSSAModel(gpu, 1, 257, 768, 48, 64, 128, tau_mem=0.1, streams=48, precision=0)
+    upload(om, gm)
+    prompts = [np.random.default_rng(i).integers(1, 257, 200) for i in range(48)]
+    want = gm.prefill_batch(prompts)[0]
+    state = gm.copy_recurrent_state_to(7)
+    gm.reset_recurrent_state()
+    got = gm.prefill_batch([prompts[7]], streams=[7])[0]
+    assert np.array_equal(got[0], want[7]) and np.array_equal(gm.copy_recurrent_state_to(7), state)
+    gm.close()
+
+
 def test_time_chunks_that_hold_no_token_leave_the_carry_as_it_is(gpu):
     """A long prompt cut into 37 time chunks beside prompts of 7, 36 and 1 tokens, most of whose chunks are empty: carries and logits
     against the same prompts read in windows too short to be cut. (A chunk's decay is one exponential where the recurrence multiplies
