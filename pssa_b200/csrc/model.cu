@@ -145,7 +145,7 @@ void pssa_b200_model_destroy(pssa_b200_model* m) {
     cudaFree(m->score.logits), cudaFree(m->score.targets), cudaFree(m->score.loss);
     cudaFree(m->sampler.recent), cudaFree(m->sampler.count), cudaFree(m->sampler.rng), cudaFree(m->sampler.ids);
     cudaFree(m->sampler.status), cudaFree(m->sampler.probs), cudaFree(m->sampler.conf);
-    cudaFree(m->chunks.off), cudaFree(m->chunks.len), cudaFree(m->chunks.records), cudaFree(m->chunks.carry_in);
+    cudaFree(m->chunks.host.off), cudaFree(m->chunks.dev.off), cudaFree(m->chunks.records), cudaFree(m->chunks.carry_in);
     cudaFree(m->step_barrier);
     for (auto& b : m->blocks) {
         for (int id : kBlockTensors) cudaFree(b.w[id]);
@@ -314,7 +314,7 @@ int32_t pssa_b200_model_set_option(pssa_b200_model* m, int32_t option, int32_t v
             // the extra feature buffer of the passes lives in the activation workspace: rebuild it on the next call
             if (m->ws.base) cudaFree(m->ws.base);
             m->ws = pssa::Workspace();
-            m->dev_layout.ws_base = nullptr;
+            m->dev_layout.valid = false;
             return PSSA_B200_OK;
         }
         case 5:  // lane groups (not a reference option): 0 = by shape, 1 = one stream, 2..4 = that many groups

@@ -51,11 +51,20 @@ struct DeviceBlock {
     bool keys_t_dirty = true;
 };
 
+// what the device knows of a call: its ids, its lanes as the SSM stage takes them, and the rows and streams of its steps and heads
+struct LaneTables {
+    uint32_t *off = nullptr, *len = nullptr, *slot = nullptr, *last_rows = nullptr,
+             *row_slot = nullptr,   // stream of each row of a decode step
+             *head_slot = nullptr,  // stream of each row the head emits
+             *ids = nullptr;
+};
+
 struct Workspace {
     size_t rows = 0, lanes = 0;
-    uint32_t *ids = nullptr, *lane_off = nullptr, *lane_len = nullptr, *lane_slot = nullptr, *last_rows = nullptr,
-             *greedy = nullptr, *row_slot = nullptr,  // row_slot: stream of each row of a decode step
-             *head_slot = nullptr;                    // stream of each row the head emits
+    // The host entry points and the device-resident one have a description each: a call of the latter may have been captured, and
+    // its replays read these tables whatever host calls came in between.
+    LaneTables host, dev;
+    uint32_t* greedy = nullptr;
     float* feat_c = nullptr;  // Ouro passes only: a block's input features, kept for its depth residual
     float *feat_a = nullptr, *feat_b = nullptr, *x_norm = nullptr, *proj = nullptr, *y = nullptr, *weights = nullptr,
           *m_val = nullptr, *m_proj = nullptr, *z = nullptr, *mlp_act = nullptr, *last_feat = nullptr, *logits = nullptr;
@@ -102,9 +111,9 @@ struct pssa_b200_model {
         void* arg = nullptr;
         bool active = false;        // set for the duration of a sharded prefill call only (decode steps stay local)
     } sp;
-    // lane description last uploaded by the device-resident entry point (skipped when unchanged: graph capture)
+    // caller's lanes whose description ws.dev holds (nothing is uploaded when they are unchanged: graph capture)
     struct DevLayout {
-        const char* ws_base = nullptr;
+        bool valid = false;
         std::vector<uint32_t> off, len, slot;
     } dev_layout;
     // scorer buffers: a tile of full-vocabulary logits, targets and per-row losses
@@ -137,8 +146,10 @@ struct pssa_b200_model {
     // time chunks ("virtual lanes") of the two-pass SSM: chunk maps, chunk carry-ins and the chunk row ranges
     struct Chunks {
         size_t capacity = 0;        // virtual lanes the buffers hold
-        uint32_t *off = nullptr, *len = nullptr;
-        std::vector<uint32_t> host_off, host_len;  // what `off` / `len` hold on the device: an unchanged description is not uploaded again
+        struct Ranges {             // the chunks' rows, for host calls and for the device-resident entry point (see Workspace)
+            uint32_t *off = nullptr, *len = nullptr;
+            std::vector<uint32_t> host_off, host_len;  // what they hold on the device: an unchanged description is not uploaded again
+        } host, dev;
         float* records = nullptr;   // [capacity][d + d*s]  (local mode; the sharded mode uses sp.send)
         float* carry_in = nullptr;  // [capacity][d*s]
     } chunks;

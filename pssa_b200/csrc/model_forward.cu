@@ -35,8 +35,12 @@ int32_t ensure_workspace(pssa_b200_model* m, size_t rows, size_t lanes) {
     const size_t d = m->d, f = sizeof(float);
     Carver c;
     // a call's description side by side, the ids last: the host entry points send it in one copy (send_description)
-    size_t o_off = c.take(lanes * 4), o_len = c.take(lanes * 4), o_slot = c.take(lanes * 4), o_last = c.take(lanes * 4),
-           o_rslot = c.take(lanes * 4), o_hslot = c.take(lanes * 4), o_ids = c.take(rows * 4), o_greedy = c.take(lanes * 4);
+    struct { size_t off, len, slot, last, row, head, ids; } o_host, o_dev;
+    for (auto* o : {&o_host, &o_dev}) {
+        o->off = c.take(lanes * 4), o->len = c.take(lanes * 4), o->slot = c.take(lanes * 4), o->last = c.take(lanes * 4);
+        o->row = c.take(lanes * 4), o->head = c.take(lanes * 4), o->ids = c.take(rows * 4);
+    }
+    size_t o_greedy = c.take(lanes * 4);
     size_t o_fc = c.take(m->loops > 1 ? rows * d * f : 0);
     size_t o_fa = c.take(rows * d * f), o_fb = c.take(rows * d * f), o_xn = c.take(rows * d * f),
            o_proj = c.take(rows * m->ncat * f), o_y = c.take(rows * d * f), o_w = c.take(rows * m->cap * f),
@@ -51,6 +55,7 @@ int32_t ensure_workspace(pssa_b200_model* m, size_t rows, size_t lanes) {
     PSSA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     if (ws.base) cudaFree(ws.base);
     ws = Workspace();
+    m->dev_layout.valid = false;
     cudaError_t e = cudaMalloc((void**)&ws.base, total);
     if (e != cudaSuccess) {
         ws = Workspace();
@@ -60,9 +65,11 @@ int32_t ensure_workspace(pssa_b200_model* m, size_t rows, size_t lanes) {
     PSSA_CUDA(ctx, cudaMemsetAsync(ws.base, 0, total, ctx->stream));
     ws.bytes = total, ws.rows = rows, ws.lanes = lanes;
     char* b = ws.base;
-    ws.ids = (uint32_t*)(b + o_ids), ws.lane_off = (uint32_t*)(b + o_off), ws.lane_len = (uint32_t*)(b + o_len);
-    ws.lane_slot = (uint32_t*)(b + o_slot), ws.last_rows = (uint32_t*)(b + o_last), ws.greedy = (uint32_t*)(b + o_greedy);
-    ws.row_slot = (uint32_t*)(b + o_rslot), ws.head_slot = (uint32_t*)(b + o_hslot);
+    auto tables = [&](const auto& o) {
+        return LaneTables{(uint32_t*)(b + o.off), (uint32_t*)(b + o.len), (uint32_t*)(b + o.slot), (uint32_t*)(b + o.last),
+                          (uint32_t*)(b + o.row), (uint32_t*)(b + o.head), (uint32_t*)(b + o.ids)};
+    };
+    ws.host = tables(o_host), ws.dev = tables(o_dev), ws.greedy = (uint32_t*)(b + o_greedy);
     ws.step = (float*)(b + o_step), ws.step_rows = step_rows;
     ws.feat_c = m->loops > 1 ? (float*)(b + o_fc) : nullptr;
     ws.feat_a = (float*)(b + o_fa), ws.feat_b = (float*)(b + o_fb), ws.x_norm = (float*)(b + o_xn);
@@ -80,11 +87,13 @@ int32_t ensure_chunks(pssa_b200_model* m, size_t vlanes) {
     if (vlanes <= c.capacity) return PSSA_B200_OK;
     pssa_b200_ctx* ctx = m->ctx;
     PSSA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    cudaFree(c.off), cudaFree(c.len), cudaFree(c.records), cudaFree(c.carry_in);
+    cudaFree(c.host.off), cudaFree(c.dev.off), cudaFree(c.records), cudaFree(c.carry_in);
     c = pssa_b200_model::Chunks{};
     const size_t ds = m->d * m->s;
-    PSSA_CUDA(ctx, cudaMalloc((void**)&c.off, vlanes * 4));
-    PSSA_CUDA(ctx, cudaMalloc((void**)&c.len, vlanes * 4));
+    for (auto* r : {&c.host, &c.dev}) {
+        PSSA_CUDA(ctx, cudaMalloc((void**)&r->off, 2 * vlanes * 4));
+        r->len = r->off + vlanes;
+    }
     PSSA_CUDA(ctx, cudaMalloc((void**)&c.records, vlanes * (m->d + ds) * sizeof(float)));
     PSSA_CUDA(ctx, cudaMalloc((void**)&c.carry_in, vlanes * ds * sizeof(float)));
     c.capacity = vlanes;
@@ -175,12 +184,13 @@ void longest_first(const pssa_b200_model* m, std::vector<uint32_t>& off, std::ve
     }
 }
 
-// One pass: `rows` packed token rows of `lanes` lanes already described in the workspace (ids, lane_off, lane_len,
-// lane_slot, last_rows). Leaves the final features of every row in ws.feat_a or feat_b (returned).
-int32_t forward_rows(pssa_b200_model* m, size_t rows, size_t lanes, const uint32_t* h_off, const uint32_t* h_len, float** feats_out,
-                     size_t n_obs = 0) {
+// One pass: `rows` packed token rows of `lanes` lanes, described on the device by `lt` (ws.host or ws.dev) and here by the offsets and
+// lengths that lie there. Leaves the final features of every row in ws.feat_a or feat_b (returned).
+int32_t forward_rows(pssa_b200_model* m, size_t rows, size_t lanes, const LaneTables& lt, const uint32_t* h_off, const uint32_t* h_len,
+                     float** feats_out, size_t n_obs = 0) {
     pssa_b200_ctx* ctx = m->ctx;
     Workspace& ws = m->ws;
+    auto& chunks = &lt == &ws.dev ? m->chunks.dev : m->chunks.host;
     const bool exact = m->precision == PSSA_B200_PRECISION_FP32_EXACT;
     const int d = (int)m->d, s = (int)m->s, k = (int)m->k;
     const size_t nc = m->ncat, ds = m->d * m->s;
@@ -197,8 +207,8 @@ int32_t forward_rows(pssa_b200_model* m, size_t rows, size_t lanes, const uint32
     SsmParams ssm{};
     ssm.delta = ws.proj + m->off_delta, ssm.x_norm = ws.x_norm, ssm.b_proj = ws.proj + m->off_b, ssm.c_proj = ws.proj + m->off_c;
     ssm.rates = m->blocks[0].rates, ssm.y = ws.y, ssm.y_bf16 = exact ? nullptr : ws.y_bf16;
-    ssm.offsets = ws.lane_off, ssm.lengths = ws.lane_len, ssm.rows = rows, ssm.d = d, ssm.s = s, ssm.lanes = (int)lanes;
-    ssm.ld_delta = nc, ssm.ld_bc = nc, ssm.lane_slots = ws.lane_slot, ssm.carry_stride = m->depth * m->loops * ds;
+    ssm.offsets = lt.off, ssm.lengths = lt.len, ssm.rows = rows, ssm.d = d, ssm.s = s, ssm.lanes = (int)lanes;
+    ssm.ld_delta = nc, ssm.ld_bc = nc, ssm.lane_slots = lt.slot, ssm.carry_stride = m->depth * m->loops * ds;
     ssm.aligned = ssm_vector_ok(ssm);
     ssm.single_token = single_token, ssm.max_len = (int)max_len;
     ssm.ragged = lanes > 1 && 8 * rows < 7 * lanes * max_len && std::is_sorted(h_len, h_len + lanes, [](uint32_t a, uint32_t b) { return a > b; });
@@ -236,11 +246,11 @@ int32_t forward_rows(pssa_b200_model* m, size_t rows, size_t lanes, const uint32
         // Uploaded only when the description changed: a repeated call (every step of a benchmark, every pass of a long
         // prompt with equal pass lengths) makes no copy and no synchronisation. The source vectors live in the model;
         // the one wait below is for earlier copies that may still read the vectors about to be replaced.
-        if (v_off != m->chunks.host_off || v_len != m->chunks.host_len) {
+        if (v_off != chunks.host_off || v_len != chunks.host_len) {
             PSSA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));  // earlier copies out of the vectors about to be replaced
-            m->chunks.host_off.swap(v_off), m->chunks.host_len.swap(v_len);
-            PSSA_CUDA(ctx, cudaMemcpyAsync(m->chunks.off, m->chunks.host_off.data(), vlanes * 4, cudaMemcpyHostToDevice, ctx->stream));
-            PSSA_CUDA(ctx, cudaMemcpyAsync(m->chunks.len, m->chunks.host_len.data(), vlanes * 4, cudaMemcpyHostToDevice, ctx->stream));
+            chunks.host_off.swap(v_off), chunks.host_len.swap(v_len);
+            PSSA_CUDA(ctx, cudaMemcpyAsync(chunks.off, chunks.host_off.data(), vlanes * 4, cudaMemcpyHostToDevice, ctx->stream));
+            PSSA_CUDA(ctx, cudaMemcpyAsync(chunks.len, chunks.host_len.data(), vlanes * 4, cudaMemcpyHostToDevice, ctx->stream));
         }
     }
     const bool observe = m->obs.enabled && n_obs > 0;
@@ -306,12 +316,13 @@ int32_t forward_rows(pssa_b200_model* m, size_t rows, size_t lanes, const uint32
     // the slice the stages below work on (set per group by the driver loop)
     size_t r0 = 0, nr = rows, l0 = 0, nl = lanes, gi = 0;
     Workspace v = ws;
+    const uint32_t* ids = lt.ids;
     auto select = [&](size_t g) {
         const Group& gr = groups[g];
         gi = g, r0 = gr.r0, nr = gr.nr, l0 = gr.l0, nl = gr.nl;
-        v = ws;
+        v = ws, ids = lt.ids + r0;
         const size_t dd = m->d;
-        v.ids += r0, v.x_norm += r0 * dd, v.proj += r0 * nc, v.y += r0 * dd, v.weights += r0 * m->cap, v.m_val += r0 * dd, v.m_proj += r0 * dd;
+        v.x_norm += r0 * dd, v.proj += r0 * nc, v.y += r0 * dd, v.weights += r0 * m->cap, v.m_val += r0 * dd, v.m_proj += r0 * dd;
         v.z += r0 * dd, v.mlp_act += r0 * 2 * dd, v.q_stat += r0;
         v.x_bf16 = (char*)ws.x_bf16 + r0 * dd * 2, v.y_bf16 = (char*)ws.y_bf16 + r0 * dd * 2, v.m_bf16 = (char*)ws.m_bf16 + r0 * dd * 2;
         v.z_bf16 = (char*)ws.z_bf16 + r0 * (dd + 64) * 2, v.act_bf16 = (char*)ws.act_bf16 + r0 * (2 * dd + 64) * 2;
@@ -348,7 +359,7 @@ int32_t forward_rows(pssa_b200_model* m, size_t rows, size_t lanes, const uint32
         if (res_in) res_in += r0 * (size_t)d;
         feat_out += r0 * (size_t)d;
         // stage 1: gather + RMSNorm (src/gpu_batch.rs:445-472)
-        if ((rc = launch_embed_norm(ctx, m->embed, feat_in ? nullptr : v.ids, feat_in, b.w[T_NORM_GAMMA], b.w[T_NORM_BETA],
+        if ((rc = launch_embed_norm(ctx, m->embed, feat_in ? nullptr : ids, feat_in, b.w[T_NORM_GAMMA], b.w[T_NORM_BETA],
                                     v.x_norm, exact ? nullptr : v.x_bf16, nr, d, exact, m->v)))
             return rc;
         // stage 2: x-side projections (src/gpu_batch.rs:477-536 plus the query/gate/adapter rows that read x_norm)
@@ -367,14 +378,14 @@ int32_t forward_rows(pssa_b200_model* m, size_t rows, size_t lanes, const uint32
         // stage 3: SSM with the lane carries of this block (src/gpu_batch.rs:582-619)
         SsmParams sp = ssm;
         sp.rates = b.rates, sp.carry = carry_base;
-        sp.offsets = ws.lane_off + l0, sp.lengths = ws.lane_len + l0, sp.lane_slots = ws.lane_slot + l0;
+        sp.offsets = lt.off + l0, sp.lengths = lt.len + l0, sp.lane_slots = lt.slot + l0;
         sp.lanes = (int)nl, sp.rows = nr;  // of this group; row numbers stay absolute
         if (two_pass) {
             // pass 1: every chunk's affine map (sum of delta, end state from a zero carry), one record per virtual lane
             const size_t rec = (size_t)d + ds;
             float* records = m->sp.active ? m->sp.send : m->chunks.records;
             SsmParams ag = sp;
-            ag.offsets = m->chunks.off, ag.lengths = m->chunks.len, ag.lanes = (int)vlanes, ag.max_len = chunk_len, ag.tiled = 1;
+            ag.offsets = chunks.off, ag.lengths = chunks.len, ag.lanes = (int)vlanes, ag.max_len = chunk_len, ag.tiled = 1;
             ag.carry = records + d, ag.carry_stride = rec, ag.lane_slots = nullptr;
             ag.sum_delta = records, ag.sum_delta_stride = rec;
             ag.y_bf16 = nullptr, ag.single_token = 0;  // y of this pass is scratch: the real pass below overwrites it
@@ -390,10 +401,10 @@ int32_t forward_rows(pssa_b200_model* m, size_t rows, size_t lanes, const uint32
             }
             // fold in time order: carry-in of each of this rank's chunks, and the lanes' final state
             if ((rc = launch_seqpar_fold(ctx, gathered, rec, world, rank, (int)n_chunks, (int)lanes, vlanes * rec, b.rates,
-                                         carry_base, carry_stride, ws.lane_slot, m->chunks.carry_in, d, s)))
+                                         carry_base, carry_stride, lt.slot, m->chunks.carry_in, d, s)))
                 return rc;
             // pass 2: the real one, over the virtual lanes with their carry-ins (carry-outs are scratch)
-            sp.offsets = m->chunks.off, sp.lengths = m->chunks.len, sp.lanes = (int)vlanes, sp.max_len = chunk_len, sp.tiled = 1;
+            sp.offsets = chunks.off, sp.lengths = chunks.len, sp.lanes = (int)vlanes, sp.max_len = chunk_len, sp.tiled = 1;
             sp.carry = m->chunks.carry_in, sp.carry_stride = ds, sp.lane_slots = nullptr, sp.single_token = 0;
         }
         if ((rc = launch_ssm_fused(ctx, sp, exact))) return rc;
@@ -468,7 +479,7 @@ int32_t forward_rows(pssa_b200_model* m, size_t rows, size_t lanes, const uint32
                                                 res_in, rscale, nr, m->d, lda, ldz)))
                 return rc;
         }
-        if (obs_now && (rc = launch_observe_rows(ctx, ws.last_rows, n_obs, v.weights, (int)m->cap, m->obs.q_pnc, k, v.m_val,
+        if (obs_now && (rc = launch_observe_rows(ctx, lt.last_rows, n_obs, v.weights, (int)m->cap, m->obs.q_pnc, k, v.m_val,
                                                  exact ? v.z : nullptr, feat_out, res_in, rscale, d,
                                                  m->obs.buf + l * m->obs.lanes * obs_rec)))
             return rc;
@@ -500,7 +511,7 @@ int32_t forward_rows(pssa_b200_model* m, size_t rows, size_t lanes, const uint32
         // features = input + scale * features.
         const float loop_scale = 1.0f / (float)m->loops;
         float* feat = ws.feat_a;
-        rc = each_group([&] { return launch_gather_rows(ctx, m->embed, v.ids, feat + r0 * (size_t)d, nr, d, m->v); });
+        rc = each_group([&] { return launch_gather_rows(ctx, m->embed, ids, feat + r0 * (size_t)d, nr, d, m->v); });
         for (size_t l = 0; l < m->depth && rc == PSSA_B200_OK; ++l) {
             if (l > 0)  // keep the block's input
                 rc = each_group([&] { return launch_residual(ctx, nullptr, feat + r0 * (size_t)d, ws.feat_c + r0 * (size_t)d, nr * (size_t)d, 1.0f); });
@@ -528,14 +539,14 @@ int32_t forward_rows(pssa_b200_model* m, size_t rows, size_t lanes, const uint32
 }
 
 // head for the last row of every non-empty lane (src/pssa.rs:2379-2385, 2438-2440)
-int32_t head_rows(pssa_b200_model* m, const float* feats, size_t n_heads, bool want_greedy) {
+int32_t head_rows(pssa_b200_model* m, const float* feats, const uint32_t* last_rows, size_t n_heads, bool want_greedy) {
     pssa_b200_ctx* ctx = m->ctx;
     Workspace& ws = m->ws;
     int32_t rc;
     const bool exact = m->precision == PSSA_B200_PRECISION_FP32_EXACT;
     // the last rows of the lanes; the tensor-core head takes them as bf16 straight from the gather, in place of the normalised rows
     // (not in the MLP operands, whose pad columns meet weights of zero and must stay finite)
-    if ((rc = launch_gather_rows(ctx, feats, ws.last_rows, exact ? ws.last_feat : nullptr, n_heads, (int)m->d, 0, exact ? nullptr : ws.x_bf16)))
+    if ((rc = launch_gather_rows(ctx, feats, last_rows, exact ? ws.last_feat : nullptr, n_heads, (int)m->d, 0, exact ? nullptr : ws.x_bf16)))
         return rc;
     const float scale = 1.0f / std::sqrt((float)m->d);
     if (exact) {
@@ -563,10 +574,10 @@ bool is_decode_step(const pssa_b200_model* m, size_t lanes, const uint32_t* h_le
     return true;
 }
 
-// logits [rows, vocab] (null: not wanted); ids [rows] is a device array, ws.row_slot [rows] holds the rows' streams; or ids is null and
-// both are host arrays of at most kStepOwnRows
-int32_t run_decode_step(pssa_b200_model* m, size_t rows, const uint32_t* ids, float* logits, const uint32_t* host_ids = nullptr,
-                        const uint32_t* host_slots = nullptr) {
+// logits [rows, vocab] (null: not wanted); ids [rows] and the rows' streams are device arrays, or both are null and come as host
+// arrays of at most kStepOwnRows
+int32_t run_decode_step(pssa_b200_model* m, size_t rows, const uint32_t* ids, const uint32_t* row_slot, float* logits,
+                        const uint32_t* host_ids = nullptr, const uint32_t* host_slots = nullptr) {
     pssa_b200_ctx* ctx = m->ctx;
     Workspace& ws = m->ws;
     int32_t rc;
@@ -593,7 +604,7 @@ int32_t run_decode_step(pssa_b200_model* m, size_t rows, const uint32_t* ids, fl
     p.qpart = ws.step, p.ssq = p.qpart + ws.step_rows * (m->d / 8 * m->k), p.inv = p.ssq + ws.step_rows * (m->d / 16);
     p.x = ws.x_bf16, p.w = ws.w_split, p.z = ws.z_bf16, p.act = ws.act_bf16, p.barrier = m->step_barrier, p.blocks = blocks;
     for (size_t r0 = 0; r0 < rows; r0 += kStepSlice) {  // rows share nothing: slices keep the scratch small
-        p.rows = (int)std::min(kStepSlice, rows - r0), p.ids = ids ? ids + r0 : nullptr, p.slots = ids ? ws.row_slot + r0 : nullptr;
+        p.rows = (int)std::min(kStepSlice, rows - r0), p.ids = ids ? ids + r0 : nullptr, p.slots = ids ? row_slot + r0 : nullptr;
         p.host_ids = host_ids, p.host_slots = host_slots;
         p.logits = logits ? logits + r0 * m->v : nullptr;
         if ((rc = launch_decode_step(ctx, p))) return rc;
@@ -634,21 +645,21 @@ int32_t ensure_sampler(pssa_b200_model* m, size_t lanes) {
 int32_t send_description(pssa_b200_model* m, const std::vector<uint32_t>& ids, const std::vector<uint32_t>& off, const std::vector<uint32_t>& len,
                          const std::vector<uint32_t>& slot, const std::vector<uint32_t>& last, const std::vector<uint32_t>& row_slot,
                          const std::vector<uint32_t>& head_slot, const std::vector<uint32_t>* also = nullptr, void* also_dev = nullptr) {
-    Workspace& ws = m->ws;
-    const size_t bytes = ((const char*)ws.ids - (const char*)ws.lane_off) + ids.size() * 4, more = also ? also->size() * 4 : 0;
+    const LaneTables& t = m->ws.host;
+    const size_t bytes = ((const char*)t.ids - (const char*)t.off) + ids.size() * 4, more = also ? also->size() * 4 : 0;
     int32_t rc = pinned_reserve(m->ctx, bytes + more);
     if (rc) return rc;
     char* const h = m->ctx->pinned;
     auto put = [&](const uint32_t* dev, const std::vector<uint32_t>& v) {
-        if (!v.empty()) std::memcpy(h + ((const char*)dev - (const char*)ws.lane_off), v.data(), v.size() * 4);
+        if (!v.empty()) std::memcpy(h + ((const char*)dev - (const char*)t.off), v.data(), v.size() * 4);
     };
-    put(ws.lane_off, off), put(ws.lane_len, len), put(ws.lane_slot, slot), put(ws.last_rows, last);
-    put(ws.row_slot, row_slot), put(ws.head_slot, head_slot), put(ws.ids, ids);
+    put(t.off, off), put(t.len, len), put(t.slot, slot), put(t.last_rows, last);
+    put(t.row_slot, row_slot), put(t.head_slot, head_slot), put(t.ids, ids);
     if (more) {
         std::memcpy(h + bytes, also->data(), more);
         if ((rc = pinned_send(m->ctx, also_dev, bytes, more))) return rc;
     }
-    return pinned_send(m->ctx, ws.lane_off, 0, bytes);
+    return pinned_send(m->ctx, t.off, 0, bytes);
 }
 
 int32_t run_lanes(pssa_b200_model* m, const uint64_t* ids, const uint32_t* offsets, const uint32_t* lengths, const uint32_t* streams,
@@ -692,7 +703,6 @@ int32_t run_lanes(pssa_b200_model* m, const uint64_t* ids, const uint32_t* offse
         if ((rc = ensure_workspace(m, rows, n_lanes))) return rc;
         Workspace& ws = m->ws;
         cudaStream_t st = ctx->stream;
-        m->dev_layout.ws_base = nullptr;  // the cached layout of the device-resident entry no longer holds
         float* feats = nullptr;
         const bool step = is_decode_step(m, n_lanes, h_len.data()), want_head = logits || greedy || sampling;
         h_row_slot.clear(), head_slot.clear();
@@ -711,13 +721,13 @@ int32_t run_lanes(pssa_b200_model* m, const uint64_t* ids, const uint32_t* offse
         if (!own && (rc = send_description(m, h_ids, s_off, s_len, s_slot, h_last, h_row_slot, head_slot))) return rc;
         if (step) {
             float* const out = !want_head || h_last.empty() ? nullptr : direct ? reinterpret_cast<float*>(ctx->pinned + o_logits) : ws.logits;
-            if ((rc = run_decode_step(m, rows, own ? nullptr : ws.ids, out, h_ids.data(), h_row_slot.data()))) return rc;
+            if ((rc = run_decode_step(m, rows, own ? nullptr : ws.host.ids, own ? nullptr : ws.host.row_slot, out, h_ids.data(), h_row_slot.data()))) return rc;
         } else {
-            if ((rc = forward_rows(m, rows, n_lanes, s_off.data(), s_len.data(), &feats, h_last.size()))) return rc;
+            if ((rc = forward_rows(m, rows, n_lanes, ws.host, s_off.data(), s_len.data(), &feats, h_last.size()))) return rc;
         }
         if (!h_last.empty() && want_head) {
             const bool want_greedy = greedy != nullptr && !sampling;
-            if (!step && (rc = head_rows(m, feats, h_last.size(), want_greedy))) return rc;
+            if (!step && (rc = head_rows(m, feats, ws.host.last_rows, h_last.size(), want_greedy))) return rc;
             if (step && want_greedy && (rc = launch_greedy(ctx, ws.logits, ws.greedy, rows, (int)m->v))) return rc;
             if (sampling) {
                 // sample on the device from the logits the head just wrote; only ids come back
@@ -728,9 +738,9 @@ int32_t run_lanes(pssa_b200_model* m, const uint64_t* ids, const uint32_t* offse
                 sp.temperature = sampling->temperature, sp.top_p = sampling->top_p, sp.repetition_penalty = sampling->repetition_penalty;
                 sp.recent_ids = m->sampler.recent, sp.recent_count = m->sampler.count, sp.rng_state = m->sampler.rng;
                 sp.ids_out = m->sampler.ids, sp.status_out = m->sampler.status, sp.exact = (sample_flags & PSSA_B200_SAMPLE_EXACT) != 0;
-                sp.slots = ws.head_slot, sp.confidence_out = confidence ? m->sampler.conf : nullptr;
+                sp.slots = ws.host.head_slot, sp.confidence_out = confidence ? m->sampler.conf : nullptr;
                 if ((rc = launch_sample(ctx, sp))) return rc;
-                if ((rc = launch_push_recent(ctx, m->sampler.ids, ws.head_slot, m->sampler.recent, m->sampler.count, nh))) return rc;
+                if ((rc = launch_push_recent(ctx, m->sampler.ids, ws.host.head_slot, m->sampler.recent, m->sampler.count, nh))) return rc;
             }
             // results through pinned memory: ids, sampler status, confidences, then the logits, at once or in as many rows at a time as
             // the smallest buffer holds (growing it in a first call would cost more than it ever gives back)
@@ -841,13 +851,14 @@ int32_t pssa_b200_model_prefill_batch_dev(pssa_b200_model* m, const uint32_t* id
     s_off = h_off, s_len = h_len, s_slot = h_slot;
     longest_first(m, s_off, s_len, s_slot);
     auto& lay = m->dev_layout;
-    if (lay.ws_base != ws.base || lay.off != h_off || lay.len != h_len || lay.slot != h_slot) {
-        PSSA_CUDA(ctx, cudaMemcpyAsync(ws.lane_off, s_off.data(), n_lanes * 4, cudaMemcpyHostToDevice, st));
-        PSSA_CUDA(ctx, cudaMemcpyAsync(ws.lane_len, s_len.data(), n_lanes * 4, cudaMemcpyHostToDevice, st));
-        PSSA_CUDA(ctx, cudaMemcpyAsync(ws.lane_slot, s_slot.data(), n_lanes * 4, cudaMemcpyHostToDevice, st));
-        PSSA_CUDA(ctx, cudaMemcpyAsync(ws.last_rows, h_last.data(), h_last.size() * 4, cudaMemcpyHostToDevice, st));
-        PSSA_CUDA(ctx, cudaMemcpyAsync(ws.row_slot, h_row_slot.data(), h_row_slot.size() * 4, cudaMemcpyHostToDevice, st));
-        lay.ws_base = ws.base, lay.off = h_off, lay.len = h_len, lay.slot = h_slot;
+    if (!lay.valid || lay.off != h_off || lay.len != h_len || lay.slot != h_slot) {
+        lay.valid = false;
+        PSSA_CUDA(ctx, cudaMemcpyAsync(ws.dev.off, s_off.data(), n_lanes * 4, cudaMemcpyHostToDevice, st));
+        PSSA_CUDA(ctx, cudaMemcpyAsync(ws.dev.len, s_len.data(), n_lanes * 4, cudaMemcpyHostToDevice, st));
+        PSSA_CUDA(ctx, cudaMemcpyAsync(ws.dev.slot, s_slot.data(), n_lanes * 4, cudaMemcpyHostToDevice, st));
+        PSSA_CUDA(ctx, cudaMemcpyAsync(ws.dev.last_rows, h_last.data(), h_last.size() * 4, cudaMemcpyHostToDevice, st));
+        PSSA_CUDA(ctx, cudaMemcpyAsync(ws.dev.row_slot, h_row_slot.data(), h_row_slot.size() * 4, cudaMemcpyHostToDevice, st));
+        lay.valid = true, lay.off = h_off, lay.len = h_len, lay.slot = h_slot;
     }
     float* feats = nullptr;
     // logits and greedy ids of the rows in ws.logits, to the places of their lanes: contiguous runs of non-empty lanes in one copy
@@ -873,25 +884,25 @@ int32_t pssa_b200_model_prefill_batch_dev(pssa_b200_model* m, const uint32_t* id
         if (!in_order) {
             for (size_t i = 0, j; i < rows; i = j) {
                 for (j = i + 1; j < rows && h_last[j] == h_last[j - 1] + 1; ++j) {}
-                PSSA_CUDA(ctx, cudaMemcpyAsync(ws.ids + i, ids_dev + h_last[i], (j - i) * 4, cudaMemcpyDeviceToDevice, st));
+                PSSA_CUDA(ctx, cudaMemcpyAsync(ws.dev.ids + i, ids_dev + h_last[i], (j - i) * 4, cudaMemcpyDeviceToDevice, st));
             }
-            ids = ws.ids;
+            ids = ws.dev.ids;
         }
         const bool whole = rows == n_lanes && logits_dev;  // rows are lanes: no copy
         float* out = whole ? logits_dev : ws.logits;
-        if ((rc = run_decode_step(m, rows, ids, logits_dev || greedy_dev ? out : nullptr))) return rc;
+        if ((rc = run_decode_step(m, rows, ids, ws.dev.row_slot, logits_dev || greedy_dev ? out : nullptr))) return rc;
         if (greedy_dev && (rc = launch_greedy(ctx, out, ws.greedy, rows, (int)m->v))) return rc;
         if (!whole) return rows_to_lanes();
         if (greedy_dev) PSSA_CUDA(ctx, cudaMemcpyAsync(greedy_dev, ws.greedy, rows * 4, cudaMemcpyDeviceToDevice, st));
         return PSSA_B200_OK;
     }
-    PSSA_CUDA(ctx, cudaMemcpyAsync(ws.ids, ids_dev, span * 4, cudaMemcpyDeviceToDevice, st));
+    PSSA_CUDA(ctx, cudaMemcpyAsync(ws.dev.ids, ids_dev, span * 4, cudaMemcpyDeviceToDevice, st));
     m->sp.active = m->sp.world > 1;
-    rc = forward_rows(m, span, n_lanes, s_off.data(), s_len.data(), &feats, h_last.size());
+    rc = forward_rows(m, span, n_lanes, ws.dev, s_off.data(), s_len.data(), &feats, h_last.size());
     m->sp.active = false;
     if (rc) return rc;
     if (logits_dev || greedy_dev) {
-        if ((rc = head_rows(m, feats, h_last.size(), greedy_dev != nullptr))) return rc;
+        if ((rc = head_rows(m, feats, ws.dev.last_rows, h_last.size(), greedy_dev != nullptr))) return rc;
         return rows_to_lanes();
     }
     return PSSA_B200_OK;
@@ -934,11 +945,10 @@ int32_t pssa_b200_model_score(pssa_b200_model* m, uint32_t stream, const uint64_
         if ((rc = ensure_workspace(m, rows, 1))) return rc;
         Workspace& ws = m->ws;
         const uint32_t off = 0, len = (uint32_t)rows;
-        m->dev_layout.ws_base = nullptr;
         h_ids.resize(rows), h_tgt.resize(rows);
         if ((rc = send_description(m, h_ids, {off}, {len}, {stream}, {}, {}, {}, &h_tgt, sc.targets))) return rc;
         float* feats = nullptr;
-        if ((rc = forward_rows(m, rows, 1, &off, &len, &feats))) return rc;
+        if ((rc = forward_rows(m, rows, 1, ws.host, &off, &len, &feats))) return rc;
         for (size_t r0 = 0; r0 < rows; r0 += tile) {
             const size_t nr = std::min(tile, rows - r0);
             if (exact) {
@@ -1121,7 +1131,7 @@ int32_t pssa_b200_model_set_seqpar(pssa_b200_model* m, uint32_t rank, uint32_t w
     PSSA_CUDA(ctx, cudaSetDevice(ctx->device));
     PSSA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     m->sp = pssa_b200_model::SeqPar{};
-    m->dev_layout.ws_base = nullptr;  // ranks keep the caller's order of lanes
+    m->dev_layout.valid = false;  // ranks keep the caller's order of lanes
     if (world <= 1 || !exchange) return PSSA_B200_OK;
     if (rank >= world) return fail(ctx, PSSA_B200_ERR_INVALID_ARGUMENT, "sequence-parallel rank %u outside world of %u", rank, world);
     if (!send_dev || !recv_dev || capacity == 0)

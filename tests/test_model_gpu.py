@@ -637,6 +637,63 @@ def test_decode_graph_with_lane_groups_replays_the_eager_tokens(gpu):
     gm2.close()
 
 
+@pytest.mark.parametrize("d,s,k,cap,precision", [(192, 64, 64, 512, 0), (32, 16, 8, 16, 0), (32, 16, 8, 16, 1)])
+def test_decode_graph_beside_host_calls_equals_eager_steps(gpu, d, s, k, cap, precision):
+    """Host calls on other streams between two replays (a prompt cut into time chunks, a score, a ragged batch, a step of more rows
+    than travel with the launch) leave the description that a captured step reads alone: tokens and every carry equal
+    those of a model that takes eager steps in place of the replays. Shapes with and without the decode step of its own."""
+    import torch
+    gpu.set_stream(torch.cuda.current_stream())
+    streams, mine = 40, [4, 1, 3]
+    others = [i for i in range(streams) if i not in mine]
+    _, gm = make_pair(gpu, 2, 97, d, s, k, cap, seed=31, streams=streams, precision=precision)
+    _, gm2 = make_pair(gpu, 2, 97, d, s, k, cap, seed=31, streams=streams, precision=precision)
+    for m in (gm, gm2):
+        m.reserve(2048, streams)
+        _, first = m.prefill_batch([[5, 9, 2], [11, 3], [7]], streams=mine, want_logits=False, want_greedy=True)
+    ids_dev = torch.tensor(first.astype(np.int32), device="cuda", dtype=torch.int32)
+    graph = gm.capture_greedy_decode_graph(ids_dev, mine)  # takes one real step
+    ids = gm2.decode_step(first, mine, want_logits=False, want_greedy=True)
+    rng = np.random.default_rng(6)
+    long, text = rng.integers(1, 97, 1500), rng.integers(1, 97, 301)
+    turns = [rng.integers(1, 97, n) for n in (70, 3, 33, 1)]
+    between = [lambda m: m.prefill_inference(long, stream=0), lambda m: m.score(text[:-1], text[1:], stream=2),
+               lambda m: m.prefill_batch(turns, streams=[7, 0, 39, 2]), lambda m: m.decode_step(np.arange(1, 38), others),
+               lambda m: m.forward_inference(5, 8)]
+    for call in between:
+        call(gm), call(gm2)
+        graph.replay()
+        ids = gm2.decode_step(ids, mine, want_logits=False, want_greedy=True)
+        torch.cuda.synchronize()
+        assert np.array_equal(ids_dev.cpu().numpy().astype(np.uint64), ids)
+    for i in range(streams):
+        a, b = gm.copy_recurrent_state_to(i), gm2.copy_recurrent_state_to(i)
+        assert np.array_equal(a.view(np.uint32), b.view(np.uint32)), i
+    gpu.poll_status()
+    gpu.set_stream(None)
+    gm.close()
+    gm2.close()
+
+
+def test_device_lanes_are_described_again_after_the_workspace_grew(gpu):
+    """The description on the device goes with the workspace that holds it: the same lanes after `reserve` made a larger one."""
+    import torch
+    gpu.set_stream(torch.cuda.current_stream())
+    _, gm = make_pair(gpu, 2, 97, 32, 16, 8, 16, seed=31, streams=3, precision=0)
+    ids = torch.arange(1, 61, device="cuda", dtype=torch.int32)
+    off, length = np.array([0, 25, 30], np.uint32), np.array([25, 5, 30], np.uint32)
+    got = []
+    for rows in (60, 61, 4000):
+        gm.reserve(rows, 3)
+        gm.reset_recurrent_state()
+        out = torch.zeros(3, 97, device="cuda")
+        gm.prefill_batch_dev(ids, off, length, [2, 0, 1], out)
+        got.append(out.cpu().numpy())
+    assert np.any(got[0]) and all(np.array_equal(got[0], x) for x in got[1:])
+    gpu.set_stream(None)
+    gm.close()
+
+
 def test_reserved_model_allocates_nothing_during_calls(gpu):
     """`pssa_b200_model_reserve`: after it, prefill (plain and time-chunked) and decode calls within the reserved size
     leave the device's free memory unchanged (growth of the workspace, the chunk buffers and the sampler state is what
