@@ -111,10 +111,11 @@ struct pssa_b200_model {
         void* arg = nullptr;
         bool active = false;        // set for the duration of a sharded prefill call only (decode steps stay local)
     } sp;
-    // caller's lanes whose description ws.dev holds (nothing is uploaded when they are unchanged: graph capture)
+    // what ws.dev holds, word for word (nothing is uploaded when a call would send the same: graph capture). The caller's lanes would
+    // not do as a key: their order on the device depends on the options.
     struct DevLayout {
         bool valid = false;
-        std::vector<uint32_t> off, len, slot;
+        std::vector<uint32_t> off, len, slot, last_rows, row_slot;
     } dev_layout;
     // scorer buffers: a tile of full-vocabulary logits, targets and per-row losses
     struct Score {

@@ -851,14 +851,18 @@ int32_t pssa_b200_model_prefill_batch_dev(pssa_b200_model* m, const uint32_t* id
     s_off = h_off, s_len = h_len, s_slot = h_slot;
     longest_first(m, s_off, s_len, s_slot);
     auto& lay = m->dev_layout;
-    if (!lay.valid || lay.off != h_off || lay.len != h_len || lay.slot != h_slot) {
+    struct { std::vector<uint32_t>&sent, &now; uint32_t* dev; } tables[] = {
+        {lay.off, s_off, ws.dev.off}, {lay.len, s_len, ws.dev.len}, {lay.slot, s_slot, ws.dev.slot},
+        {lay.last_rows, h_last, ws.dev.last_rows}, {lay.row_slot, h_row_slot, ws.dev.row_slot}};
+    bool known = lay.valid;
+    for (auto& t : tables) known = known && t.sent == t.now;
+    if (!known) {
         lay.valid = false;
-        PSSA_CUDA(ctx, cudaMemcpyAsync(ws.dev.off, s_off.data(), n_lanes * 4, cudaMemcpyHostToDevice, st));
-        PSSA_CUDA(ctx, cudaMemcpyAsync(ws.dev.len, s_len.data(), n_lanes * 4, cudaMemcpyHostToDevice, st));
-        PSSA_CUDA(ctx, cudaMemcpyAsync(ws.dev.slot, s_slot.data(), n_lanes * 4, cudaMemcpyHostToDevice, st));
-        PSSA_CUDA(ctx, cudaMemcpyAsync(ws.dev.last_rows, h_last.data(), h_last.size() * 4, cudaMemcpyHostToDevice, st));
-        PSSA_CUDA(ctx, cudaMemcpyAsync(ws.dev.row_slot, h_row_slot.data(), h_row_slot.size() * 4, cudaMemcpyHostToDevice, st));
-        lay.valid = true, lay.off = h_off, lay.len = h_len, lay.slot = h_slot;
+        for (auto& t : tables) {
+            PSSA_CUDA(ctx, cudaMemcpyAsync(t.dev, t.now.data(), t.now.size() * 4, cudaMemcpyHostToDevice, st));
+            t.sent = t.now;
+        }
+        lay.valid = true;
     }
     float* feats = nullptr;
     // logits and greedy ids of the rows in ws.logits, to the places of their lanes: contiguous runs of non-empty lanes in one copy
@@ -1131,7 +1135,6 @@ int32_t pssa_b200_model_set_seqpar(pssa_b200_model* m, uint32_t rank, uint32_t w
     PSSA_CUDA(ctx, cudaSetDevice(ctx->device));
     PSSA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     m->sp = pssa_b200_model::SeqPar{};
-    m->dev_layout.valid = false;  // ranks keep the caller's order of lanes
     if (world <= 1 || !exchange) return PSSA_B200_OK;
     if (rank >= world) return fail(ctx, PSSA_B200_ERR_INVALID_ARGUMENT, "sequence-parallel rank %u outside world of %u", rank, world);
     if (!send_dev || !recv_dev || capacity == 0)

@@ -675,6 +675,29 @@ def test_decode_graph_beside_host_calls_equals_eager_steps(gpu, d, s, k, cap, pr
     gm2.close()
 
 
+@pytest.mark.parametrize("precision,lengths", [(1, (20, 65, 3, 140, 90)), (0, (20, 65, 3, 140, 90)), (0, (1100, 1400))])
+def test_device_lanes_follow_a_change_of_the_lane_groups(gpu, precision, lengths):
+    """The order in which lanes lie on the device depends on the lane groups: the same ragged call with 1, 2, 1 and the automatic
+    number of groups, the last lengths cut into time chunks, gives the same logits and carries."""
+    import torch
+    gpu.set_stream(torch.cuda.current_stream())
+    n = len(lengths)
+    _, gm = make_pair(gpu, 2, 97, 192, 64, 64, 512, seed=32, streams=n, precision=precision)
+    ids = torch.from_numpy(np.random.default_rng(7).integers(1, 97, sum(lengths)).astype(np.int32)).cuda()
+    off = np.concatenate([[0], np.cumsum(lengths)[:-1]]).astype(np.uint32)
+    got = []
+    for groups in (1, 2, 1, 0, 2):
+        gm.set_lane_groups(groups)
+        gm.reset_recurrent_state()
+        out = torch.zeros(n, 97, device="cuda")
+        gm.prefill_batch_dev(ids, off, np.array(lengths, np.uint32), list(range(n))[::-1], out)
+        got.append(np.concatenate([out.cpu().numpy().ravel()] + [gm.copy_recurrent_state_to(i) for i in range(n)]).view(np.uint32))
+    assert all(np.array_equal(got[0], x) for x in got[1:])
+    gpu.poll_status()
+    gpu.set_stream(None)
+    gm.close()
+
+
 def test_device_lanes_are_described_again_after_the_workspace_grew(gpu):
     """The description on the device goes with the workspace that holds it: the same lanes after `reserve` made a larger one."""
     import torch
