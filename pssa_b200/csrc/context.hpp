@@ -104,6 +104,24 @@ struct PerDeviceOnce {
     }
 };
 
+// CTAs of a kernel to an SM, asked for once per device and size of dynamic shared memory (a width of the model is a size of its own):
+// one word a device, the size above the count, so that another size asks again instead of taking the count of the one before.
+struct PerDeviceCount {
+    std::atomic<unsigned long long> word[64]{};
+    template <typename Ask>  // ask(&count) -> 0 or an error
+    auto get(int device, size_t smem, int* count, Ask ask) -> decltype(ask(count)) {
+        const bool known = device >= 0 && device < 64;
+        if (known) {
+            const unsigned long long w = word[device].load(std::memory_order_relaxed);
+            *count = (int)(w & 0xffff);
+            if (w != 0 && w >> 16 == smem) return {};
+        }
+        const auto e = ask(count);
+        if (e == decltype(e){} && known) word[device].store((unsigned long long)smem << 16 | (unsigned)*count, std::memory_order_relaxed);
+        return e;
+    }
+};
+
 // Arena: reset at the start of an entry point, then bump-allocate 256-byte aligned blocks.
 int32_t arena_reserve(pssa_b200_ctx* ctx, size_t bytes);
 inline void arena_reset(pssa_b200_ctx* ctx) { ctx->arena_used = 0; }
@@ -138,21 +156,15 @@ inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 bl
 // An early dependent start places CTAs on whichever SMs the predecessor frees first, as many as fit: a grid that does not fill the
 // machine then crowds on some SMs and leaves others empty (the fused SSM of 16 lanes of 1024 tokens at d 768: 635 us a launch in a
 // stream where it takes 435 evenly spread). So a long kernel of several small CTAs to an SM starts early only when the fullest
-// SM is as full either way, or holds at least 1 / `slack` of what fits, where that many hide its latency (0: never). `resident`: the kernel's
-// CTAs to an SM, asked for once per device.
-struct PerDeviceCount {
-    std::atomic<int> n[64]{};
-};
+// SM is as full either way, or holds at least 1 / `slack` of what fits, where that many hide its latency (0: never).
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_spread(PerDeviceCount& resident, int slack, int device, int sm_count, void (*kernel)(KArgs...), dim3 grid, dim3 block,
                                  size_t smem, cudaStream_t stream, Args... args) {
-    const bool known = device >= 0 && device < 64;
-    int per_sm = known ? resident.n[device].load(std::memory_order_relaxed) : 0;
-    if (per_sm == 0) {
-        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, (int)(block.x * block.y * block.z), smem);
-        if (e != cudaSuccess) return e;
-        if (known) resident.n[device].store(per_sm, std::memory_order_relaxed);
-    }
+    int per_sm = 0;
+    const cudaError_t e = resident.get(device, smem, &per_sm, [&](int* n) {
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, kernel, (int)(block.x * block.y * block.z), smem);
+    });
+    if (e != cudaSuccess) return e;
     const size_t blocks = (size_t)grid.x * grid.y * grid.z, even = (blocks + sm_count - 1) / sm_count;
     if (even * slack >= (size_t)per_sm) return launch_dependent(kernel, grid, block, smem, stream, args...);
     cudaLaunchConfig_t cfg{};
