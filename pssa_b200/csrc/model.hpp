@@ -59,11 +59,23 @@ struct LaneTables {
              *ids = nullptr;
 };
 
+// Where a host call's tables lie: one behind another, each on 16 bytes, no longer than the call needs. Returns the words of all.
+constexpr size_t kHostTables = 7;  // six of lanes, the ids
+constexpr size_t table_words(size_t n) { return (n + 3) & ~size_t(3); }
+inline size_t lay_host_tables(const size_t (&sizes)[kHostTables], size_t (&at)[kHostTables]) {
+    size_t words = 0;
+    for (size_t i = 0; i < kHostTables; ++i) at[i] = words, words += table_words(sizes[i]);
+    return words;
+}
+// what the longest call of so many rows and lanes needs
+constexpr size_t host_tables_words(size_t rows, size_t lanes) { return (kHostTables - 1) * table_words(lanes) + table_words(rows); }
+
 struct Workspace {
     size_t rows = 0, lanes = 0;
     // The host entry points and the device-resident one have a description each: a call of the latter may have been captured, and
-    // its replays read these tables whatever host calls came in between.
+    // its replays read these tables whatever host calls came in between. The host ones lie in `host_words`, anew for each call.
     LaneTables host, dev;
+    uint32_t* host_words = nullptr;
     uint32_t* greedy = nullptr;
     float* feat_c = nullptr;  // Ouro passes only: a block's input features, kept for its depth residual
     float *feat_a = nullptr, *feat_b = nullptr, *x_norm = nullptr, *proj = nullptr, *y = nullptr, *weights = nullptr,

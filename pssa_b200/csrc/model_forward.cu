@@ -34,13 +34,10 @@ int32_t ensure_workspace(pssa_b200_model* m, size_t rows, size_t lanes) {
     lanes = std::max(lanes, ws.lanes);
     const size_t d = m->d, f = sizeof(float);
     Carver c;
-    // a call's description side by side, the ids last: the host entry points send it in one copy (send_description)
-    struct { size_t off, len, slot, last, row, head, ids; } o_host, o_dev;
-    for (auto* o : {&o_host, &o_dev}) {
-        o->off = c.take(lanes * 4), o->len = c.take(lanes * 4), o->slot = c.take(lanes * 4), o->last = c.take(lanes * 4);
-        o->row = c.take(lanes * 4), o->head = c.take(lanes * 4), o->ids = c.take(rows * 4);
-    }
-    size_t o_greedy = c.take(lanes * 4);
+    // what the device has to know of a call: host calls lay theirs out as long as each needs it (send_description)
+    size_t o_host = c.take(host_tables_words(rows, lanes) * 4);
+    size_t o_off = c.take(lanes * 4), o_len = c.take(lanes * 4), o_slot = c.take(lanes * 4), o_last = c.take(lanes * 4),
+           o_row = c.take(lanes * 4), o_ids = c.take(rows * 4), o_greedy = c.take(lanes * 4);
     size_t o_fc = c.take(m->loops > 1 ? rows * d * f : 0);
     size_t o_fa = c.take(rows * d * f), o_fb = c.take(rows * d * f), o_xn = c.take(rows * d * f),
            o_proj = c.take(rows * m->ncat * f), o_y = c.take(rows * d * f), o_w = c.take(rows * m->cap * f),
@@ -65,11 +62,9 @@ int32_t ensure_workspace(pssa_b200_model* m, size_t rows, size_t lanes) {
     PSSA_CUDA(ctx, cudaMemsetAsync(ws.base, 0, total, ctx->stream));
     ws.bytes = total, ws.rows = rows, ws.lanes = lanes;
     char* b = ws.base;
-    auto tables = [&](const auto& o) {
-        return LaneTables{(uint32_t*)(b + o.off), (uint32_t*)(b + o.len), (uint32_t*)(b + o.slot), (uint32_t*)(b + o.last),
-                          (uint32_t*)(b + o.row), (uint32_t*)(b + o.head), (uint32_t*)(b + o.ids)};
-    };
-    ws.host = tables(o_host), ws.dev = tables(o_dev), ws.greedy = (uint32_t*)(b + o_greedy);
+    ws.host_words = (uint32_t*)(b + o_host), ws.greedy = (uint32_t*)(b + o_greedy);
+    ws.dev.off = (uint32_t*)(b + o_off), ws.dev.len = (uint32_t*)(b + o_len), ws.dev.slot = (uint32_t*)(b + o_slot);
+    ws.dev.last_rows = (uint32_t*)(b + o_last), ws.dev.row_slot = (uint32_t*)(b + o_row), ws.dev.ids = (uint32_t*)(b + o_ids);
     ws.step = (float*)(b + o_step), ws.step_rows = step_rows;
     ws.feat_c = m->loops > 1 ? (float*)(b + o_fc) : nullptr;
     ws.feat_a = (float*)(b + o_fa), ws.feat_b = (float*)(b + o_fb), ws.x_norm = (float*)(b + o_xn);
@@ -640,26 +635,31 @@ int32_t ensure_sampler(pssa_b200_model* m, size_t lanes) {
     return PSSA_B200_OK;
 }
 
-// What the device has to know of a host call -- lanes, rows of the heads, ids -- in one copy out of pinned memory. (Five or six copies
-// from pageable memory at 4 to 5 us of this thread's time each before.) With `also`, that many words go to `also_dev` too.
+// What the device has to know of a host call -- lanes, rows of the heads, ids -- one table behind another in one copy out of pinned
+// memory, as long as this call needs it. (Five or six copies from pageable memory at 4 to 5 us of this thread's time each before. A place
+// per table for as many lanes as the workspace holds: 400 KB for one lane after room was reserved for 16384, and a pinned buffer
+// grown for it, which made the first prompt 2.7 ms instead of 0.15.) With `also`, that many words go to `also_dev` too.
 int32_t send_description(pssa_b200_model* m, const std::vector<uint32_t>& ids, const std::vector<uint32_t>& off, const std::vector<uint32_t>& len,
                          const std::vector<uint32_t>& slot, const std::vector<uint32_t>& last, const std::vector<uint32_t>& row_slot,
                          const std::vector<uint32_t>& head_slot, const std::vector<uint32_t>* also = nullptr, void* also_dev = nullptr) {
-    const LaneTables& t = m->ws.host;
-    const size_t bytes = ((const char*)t.ids - (const char*)t.off) + ids.size() * 4, more = also ? also->size() * 4 : 0;
+    uint32_t* const base = m->ws.host_words;
+    LaneTables& t = m->ws.host;
+    struct { uint32_t*& dev; const std::vector<uint32_t>& words; } tables[] = {{t.off, off}, {t.len, len}, {t.slot, slot}, {t.last_rows, last},
+                                                                               {t.row_slot, row_slot}, {t.head_slot, head_slot}, {t.ids, ids}};
+    size_t sizes[kHostTables], at[kHostTables];
+    for (size_t i = 0; i < kHostTables; ++i) sizes[i] = tables[i].words.size();
+    const size_t bytes = lay_host_tables(sizes, at) * 4, more = also ? also->size() * 4 : 0;
+    for (size_t i = 0; i < kHostTables; ++i) tables[i].dev = base + at[i];
     int32_t rc = pinned_reserve(m->ctx, bytes + more);
     if (rc) return rc;
     char* const h = m->ctx->pinned;
-    auto put = [&](const uint32_t* dev, const std::vector<uint32_t>& v) {
-        if (!v.empty()) std::memcpy(h + ((const char*)dev - (const char*)t.off), v.data(), v.size() * 4);
-    };
-    put(t.off, off), put(t.len, len), put(t.slot, slot), put(t.last_rows, last);
-    put(t.row_slot, row_slot), put(t.head_slot, head_slot), put(t.ids, ids);
+    for (auto& x : tables)
+        if (!x.words.empty()) std::memcpy(h + (x.dev - base) * 4, x.words.data(), x.words.size() * 4);
     if (more) {
         std::memcpy(h + bytes, also->data(), more);
         if ((rc = pinned_send(m->ctx, also_dev, bytes, more))) return rc;
     }
-    return pinned_send(m->ctx, t.off, 0, bytes);
+    return pinned_send(m->ctx, base, 0, bytes);
 }
 
 int32_t run_lanes(pssa_b200_model* m, const uint64_t* ids, const uint32_t* offsets, const uint32_t* lengths, const uint32_t* streams,

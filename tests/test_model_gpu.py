@@ -740,6 +740,24 @@ def test_reserved_model_allocates_nothing_during_calls(gpu):
     gm.close()
 
 
+def test_host_calls_of_any_length_after_room_for_many_lanes(gpu):
+    """Host calls lay their tables out as long as each needs them: prompts, scores and steps of few and many lanes in turn, with room
+    for 600 lanes and for as many as each call has, give the same logits and carries."""
+    rng = np.random.default_rng(4)
+    prompt, text, steps = rng.integers(1, 97, 200), rng.integers(1, 97, 62), rng.integers(1, 97, 40)
+    turns = [rng.integers(1, 97, n) for n in (7, 0, 33, 1, 12)]
+    got = []
+    for lanes in (0, 600):
+        _, gm = make_pair(gpu, 2, 97, 32, 16, 8, 16, seed=33, streams=40, precision=0)
+        if lanes:
+            gm.reserve(2000, lanes)
+        out = [gm.prefill_inference(prompt)[1], gm.decode_step(steps), gm.score(text[:-1], text[1:], stream=3)[1],
+               gm.prefill_batch(turns, streams=[9, 1, 0, 39, 4])[0], gm.decode_step(steps[:18], list(range(22, 40))), gm.prefill_inference(prompt[:5], stream=2)[1]]
+        got.append(np.concatenate([np.ravel(x) for x in out] + [gm.copy_recurrent_state_to(i) for i in range(40)]).view(np.uint32))
+        gm.close()
+    assert np.array_equal(got[0], got[1])
+
+
 @pytest.mark.parametrize("k,cap,tau", [(64, 256, 0.1), (128, 128, 0.13), (128, 512, 0.1), (64, 512, 0.25)])
 def test_one_kernel_all_slots_read_agrees_with_the_separate_kernels(gpu, monkeypatch, k, cap, tau):
     """The bf16 mode's all-slots read runs projection, distances, softmax and the bf16 weight rows as one kernel when
