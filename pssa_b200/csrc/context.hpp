@@ -25,6 +25,7 @@ struct pssa_b200_ctx {
     std::vector<cudaEvent_t> io_events;
     cudaEvent_t staged_ev = nullptr;  // behind the last copy out of `pinned` that nobody has waited for yet
     bool staged = false;
+    bool asked[2][2] = {};  // [in, out][first buffer, largest]: a model's host call has gone without it before (want_pinned)
     std::string error;
     std::string label;
     uint64_t launches = 0;

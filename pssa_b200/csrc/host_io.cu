@@ -13,7 +13,7 @@ namespace pssa {
 namespace {
 
 constexpr size_t kKeepDevice = (size_t)256 << 20;  // device region kept between calls, at most
-constexpr size_t kPinnedMax = (size_t)4 << 20;     // a context's pinned buffer: larger transfers go through it in windows
+constexpr size_t kThreadsFrom = (size_t)1 << 20;   // outputs from here on are copied by several threads
 constexpr size_t kPinnedKept = 4;                  // pinned buffers kept for the next context, while any context lives
 constexpr size_t kPinnedInputs = (size_t)2 << 20;  // above this the driver's own pipelined pageable copy is as fast
 constexpr size_t kPiece = (size_t)512 << 10;       // one device copy of a large transfer
@@ -158,6 +158,12 @@ int32_t pinned_reserve(pssa_b200_ctx* ctx, size_t bytes) {
     return PSSA_B200_OK;
 }
 
+bool want_pinned(pssa_b200_ctx* ctx, size_t bytes, bool out) {
+    if (bytes <= ctx->pinned_bytes) return true;
+    if (bytes > kPinnedMax) return false;
+    return std::exchange(ctx->asked[out][bytes > kPinnedMin], true);
+}
+
 int32_t pinned_send(pssa_b200_ctx* ctx, void* dst_dev, size_t off, size_t bytes) {
     if (!ctx->staged_ev) PSSA_CUDA(ctx, cudaEventCreateWithFlags(&ctx->staged_ev, cudaEventDisableTiming));
     PSSA_CUDA(ctx, cudaMemcpyAsync(dst_dev, ctx->pinned + off, bytes, cudaMemcpyHostToDevice, ctx->stream));
@@ -247,6 +253,11 @@ int32_t copy_to_host(pssa_b200_ctx* ctx, void* dst, const void* src_dev, size_t 
 // In pieces, each copied into the pinned buffer by several threads while the one before is on the link: a carry of 2.4 MB in 75 us
 // instead of the driver's 142 for pageable memory.
 int32_t copy_to_device(pssa_b200_ctx* ctx, void* dst_dev, const void* src, size_t bytes) {
+    if (!want_pinned(ctx, std::min(bytes, kPinnedMax), false)) {
+        PSSA_CUDA(ctx, cudaMemcpyAsync(dst_dev, src, bytes, cudaMemcpyHostToDevice, ctx->stream));
+        PSSA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        return PSSA_B200_OK;
+    }
     for (size_t w0 = 0; w0 < bytes; w0 += kPinnedMax) {
         const size_t wn = std::min(kPinnedMax, bytes - w0);
         int32_t rc = pinned_reserve(ctx, wn);

@@ -49,15 +49,18 @@ class HostCall {
 
 // device -> host through the context's pinned buffer, in stream order; waits for the stream
 int32_t copy_to_host(pssa_b200_ctx* ctx, void* dst, const void* src_dev, size_t bytes);
-// host -> device through the context's pinned buffer; waits for the stream
+// host -> device through the context's pinned buffer (see want_pinned); waits for the stream
 int32_t copy_to_device(pssa_b200_ctx* ctx, void* dst_dev, const void* src, size_t bytes);
-// outputs from here on are copied by several threads
-constexpr size_t kThreadsFrom = (size_t)1 << 20;
-// the pinned buffer that every context starts with: a larger one costs milliseconds to pin
-constexpr size_t kPinnedMin = (size_t)256 << 10;
+// a context's first pinned buffer, and its largest: longer transfers go through it in windows
+constexpr size_t kPinnedMin = (size_t)256 << 10, kPinnedMax = (size_t)4 << 20;
 // pinned host memory of the context, at least `bytes`, valid until the next call; waits for the stream when it has to grow, and for
 // a copy that pinned_send left behind
 int32_t pinned_reserve(pssa_b200_ctx* ctx, size_t bytes);
+// Whether words of a model's host call should pass through pinned memory: yes where the buffer holds them; otherwise a context's first
+// such call goes without and the next one pins it. Pinning takes 0.9 to 2.6 ms for the first buffer and 1.5 to 4.5 for the largest, and
+// saves a call 10 us at 256 KB and 150 at 4 MB: a program that makes one call never gets it back (the small model's first step 2.8
+// ms with it and 0.2 without), one that makes many pays once.
+bool want_pinned(pssa_b200_ctx* ctx, size_t bytes, bool out);
 // enqueues the copy of `bytes` at `off` of the pinned buffer to the device and returns
 int32_t pinned_send(pssa_b200_ctx* ctx, void* dst_dev, size_t off, size_t bytes);
 void host_io_create();  // once per context

@@ -167,5 +167,6 @@ struct pssa_b200_model {
         float* carry_in = nullptr;  // [capacity][d*s]
     } chunks;
     void* step_barrier = nullptr;  // grid barrier of the decode step in one kernel (step_decode.cu)
+    std::vector<char> sent;  // a host call's description that went over from pageable memory
     std::vector<bool> tensor_set;  // [depth * T_COUNT + id] upload bookkeeping
 };

@@ -635,10 +635,10 @@ int32_t ensure_sampler(pssa_b200_model* m, size_t lanes) {
     return PSSA_B200_OK;
 }
 
-// What the device has to know of a host call -- lanes, rows of the heads, ids -- one table behind another in one copy out of pinned
-// memory, as long as this call needs it. (Five or six copies from pageable memory at 4 to 5 us of this thread's time each before. A place
-// per table for as many lanes as the workspace holds: 400 KB for one lane after room was reserved for 16384, and a pinned buffer
-// grown for it, which made the first prompt 2.7 ms instead of 0.15.) With `also`, that many words go to `also_dev` too.
+// What the device has to know of a host call -- lanes, rows of the heads, ids -- one table behind another in one copy, as long as this
+// call needs it, out of pinned memory where the context has enough. (Five or six copies from pageable memory at 4 to 5 us of this
+// thread's time each before. A place per table for as many lanes as the workspace holds: 400 KB for one lane after room was reserved for
+// 16384, and a pinned buffer grown for it, which made the first prompt 2.7 ms instead of 0.15.) With `also`, that many words go to `also_dev` too.
 int32_t send_description(pssa_b200_model* m, const std::vector<uint32_t>& ids, const std::vector<uint32_t>& off, const std::vector<uint32_t>& len,
                          const std::vector<uint32_t>& slot, const std::vector<uint32_t>& last, const std::vector<uint32_t>& row_slot,
                          const std::vector<uint32_t>& head_slot, const std::vector<uint32_t>* also = nullptr, void* also_dev = nullptr) {
@@ -650,16 +650,25 @@ int32_t send_description(pssa_b200_model* m, const std::vector<uint32_t>& ids, c
     for (size_t i = 0; i < kHostTables; ++i) sizes[i] = tables[i].words.size();
     const size_t bytes = lay_host_tables(sizes, at) * 4, more = also ? also->size() * 4 : 0;
     for (size_t i = 0; i < kHostTables; ++i) tables[i].dev = base + at[i];
-    int32_t rc = pinned_reserve(m->ctx, bytes + more);
-    if (rc) return rc;
-    char* const h = m->ctx->pinned;
-    for (auto& x : tables)
-        if (!x.words.empty()) std::memcpy(h + (x.dev - base) * 4, x.words.data(), x.words.size() * 4);
-    if (more) {
-        std::memcpy(h + bytes, also->data(), more);
-        if ((rc = pinned_send(m->ctx, also_dev, bytes, more))) return rc;
+    int32_t rc;
+    const bool pinned = want_pinned(m->ctx, bytes + more, false);
+    if (pinned) {
+        if ((rc = pinned_reserve(m->ctx, bytes + more))) return rc;
+    } else {
+        if (!m->sent.empty()) PSSA_CUDA(m->ctx, cudaStreamSynchronize(m->ctx->stream));  // an earlier copy may still read them
+        m->sent.resize(bytes + more);
     }
-    return pinned_send(m->ctx, base, 0, bytes);
+    char* const h = pinned ? m->ctx->pinned : m->sent.data();
+    for (size_t i = 0; i < kHostTables; ++i)
+        if (sizes[i]) std::memcpy(h + at[i] * 4, tables[i].words.data(), sizes[i] * 4);
+    if (more) std::memcpy(h + bytes, also->data(), more);
+    auto send = [&](void* dev, size_t off, size_t n) -> int32_t {
+        if (pinned) return pinned_send(m->ctx, dev, off, n);
+        PSSA_CUDA(m->ctx, cudaMemcpyAsync(dev, h + off, n, cudaMemcpyHostToDevice, m->ctx->stream));
+        return PSSA_B200_OK;
+    };
+    if (more && (rc = send(also_dev, bytes, more))) return rc;
+    return send(base, 0, bytes);
 }
 
 int32_t run_lanes(pssa_b200_model* m, const uint64_t* ids, const uint32_t* offsets, const uint32_t* lengths, const uint32_t* streams,
@@ -716,7 +725,7 @@ int32_t run_lanes(pssa_b200_model* m, const uint64_t* ids, const uint32_t* offse
         // A step of a few streams takes its ids along with the launch and leaves logits that nothing on the device reads in pinned
         // memory itself: no copy before it and none behind (chat on the small model 56 -> 45 us a token, on the large one 306 -> 291).
         const bool own = step && rows <= kStepOwnRows && !sampling;
-        const bool direct = own && logits && !greedy && o_logits + nh * row <= kPinnedMin;
+        const bool direct = own && logits && !greedy && o_logits + nh * row <= std::min(kPinnedMin, ctx->pinned_bytes);
         if (direct && (rc = pinned_reserve(ctx, o_logits + nh * row))) return rc;
         if (!own && (rc = send_description(m, h_ids, s_off, s_len, s_slot, h_last, h_row_slot, head_slot))) return rc;
         if (step) {
@@ -745,8 +754,11 @@ int32_t run_lanes(pssa_b200_model* m, const uint64_t* ids, const uint32_t* offse
             // results through pinned memory: ids, sampler status, confidences, then the logits, at once or in as many rows at a time as
             // the smallest buffer holds (growing it in a first call would cost more than it ever gives back)
             const bool together = logits && o_logits + nh * row <= kPinnedMin;
-            if ((rc = pinned_reserve(ctx, o_logits + (together ? nh * row : 0)))) return rc;
-            char* const h = ctx->pinned;
+            const size_t landing = o_logits + (together ? nh * row : 0);
+            const bool pinned = want_pinned(ctx, landing, true);
+            if (pinned && (rc = pinned_reserve(ctx, landing))) return rc;
+            std::vector<char> pageable(pinned ? 0 : landing);
+            char* const h = pinned ? ctx->pinned : pageable.data();
             if (greedy) PSSA_CUDA(ctx, cudaMemcpyAsync(h, sampling ? m->sampler.ids : ws.greedy, nh * 4, cudaMemcpyDeviceToHost, st));
             if (sampling) PSSA_CUDA(ctx, cudaMemcpyAsync(h + nh * 4, m->sampler.status, nh * 4, cudaMemcpyDeviceToHost, st));
             if (sampling && confidence) PSSA_CUDA(ctx, cudaMemcpyAsync(h + o_conf, m->sampler.conf, nh * 4, cudaMemcpyDeviceToHost, st));
@@ -965,7 +977,12 @@ int32_t pssa_b200_model_score(pssa_b200_model* m, uint32_t stream, const uint64_
             if (logits_out)
                 PSSA_CUDA(ctx, cudaMemcpyAsync(logits_out + (t0 + r0) * m->v, sc.logits, nr * m->v * sizeof(float), cudaMemcpyDeviceToHost, st));
         }
-        if ((rc = copy_to_host(ctx, h_loss.data(), sc.loss, rows * 4))) return rc;
+        if (want_pinned(ctx, std::min(rows * 4, kPinnedMax), true)) {
+            if ((rc = copy_to_host(ctx, h_loss.data(), sc.loss, rows * 4))) return rc;
+        } else {
+            PSSA_CUDA(ctx, cudaMemcpyAsync(h_loss.data(), sc.loss, rows * 4, cudaMemcpyDeviceToHost, st));
+            PSSA_CUDA(ctx, cudaStreamSynchronize(st));
+        }
         for (size_t t = 0; t < rows; ++t) {
             if (!std::isfinite(h_loss[t])) return fail(ctx, PSSA_B200_ERR_INVALID_ARGUMENT, "model emitted non-finite logits at token %zu", t0 + t);
             total += (double)h_loss[t];
