@@ -174,11 +174,7 @@ int32_t pinned_send(pssa_b200_ctx* ctx, void* dst_dev, size_t off, size_t bytes)
 
 // Copies `bytes` from consecutive device memory at `src` to the arrays in `to` (consecutive in the device order, with gaps).
 namespace {
-struct Target {
-    char* dst;
-    size_t off, bytes;
-};
-int32_t scatter(pssa_b200_ctx* ctx, const char* src, size_t bytes, const std::vector<Target>& to) {
+int32_t scatter(pssa_b200_ctx* ctx, const char* src, size_t bytes, const std::vector<HostSpan>& to) {
     cudaStream_t st = ctx->stream;
     for (size_t w0 = 0; w0 < bytes; w0 += kPinnedMax) {
         const size_t wn = std::min(kPinnedMax, bytes - w0);
@@ -187,7 +183,7 @@ int32_t scatter(pssa_b200_ctx* ctx, const char* src, size_t bytes, const std::ve
         if (wn < kThreadsFrom) {
             PSSA_CUDA(ctx, cudaMemcpyAsync(ctx->pinned, src + w0, wn, cudaMemcpyDeviceToHost, st));
             PSSA_CUDA(ctx, cudaStreamSynchronize(st));
-            for (const Target& t : to) {
+            for (const HostSpan& t : to) {
                 const size_t a = std::max(t.off, w0), b = std::min(t.off + t.bytes, w0 + wn);
                 if (a < b) std::memcpy(t.dst + (a - t.off), ctx->pinned + (a - w0), b - a);
             }
@@ -247,7 +243,18 @@ int32_t scatter(pssa_b200_ctx* ctx, const char* src, size_t bytes, const std::ve
 }  // namespace
 
 int32_t copy_to_host(pssa_b200_ctx* ctx, void* dst, const void* src_dev, size_t bytes) {
-    return scatter(ctx, (const char*)src_dev, bytes, {Target{(char*)dst, 0, bytes}});
+    return scatter(ctx, (const char*)src_dev, bytes, {HostSpan{(char*)dst, 0, bytes}});
+}
+
+int32_t copy_spans_to_host(pssa_b200_ctx* ctx, const void* src_dev, size_t bytes, const std::vector<HostSpan>& to) {
+    // Up to a megabyte a larger buffer would save 8 to 28 us a call and is not pinned for it: the driver's own copy then. Us a decode step
+    // with logits of 16384 words, rounds of 256 KB by one thread -> this: 16 lanes 160 -> 139 (112 where the buffer is there), 32 lanes 322 ->
+    // 168, 64 582 -> 245, 256 2065 -> 740, 512 4020 -> 1370.
+    if (bytes > kThreadsFrom ? want_pinned(ctx, std::min(bytes, kPinnedMax), true) : bytes <= ctx->pinned_bytes)
+        return scatter(ctx, (const char*)src_dev, bytes, to);
+    for (const HostSpan& t : to) PSSA_CUDA(ctx, cudaMemcpyAsync(t.dst, (const char*)src_dev + t.off, t.bytes, cudaMemcpyDeviceToHost, ctx->stream));
+    PSSA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    return PSSA_B200_OK;
 }
 
 // In pieces, each copied into the pinned buffer by several threads while the one before is on the link: a carry of 2.4 MB in 75 us
@@ -334,14 +341,14 @@ int32_t HostCall::upload() {
 }
 
 int32_t HostCall::download(const char* what) {
-    std::vector<Target> to;
+    std::vector<HostSpan> to;
     size_t lo = SIZE_MAX, hi = 0;
     for (const Array& a : arrays_)
         if (a.dst && a.bytes) lo = std::min(lo, a.off), hi = std::max(hi, a.off + a.bytes);
     if (lo == SIZE_MAX) lo = hi = 0;
     for (const Array& a : arrays_)
         if (a.dst && a.bytes) to.push_back({(char*)a.dst, a.off - lo, a.bytes});
-    std::sort(to.begin(), to.end(), [](const Target& x, const Target& y) { return x.off < y.off; });
+    std::sort(to.begin(), to.end(), [](const HostSpan& x, const HostSpan& y) { return x.off < y.off; });
     // With `what`, the status word comes back too and outputs stay untouched when a bounded wait has expired. The pinned
     // buffer may still be the source of the inputs' copy: it is only written by copies behind that one on the stream.
     int32_t rc;
@@ -358,7 +365,7 @@ int32_t HostCall::download(const char* what) {
         return fail(ctx_, status, "%s: a bounded device-side wait expired", what);
     }
     if (!small) return scatter(ctx_, base_ + lo, bytes, to);
-    for (const Target& t : to) std::memcpy(t.dst, ctx_->pinned + 64 + t.off, t.bytes);
+    for (const HostSpan& t : to) std::memcpy(t.dst, ctx_->pinned + 64 + t.off, t.bytes);
     return PSSA_B200_OK;
 }
 

@@ -49,6 +49,12 @@ class HostCall {
 
 // device -> host through the context's pinned buffer, in stream order; waits for the stream
 int32_t copy_to_host(pssa_b200_ctx* ctx, void* dst, const void* src_dev, size_t bytes);
+// The same to several arrays, through pinned memory where that pays: `to` in the order of `off`, the places in `src_dev`.
+struct HostSpan {
+    char* dst;
+    size_t off, bytes;
+};
+int32_t copy_spans_to_host(pssa_b200_ctx* ctx, const void* src_dev, size_t bytes, const std::vector<HostSpan>& to);
 // host -> device through the context's pinned buffer (see want_pinned); waits for the stream
 int32_t copy_to_device(pssa_b200_ctx* ctx, void* dst_dev, const void* src, size_t bytes);
 // a context's first pinned buffer, and its largest: longer transfers go through it in windows

@@ -671,6 +671,15 @@ int32_t send_description(pssa_b200_model* m, const std::vector<uint32_t>& ids, c
     return send(base, 0, bytes);
 }
 
+// Logits of many lanes, `row` bytes each, to the places of their lanes.
+int32_t logits_to_host(pssa_b200_ctx* ctx, float* logits, const float* src, const std::vector<size_t>& lanes, size_t row) {
+    std::vector<HostSpan> to;  // neighbouring lanes in one piece
+    for (size_t i = 0; i < lanes.size(); ++i)
+        if (i > 0 && lanes[i] == lanes[i - 1] + 1) to.back().bytes += row;
+        else to.push_back({(char*)logits + lanes[i] * row, i * row, row});
+    return copy_spans_to_host(ctx, src, lanes.size() * row, to);
+}
+
 int32_t run_lanes(pssa_b200_model* m, const uint64_t* ids, const uint32_t* offsets, const uint32_t* lengths, const uint32_t* streams,
                   size_t n_lanes, float* logits, uint64_t* greedy, int32_t (*cancelled)(void*), void* cancel_arg, size_t* processed,
                   const pssa_b200_sampling* sampling = nullptr, uint32_t sample_flags = 0, float* confidence = nullptr) {
@@ -751,8 +760,7 @@ int32_t run_lanes(pssa_b200_model* m, const uint64_t* ids, const uint32_t* offse
                 if ((rc = launch_sample(ctx, sp))) return rc;
                 if ((rc = launch_push_recent(ctx, m->sampler.ids, ws.host.head_slot, m->sampler.recent, m->sampler.count, nh))) return rc;
             }
-            // results through pinned memory: ids, sampler status, confidences, then the logits, at once or in as many rows at a time as
-            // the smallest buffer holds (growing it in a first call would cost more than it ever gives back)
+            // results through pinned memory: ids, sampler status, confidences and then the logits, where the smallest buffer holds them
             const bool together = logits && o_logits + nh * row <= kPinnedMin;
             const size_t landing = o_logits + (together ? nh * row : 0);
             const bool pinned = want_pinned(ctx, landing, true);
@@ -767,14 +775,7 @@ int32_t run_lanes(pssa_b200_model* m, const uint64_t* ids, const uint32_t* offse
             if (together)
                 for (size_t i = 0; i < nh; ++i) std::memcpy(logits + head_lane[i] * m->v, h + o_logits + i * row, row);
             const std::vector<uint32_t> got((const uint32_t*)h, (const uint32_t*)(h + 3 * nh * 4));
-            if (logits && !together)
-                for (size_t i = 0, n; i < nh; i += n) {
-                    n = std::min(nh - i, std::max<size_t>(1, kPinnedMin / row));
-                    if ((rc = pinned_reserve(ctx, n * row))) return rc;
-                    PSSA_CUDA(ctx, cudaMemcpyAsync(ctx->pinned, ws.logits + i * m->v, n * row, cudaMemcpyDeviceToHost, st));
-                    PSSA_CUDA(ctx, cudaStreamSynchronize(st));
-                    for (size_t j = 0; j < n; ++j) std::memcpy(logits + head_lane[i + j] * m->v, ctx->pinned + j * row, row);
-                }
+            if (logits && !together && (rc = logits_to_host(ctx, logits, ws.logits, head_lane, row))) return rc;
             if (greedy)
                 for (size_t i = 0; i < nh; ++i) {
                     if (got[i] == 0xffffffffu) {  // src/inference.rs:111-113, 146-147, 153-154

@@ -97,3 +97,32 @@ def test_one_thread_waits_for_the_kernels_in_front_of_a_large_output():
     gpu.close()
     assert wall > 0.15
     assert cpu <= 1.5 * wall, (cpu, wall)
+
+
+@pytest.mark.parametrize("vocab,lanes", [(16384, 4), (16384, 5), (16384, 17), (4099, 63), (4099, 130), (16384, 70)])
+def test_logits_of_many_lanes_reach_their_places(vocab, lanes):
+    """Logits that the first pinned buffer holds, that it does not hold (the driver's copy, and the largest buffer from the second call on)
+    and of more than one window of that: a step of every lane and ragged calls with empty lanes between them, in a new context and
+    again, equal the device-resident entry point's logits."""
+    import torch
+    import pssa_b200
+    gpu = pssa_b200.B200Dispatch(0, torch.cuda.current_stream())
+    d, s, k, cap = 32, 16, 8, 16
+    m = pssa_b200.PSSAModel(gpu, 1, vocab, d, s, k, cap, tau_mem=0.1, streams=lanes, precision=0)
+    m.init_random(5)
+    rng = np.random.default_rng(lanes)
+    keys = (rng.standard_normal((cap, k)) * 0.1).astype(np.float32)
+    m.set_bank(0, keys, (keys ** 2).sum(1).astype(np.float32), rng.standard_normal((cap, d)).astype(np.float32), cap)
+    for lengths in (np.ones(lanes, int), np.where(np.arange(lanes) % 5 == 2, 0, 1 + np.arange(lanes) % 3), np.arange(lanes) % 2):
+        ids = [rng.integers(1, vocab, n) for n in lengths]
+        flat = torch.from_numpy(np.concatenate(ids).astype(np.int32)).cuda()
+        off = np.concatenate([[0], np.cumsum(lengths)[:-1]]).astype(np.uint32)
+        want = torch.zeros(lanes, vocab, device="cuda")
+        m.reset_recurrent_state()
+        m.prefill_batch_dev(flat, off, lengths.astype(np.uint32), None, want)
+        want = want.cpu().numpy()
+        for _ in range(3):
+            m.reset_recurrent_state()
+            assert np.array_equal(m.prefill_batch(ids)[0], want)
+    m.close()
+    gpu.close()
