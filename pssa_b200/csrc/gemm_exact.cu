@@ -396,7 +396,18 @@ int32_t launch_parts(pssa_b200_ctx* ctx, const float* x, ExactParts& parts, size
     if (M <= 4 && 4 * K * 4 <= kMaxStagedX) return launch_tiled<4, 2, 24>(ctx, x, parts, M, K, ldo, alpha);
     bool vec = K % 4 == 0 && K >= 32 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
     for (int i = 0; i < parts.count; ++i) vec = vec && (reinterpret_cast<uintptr_t>(parts.p[i].w) & 15) == 0;
-    if (!vec) return launch_tiled<8, 4, 0>(ctx, x, parts, M, K, ldo, alpha);
+    if (!vec) {
+        // Rows that the ring cannot copy. Tiles of 8 x 8 load a word for four multiply-adds instead of 2.7, but hold twice the registers (16
+        // warps to an SM) and leave more of a last wave empty; short sums hide that sooner. Us, 8 x 4 and 8 x 8: 1000 x 192 x 16 6.4 and
+        // 5.7, 4096 x 768 x 16 79 and 64, 2048 x 1536 x 191 169 and 149, 1000 x 1536 x 767 175 and 167; under the line 300 x 768 x 191 15.3 and
+        // 15.5, 300 x 592 x 767 24.4 and 26.8, 300 x 1536 x 767 57.1 and 57.6. Few rows need nothing of their own (16 x 16384 x 767 32; 40
+        // with X staged in shared memory).
+        size_t n = 0;
+        for (int i = 0; i < parts.count; ++i) n += parts.p[i].n;
+        const size_t wide = (M + 7) / 8 * ((n + 7) / 8);
+        if (wide >= (K < 64 ? 20 : K < 256 ? 30 : 56) * (size_t)ctx->sm_count) return launch_tiled<8, 8, 0>(ctx, x, parts, M, K, ldo, alpha);
+        return launch_tiled<8, 4, 0>(ctx, x, parts, M, K, ldo, alpha);
+    }
     if (M <= 8 || (M > 16 && M <= 24)) return launch_ring<8, 4, 1, 4, 64>(ctx, x, parts, M, K, ldo, alpha);
     return launch_ring<8, 8, 2, 2, 128>(ctx, x, parts, M, K, ldo, alpha);
 }

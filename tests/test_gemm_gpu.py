@@ -58,6 +58,23 @@ def test_exact_gemm_ring_tiles_are_dot_slice_bit_for_bit(gpu, m, n, k):
     assert np.array_equal(bits(got), bits(want + want))
 
 
+@pytest.mark.parametrize("m,n,k,offset", [(977, 190, 17, 0), (985, 190, 17, 0), (1501, 185, 64, 1), (2873, 181, 259, 0), (2999, 181, 258, 0), (37, 50, 96, 1)])
+def test_exact_gemm_of_many_unaligned_rows_is_dot_slice_bit_for_bit(gpu, m, n, k, offset):
+    """Rows that are not 16-byte aligned, by their length or where the arrays begin: both sides of the line between tiles of four and
+    of eight columns (2960 tiles of 8 x 8 for short sums, 4440 below 256 columns, 8288 above, on 148 SMs), ragged in rows and columns."""
+    import torch
+    from pssa_b200 import _native as N
+    rng = np.random.default_rng(m + k)
+    x, w = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((n, k)).astype(np.float32)
+    xd, wd = (torch.cat([torch.zeros(offset), torch.from_numpy(a).ravel()]).cuda() for a in (x, w))
+    out = torch.full((m * n + 1,), 7.0, device="cuda")
+    torch.cuda.synchronize()
+    gpu.gemm_xwt_dev(xd[offset:], wd[offset:], m, n, k, out, precision=N.PRECISION_FP32_EXACT)
+    gpu.synchronize()
+    got = out.cpu().numpy()
+    assert np.array_equal(bits(got[:-1].reshape(m, n)), bits(O.gemm_xwt(x, w))) and got[-1] == 7.0
+
+
 def test_batch_folds_into_rows_and_bad_lengths_leave_output_untouched(gpu):
     # tests/backend.rs:9-82
     import pssa_b200
