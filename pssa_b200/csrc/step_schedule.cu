@@ -356,10 +356,12 @@ int32_t launch_step_schedule(pssa_b200_ctx* ctx, const StepLaunch& p) {
         const StepBlock b = step_block(p.blocks[l]);
         float* const out = in == a.feat_a ? a.feat_b : a.feat_a;
         const unsigned* const ids = l == 0 ? a.ids : nullptr;
-        // started early its few CTAs crowd on the SMs that the product before leaves first (256 streams of 12 blocks of d 768: 1114 -> 1074
-        // us a step, 64 871 -> 858; 128 of 4 blocks of d 384 231 -> 228); at d 192 the launch's latency is more (200 streams 66.5, 68.4)
+        // Started early its few CTAs crowd on the SMs that the product before leaves first, at every width and number of rows: us a step as a
+        // graph, early -> in order, 4 blocks: d 64 x 256 rows 193 -> 177, d 192 x 200 219 -> 204, d 384 x 512 345 -> 331, d 768 x 256 374 -> 356,
+        // x 2048 988 -> 968. The first block's follows another call: early saves 2 us of an eager step of 200 to 512 rows and costs 1 to 3
+        // with fewer rows or as a graph; of 1024 rows and more of wide models it costs 3 to 7.
         const dim3 norm_grid(((unsigned)a.rows + kWarps - 1) / kWarps);
-        if (d > 256) step_norm_kernel<<<norm_grid, kThreads, 0, ctx->stream>>>(a, b, ids, in);
+        if (l > 0 || d > 256) step_norm_kernel<<<norm_grid, kThreads, 0, ctx->stream>>>(a, b, ids, in);
         else PSSA_CUDA(ctx, launch_dependent(step_norm_kernel, norm_grid, dim3(kThreads), 0, ctx->stream, a, b, ids, in));
         if ((rc = after_launch(ctx, "step_norm_kernel"))) return rc;
         if ((rc = narrow(ctx, a, a.nc) ? product<32, 9, PutXside>(ctx, a, a.x, d, b.wcat, d, a.nc, d, "step_product_kernel[x-side]")
