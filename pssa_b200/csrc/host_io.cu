@@ -112,7 +112,7 @@ CopyPool& copy_pool() {
 struct PinnedCache {
     std::mutex m;
     std::vector<std::pair<char*, size_t>> kept;
-    size_t contexts = 0;
+    size_t contexts = 0, pinned = 0;  // buffers that are pinned now, kept or in use
 };
 PinnedCache& pinned_cache() {
     static PinnedCache* c = new PinnedCache();
@@ -122,7 +122,7 @@ void pinned_give_back(char* p, size_t bytes) {
     PinnedCache& c = pinned_cache();
     std::lock_guard<std::mutex> l(c.m);
     if (bytes <= kPinnedMax && c.contexts > 0 && c.kept.size() < kPinnedKept) c.kept.push_back({p, bytes});
-    else cudaFreeHost(p);
+    else cudaFreeHost(p), --c.pinned;
 }
 }  // namespace
 
@@ -155,12 +155,22 @@ int32_t pinned_reserve(pssa_b200_ctx* ctx, size_t bytes) {
         return cuda_fail(ctx, e, "pinned staging allocation");
     }
     ctx->pinned_bytes = want;
+    PinnedCache& c = pinned_cache();
+    std::lock_guard<std::mutex> l(c.m);
+    ++c.pinned;
     return PSSA_B200_OK;
 }
 
 bool want_pinned(pssa_b200_ctx* ctx, size_t bytes, bool out) {
     if (bytes <= ctx->pinned_bytes) return true;
     if (bytes > kPinnedMax) return false;
+    {
+        PinnedCache& c = pinned_cache();
+        std::lock_guard<std::mutex> l(c.m);
+        if (bytes <= kPinnedMin && c.pinned > 0) return true;
+        for (auto& k : c.kept)
+            if (k.second >= bytes) return true;
+    }
     return std::exchange(ctx->asked[out][bytes > kPinnedMin], true);
 }
 
@@ -174,10 +184,10 @@ int32_t pinned_send(pssa_b200_ctx* ctx, void* dst_dev, size_t off, size_t bytes)
 
 // Copies `bytes` from consecutive device memory at `src` to the arrays in `to` (consecutive in the device order, with gaps).
 namespace {
-int32_t scatter(pssa_b200_ctx* ctx, const char* src, size_t bytes, const std::vector<HostSpan>& to) {
+int32_t scatter(pssa_b200_ctx* ctx, const char* src, size_t bytes, const std::vector<HostSpan>& to, size_t window = kPinnedMax) {
     cudaStream_t st = ctx->stream;
-    for (size_t w0 = 0; w0 < bytes; w0 += kPinnedMax) {
-        const size_t wn = std::min(kPinnedMax, bytes - w0);
+    for (size_t w0 = 0; w0 < bytes; w0 += window) {
+        const size_t wn = std::min(window, bytes - w0);
         int32_t rc = pinned_reserve(ctx, wn);
         if (rc) return rc;
         if (wn < kThreadsFrom) {
@@ -247,11 +257,12 @@ int32_t copy_to_host(pssa_b200_ctx* ctx, void* dst, const void* src_dev, size_t 
 }
 
 int32_t copy_spans_to_host(pssa_b200_ctx* ctx, const void* src_dev, size_t bytes, const std::vector<HostSpan>& to) {
-    // Up to a megabyte a larger buffer would save 8 to 28 us a call and is not pinned for it: the driver's own copy then. Us a decode step
-    // with logits of 16384 words, rounds of 256 KB by one thread -> this: 16 lanes 160 -> 139 (112 where the buffer is there), 32 lanes 322 ->
-    // 168, 64 582 -> 245, 256 2065 -> 740, 512 4020 -> 1370.
-    if (bytes > kThreadsFrom ? want_pinned(ctx, std::min(bytes, kPinnedMax), true) : bytes <= ctx->pinned_bytes)
-        return scatter(ctx, (const char*)src_dev, bytes, to);
+    // Up to a megabyte through what the context has: a larger buffer would save 8 to 45 us a call and is not pinned for it. Us a decode step with
+    // logits of 16384 words, rounds of 256 KB by one thread -> this: 32 lanes 322 -> 168, 64 582 -> 245, 256 2065 -> 740, 512 4020 -> 1370.
+    // (The driver's own copy, for comparison: 224, 345, 1060, 2000; seven prompts into pages that nothing has touched 50 us slower than
+    // two rounds.)
+    if (bytes <= kThreadsFrom && ctx->pinned_bytes > 0) return scatter(ctx, (const char*)src_dev, bytes, to, ctx->pinned_bytes);
+    if (bytes > kThreadsFrom && want_pinned(ctx, std::min(bytes, kPinnedMax), true)) return scatter(ctx, (const char*)src_dev, bytes, to);
     for (const HostSpan& t : to) PSSA_CUDA(ctx, cudaMemcpyAsync(t.dst, (const char*)src_dev + t.off, t.bytes, cudaMemcpyDeviceToHost, ctx->stream));
     PSSA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     return PSSA_B200_OK;
@@ -393,6 +404,7 @@ void host_io_destroy(pssa_b200_ctx* ctx) {
     std::lock_guard<std::mutex> l(c.m);
     if (--c.contexts == 0) {
         for (auto& k : c.kept) cudaFreeHost(k.first);
+        c.pinned -= c.kept.size();
         c.kept.clear();
     }
 }

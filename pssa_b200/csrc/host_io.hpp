@@ -63,9 +63,9 @@ constexpr size_t kPinnedMin = (size_t)256 << 10, kPinnedMax = (size_t)4 << 20;
 // a copy that pinned_send left behind
 int32_t pinned_reserve(pssa_b200_ctx* ctx, size_t bytes);
 // Whether words of a model's host call should pass through pinned memory: yes where the buffer holds them; otherwise a context's first
-// such call goes without and the next one pins it. Pinning takes 0.9 to 2.6 ms for the first buffer and 1.5 to 4.5 for the largest, and
-// saves a call 10 us at 256 KB and 150 at 4 MB: a program that makes one call never gets it back (the small model's first step 2.8
-// ms with it and 0.2 without), one that makes many pays once.
+// such call goes without and the next one pins it. Pinning a process's first buffer takes 0.9 to 2.6 ms (3 us while another one is
+// pinned: then at once), the largest 1.5 to 4.5 ms, and saves a call 10 us at 256 KB and 150 at 4 MB: a program that makes one call never
+// gets it back (the small model's first step 2.8 ms with it and 0.2 without), one that makes many pays once.
 bool want_pinned(pssa_b200_ctx* ctx, size_t bytes, bool out);
 // enqueues the copy of `bytes` at `off` of the pinned buffer to the device and returns
 int32_t pinned_send(pssa_b200_ctx* ctx, void* dst_dev, size_t off, size_t bytes);

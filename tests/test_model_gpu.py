@@ -758,33 +758,43 @@ def test_host_calls_of_any_length_after_room_for_many_lanes(gpu):
     assert np.array_equal(got[0], got[1])
 
 
-@pytest.mark.parametrize("first", ["step", "prompt", "score", "passes", "sampled"])
-def test_first_call_of_a_context_gives_what_later_ones_give(first):
-    """A context's first host call has no pinned buffer, its second pins one and its third finds it (a step then writes its logits there).
-    Logits and carries are the same each time, whatever carry was set before (`passes`: one prompt in several passes, none but the
-    last of which has results, of more words than the first buffer holds)."""
+def first_calls_of_contexts():
     import pssa_b200
-    rng = np.random.default_rng(9)
-    ids = rng.integers(1, 97, 70000 if first == "passes" else 70)
-    calls = {"step": lambda m: m.forward_inference(5), "prompt": lambda m: m.prefill_inference(ids)[1], "score": lambda m: m.score(ids[:-1], ids[1:])[1],
-             "passes": lambda m: m.prefill_inference(ids)[1], "sampled": lambda m: m.decode_step_sampled(np.array([3]))}
-    ctx = pssa_b200.B200Dispatch(0)
-    _, gm = make_pair(ctx, 2, 97, 32, 16, 8, 16, seed=34, precision=0)
-    gm.set_max_rows(69000 if first == "passes" else 65536)
-    gm.sampler_seed(0, 7)
-    carry = rng.standard_normal(gm.recurrent_state_len()).astype(np.float32)
-    got = []
-    for _ in range(4):
-        if first in ("step", "sampled"):  # the others' own words are the first to ask for the buffer
-            gm.copy_recurrent_state_from(carry, 0)
-        else:
-            gm.reset_recurrent_state()
+    for first in ("step", "prompt", "score", "passes", "sampled"):
+        rng = np.random.default_rng(9)
+        ids = rng.integers(1, 97, 70000 if first == "passes" else 70)
+        calls = {"step": lambda m: m.forward_inference(5), "prompt": lambda m: m.prefill_inference(ids)[1], "score": lambda m: m.score(ids[:-1], ids[1:])[1],
+                 "passes": lambda m: m.prefill_inference(ids)[1], "sampled": lambda m: m.decode_step_sampled(np.array([3]))}
+        ctx = pssa_b200.B200Dispatch(0)
+        _, gm = make_pair(ctx, 2, 97, 32, 16, 8, 16, seed=34, precision=0)
+        gm.set_max_rows(69000 if first == "passes" else 65536)
         gm.sampler_seed(0, 7)
-        out = [np.ravel(calls[first](gm)).astype(np.float32)]
-        got.append(np.concatenate(out + [gm.copy_recurrent_state_to(0)]).view(np.uint32))
-    gm.close()
-    ctx.close()
-    assert all(np.array_equal(got[0], x) for x in got[1:])
+        carry = rng.standard_normal(gm.recurrent_state_len()).astype(np.float32)
+        got = []
+        for _ in range(4):
+            if first in ("step", "sampled"):  # the others' own words are the first to ask for the buffer
+                gm.copy_recurrent_state_from(carry, 0)
+            else:
+                gm.reset_recurrent_state()
+            gm.sampler_seed(0, 7)
+            out = [np.ravel(calls[first](gm)).astype(np.float32)]
+            got.append(np.concatenate(out + [gm.copy_recurrent_state_to(0)]).view(np.uint32))
+        gm.close()
+        ctx.close()
+        assert all(np.array_equal(got[0], x) for x in got[1:]), first
+
+
+def test_first_call_of_a_context_gives_what_later_ones_give():
+    """In a process with no other context: a context's first host call has no pinned buffer, its second pins one and its third finds it
+    (a step then writes its logits there). Logits and carries are the same each time, whatever carry was set before (`passes`: one
+    prompt in several passes, none but the last of which has results, of more words than the first buffer holds)."""
+    import os
+    import pathlib
+    import subprocess
+    import sys
+    ran = subprocess.run([sys.executable, "-c", "import test_model_gpu as t; t.first_calls_of_contexts()"], cwd=pathlib.Path(__file__).parent,
+                         env=dict(os.environ, PYTHONPATH=str(pathlib.Path(__file__).parent.parent)), capture_output=True, text=True, timeout=300)
+    assert ran.returncode == 0, ran.stderr[-2000:]
 
 
 @pytest.mark.parametrize("k,cap,tau", [(64, 256, 0.1), (128, 128, 0.13), (128, 512, 0.1), (64, 512, 0.25)])
