@@ -734,7 +734,8 @@ int32_t run_lanes(pssa_b200_model* m, const uint64_t* ids, const uint32_t* offse
         // A step of a few streams takes its ids along with the launch and leaves logits that nothing on the device reads in pinned
         // memory itself: no copy before it and none behind (chat on the small model 56 -> 45 us a token, on the large one 306 -> 291).
         const bool own = step && rows <= kStepOwnRows && !sampling;
-        const bool direct = own && logits && !greedy && o_logits + nh * row <= std::min(kPinnedMin, ctx->pinned_bytes);
+        // (A step has logits for every row. Where lanes go on behind a pass of one token, the heads are some of them.)
+        const bool direct = own && logits && !greedy && nh == rows && o_logits + nh * row <= std::min(kPinnedMin, ctx->pinned_bytes);
         if (direct && (rc = pinned_reserve(ctx, o_logits + nh * row))) return rc;
         if (!own && (rc = send_description(m, h_ids, s_off, s_len, s_slot, h_last, h_row_slot, head_slot))) return rc;
         if (step) {
@@ -746,7 +747,11 @@ int32_t run_lanes(pssa_b200_model* m, const uint64_t* ids, const uint32_t* offse
         if (!h_last.empty() && want_head) {
             const bool want_greedy = greedy != nullptr && !sampling;
             if (!step && (rc = head_rows(m, feats, ws.host.last_rows, h_last.size(), want_greedy))) return rc;
-            if (step && want_greedy && (rc = launch_greedy(ctx, ws.logits, ws.greedy, rows, (int)m->v))) return rc;
+            if (step && nh < rows)  // the heads' rows one behind another, in order: none is overwritten before it has moved
+                for (size_t i = 0; i < nh; ++i)
+                    if (h_last[i] != i)
+                        PSSA_CUDA(ctx, cudaMemcpyAsync(ws.logits + i * m->v, ws.logits + h_last[i] * m->v, row, cudaMemcpyDeviceToDevice, st));
+            if (step && want_greedy && (rc = launch_greedy(ctx, ws.logits, ws.greedy, nh, (int)m->v))) return rc;
             if (sampling) {
                 // sample on the device from the logits the head just wrote; only ids come back
                 if ((rc = ensure_sampler(m, n_lanes))) return rc;

@@ -758,6 +758,28 @@ def test_host_calls_of_any_length_after_room_for_many_lanes(gpu):
     assert np.array_equal(got[0], got[1])
 
 
+@pytest.mark.parametrize("lanes,vocab", [(5, 257), (16, 16384), (32, 4099), (40, 4099)])
+def test_lanes_that_go_on_behind_a_pass_of_one_token_keep_their_results_apart(gpu, lanes, vocab):
+    """Room for one token of each lane a pass: a pass then is a step of every lane that is left, of which some end in it. Logits and ids
+    of lanes of 0 to 3 tokens, asked for together and apart in calls before and behind the context's pinned buffer, and the carries
+    are those of every lane by itself."""
+    _, gm = make_pair(gpu, 1, vocab, 32, 16, 64, 64, seed=35, streams=lanes, precision=0)
+    rng = np.random.default_rng(lanes)
+    prompts = [rng.integers(1, vocab, n) for n in [2, 1, 0, 3] + [int(x) for x in rng.integers(1, 4, lanes - 4)]]
+    gm.set_max_rows(1)
+    want = [np.zeros(vocab, np.float32) if len(p) == 0 else gm.prefill_batch([p], streams=[i])[0][0] for i, p in enumerate(prompts)]
+    state = [gm.copy_recurrent_state_to(i) for i in range(lanes)]
+    ids = [int(w[1:].argmax()) + 1 if len(p) else 0 for w, p in zip(want, prompts)]
+    gm.set_max_rows(lanes)
+    for want_logits, want_greedy in ((True, False), (True, True), (False, True), (True, False)):
+        gm.reset_recurrent_state()
+        logits, greedy = gm.prefill_batch(prompts, want_logits=want_logits, want_greedy=want_greedy)
+        assert logits is None or np.array_equal(logits, want)
+        assert greedy is None or list(greedy) == ids
+        assert all(np.array_equal(gm.copy_recurrent_state_to(i), s) for i, s in enumerate(state))
+    gm.close()
+
+
 def first_calls_of_contexts():
     import pssa_b200
     for first in ("step", "prompt", "score", "passes", "sampled"):
