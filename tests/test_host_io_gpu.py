@@ -107,11 +107,11 @@ def test_logits_of_many_lanes_reach_their_places(vocab, lanes):
     import torch
     import pssa_b200
     gpu = pssa_b200.B200Dispatch(0, torch.cuda.current_stream())
-    d, s, k, cap = 32, 16, 8, 16
+    d, s, k, cap = 32, 16, 64, 64
     m = pssa_b200.PSSAModel(gpu, 1, vocab, d, s, k, cap, tau_mem=0.1, streams=lanes, precision=0)
     m.init_random(5)
     rng = np.random.default_rng(lanes)
-    keys = (rng.standard_normal((cap, k)) * 0.1).astype(np.float32)
+    keys = (rng.standard_normal((cap, k)) * 0.05).astype(np.float32)
     m.set_bank(0, keys, (keys ** 2).sum(1).astype(np.float32), rng.standard_normal((cap, d)).astype(np.float32), cap)
     for lengths in (np.ones(lanes, int), np.where(np.arange(lanes) % 5 == 2, 0, 1 + np.arange(lanes) % 3), np.arange(lanes) % 2):
         ids = [rng.integers(1, vocab, n) for n in lengths]

@@ -748,7 +748,7 @@ def test_host_calls_of_any_length_after_room_for_many_lanes(gpu):
     turns = [rng.integers(1, 97, n) for n in (7, 0, 33, 1, 12)]
     got = []
     for lanes in (0, 600):
-        _, gm = make_pair(gpu, 2, 97, 32, 16, 8, 16, seed=33, streams=40, precision=0)
+        _, gm = make_pair(gpu, 2, 97, 32, 16, 64, 64, seed=33, streams=40, precision=0)
         if lanes:
             gm.reserve(2000, lanes)
         out = [gm.prefill_inference(prompt)[1], gm.decode_step(steps), gm.score(text[:-1], text[1:], stream=3)[1],
@@ -788,7 +788,7 @@ def first_calls_of_contexts():
         calls = {"step": lambda m: m.forward_inference(5), "prompt": lambda m: m.prefill_inference(ids)[1], "score": lambda m: m.score(ids[:-1], ids[1:])[1],
                  "passes": lambda m: m.prefill_inference(ids)[1], "sampled": lambda m: m.decode_step_sampled(np.array([3]))}
         ctx = pssa_b200.B200Dispatch(0)
-        _, gm = make_pair(ctx, 2, 97, 32, 16, 8, 16, seed=34, precision=0)
+        _, gm = make_pair(ctx, 2, 97, 32, 16, 64, 64, seed=34, precision=0)
         gm.set_max_rows(69000 if first == "passes" else 65536)
         gm.sampler_seed(0, 7)
         carry = rng.standard_normal(gm.recurrent_state_len()).astype(np.float32)

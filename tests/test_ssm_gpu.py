@@ -198,28 +198,38 @@ def test_edge_values_of_the_decay_reach_every_state(gpu, s, exact):
         assert np.array_equal(np.isnan(y.cpu().numpy()[1]), np.isnan((want * c[1]).sum(1)))
 
 
-# (lanes, d): two channels a thread, 352 and 256 threads a CTA (one, 16 and 48 lanes of 768 channels); whole tiles, a tail, ragged states
-@pytest.mark.parametrize("lanes,d,s,T", [(1, 68, 48, 101), (16, 768, 36, 64), (48, 768, 48, 35)])
+# two channels a thread, 352 and 256 threads a CTA (one, 16 and 48 lanes of up to 768 channels); tiles of 32 tokens and a tail; the last states
+# of a thread whole, in part, and those of a width that shorter calls take to another kernel
+@pytest.mark.parametrize("lanes,d,s,T", [(1, 68, 60, 261), (16, 768, 52, 256), (48, 768, 60, 291), (48, 768, 64, 263)])
 def test_small_argument_tiles_and_their_borders(gpu, lanes, d, s, T):
-    """Tiles whose exponents allow the polynomial of small arguments beside tiles that do not: a delta at, past and far past its
-    limit, negative, infinite and NaN deltas, rates of zero, of the other sign and NaN among the states it serves."""
+    """Calls of 256 tokens a lane or more, whose tiles take the polynomial of small arguments for states 48 to 63 where a warp's exponents
+    allow it: rates of zero and at the limit (channels 4 and 5), of the other sign and NaN (20 and 36, whose warps never take
+    it), and a delta at, past and far past the limit, negative, infinite and NaN (50 to 55), each in a tile of its own between
+    tiles that do. The same tokens in two shorter calls, which never take it, give other bits exactly there."""
     import torch
     g = torch.Generator(device="cuda").manual_seed(d + s)
     f = lambda *sh: torch.randn(*sh, device="cuda", generator=g)  # noqa: E731
     rows = lanes * T
     delta = torch.rand(rows, d, device="cuda", generator=g)
     rates = -torch.exp(torch.empty(d, s, device="cuda").uniform_(-5.0, -1.4, generator=g))  # all below 0.4 / log2(e) = 0.277
-    rates[4, 33], rates[5, 34], rates[6, 33], rates[7, 35] = 0.0, 0.02, float("nan"), 0.277
-    t = T - 1 if T < 64 else 40  # in the tail or in the second tile; the first whole tile stays small
-    for ch, v in ((8, 0.4 / 1.4427 / 0.25), (9, 3.0), (10, -1.0), (11, float("inf")), (12, float("nan")), (13, 60.0)):
-        delta[t, ch] = v
+    rates[4, 50], rates[5, 49], rates[20, 50], rates[36, 49], rates[50, 48:] = 0.0, -0.277, 0.02, float("nan"), -0.25
+    special = ((1, 50, 0.4 / 1.4427 / 0.25), (2, 50, 0.401 / 1.4427 / 0.25), (3, 51, 3.0), (4, 52, -1.0), (5, 53, float("inf")), (6, 54, float("nan")), (7, 55, 60.0))
+    for tile, ch, v in special:
+        delta[tile * 32 + tile, ch] = v
     bp, cp, x, h0 = f(rows, s), f(rows, s), f(rows, d), f(lanes, d * s)
-    off, ln = (np.arange(lanes) * T).astype(np.uint32), np.full(lanes, T, np.uint32)
-    carry, y = h0.clone(), torch.zeros(rows, d, device="cuda")
+    carry, y, carry2, y2 = h0.clone(), torch.zeros(rows, d, device="cuda"), h0.clone(), torch.zeros(rows, d, device="cuda")
+    off = np.arange(lanes) * T
     gpu.set_stream(torch.cuda.current_stream())
-    gpu.ssm_forward_dev(delta, bp, cp, x, rates, carry, y, off, ln, rows, d, s)
+    for c, out, parts in ((carry, y, ((0, T),)), (carry2, y2, ((0, 128), (128, T - 128)))):
+        for t0, n in parts:
+            gpu.ssm_forward_dev(delta, bp, cp, x, rates, c, out, (off + t0).astype(np.uint32), np.full(lanes, n, np.uint32), rows, d, s)
     torch.cuda.synchronize()
     gpu.set_stream(None)
+    if s != 64:  # (64 states: the two shorter calls are the few-lanes kernel's)
+        a, b = (v.reshape(lanes, d, s).view(torch.int32) for v in (carry, carry2))
+        assert not torch.equal(a[:, :8, 48:], b[:, :8, 48:])
+        never = [ch for ch in list(range(16, 24)) + list(range(32, 40)) if ch != 36]
+        assert torch.equal(a[:, never], b[:, never])
     q = lambda a, w: a.double().reshape(lanes, T, w)  # noqa: E731
     dl, b, c, xv, want = q(delta, d), q(bp, s), q(cp, s), q(x, d), h0.double().reshape(lanes, d, s)
     size = want.abs()  # of the terms: they can cancel
@@ -232,7 +242,7 @@ def test_small_argument_tiles_and_their_borders(gpu, lanes, d, s, T):
         # a token: the argument's two roundings (2^-24 of at most 60 * 0.25 / ln 2 = 22) and the exponential's 2^-22; sums 2^-24 each
         fin = torch.isfinite(ref)
         assert float(((got - ref).abs() / mag)[fin].max()) <= (i + 1) * 2.0 ** -22 + (2 * 22 + s) * 2.0 ** -24
-    got, want, size = carry.double().reshape(lanes, d, s), want, size
+    got = carry.double().reshape(lanes, d, s)
     assert torch.equal(torch.isnan(got), torch.isnan(want))
     fin = torch.isfinite(want)
     assert float(((got - want).abs() / size)[fin].max()) <= T * 2.0 ** -22 + 2 * 22 * 2.0 ** -24
