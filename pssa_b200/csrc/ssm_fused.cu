@@ -10,10 +10,10 @@
 // the exp throughput (d*s per token), not by HBM.
 //
 // Work split: one CTA = one lane (independent sequence) x CH consecutive channels i; a channel's
-// s states are spread over G threads of one warp holding ST states each (G*ST >= s). Inside a warp
-// the 32/G threads that own the same state group sit in adjacent lanes, so the B_j / C_j vectors a
-// thread needs are one shared-memory address per quarter warp (a broadcast, no bank conflicts; the
-// groups are padded apart by 4 floats), and y is completed by a shuffle tree over the G groups.
+// s states are spread over G threads of one warp holding ST states each (G*ST >= s), in pieces of four that
+// alternate between the groups. Inside a warp the 32/G threads that own the same group sit in adjacent lanes, so the
+// B_j / C_j pieces a thread needs are one shared-memory address per group (a broadcast) and the groups' pieces lie side
+// by side (no bank conflicts); y is completed over the G groups by shuffles.
 // Time is walked serially by every thread; token tiles (delta, x, B, C rows) are staged through a
 // cp.async ring in shared memory so the global-load latency is hidden behind the previous tile's exps.
 //
@@ -1247,8 +1247,10 @@ int32_t launch_ssm_fused(pssa_b200_ctx* ctx, const SsmParams& p, bool exact) {
         if (channels <= (exact ? 2 : 1) * schedulers && !by_shape) return launch_wide<32, 2, 32>(ctx, p, exact);
         // (resident CTAs count every lane, however short)
         if (channels <= 4 * schedulers && (size_t)p.lanes * p.d <= 4 * schedulers) return launch_wide<16, 4, 32>(ctx, p, exact);
-        // (five CTAs of the 16 x 4 split fit an SM: a sixth would run behind them. Four channels a warp then, 8 x 8, three CTAs to an SM;
-        // 8 lanes of d 768, 1024 tokens 174 -> 148 us, but 7 lanes 142 and 148, 10 lanes 192 and 204)
+        // (five CTAs of the 16 x 4 split fit an SM: a sixth would run behind them. Four channels a warp then, 8 x 8, three CTAs to an SM. Us
+        // a launch of 1024 tokens, inputs from HBM: 8 and 9 lanes of d 768 185 -> 169, 31 of d 192 182 -> 167, 16 and 18 of d 384 184 -> 168, 4 of
+        // d 1536 183 -> 166, 6 of d 1024 182 -> 167, 62 and 74 of d 96 183 -> 166, 24 and 27 of d 256 183 -> 166; 300 tokens 68 to 71 -> 63 to 65. Below
+        // and above it loses at each of these widths: 7 lanes of d 768 155 and 168, 10 lanes 202 and 233)
         const size_t ctas = channels / 8, sms = (size_t)ctx->sm_count;
         if (!exact && !tape && !by_shape && !p.ragged && ctas > 5 * sms && ctas <= 6 * sms) return launch_wide<8, 8, 16>(ctx, p, exact);
         const double wide_us = 13.8 * (double)channels / (double)schedulers;
